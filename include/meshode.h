@@ -616,6 +616,43 @@ size_t mo_mlp_wgrad_partial_bytes(int splits);
 int mo_mlp_wgrad(const float* A, const float* B, int64_t rows, int splits, float* partial, float* dW,
                  void* stream);
 
+/* The same operations on the tensor cores, in FP16 pairs that carry 22 bits of
+ * every operand (a layer's hidden width m <= 256 runs zero-padded to
+ * W = mo_mlp_tc_width(m) = 64, 128 or 256; -1 for other m).  Arrays of n rows x
+ * W columns are padded to mo_mlp_tc_rows(n) rows (whole 128-row tiles) and
+ * stored in blocks of 8 columns: element (row, c) of tile t at
+ * ((t*(W/8) + c/8)*128 + row)*8 + c%8. */
+int mo_mlp_tc_width(int m);
+int64_t mo_mlp_tc_rows(int64_t n);
+size_t mo_mlp_tc_pack_bytes(int W);
+/* Floats of the partial sums of mo_mlp_tc_bwd over n rows, and of
+ * mo_mlp_tc_wgrad over `rows` padded rows. */
+int64_t mo_mlp_tc_partial_floats(int64_t n, int W);
+int64_t mo_mlp_tc_wgrad_floats(int64_t rows, int W);
+/* The parameters (W1 [m,3], W2, W3 [m,m], W4 [3,m], biases) as the kernels take
+ * them; pack (128-byte aligned) also keeps the largest activations and
+ * gradients that the following calls see. */
+int mo_mlp_tc_pack(const float* W1, const float* b1, const float* W2, const float* b2, const float* W3,
+                   const float* b3, const float* W4, const float* b4, int m, void* pack, void* stream);
+/* mo_mlp_fwd; store (may be NULL): H1, H2, H3 at store + l*astride. */
+int mo_mlp_tc_fwd(const float* u, const float* x, int64_t n, void* pack, int W, float a, float w, int init_acc,
+                  float* unext, float* acc, float* store, int64_t astride, void* stream);
+/* The vector-Jacobian product of one evaluation for dL/dk = ca*a + cg*gprev
+ * (gprev may be NULL): gu = dL/du, dx_out = dx_in + gu, gz2 and gz3 for
+ * mo_mlp_tc_wgrad; partial holds (first) or gets added (else) the sums of dW4,
+ * db4, dW1 and db1. */
+int mo_mlp_tc_bwd(const float* a, float ca, const float* gprev, float cg, const float* u, int64_t n, void* pack,
+                  int W, const float* store, int64_t astride, float* gz2, float* gz3, const float* dx_in,
+                  float* dx_out, float* gu, float* partial, int first, void* stream);
+/* partial (set or added to): G^T H and the column sums of G over `rows` padded
+ * rows; layer 2: G = gz2, H = H1; layer 3: G = gz3, H = H2. */
+int mo_mlp_tc_wgrad(const float* G, const float* H, int64_t rows, void* pack, int W, int layer, float* partial,
+                    int first, void* stream);
+/* The gradients (shapes of the parameters) from the partial sums. */
+int mo_mlp_tc_reduce(const float* partial, int64_t n, const float* wpart2, const float* wpart3, int64_t rows, int W,
+                     int m, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3, float* dW4,
+                     float* db4, void* stream);
+
 /* sizeof(MoPair) and sizeof(MoTile) as compiled (host pointers), so that
  * bindings in other languages can check their struct layout. */
 int mo_abi_sizes(size_t* pair_bytes, size_t* tile_bytes);

@@ -135,6 +135,16 @@ _SIGS = {
     "mo_mlp_partial_reduce": (_I, [_P, _I64, _P, _P, _P, _P, _P, _P, _P, _P]),
     "mo_mlp_wgrad_partial_bytes": (_SZ, [_I]),
     "mo_mlp_wgrad": (_I, [_P, _P, _I64, _I, _P, _P, _P]),
+    "mo_mlp_tc_width": (_I, [_I]),
+    "mo_mlp_tc_rows": (_I64, [_I64]),
+    "mo_mlp_tc_pack_bytes": (_SZ, [_I]),
+    "mo_mlp_tc_partial_floats": (_I64, [_I64, _I]),
+    "mo_mlp_tc_wgrad_floats": (_I64, [_I64, _I]),
+    "mo_mlp_tc_pack": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P]),
+    "mo_mlp_tc_fwd": (_I, [_P, _P, _I64, _P, _I, _F, _F, _I, _P, _P, _P, _I64, _P]),
+    "mo_mlp_tc_bwd": (_I, [_P, _F, _P, _F, _P, _I64, _P, _I, _P, _I64, _P, _P, _P, _P, _P, _P, _I, _P]),
+    "mo_mlp_tc_wgrad": (_I, [_P, _P, _I64, _P, _I, _I, _P, _I, _P]),
+    "mo_mlp_tc_reduce": (_I, [_P, _I64, _P, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "mo_pack_pos": (_I, [_P, _I64, _P, _P]),
     "mo_unpack_pos": (_I, [_P, _I64, _P, _P]),
     "mo_nn_scratch_bytes": (_SZ, [_I64, _I64]),

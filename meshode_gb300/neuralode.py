@@ -18,11 +18,12 @@ the graph/DF losses, back-propagating through the stored RK4 graph.  Here:
   from the forward instead: plain autograd's memory, no recompute, the same
   gradients bit for bit).
 
-Every evaluation of the MLP is one fused libmeshode kernel (mo_mlp_fwd:
-the four layers of a 64-vertex tile with its activations kept on chip, and
-the RK4 stage update), its vector-Jacobian product another (mo_mlp_bwd), and
-the 256x256 weight gradients a split-K kernel over the four stages of a step
-(mo_mlp_wgrad); all FP32 (packed FFMA2), no library GEMM.
+Every evaluation of the MLP is one fused libmeshode kernel (mo_mlp_tc_fwd:
+the four layers of 128-vertex tiles with their activations kept on chip, and
+the RK4 stage update), its vector-Jacobian product another (mo_mlp_tc_bwd), and
+the hidden weights' gradients a split-K kernel over the four stages of a step
+(mo_mlp_tc_wgrad).  Their contractions run on the tensor cores in FP16 pairs
+that carry 22 bits, accumulated in FP32; everything else is FP32.
 """
 import math
 
@@ -52,71 +53,52 @@ MLP_WIDTH = 256  # the fused kernels' hidden width; narrower MLPs run zero-padde
 
 
 class _Packed:
-    """The parameters as the fused kernels take them: zero-padded to the
-    kernels' width (exact: a padded unit's pre-activation and outgoing
-    weights are 0), with W2 and W3 also transposed for the forward."""
+    """The parameters as the fused kernels take them (mo_mlp_tc_pack): split
+    and laid out for the tensor cores, zero-padded to the kernels' width
+    (exact: a padded unit's pre-activation and outgoing weights are 0)."""
 
     def __init__(self, params):
-        W1, b1, W2, b2, W3, b3, W4, b4 = [p.detach() for p in params]
-        m = W1.shape[0]
-        M = L.lib().mo_mlp_width()
-        if m > M:
-            raise RuntimeError("hidden width %d exceeds the fused kernels' %d" % (m, M))
-        self.m, self.M = m, M
-        dev = W1.device
-
-        def pad(t, shape):
-            out = torch.zeros(shape, dtype=torch.float32, device=dev)
-            out[tuple(slice(0, k) for k in t.shape)] = t
-            return out
-
-        self.W1, self.b1 = pad(W1, (M, 3)), pad(b1, (M,))
-        self.W2, self.b2 = pad(W2, (M, M)), pad(b2, (M,))
-        self.W3, self.b3 = pad(W3, (M, M)), pad(b3, (M,))
-        self.W4, self.b4 = pad(W4, (3, M)), b4.contiguous().float()
-        self.W2T = torch.empty_like(self.W2)
-        self.W3T = torch.empty_like(self.W3)
-        s = stream_ptr()
-        call("mo_mlp_transpose", ptr(self.W2), ptr(self.W2T), s)
-        call("mo_mlp_transpose", ptr(self.W3), ptr(self.W3T), s)
+        params = [p.detach().float().contiguous() for p in params]
+        m = params[0].shape[0]
+        if m > MLP_WIDTH:
+            raise RuntimeError("hidden width %d exceeds the fused kernels' %d" % (m, MLP_WIDTH))
+        self.m = m
+        self.M = int(L.lib().mo_mlp_tc_width(m))
+        self.dev = params[0].device
+        self.buf = torch.empty(int(L.lib().mo_mlp_tc_pack_bytes(self.M)), dtype=torch.uint8, device=self.dev)
+        call("mo_mlp_tc_pack", *[ptr(p) for p in params], m, ptr(self.buf), stream_ptr())
 
     def grads(self):
-        M = self.M
-        return [torch.zeros(sh, dtype=torch.float32, device=self.W1.device)
-                for sh in ((M, 3), (M,), (M, M), (M,), (M, M), (M,), (3, M), (3,))]
-
-    def unpad(self, g):
         m = self.m
-        return [g[0][:m].contiguous(), g[1][:m].contiguous(), g[2][:m, :m].contiguous(), g[3][:m].contiguous(),
-                g[4][:m, :m].contiguous(), g[5][:m].contiguous(), g[6][:, :m].contiguous(), g[7]]
+        return [torch.zeros(sh, dtype=torch.float32, device=self.dev)
+                for sh in ((m, 3), (m,), (m, m), (m,), (m, m), (m,), (3, m), (3,))]
 
 
 def _fwd(P, u, x, a, w, init_acc, unext, acc, store=None, astride=0):
     """One fused MLP evaluation k = f(u) with the RK4 update
-    unext = x + a*k, acc = (init ? x : acc) + w*k (mo_mlp_fwd); store: the
-    stage's Z1 H1 Z2 H2 Z3 H3 at stride astride."""
-    call("mo_mlp_fwd", ptr(u), ptr(x), u.shape[0], ptr(P.W1), ptr(P.b1), ptr(P.W2T), ptr(P.b2), ptr(P.W3T),
-         ptr(P.b3), ptr(P.W4), ptr(P.b4), float(a), float(w), int(init_acc), ptr(unext), ptr(acc), ptr(store),
-         int(astride), stream_ptr())
+    unext = x + a*k, acc = (init ? x : acc) + w*k (mo_mlp_tc_fwd); store: the
+    stage's H1 H2 H3 at stride astride."""
+    call("mo_mlp_tc_fwd", ptr(u), ptr(x), u.shape[0], ptr(P.buf), P.M, float(a), float(w), int(init_acc), ptr(unext),
+         ptr(acc), ptr(store), int(astride), stream_ptr())
 
 
 class _StepStore:
     """The activations of one RK4 step's four evaluations:
-    act [6][4][n][M] (Z1 H1 Z2 H2 Z3 H3 of stages 1..4) and the stage
-    inputs u2..u4."""
+    act [3][4][rows][M] (H1 H2 H3 of stages 1..4; rows: n padded to whole
+    tiles) and the stage inputs u2..u4."""
 
     def __init__(self, n, M, dev):
-        self.n, self.M = n, M
-        self.act = torch.empty(6 * 4 * n * M, dtype=torch.float32, device=dev)
+        self.n = int(L.lib().mo_mlp_tc_rows(n)) * M  # floats of one array of one stage
+        self.act = torch.empty(3 * 4 * self.n, dtype=torch.float32, device=dev)
         self.u = [None, torch.empty(n, 3, dtype=torch.float32, device=dev),
                   torch.empty(n, 3, dtype=torch.float32, device=dev), torch.empty(n, 3, dtype=torch.float32, device=dev)]
 
     def stage(self, s):
-        return self.act[s * self.n * self.M:], 4 * self.n * self.M
+        return self.act[s * self.n:], 4 * self.n
 
     def array(self, a):
-        """Array a (0 Z1, 1 H1, 2 Z2, 3 H2, 4 Z3, 5 H3) of all four stages, [4n, M]."""
-        return self.act[a * 4 * self.n * self.M:(a + 1) * 4 * self.n * self.M]
+        """Array a (0 H1, 1 H2, 2 H3) of all four stages."""
+        return self.act[a * 4 * self.n:(a + 1) * 4 * self.n]
 
 
 def _rk4_step(P, x, h, st=None):
@@ -136,46 +118,48 @@ def _rk4_step(P, x, h, st=None):
 
 
 class _Backward:
-    """Work buffers of the adjoint: the stage gradients g_z3, g_z2 of the
-    four evaluations of a step ([2][4][n][M]), the per-warp partial rows of
-    the small gradients and the split partials of the weight gradients."""
+    """Work buffers of the adjoint: the stage gradients g_z2, g_z3 of the
+    four evaluations of a step ([2][4][rows][M]) and the partial sums of the
+    parameter gradients, added to by every step (each block and split of the
+    kernels adds to its own, in step order) and reduced once at the end."""
 
     def __init__(self, n, M, dev):
         lib = L.lib()
-        self.n, self.M = n, M
-        self.tiles = int(lib.mo_mlp_tiles(n))
-        self.pw = int(lib.mo_mlp_partial_floats())
-        self.gz = torch.empty(2 * 4 * n * M, dtype=torch.float32, device=dev)
-        self.partial = torch.empty(4 * self.tiles * 8 * self.pw, dtype=torch.float32, device=dev)
-        self.splits = max(1, min(2 * torch.cuda.get_device_properties(dev).multi_processor_count // 4,
-                                 (4 * n) // 256))
-        self.wpart = torch.empty(int(lib.mo_mlp_wgrad_partial_bytes(self.splits)) // 4, dtype=torch.float32,
-                                 device=dev)
-        self.gu = [torch.empty(n, 3, dtype=torch.float32, device=dev) for _ in range(4)]
-        self.red = torch.empty(int(lib.mo_mlp_partial_reduce_bytes()) // 4, dtype=torch.float32, device=dev)
+        self.n = n
+        self.rows = int(lib.mo_mlp_tc_rows(n))
+        self.size = self.rows * M
 
-    def stage_vjp(self, P, st, s, u, gk):
-        """dL/du of evaluation s (0..3) of the step for dL/dk = gk."""
-        n, M = self.n, self.M
+        def floats(k):
+            return torch.empty(int(k), dtype=torch.float32, device=dev)
+
+        self.gz = floats(2 * 4 * self.size)
+        self.partial = floats(lib.mo_mlp_tc_partial_floats(n, M))
+        self.wpart = [floats(lib.mo_mlp_tc_wgrad_floats(4 * self.rows, M)) for _ in range(2)]
+        self.gu = [torch.empty(n, 3, dtype=torch.float32, device=dev) for _ in range(2)]
+        self.dx = [torch.empty(n, 3, dtype=torch.float32, device=dev) for _ in range(2)]
+        self.evals = self.steps = 0
+
+    def stage_vjp(self, P, st, s, u, a, ca, cg, dx_in, dx_out):
+        """Evaluation s (0..3) of the step: dL/dk = ca*a + cg*(dL/du of the
+        evaluation handled before); dx_out = dx_in + dL/du."""
         act, astride = st.stage(s)
-        gz3 = self.gz[s * n * M:]
-        gz2 = self.gz[(4 + s) * n * M:]
-        part = self.partial[s * self.tiles * 8 * self.pw:]
-        call("mo_mlp_bwd", ptr(gk), ptr(u), n, ptr(P.W1), ptr(P.W2), ptr(P.W3), ptr(P.W4), ptr(act), int(astride),
-             ptr(gz3), ptr(gz2), ptr(self.gu[s]), ptr(part), stream_ptr())
-        return self.gu[s]
+        prev, out = self.gu[self.evals & 1], self.gu[1 - (self.evals & 1)]
+        call("mo_mlp_tc_bwd", ptr(a), float(ca), ptr(prev) if cg else None, float(cg), ptr(u), self.n, ptr(P.buf), P.M,
+             ptr(act), int(astride), ptr(self.gz[s * self.size:]), ptr(self.gz[(4 + s) * self.size:]), ptr(dx_in),
+             ptr(dx_out), ptr(out), ptr(self.partial), int(self.evals == 0), stream_ptr())
+        self.evals += 1
 
-    def weights(self, st, grads, stream=None):
-        """The parameter gradients of the step's four evaluations, added to
-        grads (on `stream`, default the current one)."""
-        n, M = self.n, self.M
-        dW1, db1, dW2, db2, dW3, db3, dW4, db4 = grads
-        s = stream_ptr(stream)
-        call("mo_mlp_partial_reduce", ptr(self.partial), 4 * self.tiles * 8, ptr(self.red), ptr(dW4), ptr(db4),
-             ptr(db3), ptr(db2), ptr(db1), ptr(dW1), s)
-        call("mo_mlp_wgrad", ptr(self.gz), ptr(st.array(3)), 4 * n, self.splits, ptr(self.wpart), ptr(dW3), s)
-        call("mo_mlp_wgrad", ptr(self.gz[4 * n * M:]), ptr(st.array(1)), 4 * n, self.splits, ptr(self.wpart),
-             ptr(dW2), s)
+    def weights(self, P, st):
+        """The hidden weights' gradients of the step's four evaluations."""
+        s = stream_ptr()
+        for k, layer in ((0, 2), (1, 3)):
+            call("mo_mlp_tc_wgrad", ptr(self.gz[4 * k * self.size:]), ptr(st.array(k)), 4 * self.rows, ptr(P.buf), P.M,
+                 layer, ptr(self.wpart[k]), int(self.steps == 0), s)
+        self.steps += 1
+
+    def reduce(self, P, grads):
+        call("mo_mlp_tc_reduce", ptr(self.partial), self.n, ptr(self.wpart[0]), ptr(self.wpart[1]), 4 * self.rows, P.M,
+             P.m, *[ptr(g) for g in grads], stream_ptr())
 
 
 class ODEFlow(Function):
@@ -215,53 +199,30 @@ class ODEFlow(Function):
         n = ckpt.shape[1]
         grads = P.grads()
         a = a_out.contiguous().float()
-        dev = a.device
-        main = torch.cuda.current_stream(dev)
-        # The weight gradients of step k (reads of its activations and stage
-        # gradients, adds into grads) run on a side stream while the main
-        # stream recomputes and back-propagates step k-1 into the other of
-        # two buffer sets; they fill the tail waves of those launches.  All
-        # additions into grads are on the side stream, in step order.
-        side = torch.cuda.Stream(device=dev)
-        Bs = [_Backward(n, P.M, dev), _Backward(n, P.M, dev)]
-        works = [None, None] if ctx.stores is not None else [_StepStore(n, P.M, dev), _StepStore(n, P.M, dev)]
-        done = [None, None]   # side-stream event after the last use of each buffer set
-        held = [None, None]   # stored activations kept alive until the side stream is past them
-        for k in reversed(range(steps)):
-            j = k & 1
-            if done[j] is not None:
-                main.wait_event(done[j])
-            B = Bs[j]
-            xk = ckpt[k]
-            if ctx.stores is not None:
-                st = ctx.stores[k]
-                ctx.stores[k] = None
-                held[j] = st  # freed once its weight gradients have run
-            else:
-                st = works[j]
-                _rk4_step(P, xk, h, st)
-            us = [xk, st.u[1], st.u[2], st.u[3]]
-            dk4 = a * (h / 6)
-            g4 = B.stage_vjp(P, st, 3, us[3], dk4)
-            dx = a + g4
-            g3 = B.stage_vjp(P, st, 2, us[2], a * (h / 3) + h * g4)
-            dx += g3
-            g2 = B.stage_vjp(P, st, 1, us[1], a * (h / 3) + (h / 2) * g3)
-            dx += g2
-            g1 = B.stage_vjp(P, st, 0, us[0], a * (h / 6) + (h / 2) * g2)
-            dx += g1
-            ready = torch.cuda.Event()
-            ready.record(main)
-            side.wait_event(ready)
-            B.weights(st, grads, stream=side)
-            done[j] = torch.cuda.Event()
-            done[j].record(side)
-            a = dx
-        main.wait_stream(side)
-        held = None
+        if n > 0 and steps > 0:
+            B = _Backward(n, P.M, a.device)
+            work = None if ctx.stores is not None else _StepStore(n, P.M, a.device)
+            for k in reversed(range(steps)):
+                xk = ckpt[k]
+                if ctx.stores is not None:
+                    st = ctx.stores[k]
+                    ctx.stores[k] = None
+                else:
+                    st = work
+                    _rk4_step(P, xk, h, st)
+                # dk4 = a h/6, dk3 = a h/3 + h g4, dk2 = a h/3 + h/2 g3, dk1 = a h/6 + h/2 g2;
+                # dL/dx = a + g4 + g3 + g2 + g1
+                dx = B.dx[k & 1]
+                B.stage_vjp(P, st, 3, st.u[3], a, h / 6, 0.0, a, dx)
+                B.stage_vjp(P, st, 2, st.u[2], a, h / 3, h, dx, dx)
+                B.stage_vjp(P, st, 1, st.u[1], a, h / 3, h / 2, dx, dx)
+                B.stage_vjp(P, st, 0, xk, a, h / 6, h / 2, dx, dx)
+                B.weights(P, st)
+                a = dx
+            B.reduce(P, grads)
         ctx.stores = None
         ctx.P = None
-        return (a, None, None) + tuple(P.unpad(grads))
+        return (a, None, None) + tuple(grads)
 
 
 class FitLossFunction(Function):
