@@ -15,10 +15,10 @@
 //
 // The reference assembles A and factorises it with SimplicialLDLT.  Here the
 // normal equations A x = B are solved matrix-free with Jacobi-preconditioned
-// conjugate gradients in double: A x is gathered per vertex over the
-// deterministic vertex -> edge CSR (and, for the cell term, a cell -> vertex
-// CSR), every dot product is a fixed-order reduction, and one CG iteration
-// is a captured CUDA graph of five launches.
+// conjugate gradients in double: A x is gathered per vertex over its unique
+// neighbours (and, for the cell term, a cell -> vertex CSR), every dot product is
+// a fixed-order reduction, and all iterations run in one cooperative launch
+// (k_lin_cg).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -29,8 +29,11 @@
 namespace mo {
 namespace {
 
-constexpr int LT = 256;        // threads per block
-constexpr int LBLOCKS = 512;   // blocks of the dot-product partials
+constexpr int CG_ROWS = 341;      // vertices a block of the solver handles at a time, a thread per coordinate
+constexpr int CG_THREADS = 1024;  // one block per SM
+constexpr int CG_MIN_ROWS = 64;   // vertices a block should have before another block is used
+constexpr int CG_CHECK = 32;      // iterations between convergence checks
+constexpr int CG_MAX_BLOCKS = 512;
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -47,13 +50,16 @@ struct LinScratch {
     int32_t* cell_mem; // [nv] vertices by cell, increasing
     double* cellsum;   // [ng, 3]
     double* rot;       // [nv, 9] s_i * R_i (row-major)
+    int4* nbr;         // [2 nh] unique neighbours: (vertex, -, weight as a double)
+    int32_t* nnbr;     // [nv] their number
     double* x;         // [nv, 3]
-    double* r;
-    double* z;
-    double* p;
-    double* Ap;
-    double* partial;   // [LBLOCKS, 3]
-    double* scal;      // rz[3], pAp[3], alpha[3], beta[3], rz0[3], bb[3]
+    double* r;         // [nv, 3]
+    double* dinv;      // [nv, 3]
+    double* z;         // [nv, 4]
+    double* p;         // [2, nv, 4]
+    double* partial;   // [3][CG_MAX_BLOCKS, 3]
+    double* result;    // iterations, relative residual
+    unsigned* bar;     // grid barrier count, then its abort flag
     int* status;
     uint32_t* keys_a;  // cell sort
     uint32_t* keys_b;
@@ -84,13 +90,16 @@ LinScratch plan(char* base, int64_t nv, int64_t nf, int64_t ne, int64_t ng, int 
     s.cell_mem = reinterpret_cast<int32_t*>(take(4 * (size_t)nv));
     s.cellsum = reinterpret_cast<double*>(take(24 * (size_t)ng));
     s.rot = reinterpret_cast<double*>(take(with_rot ? 72 * (size_t)nv : 0));
+    s.nbr = reinterpret_cast<int4*>(take(32 * (size_t)nh));
+    s.nnbr = reinterpret_cast<int32_t*>(take(4 * (size_t)nv));
     s.x = reinterpret_cast<double*>(take(24 * (size_t)nv));
     s.r = reinterpret_cast<double*>(take(24 * (size_t)nv));
-    s.z = reinterpret_cast<double*>(take(24 * (size_t)nv));
-    s.p = reinterpret_cast<double*>(take(24 * (size_t)nv));
-    s.Ap = reinterpret_cast<double*>(take(24 * (size_t)nv));
-    s.partial = reinterpret_cast<double*>(take(48 * (size_t)LBLOCKS));  // two sets of 3 per block
-    s.scal = reinterpret_cast<double*>(take(8 * 18));
+    s.dinv = reinterpret_cast<double*>(take(24 * (size_t)nv));
+    s.z = reinterpret_cast<double*>(take(32 * (size_t)nv));
+    s.p = reinterpret_cast<double*>(take(64 * (size_t)nv));
+    s.partial = reinterpret_cast<double*>(take(8 * 9 * (size_t)CG_MAX_BLOCKS));
+    s.result = reinterpret_cast<double*>(take(16));
+    s.bar = reinterpret_cast<unsigned*>(take(16));
     s.status = reinterpret_cast<int*>(take(16));
     s.keys_a = reinterpret_cast<uint32_t*>(take(4 * (size_t)nv));
     s.keys_b = reinterpret_cast<uint32_t*>(take(4 * (size_t)nv));
@@ -353,179 +362,320 @@ __global__ void k_lin_rhs_rot(int64_t nv, const int* __restrict__ row_ptr, const
 }
 
 // ---- CG --------------------------------------------------------------------
-// Ap = A p for both systems; partial[block] = sum p.Ap per column.
-__global__ void __launch_bounds__(LT) k_lin_apply(int64_t nv, const int* __restrict__ row_ptr,
-                                                  const int* __restrict__ other, const int* __restrict__ key,
-                                                  const double* __restrict__ w, const int32_t* __restrict__ ref,
-                                                  const double* __restrict__ cellw, const double* __restrict__ cellsum,
-                                                  double c0, const double* __restrict__ p, double* __restrict__ Ap,
-                                                  double* __restrict__ partial) {
-    __shared__ double sh[3][LT];
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int64_t i = (int64_t)blockIdx.x * LT + threadIdx.x; i < nv; i += (int64_t)gridDim.x * LT) {
-        double y[3];
-        for (int c = 0; c < 3; ++c) y[c] = c0 * p[3 * i + c];
-        if (ref) {
-            const int64_t g = ref[i];
-            const double w2 = cellw[g] * cellw[g];
-            for (int c = 0; c < 3; ++c) y[c] += w2 * cellsum[3 * g + c];
-        }
-        for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
-            const int64_t o = other[k];
-            const double we = w[key[k] >> 1];
-            for (int c = 0; c < 3; ++c) y[c] += we * (p[3 * i + c] - p[3 * o + c]);
-        }
-        for (int c = 0; c < 3; ++c) {
-            Ap[3 * i + c] = y[c];
-            acc[c] += p[3 * i + c] * y[c];
-        }
+// A vertex's unique neighbours with their summed weights, in the order of
+// their first half-edge: a closed mesh names every neighbour twice, and the
+// product with A is bound by the FP64 pipe (2 lanes a clock and SM).
+__global__ void k_lin_merge(int64_t nv, const int* __restrict__ row_ptr, const int* __restrict__ other,
+                            const int* __restrict__ key, const double* __restrict__ w, int4* __restrict__ nbr,
+                            int32_t* __restrict__ nnbr) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nv) return;
+    const int b = row_ptr[i], e = row_ptr[i + 1];
+    int n = 0;
+    for (int k = b; k < e; ++k) {
+        const int o = other[k];
+        if (o == i) continue;  // a self-loop's entries cancel
+        bool seen = false;
+        for (int j = b; j < k && !seen; ++j) seen = other[j] == o;
+        if (seen) continue;
+        double s = w[key[k] >> 1];
+        for (int j = k + 1; j < e; ++j)
+            if (other[j] == o) s += w[key[j] >> 1];
+        nbr[b + n] = make_int4(o, 0, __double2loint(s), __double2hiint(s));
+        ++n;
     }
-    for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = acc[c];
+    nnbr[i] = n;
+}
+
+struct CgArgs {
+    int64_t nv, ng;
+    const int* row_ptr;
+    const int4* nbr;
+    const int32_t *nnbr, *ref;  // ref NULL: no cell term
+    const double* cellw;
+    const int32_t *cell_ptr, *cell_mem;
+    double c0;
+    const double *V0, *diag;
+    double *x, *r, *dinv, *z, *p, *cellsum, *partial, *result;
+    unsigned* bar;
+    double tol;
+    int max_iter;
+};
+
+// All blocks of the (cooperative) grid; `target` grows by gridDim.x per call.
+// A wait of more than two seconds, or another block's, ends the solve: false.
+__device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned target) {
+    __shared__ int ok;
     __syncthreads();
-    for (int o = LT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 3; ++c) partial[3 * blockIdx.x + c] = sh[c][0];
-}
-
-// cellsum[g] = sum of p over cell g's members, in vertex order.
-__global__ void k_lin_cellsum(int64_t ng, const int32_t* __restrict__ cell_ptr, const int32_t* __restrict__ mem,
-                              const double* __restrict__ p, double* __restrict__ cellsum) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ng) return;
-    double s[3] = {0.0, 0.0, 0.0};
-    for (int k = cell_ptr[g]; k < cell_ptr[g + 1]; ++k) {
-        const int64_t j = mem[k];
-        for (int c = 0; c < 3; ++c) s[c] += p[3 * j + c];
-    }
-    for (int c = 0; c < 3; ++c) cellsum[3 * g + c] = s[c];
-}
-
-// Fixed-order sum of the block partials into out[3].
-__global__ void __launch_bounds__(LT) k_lin_reduce(const double* __restrict__ partial, int nblocks,
-                                                   double* __restrict__ out) {
-    __shared__ double sh[3][LT];
-    for (int c = 0; c < 3; ++c) {
-        double a = 0.0;
-        for (int b = threadIdx.x; b < nblocks; b += LT) a += partial[3 * b + c];
-        sh[c][threadIdx.x] = a;
-    }
-    __syncthreads();
-    for (int o = LT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 3; ++c) out[c] = sh[c][0];
-}
-
-// scal: rz[0..2] pAp[3..5] alpha[6..8] beta[9..11] rz_new[12..14] bb[15..17]
-// x += alpha p, r -= alpha Ap, z = r / diag; partial = r.z per column.
-__global__ void __launch_bounds__(LT) k_lin_update(int64_t nv, double* __restrict__ scal, double* __restrict__ x,
-                                                   double* __restrict__ r, double* __restrict__ z,
-                                                   const double* __restrict__ p, const double* __restrict__ Ap,
-                                                   const double* __restrict__ diag, double* __restrict__ partial) {
-    __shared__ double sh[3][LT];
-    __shared__ double alpha[3];
-    if (threadIdx.x < 3) {
-        const double pap = scal[3 + threadIdx.x];
-        alpha[threadIdx.x] = pap > 0.0 ? scal[threadIdx.x] / pap : 0.0;
-    }
-    __syncthreads();
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int64_t i = (int64_t)blockIdx.x * LT + threadIdx.x; i < nv; i += (int64_t)gridDim.x * LT) {
-        const double di = diag[i];
-        for (int c = 0; c < 3; ++c) {
-            const int64_t k = 3 * i + c;
-            x[k] += alpha[c] * p[k];
-            const double rk = r[k] - alpha[c] * Ap[k];
-            r[k] = rk;
-            const double zk = rk / di;
-            z[k] = zk;
-            acc[c] += rk * zk;
-        }
-    }
-    for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = acc[c];
-    __syncthreads();
-    for (int o = LT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 3; ++c) partial[3 * blockIdx.x + c] = sh[c][0];
-}
-
-// p = z + beta p with beta = rz_new / rz; then rz = rz_new.  Block 0 thread c
-// rolls the scalars after every block has read them (next launch).
-__global__ void __launch_bounds__(LT) k_lin_direction(int64_t nv, const double* __restrict__ scal,
-                                                      const double* __restrict__ z, double* __restrict__ p) {
-    double beta[3];
-    for (int c = 0; c < 3; ++c) beta[c] = scal[c] > 0.0 ? scal[12 + c] / scal[c] : 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * LT + threadIdx.x; i < nv; i += (int64_t)gridDim.x * LT)
-        for (int c = 0; c < 3; ++c) p[3 * i + c] = z[3 * i + c] + beta[c] * p[3 * i + c];
-}
-
-__global__ void k_lin_roll(double* scal) {
-    if (threadIdx.x < 3) scal[threadIdx.x] = scal[12 + threadIdx.x];
-}
-
-// r = B - A x (B in r), z = r / diag, p = z; partial = r.z and b.b per column.
-__global__ void __launch_bounds__(LT) k_lin_start(int64_t nv, double* __restrict__ r, const double* __restrict__ Ax,
-                                                  const double* __restrict__ diag, double* __restrict__ z,
-                                                  double* __restrict__ p, double* __restrict__ partial) {
-    __shared__ double sh[6][LT];
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int64_t i = (int64_t)blockIdx.x * LT + threadIdx.x; i < nv; i += (int64_t)gridDim.x * LT) {
-        for (int c = 0; c < 3; ++c) {
-            const int64_t k = 3 * i + c;
-            const double b = r[k];
-            const double rk = b - Ax[k];
-            r[k] = rk;
-            const double zk = rk / diag[i];
-            z[k] = zk;
-            p[k] = zk;
-            acc[c] += rk * zk;
-            acc[3 + c] += b * b;
-        }
-    }
-    for (int c = 0; c < 6; ++c) sh[c][threadIdx.x] = acc[c];
-    __syncthreads();
-    for (int o = LT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int c = 0; c < 6; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + o];
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
-        for (int c = 0; c < 3; ++c) partial[3 * blockIdx.x + c] = sh[c][0];
-        for (int c = 0; c < 3; ++c) partial[3 * (LBLOCKS + blockIdx.x) + c] = sh[3 + c][0];
+        __threadfence();
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+        ok = 1;
+        unsigned v, stop;
+        unsigned long long t0 = 0, t;
+        for (int n = 0;; ++n) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((n & 1023) == 1023) {
+                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+                if (t0 == 0) t0 = t;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(stop) : "l"(bar + 1) : "memory");
+                if (stop || t - t0 > 2000000000ull) {
+                    atomicExch(bar + 1, 1u);
+                    ok = 0;
+                    break;
+                }
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// Per coordinate: the block's sum of v (thread t holds coordinate t % 3), in a
+// fixed order, into out[0..2] of shared memory.  FP64 instructions are the scarce
+// resource (a warp's takes 64 clocks of its scheduler), so three warps add what
+// all threads put into shared memory instead of every warp shuffling.
+__device__ __forceinline__ void block_sum3(double v, double* sh, double* out) {
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (c < 3) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 0; k < (CG_ROWS + 31) / 32; ++k) {
+            const int row = lane + 32 * k;
+            if (row < CG_ROWS) s += sh[3 * row + c];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[c] = s;
+    }
+    __syncthreads();
+}
+
+// The totals of the blocks' partial sums (every block adds them in the same order).
+__device__ __forceinline__ void grid_sum3(const double* part, double* out) {
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (c < 3) {
+        double s = 0.0;
+#pragma unroll 4
+        for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + 3 * b + c);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) out[c] = s;
+    }
+}
+
+// Every iteration of the conjugate gradients in one cooperative launch.  (Before:
+// a graph of seven kernels, 98 us an iteration at 41k vertices and 802 cells, of
+// which the launches and the cells, each summed by one thread, were most.)
+// Three grid barriers an iteration:
+//   A p and p.Ap | alpha; x, r, z = r / diag and r.z | beta; p = z + beta p and
+//   its cell sums
+// p is double-buffered, so the cell sums can be taken of z + beta p while the
+// vertices write it.  A block owns a contiguous range of vertices, a thread one
+// coordinate of a vertex; with at most CG_ROWS vertices (ONE) x and r stay in
+// registers.  Bound: the FP64 pipe (2 lanes a clock and SM) in A p, two
+// operations a neighbour and coordinate, and the latency of the barriers.
+template <bool ONE>
+__global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
+    __shared__ double sh[CG_THREADS];
+    __shared__ double sum[3], rz[3], bb[3], coef[3];
+    __shared__ double rel_sh;
+    const int64_t per = (A.nv + gridDim.x - 1) / gridDim.x;
+    const int c = threadIdx.x % 3, tid = threadIdx.x;
+    const int64_t i0 = per * blockIdx.x + tid / 3;
+    const int64_t i1 = tid < 3 * CG_ROWS ? min(A.nv, per * (blockIdx.x + 1)) : 0;
+    double* PA = A.partial;
+    double* PU = PA + 3 * CG_MAX_BLOCKS;
+    double* PR = PU + 3 * CG_MAX_BLOCKS;
+    unsigned target = 0;
+    double x = 0, r = 0, di = 0;  // ONE: this thread's vertex
+
+    // a vertex's neighbours and cell
+    struct Row {
+        const int4* q;
+        const double* sum;
+        double w2;
+        int n;
+    };
+    auto row_of = [&](int64_t i) {
+        Row w{A.nbr + A.row_ptr[i], nullptr, 0.0, A.nnbr[i]};
+        if (A.ref) {
+            const int64_t g = A.ref[i];
+            w.sum = A.cellsum + 3 * g + c;
+            w.w2 = A.cellw[g] * A.cellw[g];
+        }
+        return w;
+    };
+    Row mine{};  // ONE
+    if (ONE && i0 < i1) mine = row_of(i0);
+    // coordinate c of A v for vertex i; v in rows of 4
+    auto apply = [&](const double* v, int64_t i, double vi) {
+        const Row w = ONE ? mine : row_of(i);
+        const double cs = w.sum ? __ldcg(w.sum) : 0.0;
+        double y = A.c0 * vi;
+        const int4* q = w.q;
+        const int n = w.n;
+#pragma unroll 6
+        for (int k = 0; k < n; ++k) {
+            const int4 e = __ldg(q + k);
+            y += __hiloint2double(e.w, e.z) * (vi - __ldcg(v + 4 * (int64_t)e.x + c));
+        }
+        y += w.w2 * cs;
+        return y;
+    };
+    // cellsum = sums of value(member, coordinate) over the cells: a warp per
+    // coordinate of a cell, its loads in flight together, or a block where cells
+    // are large
+    auto cells = [&](auto value) {
+        if (A.nv >= A.ng * 1024) {
+            for (int64_t g = blockIdx.x; g < A.ng; g += gridDim.x) {
+                double s = 0.0;
+                const int e = A.cell_ptr[g + 1];
+                if (tid < 3 * CG_ROWS)
+                    for (int k = A.cell_ptr[g] + tid / 3; k < e; k += CG_ROWS) s += value(A.cell_mem[k], c);
+                block_sum3(s, sh, sum);
+                if (tid < 3) A.cellsum[3 * g + tid] = sum[tid];
+                __syncthreads();
+            }
+            return;
+        }
+        const int lane = tid & 31;
+        for (int64_t q = blockIdx.x + gridDim.x * (int64_t)(tid >> 5); q < 3 * A.ng; q += gridDim.x * (CG_THREADS / 32)) {
+            const int64_t g = q / 3;
+            const int k0 = (int)(q - 3 * g), e = A.cell_ptr[g + 1];
+            double s = 0.0;
+#pragma unroll 4
+            for (int k = A.cell_ptr[g] + lane; k < e; k += 32) s += value(A.cell_mem[k], k0);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) A.cellsum[q] = s;
+        }
+    };
+    auto store_partial = [&](double* part, double v) {
+        block_sum3(v, sh, sum);
+        if (tid < 3) part[3 * blockIdx.x + tid] = sum[tid];
+    };
+
+    // r = B - A x0 (B in r), z = r / diag, p = z
+    double* p = A.p;
+    double* pn = A.p + 4 * A.nv;
+    if (A.ref) cells([&](int64_t j, int k) { return A.V0[3 * j + k]; });
+    for (int64_t i = i0; i < i1; i += CG_ROWS) pn[4 * i + c] = A.V0[3 * i + c];  // x0 in rows of 4
+    if (!grid_sync(A.bar, target += gridDim.x)) return;
+    double sz = 0.0, sb = 0.0;
+    for (int64_t i = i0; i < i1; i += CG_ROWS) {
+        const double x0 = A.V0[3 * i + c], b = A.r[3 * i + c], rc = b - apply(pn, i, x0);
+        const double d = 1.0 / A.diag[i], zc = rc * d;
+        if (ONE) {
+            x = x0;
+            r = rc;
+            di = d;
+        } else {
+            A.x[3 * i + c] = x0;
+            A.r[3 * i + c] = rc;
+            A.dinv[3 * i + c] = d;
+        }
+        A.z[4 * i + c] = zc;
+        p[4 * i + c] = zc;
+        sz += rc * zc;
+        sb += b * b;
+    }
+    store_partial(PU, sz);
+    store_partial(PR, sb);
+    if (!grid_sync(A.bar, target += gridDim.x)) return;
+    grid_sum3(PU, rz);
+    grid_sum3(PR, bb);
+    if (A.ref) cells([&](int64_t j, int k) { return __ldcg(A.z + 4 * j + k); });
+    if (!grid_sync(A.bar, target += gridDim.x)) return;
+
+    int it = 0;
+    double rel = INFINITY;
+    while (it < A.max_iter) {
+        const bool check = (it + 1) % CG_CHECK == 0 || it + 1 == A.max_iter;
+        double y = 0, pi = 0, acc = 0.0;
+        for (int64_t i = i0; i < i1; i += CG_ROWS) {
+            pi = p[4 * i + c];
+            y = apply(p, i, pi);
+            acc += pi * y;
+            if (!ONE) pn[4 * i + c] = y;  // A p waits where the next p will be
+        }
+        store_partial(PA, acc);
+        if (!grid_sync(A.bar, target += gridDim.x)) return;
+        grid_sum3(PA, sum);
+        if (tid < 96 && (tid & 31) == 0) coef[tid >> 5] = sum[tid >> 5] > 0.0 ? rz[tid >> 5] / sum[tid >> 5] : 0.0;
+        __syncthreads();
+        const double alpha = coef[c];
+        double s = 0.0, rr = 0.0;
+        for (int64_t i = i0; i < i1; i += CG_ROWS) {
+            double rc, zc;
+            if (ONE) {
+                x += alpha * pi;
+                r -= alpha * y;
+                rc = r;
+                zc = rc * di;
+            } else {
+                A.x[3 * i + c] += alpha * p[4 * i + c];
+                rc = A.r[3 * i + c] -= alpha * pn[4 * i + c];
+                zc = rc * A.dinv[3 * i + c];
+            }
+            A.z[4 * i + c] = zc;
+            s += rc * zc;
+            if (check) rr += rc * rc;
+        }
+        store_partial(PU, s);
+        if (check) store_partial(PR, rr);
+        if (!grid_sync(A.bar, target += gridDim.x)) return;
+        grid_sum3(PU, sum);
+        ++it;
+        if (check) {
+            grid_sum3(PR, coef);
+            __syncthreads();
+            if (tid == 0) {
+                double m = 0.0;
+                for (int k = 0; k < 3; ++k) {
+                    const double v = bb[k] > 0.0 ? sqrt(coef[k] / bb[k]) : sqrt(coef[k]);
+                    if (m < v) m = v;
+                }
+                rel_sh = m;
+            }
+            __syncthreads();
+            rel = rel_sh;
+            if (!(rel > A.tol)) break;
+        }
+        if (tid < 96 && (tid & 31) == 0) {
+            const int k = tid >> 5;
+            coef[k] = rz[k] > 0.0 ? sum[k] / rz[k] : 0.0;
+            rz[k] = sum[k];
+        }
+        __syncthreads();
+        const double beta = coef[c];
+        for (int64_t i = i0; i < i1; i += CG_ROWS) pn[4 * i + c] = fma(beta, p[4 * i + c], A.z[4 * i + c]);
+        if (A.ref) {
+            const double b0 = coef[0], b1 = coef[1], b2 = coef[2];
+            cells([&](int64_t j, int k) {
+                return fma(k == 0 ? b0 : k == 1 ? b1 : b2, __ldcg(p + 4 * j + k), __ldcg(A.z + 4 * j + k));
+            });
+        }
+        double* t = p;
+        p = pn;
+        pn = t;
+        if (!grid_sync(A.bar, target += gridDim.x)) return;
+    }
+    if (ONE)
+        for (int64_t i = i0; i < i1; i += CG_ROWS) A.x[3 * i + c] = x;
+    if (blockIdx.x == 0 && tid == 0) {
+        A.result[0] = (double)it;
+        A.result[1] = rel;
     }
 }
 
 __global__ void k_lin_to_float(const double* __restrict__ x, int64_t n, float* __restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = (float)x[i];
-}
-
-// ||r||^2 per column into out[3] (for the convergence check).
-__global__ void __launch_bounds__(LT) k_lin_rr(int64_t nv, const double* __restrict__ r, double* __restrict__ partial) {
-    __shared__ double sh[3][LT];
-    double acc[3] = {0, 0, 0};
-    for (int64_t i = (int64_t)blockIdx.x * LT + threadIdx.x; i < nv; i += (int64_t)gridDim.x * LT)
-        for (int c = 0; c < 3; ++c) acc[c] += r[3 * i + c] * r[3 * i + c];
-    for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = acc[c];
-    __syncthreads();
-    for (int o = LT / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] += sh[c][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 3; ++c) partial[3 * blockIdx.x + c] = sh[c][0];
 }
 
 }  // namespace
@@ -556,9 +706,8 @@ extern "C" int mo_solve_linear(float* V, int64_t nv, const int32_t* F, int64_t n
     MO_CHECK_ARG(!with_rot || ng == nv, "with_rot needs one target position per vertex (ng == nv)");
     MO_CHECK_ARG(tol > 0.0 && max_iter > 0, "bad tolerance or iteration limit");
     MO_CHECK_ARG(std::isfinite(rigidity), "bad rigidity");
-    // The iterations are captured as a CUDA graph, which the caller's stream
-    // (possibly the legacy default stream) may not allow: the solve runs on a
-    // stream of its own that first waits for the caller's work.
+    // The solve runs on a stream of its own that first waits for the caller's
+    // work.
     cudaStream_t caller = as_stream(stream);
     cudaStream_t s = nullptr;
     cudaEvent_t ready = nullptr;
@@ -593,13 +742,11 @@ int solve_on(float* V, int64_t nv, const int32_t* F, int64_t nf, const int32_t* 
     }
     LinScratch S = plan(reinterpret_cast<char*>(scratch), nv, nf, ne, ng, with_rot);
     const int64_t nh = 3 * nf + (with_rot ? 0 : ne);
-    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(LBLOCKS, (nv + LT - 1) / LT));
     int rc = MO_OK;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
     auto fail = [&](cudaError_t e, const char* where) { rc = cuda_status(e, where); };
     do {
         cudaError_t e = cudaMemsetAsync(S.status, 0, 16, s);
+        if (e == cudaSuccess) e = cudaMemsetAsync(S.bar, 0, 16, s);
         if (e != cudaSuccess) { fail(e, "memset"); break; }
         if (nh > 0) {
             k_lin_edges<<<ceil_div(nh, 256), 256, 0, s>>>(F, nf, with_rot ? nullptr : E, with_rot ? 0 : ne, S.edges);
@@ -652,63 +799,31 @@ int solve_on(float* V, int64_t nv, const int32_t* F, int64_t nf, const int32_t* 
             c0 = 1.0;
         }
         const int32_t* cref = with_rot ? nullptr : ref;
-        // start from the input positions: r = B - A x0
-        e = cudaMemcpyAsync(S.x, S.V0, 24 * (size_t)nv, cudaMemcpyDeviceToDevice, s);
-        if (e != cudaSuccess) { fail(e, "copy"); break; }
-        if (cref) {
-            k_lin_cellsum<<<ceil_div(ng, 256), 256, 0, s>>>(ng, S.cell_ptr, S.cell_mem, S.x, S.cellsum);
-            ::mo::note_launch();
-        }
-        k_lin_apply<<<blocks, LT, 0, s>>>(nv, row_ptr, other, key, S.w, cref, S.cellw, S.cellsum, c0, S.x, S.Ap,
-                                          S.partial);
+        k_lin_merge<<<ceil_div(nv, 128), 128, 0, s>>>(nv, row_ptr, other, key, S.w, S.nbr, S.nnbr); ::mo::note_launch();
+        // one block per SM, fewer where blocks would have too few vertices for the barriers to pay
+        const int blocks = (int)std::max<int64_t>(
+            1, std::min<int64_t>(std::min(device_sm_count(), CG_MAX_BLOCKS), (nv + CG_MIN_ROWS - 1) / CG_MIN_ROWS));
+        CgArgs args{nv, ng, row_ptr, S.nbr, S.nnbr, cref, S.cellw, S.cell_ptr, S.cell_mem, c0, S.V0, S.diag,
+                    S.x, S.r, S.dinv, S.z, S.p, S.cellsum, S.partial, S.result, S.bar, tol, max_iter};
+        void* argv[] = {&args};
+        const bool one = (nv + blocks - 1) / blocks <= CG_ROWS;
+        e = cudaLaunchCooperativeKernel(one ? (const void*)k_lin_cg<true> : (const void*)k_lin_cg<false>, dim3(blocks),
+                                        dim3(CG_THREADS), argv, 0, s);
         ::mo::note_launch();
-        k_lin_start<<<blocks, LT, 0, s>>>(nv, S.r, S.Ap, S.diag, S.z, S.p, S.partial); ::mo::note_launch();
-        k_lin_reduce<<<1, LT, 0, s>>>(S.partial, blocks, S.scal); ::mo::note_launch();                  // rz
-        k_lin_reduce<<<1, LT, 0, s>>>(S.partial + 3 * LBLOCKS, blocks, S.scal + 15); ::mo::note_launch(); // bb
-        e = cudaGetLastError();
-        if (e != cudaSuccess) { fail(e, "cg start"); break; }
-        // one iteration, captured once
-        e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) { fail(e, "capture"); break; }
-        if (cref) k_lin_cellsum<<<ceil_div(ng, 256), 256, 0, s>>>(ng, S.cell_ptr, S.cell_mem, S.p, S.cellsum);
-        k_lin_apply<<<blocks, LT, 0, s>>>(nv, row_ptr, other, key, S.w, cref, S.cellw, S.cellsum, c0, S.p, S.Ap,
-                                          S.partial);
-        k_lin_reduce<<<1, LT, 0, s>>>(S.partial, blocks, S.scal + 3);  // pAp
-        k_lin_update<<<blocks, LT, 0, s>>>(nv, S.scal, S.x, S.r, S.z, S.p, S.Ap, S.diag, S.partial);
-        k_lin_reduce<<<1, LT, 0, s>>>(S.partial, blocks, S.scal + 12);  // rz_new
-        k_lin_direction<<<blocks, LT, 0, s>>>(nv, S.scal, S.z, S.p);
-        k_lin_roll<<<1, 32, 0, s>>>(S.scal);
-        e = cudaStreamEndCapture(s, &graph);
-        if (e != cudaSuccess) { fail(e, "capture"); break; }
-        e = cudaGraphInstantiate(&exec, graph, 0);
-        if (e != cudaSuccess) { fail(e, "instantiate"); break; }
-        double bb[3];
-        e = cudaMemcpyAsync(bb, S.scal + 15, sizeof(bb), cudaMemcpyDeviceToHost, s);
+        if (e != cudaSuccess) { fail(e, "k_lin_cg"); break; }
+        double result[2];
+        unsigned aborted[2];
+        e = cudaMemcpyAsync(result, S.result, sizeof(result), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(aborted, S.bar, sizeof(aborted), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) { fail(e, "read"); break; }
-        // convergence: max over columns of ||r|| / ||b|| <= tol, checked every
-        // `check` iterations; the iteration count is bounded by max_iter
-        const int check = 32;
-        int it = 0;
-        double rel = INFINITY;
-        while (it < max_iter) {
-            const int n = std::min(check, max_iter - it);
-            for (int k = 0; k < n; ++k) {
-                e = cudaGraphLaunch(exec, s);
-                if (e != cudaSuccess) break;
-            }
-            if (e != cudaSuccess) { fail(e, "cg iteration"); break; }
-            it += n;
-            k_lin_rr<<<blocks, LT, 0, s>>>(nv, S.r, S.partial); ::mo::note_launch();
-            k_lin_reduce<<<1, LT, 0, s>>>(S.partial, blocks, S.scal + 6); ::mo::note_launch();
-            double rr[3];
-            e = cudaMemcpyAsync(rr, S.scal + 6, sizeof(rr), cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            if (e != cudaSuccess) { fail(e, "residual"); break; }
-            rel = 0.0;
-            for (int c = 0; c < 3; ++c) rel = std::max(rel, bb[c] > 0.0 ? std::sqrt(rr[c] / bb[c]) : std::sqrt(rr[c]));
-            if (!(rel > tol)) break;
+        if (e != cudaSuccess) { fail(e, "conjugate gradients"); break; }
+        if (aborted[1]) {
+            set_error("conjugate gradients: a grid barrier ran out of time");
+            rc = MO_ERR_DEVICE;
+            break;
         }
+        const int it = (int)result[0];
+        const double rel = result[1];
         if (rc) break;
         if (iters_out) *iters_out = it;
         if (rel_residual_out) *rel_residual_out = rel;
@@ -720,8 +835,6 @@ int solve_on(float* V, int64_t nv, const int32_t* F, int64_t nf, const int32_t* 
             rc = MO_ERR_DEVICE;
         }
     } while (0);
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
     if (owned) cudaFreeAsync(owned, s);
     return rc;
 }
