@@ -126,12 +126,13 @@ class ReverseLossFunction(Function):
         ns, nt = int(S.shape[0]), int(T.shape[0])
         s = L.stream_ptr()
         idx = torch.empty(nt, dtype=torch.int32, device=dev)
-        L.call("mo_nn_query", L.ptr(S), ns, L.ptr(T), nt, L.ptr(idx), None, None, 0, s)
-        nb = L.lib().mo_reverse_loss_scratch_bytes(ns, nt)
+        nb = max(L.lib().mo_nn_scratch_bytes(ns, nt), L.lib().mo_reverse_loss_scratch_bytes(ns, nt))
         scratch = torch.empty(max(int(nb), 1), dtype=torch.uint8, device=dev)
+        L.call("mo_nn_query", L.ptr(S), ns, L.ptr(T), nt, L.ptr(idx), None, L.ptr(scratch), nb, s)
         loss = torch.empty(1, dtype=torch.float64, device=dev)
+        st = torch.empty(1, dtype=torch.int32, device=dev)  # the query's indices are in range
         L.call("mo_reverse_loss_forward", L.ptr(S), ns, L.ptr(T), nt, L.ptr(idx), L.ptr(loss), L.ptr(scratch), nb,
-               None, s)
+               L.ptr(st), s)
         ctx.save_for_backward(S, T, idx)
         ctx.src_device = src_V.device
         return loss.to(torch.float32).reshape(()).to(src_V.device)
@@ -145,7 +146,7 @@ class ReverseLossFunction(Function):
         gs = torch.empty_like(S)
         nb = L.lib().mo_reverse_loss_scratch_bytes(ns, nt)
         scratch = torch.empty(max(int(nb), 1), dtype=torch.uint8, device=S.device)
-        st = torch.zeros(1, dtype=torch.int32, device=S.device)  # the forward checked the indices
+        st = torch.empty(1, dtype=torch.int32, device=S.device)  # the query's indices are in range
         L.call("mo_reverse_loss_backward", L.ptr(S), ns, L.ptr(T), nt, L.ptr(idx), L.ptr(g), L.ptr(gs),
                L.ptr(scratch), nb, L.ptr(st), L.stream_ptr())
         return gs.to(ctx.src_device), None
