@@ -375,6 +375,16 @@ int mo_fused_step_weighted(const MoPair* pairs, const MoTile* tiles, const int32
  * the cells the step moves vertices into (see MoPair). */
 int mo_fused_step_on_demand(const MoPair* pairs, const MoTile* tiles, const int32_t* ntiles, int max_tiles,
                             int launch_index, float* tile_loss, int grid_ctas, void* stream);
+/* The next nsteps steps of one pair (a MoPair in host memory; weighted: as
+ * mo_fused_step_weighted) in one launch whose blocks wait on one another, for
+ * pairs small enough that every vertex has a thread on the chip at once
+ * (mo_fused_run_fits).  Results are mo_fused_step's, bit for bit.  tile_loss
+ * (may be NULL): the loss partials of step k at tile_loss + k*loss_stride, as
+ * launch k of mo_fused_step leaves them for tiles of 8 slices.  sync: two words
+ * of device memory.  A wait inside that runs out leaves NaN positions. */
+int mo_fused_run_fits(int64_t nv);
+int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float* tile_loss, int64_t loss_stride,
+                 uint32_t* sync, void* stream);
 /* pair_loss[k*npairs + p] (double) = sum, in a fixed order, of the tile
  * partials of pair p (its MoPair tile0/ntiles range) for launches
  * k = 0..nlaunch-1: the layer loss 0.5*sum d^2 + w_edge*0.5*sum |r|^2 at the

@@ -6,6 +6,8 @@
 // RigidLossFunction (src/python/layers/rigid_loss_layer.py:7-27) or
 // GraphLossFunction (src/python/layers/graph_loss_layer.py:9-43) and
 // torch.optim.Adam.
+#include <algorithm>
+
 #include "mo_lazydf.cuh"
 
 namespace mo {
@@ -196,6 +198,197 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) k_fused_step(const MoPair* __
     }
 }
 
+// ---------------------------------------------------------------------------
+// Many steps of one pair in one cooperative launch, for pairs whose every vertex
+// can have a thread of its own on the chip.  A launch per step is a chain of
+// dependent loads (tile, pair, position, record, neighbour) behind a launch:
+// 7 us a step at 10k vertices.  Here a vertex's position, moments, records and
+// rest offsets stay in registers and shared memory for all steps; a step is one
+// gather of the neighbours' positions (L2), the arithmetic, one store and a grid
+// barrier, beside which the next step's distance lookup and the loss partials
+// run.  Bound: the latency of that gather and barrier.  Every operation on a
+// value is k_fused_step's, in its order.
+// ---------------------------------------------------------------------------
+constexpr int RUN_REC = 12;  // records a thread keeps (a closed mesh's six neighbours twice); further ones are re-read
+constexpr int RUN_CHUNK = 4096;  // steps of a launch
+
+__device__ __forceinline__ void run_arrive(unsigned* bar) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+    }
+}
+
+// Waits until every block has arrived `target` times in total; after two seconds
+// (or another block's) it gives up: false.
+__device__ __forceinline__ bool run_wait(unsigned* bar, unsigned target) {
+    __shared__ int ok;
+    if (threadIdx.x == 0) {
+        ok = 1;
+        unsigned v, stop;
+        unsigned long long t0 = 0, t;
+        for (int n = 0;; ++n) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if ((n & 1023) == 1023) {
+                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+                if (t0 == 0) t0 = t;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(stop) : "l"(bar + 1) : "memory");
+                if (stop || t - t0 > 2000000000ull) {
+                    atomicExch(bar + 1, 1u);
+                    ok = 0;
+                    break;
+                }
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+template <bool WEIGHTED>
+__global__ void __launch_bounds__(STEP_THREADS, 2) k_fused_run(const __grid_constant__ MoPair P, int nsteps,
+                                                               float* __restrict__ tile_loss, int64_t loss_stride,
+                                                               unsigned* bar) {
+    extern __shared__ float offs[];  // [RUN_REC][3][threads] rest offsets of the kept records
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nt = blockDim.x;
+    const int slice = blockIdx.x * (nt >> 5) + w;
+    const bool live = slice < P.nslices;  // warp-uniform
+    const int i = slice * 32 + lane;
+    const bool valid = live && i < P.nv;
+    const float4* __restrict__ R = reinterpret_cast<const float4*>(P.rest);
+    float4* const pos0 = reinterpret_cast<float4*>(P.pos0);
+    float4* const pos1 = reinterpret_cast<float4*>(P.pos1);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 p = valid ? ((P.t0 & 1) ? pos1 : pos0)[i] : zero;
+    const float4 r0 = valid ? __ldg(R + i) : zero;
+    float* Mm = P.adam_m + 3 * (int64_t)i;
+    float* Vv = P.adam_v + 3 * (int64_t)i;
+    float m0 = 0.f, m1 = 0.f, m2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f;
+    if (valid) {
+        m0 = Mm[0]; m1 = Mm[1]; m2 = Mm[2];
+        v0 = Vv[0]; v1 = Vv[1]; v2 = Vv[2];
+    }
+    const int rb = live ? P.slice_ptr[slice] : 0;
+    const int rows = live ? (P.slice_ptr[slice + 1] - rb) >> 5 : 0;
+    const int* __restrict__ rec = P.sell + rb + lane;
+    const float* __restrict__ recw = WEIGHTED && P.sell_w ? P.sell_w + rb + lane : nullptr;
+    int c[RUN_REC];
+#pragma unroll
+    for (int u = 0; u < RUN_REC; ++u) {
+        c[u] = u < rows ? __ldg(rec + u * 32) : -1;
+        if (c[u] != -1) {
+            const float4 s = __ldg(R + (c[u] & 0x7fffffff));
+            offs[(3 * u) * nt + threadIdx.x] = SUB(s.x, r0.x);
+            offs[(3 * u + 1) * nt + threadIdx.x] = SUB(s.y, r0.y);
+            offs[(3 * u + 2) * nt + threadIdx.x] = SUB(s.z, r0.z);
+        }
+    }
+    const int N = P.N;
+    const float Nf = (float)N, Cf = (float)((double)(N - 1) - 1e-3);
+    const float we = P.w_edge, gh = P.grad_scale;
+    float dsq, gdx, gdy, gdz;
+    auto lookup = [&]() {
+        const DFJet j = (P.layout == MO_LAYOUT_CELL)
+                            ? df_eval_layout<MO_LAYOUT_CELL>(P.grid, N, Nf, Cf, p.x, p.y, p.z)
+                            : (P.layout == MO_LAYOUT_BRICK4)
+                                  ? df_eval_layout<MO_LAYOUT_BRICK4>(P.grid, N, Nf, Cf, p.x, p.y, p.z)
+                                  : df_eval_layout<MO_LAYOUT_LINEAR>(P.grid, N, Nf, Cf, p.x, p.y, p.z);
+        dsq = MUL(j.d, j.d);
+        gdx = df_grad_component(j.d, j.gx);
+        gdy = df_grad_component(j.d, j.gy);
+        gdz = df_grad_component(j.d, j.gz);
+        if (P.use_mask) {
+            const float mk = (MUL(dsq, 0.5f) < P.mask_thresh) ? 1.0f : 0.0f;
+            gdx = MUL(gdx, mk); gdy = MUL(gdy, mk); gdz = MUL(gdz, mk);
+        }
+    };
+    lookup();
+    float2 ab = __ldg(reinterpret_cast<const float2*>(P.adam_tab) + P.t0);
+    for (int k = 0; k < nsteps; ++k) {
+        const int t = P.t0 + k + 1;
+        const float4* Vin = (t & 1) ? pos0 : pos1;
+        float4* Vout = (t & 1) ? pos1 : pos0;
+        float4 q[RUN_REC];
+#pragma unroll
+        for (int u = 0; u < RUN_REC; ++u) q[u] = c[u] != -1 ? Vin[c[u] & 0x7fffffff] : zero;
+        float grx = 0.f, gry = 0.f, grz = 0.f, esq = 0.f;
+        auto edge = [&](int cu, float4 qu, float ox, float oy, float oz, int row) {
+            const float rx = SUB(SUB(qu.x, p.x), ox);
+            const float ry = SUB(SUB(qu.y, p.y), oy);
+            const float rz = SUB(SUB(qu.z, p.z), oz);
+            if (WEIGHTED) {
+                const float we_ = recw ? __ldg(recw + row * 32) : 1.0f;
+                const float l2 = MUL(we_, we_);
+                grx = SUB(grx, MUL(rx, l2)); gry = SUB(gry, MUL(ry, l2)); grz = SUB(grz, MUL(rz, l2));
+                if (cu >= 0) {
+                    const float ex = MUL(rx, we_), ey = MUL(ry, we_), ez = MUL(rz, we_);
+                    esq += ex * ex + ey * ey + ez * ez;
+                }
+            } else {
+                grx = SUB(grx, rx); gry = SUB(gry, ry); grz = SUB(grz, rz);
+                if (cu >= 0) esq += rx * rx + ry * ry + rz * rz;
+            }
+        };
+#pragma unroll
+        for (int u = 0; u < RUN_REC; ++u)
+            if (c[u] != -1)
+                edge(c[u], q[u], offs[(3 * u) * nt + threadIdx.x], offs[(3 * u + 1) * nt + threadIdx.x],
+                     offs[(3 * u + 2) * nt + threadIdx.x], u);
+        for (int row = RUN_REC; row < rows; ++row) {
+            const int cu = __ldg(rec + row * 32);
+            if (cu == -1) break;  // padding follows the last record
+            const int o = cu & 0x7fffffff;
+            const float4 s = __ldg(R + o);
+            edge(cu, Vin[o], SUB(s.x, r0.x), SUB(s.y, r0.y), SUB(s.z, r0.z), row);
+        }
+        const float gx = MUL(gh, ADD(gdx, MUL(grx, we)));
+        const float gy = MUL(gh, ADD(gdy, MUL(gry, we)));
+        const float gz = MUL(gh, ADD(gdz, MUL(grz, we)));
+        const float part = valid ? 0.5f * dsq + we * (0.5f * esq) : 0.f;
+        if (valid) {
+            if (P.grad_dbg) {
+                P.grad_dbg[3 * (int64_t)i] = gx;
+                P.grad_dbg[3 * (int64_t)i + 1] = gy;
+                P.grad_dbg[3 * (int64_t)i + 2] = gz;
+            }
+            adam_elem(p.x, gx, m0, v0, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
+            adam_elem(p.y, gy, m1, v1, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
+            adam_elem(p.z, gz, m2, v2, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
+            Vout[i] = make_float4(p.x, p.y, p.z, 0.f);
+        }
+        const bool more = k + 1 < nsteps;
+        if (more) run_arrive(bar);
+        if (tile_loss && slice < P.ntiles * TILE_WARPS) {
+            float s = part;
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) tile_loss[(int64_t)k * loss_stride + slice] = s;
+        }
+        if (!more) break;
+        ab = __ldg(reinterpret_cast<const float2*>(P.adam_tab) + t);
+        lookup();
+        if (!run_wait(bar, (unsigned)(k + 1) * gridDim.x)) {  // never in a working launch: no result
+            if (valid) pos0[i] = pos1[i] = make_float4(NAN, NAN, NAN, 0.f);
+            return;
+        }
+    }
+    if (valid) {
+        Mm[0] = m0; Mm[1] = m1; Mm[2] = m2;
+        Vv[0] = v0; Vv[1] = v1; Vv[2] = v2;
+    }
+}
+
+// Warps of a block (an SM's share of the slices, at most 8) and blocks of a run
+// over nslices slices; blocks 0: they do not fit the chip at once.
+static void run_shape(int nslices, int* warps, int* blocks) {
+    const int sms = device_sm_count();
+    *warps = std::max(1, std::min(TILE_WARPS, (nslices + sms - 1) / sms));
+    *blocks = (nslices + *warps - 1) / *warps;
+    if (*blocks > 2 * sms) *blocks = 0;  // 8 warps: two blocks an SM (registers)
+}
+
 // One warp per (pair, launch): lane l sums the pair's tile partials l, l+32,
 // ... in double, then a fixed shuffle tree adds the 32 lane sums.  The order
 // is fixed, so the result does not depend on scheduling.
@@ -293,6 +486,51 @@ extern "C" int mo_fused_step_on_demand(const MoPair* pairs, const MoTile* tiles,
                                        int max_tiles, int launch_index, float* tile_loss, int grid_ctas,
                                        void* stream) {
     return launch_fused_step(1, pairs, tiles, ntiles, max_tiles, launch_index, tile_loss, grid_ctas, stream);
+}
+
+extern "C" int mo_fused_run_fits(int64_t nv) {
+    if (nv <= 0 || nv > ((int64_t)1 << 30)) return 0;
+    int warps, blocks;
+    run_shape((int)((nv + 31) / 32), &warps, &blocks);
+    return blocks > 0 ? 1 : 0;
+}
+
+extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float* tile_loss, int64_t loss_stride,
+                            uint32_t* sync, void* stream) {
+    MO_CHECK_ARG(pair && sync, "null pointer");
+    MO_CHECK_ARG(nsteps >= 0, "negative step count");
+    const MoPair& q = *pair;
+    MO_CHECK_ARG(q.nv > 0 && q.nslices == (q.nv + 31) / 32 && q.N >= 2, "bad pair sizes");
+    MO_CHECK_ARG(q.grid && q.slice_ptr && q.sell && q.rest && q.pos0 && q.pos1 && q.adam_m && q.adam_v && q.adam_tab,
+                 "null pointer in the pair");
+    MO_CHECK_ARG(!tile_loss || (q.ntiles >= (q.nslices + TILE_WARPS - 1) / TILE_WARPS &&
+                                loss_stride >= (int64_t)q.ntiles * TILE_WARPS),
+                 "loss partials need whole tiles of %d slices", TILE_WARPS);
+    MO_CHECK_ARG(q.t0 >= 0 && nsteps <= q.t_end - q.t0, "more steps than the pair has left");
+    int warps, blocks;
+    run_shape(q.nslices, &warps, &blocks);
+    MO_CHECK_ARG(blocks > 0, "%d vertices do not fit one launch (mo_fused_run_fits)", q.nv);
+    if (tile_loss) {  // the slices past the last one of its tile
+        const int pad = q.ntiles * TILE_WARPS - q.nslices;
+        if (pad > 0 && nsteps > 0)
+            MO_CUDA(cudaMemset2DAsync(tile_loss + q.nslices, sizeof(float) * loss_stride, 0, sizeof(float) * pad, nsteps,
+                                      as_stream(stream)));
+    }
+    const int smem = RUN_REC * 3 * (int)sizeof(float) * 32 * warps;
+    for (int done = 0; done < nsteps;) {
+        int n = std::min(RUN_CHUNK, nsteps - done);
+        MoPair p = q;
+        p.t0 += done;
+        float* loss = tile_loss ? tile_loss + (int64_t)done * loss_stride : nullptr;
+        unsigned* bar = sync;
+        MO_CUDA(cudaMemsetAsync(sync, 0, 8, as_stream(stream)));
+        void* args[] = {&p, &n, &loss, &loss_stride, &bar};
+        MO_CUDA(cudaLaunchCooperativeKernel(weighted ? (const void*)k_fused_run<true> : (const void*)k_fused_run<false>,
+                                            dim3(blocks), dim3(32 * warps), args, smem, as_stream(stream)));
+        ::mo::note_launch();
+        done += n;
+    }
+    return MO_OK;
 }
 
 extern "C" int mo_pair_loss(const MoPair* pairs, int npairs, int max_tiles, int nlaunch, const float* tile_loss,

@@ -168,6 +168,25 @@ class Pair:
         return p
 
 
+    def run(self, nsteps, record_loss=False):
+        """The next nsteps steps in one launch (mo_fused_run); the per-step
+        losses (float64 [nsteps]) or None."""
+        nt = tiles_for(self.nslices)
+        row = self.struct(self.t, 0, nt)
+        stride = nt * SLICES_PER_TILE
+        partial = torch.empty(nsteps * stride, dtype=torch.float32, device=self.device) if record_loss else None
+        sync = torch.empty(2, dtype=torch.int32, device=self.device)
+        call("mo_fused_run", ctypes.byref(row), int(self.sell_w is not None), int(nsteps), ptr(partial), stride,
+             ptr(sync), stream_ptr())
+        self.t += nsteps
+        if not record_loss:
+            return None
+        table = torch.from_numpy(np.frombuffer(bytes(row), np.uint8).copy()).to(self.device)
+        out = torch.empty(nsteps, dtype=torch.float64, device=self.device)
+        call("mo_pair_loss", ptr(table), 1, nt, int(nsteps), ptr(partial), ptr(out), stream_ptr())
+        return out
+
+
 def tiles_for(nslices, slices_per_tile=SLICES_PER_TILE):
     return (nslices + slices_per_tile - 1) // slices_per_tile
 
@@ -303,6 +322,10 @@ def fused_fit(pid, src_V_norm, steps, lr=1e-3, group_steps=25, use_graph=True, w
     cad_loss_layer.py:9-31, on the weighted step).  Returns
     (final normalised positions [nv,3] on the device, per-step losses or None)."""
     pr = pair_from_template(pid, src_V_norm, steps, lr=lr, w_edge=w_edge, mask_thresh=mask_thresh)
+    if pr.steps > 0 and L.lib().mo_fused_run_fits(pr.nv):
+        # every vertex has a thread on the chip: all steps in one launch
+        losses = pr.run(pr.steps, record_loss)
+        return pr.positions(), losses
     runner = StepGroupRunner(pr.device, 1, pr.ntiles, group_steps=group_steps, use_graph=use_graph,
                              weighted=pr.sell_w is not None)
     losses = []
