@@ -89,6 +89,23 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
     return ax * bx + ay * by + az * bz;
 }
 
+// a b - c d to about one unit in the last place (Kahan).
+__device__ __forceinline__ float diff_prod(float a, float b, float c, float d) {
+    const float w = __fmul_rn(c, d);
+    return __fadd_rn(__fmaf_rn(a, b, -w), __fmaf_rn(-c, d, w));
+}
+
+// A triangle whose angle at a has a sine below 0.1 gets its normal from
+// rounding-free products: the plain cross product is off by up to ~1e-7 / sine
+// in direction, and in a frame that is that far from orthonormal the distance
+// of a far point is wrong by as much (for an exactly repeated vertex the
+// contracted products leave a normal of any direction), below what the boxes
+// around the triangle bound, so the grid would depend on the visit order.
+constexpr float THIN2 = 0.01f;
+// |cross|^2 below which a thin triangle is measured by its segments: its
+// height is then below 1e-8, and the square loses digits.
+constexpr float THIN_NN = 1e-30f;
+
 __device__ Tri make_tri(const float* __restrict__ Vn, int i0, int i1, int i2, float4* lo, float4* hi) {
     const float ax = Vn[3 * (int64_t)i0], ay = Vn[3 * (int64_t)i0 + 1], az = Vn[3 * (int64_t)i0 + 2];
     const float bx = Vn[3 * (int64_t)i1], by = Vn[3 * (int64_t)i1 + 1], bz = Vn[3 * (int64_t)i1 + 2];
@@ -99,15 +116,26 @@ __device__ Tri make_tri(const float* __restrict__ Vn, int i0, int i1, int i2, fl
     const float acx = cx - ax, acy = cy - ay, acz = cz - az;
     const float lab = dot3(abx, aby, abz, abx, aby, abz);
     float nx = aby * acz - abz * acy, ny = abz * acx - abx * acz, nz = abx * acy - aby * acx;
-    const float nn = dot3(nx, ny, nz, nx, ny, nz);
+    float nn = dot3(nx, ny, nz, nx, ny, nz);
+    bool face = nn > 0.f && isfinite(nn) && lab > 0.f;
+    const bool thin = nn < THIN2 * lab * dot3(acx, acy, acz, acx, acy, acz);
+    if (face && thin) {
+        nx = diff_prod(aby, acz, abz, acy);
+        ny = diff_prod(abz, acx, abx, acz);
+        nz = diff_prod(abx, acy, aby, acx);
+        nn = dot3(nx, ny, nz, nx, ny, nz);
+        face = nn > THIN_NN;
+    }
     Tri t;
-    if (nn > 0.f && isfinite(nn) && lab > 0.f) {
+    if (face) {
         const float inn = rsqrtf(nn);
         nx *= inn; ny *= inn; nz *= inn;
         const float len = sqrtf(lab), il = 1.0f / len;
         const float ex = abx * il, ey = aby * il, ez = abz * il;
         const float yx = ny * ez - nz * ey, yy = nz * ex - nx * ez, yz = nx * ey - ny * ex;  // n x ex
-        const float c2x = dot3(acx, acy, acz, ex, ey, ez), c2y = dot3(acx, acy, acz, yx, yy, yz);
+        // thin: the height is |cross| / |ab|, which no rounding makes negative
+        const float c2x = dot3(acx, acy, acz, ex, ey, ez);
+        const float c2y = thin ? sqrtf(nn) * il : dot3(acx, acy, acz, yx, yy, yz);
         const float ebx = c2x - len;
         const float lac = c2x * c2x + c2y * c2y, lbc = ebx * ebx + c2y * c2y;
         t.r0 = make_float4(ax, ay, az, len);
