@@ -89,23 +89,6 @@ __device__ __forceinline__ float dot3(float ax, float ay, float az, float bx, fl
     return ax * bx + ay * by + az * bz;
 }
 
-// a b - c d to about one unit in the last place (Kahan).
-__device__ __forceinline__ float diff_prod(float a, float b, float c, float d) {
-    const float w = __fmul_rn(c, d);
-    return __fadd_rn(__fmaf_rn(a, b, -w), __fmaf_rn(-c, d, w));
-}
-
-// A triangle whose angle at a has a sine below 0.1 gets its normal from
-// rounding-free products: the plain cross product is off by up to ~1e-7 / sine
-// in direction, and in a frame that is that far from orthonormal the distance
-// of a far point is wrong by as much (for an exactly repeated vertex the
-// contracted products leave a normal of any direction), below what the boxes
-// around the triangle bound, so the grid would depend on the visit order.
-constexpr float THIN2 = 0.01f;
-// |cross|^2 below which a thin triangle is measured by its segments: its
-// height is then below 1e-8, and the square loses digits.
-constexpr float THIN_NN = 1e-30f;
-
 __device__ Tri make_tri(const float* __restrict__ Vn, int i0, int i1, int i2, float4* lo, float4* hi) {
     const float ax = Vn[3 * (int64_t)i0], ay = Vn[3 * (int64_t)i0 + 1], az = Vn[3 * (int64_t)i0 + 2];
     const float bx = Vn[3 * (int64_t)i1], by = Vn[3 * (int64_t)i1 + 1], bz = Vn[3 * (int64_t)i1 + 2];
@@ -116,26 +99,15 @@ __device__ Tri make_tri(const float* __restrict__ Vn, int i0, int i1, int i2, fl
     const float acx = cx - ax, acy = cy - ay, acz = cz - az;
     const float lab = dot3(abx, aby, abz, abx, aby, abz);
     float nx = aby * acz - abz * acy, ny = abz * acx - abx * acz, nz = abx * acy - aby * acx;
-    float nn = dot3(nx, ny, nz, nx, ny, nz);
-    bool face = nn > 0.f && isfinite(nn) && lab > 0.f;
-    const bool thin = nn < THIN2 * lab * dot3(acx, acy, acz, acx, acy, acz);
-    if (face && thin) {
-        nx = diff_prod(aby, acz, abz, acy);
-        ny = diff_prod(abz, acx, abx, acz);
-        nz = diff_prod(abx, acy, aby, acx);
-        nn = dot3(nx, ny, nz, nx, ny, nz);
-        face = nn > THIN_NN;
-    }
+    const float nn = dot3(nx, ny, nz, nx, ny, nz);
     Tri t;
-    if (face) {
+    if (nn > 0.f && isfinite(nn) && lab > 0.f) {
         const float inn = rsqrtf(nn);
         nx *= inn; ny *= inn; nz *= inn;
         const float len = sqrtf(lab), il = 1.0f / len;
         const float ex = abx * il, ey = aby * il, ez = abz * il;
         const float yx = ny * ez - nz * ey, yy = nz * ex - nx * ez, yz = nx * ey - ny * ex;  // n x ex
-        // thin: the height is |cross| / |ab|, which no rounding makes negative
-        const float c2x = dot3(acx, acy, acz, ex, ey, ez);
-        const float c2y = thin ? sqrtf(nn) * il : dot3(acx, acy, acz, yx, yy, yz);
+        const float c2x = dot3(acx, acy, acz, ex, ey, ez), c2y = dot3(acx, acy, acz, yx, yy, yz);
         const float ebx = c2x - len;
         const float lac = c2x * c2x + c2y * c2y, lbc = ebx * ebx + c2y * c2y;
         t.r0 = make_float4(ax, ay, az, len);
@@ -155,6 +127,70 @@ __device__ Tri make_tri(const float* __restrict__ Vn, int i0, int i1, int i2, fl
                            0.f);
     }
     return t;
+}
+
+// a b - c d to about one unit in the last place (Kahan).
+__device__ __forceinline__ float diff_prod(float a, float b, float c, float d) {
+    const float w = __fmul_rn(c, d);
+    return __fadd_rn(__fmaf_rn(a, b, -w), __fmaf_rn(-c, d, w));
+}
+
+// A triangle whose angle at a has a sine below 0.1 gets its normal from
+// rounding-free products: the plain cross product is off by up to ~1e-7 / sine
+// in direction, and in a frame that is that far from orthonormal the distance
+// of a far point is wrong by as much (for an exactly repeated vertex the
+// contracted products leave a normal of any direction), below what the boxes
+// around the triangle bound, so the grid would depend on the visit order.
+constexpr float THIN2 = 0.01f;
+// |cross|^2 below which a thin triangle is measured by its segments: its
+// height is then below 1e-8, and the square loses digits.
+constexpr float THIN_NN = 1e-30f;
+
+// ac lies within the angle of ab in whatever frame the plain normal gave.
+// (The asm keeps these products apart from make_tri's: shared, they would
+// change which of its sums are contracted, and with it every record's last
+// bits.)
+__device__ __forceinline__ bool thin(const Tri& t) {
+    float cx = t.r1.w, cy = t.r2.w;
+    asm volatile("" : "+f"(cx), "+f"(cy));
+    return t.r3.w != 0.f && cy * cy < THIN2 * (cx * cx + cy * cy);
+}
+
+__device__ __noinline__ void thin_tri(const float* __restrict__ Vn, int i0, int i1, int i2, Tri* out) {
+    const float* a = Vn + 3 * (int64_t)i0;
+    const float* b = Vn + 3 * (int64_t)i1;
+    const float* c = Vn + 3 * (int64_t)i2;
+    const float3 ab = make_float3(b[0] - a[0], b[1] - a[1], b[2] - a[2]),
+                 ac = make_float3(c[0] - a[0], c[1] - a[1], c[2] - a[2]);
+    const float lab = dot3(ab.x, ab.y, ab.z, ab.x, ab.y, ab.z);
+    float nx = diff_prod(ab.y, ac.z, ab.z, ac.y), ny = diff_prod(ab.z, ac.x, ab.x, ac.z),
+          nz = diff_prod(ab.x, ac.y, ab.y, ac.x);
+    const float nn = dot3(nx, ny, nz, nx, ny, nz);
+    Tri t;
+    if (nn > THIN_NN) {
+        const float cr = sqrtf(nn), inn = 1.0f / cr, len = sqrtf(lab), il = 1.0f / len;
+        nx *= inn; ny *= inn; nz *= inn;
+        const float ex = ab.x * il, ey = ab.y * il, ez = ab.z * il;
+        // the height as |cross| / |ab|, which no rounding makes negative
+        const float c2x = dot3(ac.x, ac.y, ac.z, ex, ey, ez), c2y = cr * il;
+        const float ebx = c2x - len;
+        const float lac = c2x * c2x + c2y * c2y, lbc = ebx * ebx + c2y * c2y;
+        t.r0 = make_float4(a[0], a[1], a[2], len);
+        t.r1 = make_float4(ex, ey, ez, c2x);
+        t.r2 = make_float4(ny * ez - nz * ey, nz * ex - nx * ez, nx * ey - ny * ex, c2y);
+        t.r3 = make_float4(nx, ny, nz, 1.f);
+        t.r4 = make_float4(il, lac > 0.f ? 1.0f / lac : 0.f, lbc > 0.f ? 1.0f / lbc : 0.f, ebx);
+    } else {
+        const float3 bc = make_float3(c[0] - b[0], c[1] - b[1], c[2] - b[2]);
+        const float lbc = dot3(bc.x, bc.y, bc.z, bc.x, bc.y, bc.z), lca = dot3(ac.x, ac.y, ac.z, ac.x, ac.y, ac.z);
+        t.r0 = make_float4(a[0], a[1], a[2], 0.f);
+        t.r1 = make_float4(b[0], b[1], b[2], 0.f);
+        t.r2 = make_float4(c[0], c[1], c[2], 0.f);
+        t.r3 = make_float4(0.f, 0.f, 0.f, 0.f);
+        t.r4 = make_float4(lab > 0.f ? 1.0f / lab : 0.f, lbc > 0.f ? 1.0f / lbc : 0.f, lca > 0.f ? 1.0f / lca : 0.f,
+                           0.f);
+    }
+    *out = t;
 }
 
 __device__ __forceinline__ void store_tri(float4* __restrict__ tris, int i, const Tri& t) {
@@ -202,7 +238,9 @@ __global__ void k_tri_records(const float* __restrict__ Vn, const int32_t* __res
     int i0 = F[3 * f], i1 = F[3 * f + 1], i2 = F[3 * f + 2];
     if (i0 < 0 || i1 < 0 || i2 < 0 || i0 >= nv || i1 >= nv || i2 >= nv) i0 = i1 = i2 = 0;  // flagged earlier
     float4 lo, hi;
-    store_tri(tris, (int)i, make_tri(Vn, i0, i1, i2, &lo, &hi));
+    Tri t = make_tri(Vn, i0, i1, i2, &lo, &hi);
+    if (thin(t)) thin_tri(Vn, i0, i1, i2, &t);
+    store_tri(tris, (int)i, t);
     if (boxes) {
         boxes[2 * i] = lo;
         boxes[2 * i + 1] = hi;
