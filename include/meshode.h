@@ -132,13 +132,17 @@ size_t mo_df_noalloc_scratch_capacity(void);
 #define MO_PACKET_LAST 9
 typedef struct MoDfOptions {
     int32_t method;   /* MO_DF_AUTO, MO_DF_BRUTE or MO_DF_LBVH */
-    int32_t packet;   /* MO_PACKET_* for MO_DF_LBVH */
+    int32_t packet;   /* MO_PACKET_* for MO_DF_LBVH; MO_DF_AUTO with
+                       * MO_PACKET_4x4x2 (0) takes mo_df_packet_for's */
     float band;       /* 0: exact grid.  > 0: voxels at distance >= band store
                        * band, except in the two lowest layers along each axis
                        * (x, y or z <= 1), whose band is band + 13/N; see
                        * mo_df_loss_band */
     int32_t reserved; /* 0 */
 } MoDfOptions;
+/* The packet shape of a build of an N^3 grid over nf triangles (band as in
+ * MoDfOptions) whose caller names none. */
+int mo_df_packet_for(int64_t nf, int N, float band);
 /* mo_df_build with explicit build options (opt == NULL: defaults).  method
  * and packet change only the speed, never the grid. */
 int mo_df_build_ex(const float* V, int64_t nv, const int32_t* F, int64_t nf, int N,
@@ -457,7 +461,7 @@ typedef struct MoRequest {
     int32_t layout;         /* -1: the pool's default */
     int32_t slices_per_tile;/* 0: the pool's default */
     int32_t df_method;      /* MO_DF_AUTO / BRUTE / LBVH */
-    int32_t df_packet;      /* MO_PACKET_* */
+    int32_t df_packet;      /* MO_PACKET_*, as MoDfOptions.packet */
     float df_band;          /* < 0: mo_df_loss_band(N); 0: exact grid; > 0: this band */
     int32_t out_on_host;    /* V_out is host memory (pinned, for the copy to overlap) */
     float* V_out;           /* optional [nv,3]: the denormalised result, written at retirement */

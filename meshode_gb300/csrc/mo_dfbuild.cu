@@ -946,6 +946,31 @@ extern "C" int mo_df_method_for(int64_t nf, int N) {
     return (nf <= 64 || pairs <= 3.0e8) ? MO_DF_BRUTE : MO_DF_LBVH;
 }
 
+// The traversal packet of a build whose caller names none.  Two things pull:
+// a warp of 64 voxels (4x4x4) walks the nodes they share once, but a coarse
+// grid then has too few warps to hide the chain of node loads (64^3: 4096 of
+// them, less than the chip holds), and where triangles are small against a
+// voxel its 64 voxels share little.  There the narrow packet that tests two
+// triangles at a time (2x4x4_TRI2) is the shortest walk.  Measured over
+// N 32..256, 1k..1.3M triangles, a sphere-like and a flat elongated target,
+// against 4x4x2 for all (ms a build):
+//   exact 128^3, 355k: 4.22 -> 3.39; 256^3, 1.3M: 35.6 -> 26.0; 96^3, 10k: 0.55 -> 0.50
+//   exact 64^3, 20k: 0.55 -> 0.48; 64^3, 456k: 2.75 -> 2.27; 32^3, 100k: 1.68 -> 1.06
+//   band 128^3, 30k: 0.92 -> 0.73; 64^3, 100k: 1.08 -> 0.86
+// The lines: below N = 72 the wide packet has too few warps at any triangle
+// count.  With a band the far voxels, whose walks are the ones 64 voxels
+// share best, are cut short, so the wide packet stops paying at N^3 / 48
+// triangles (128^3, 300k: 2.36 for 4x4x2, 2.35 wide, 2.27 for 2x4x4; flat
+// target 1.67, 1.82, 1.27) against about N^3 / 4 on an exact grid (112^3,
+// 500k: 3.89, 4.06, 3.84).
+extern "C" int mo_df_packet_for(int64_t nf, int N, float band) {
+    const double vox = (double)N * N * N;
+    if (N < 72) return MO_PACKET_2x4x4_TRI2;
+    const bool far_walks = !(band > 0.0f) && N >= 100;
+    if ((double)nf <= vox / (far_walks ? 4.0 : 48.0)) return MO_PACKET_4x4x4;
+    return N < 100 ? MO_PACKET_2x4x4_TRI2 : MO_PACKET_2x4x4;
+}
+
 extern "C" size_t mo_df_build_scratch_bytes(int64_t nv, int64_t nf, int N, int method) {
     if (nv < 0 || nf < 0) return 0;
     if (method == MO_DF_AUTO) method = mo_df_method_for(nf, N);
@@ -958,7 +983,7 @@ static int df_build_impl(const float* V, int64_t nv, const int32_t* F, int64_t n
                          const MoDfOptions* opt, void* scratch, size_t scratch_bytes, float* grid_out,
                          int32_t* status_out, unsigned long long* counts, void* stream) {
     int method = opt ? opt->method : MO_DF_AUTO;
-    const int packet = opt ? opt->packet : MO_PACKET_4x4x2;
+    int packet = opt ? opt->packet : MO_PACKET_4x4x2;
     const float band = opt ? opt->band : 0.0f;
     MO_CHECK_ARG(packet >= MO_PACKET_4x4x2 && packet <= MO_PACKET_LAST, "unknown packet shape %d", packet);
     MO_CHECK_ARG(band >= 0.0f && band <= 4.0f, "band must be in [0, 4] (0: exact grid), got %g", (double)band);
@@ -969,7 +994,10 @@ static int df_build_impl(const float* V, int64_t nv, const int32_t* F, int64_t n
     MO_CHECK_ARG(N >= 2 && N <= 2048, "grid resolution out of range (%d)", N);
     MO_CHECK_ARG(V && F && params4 && grid_out, "null pointer");
     MO_CHECK_ARG(method == MO_DF_AUTO || method == MO_DF_BRUTE || method == MO_DF_LBVH, "unknown method %d", method);
-    if (method == MO_DF_AUTO) method = mo_df_method_for(nf, N);
+    if (method == MO_DF_AUTO) {
+        method = mo_df_method_for(nf, N);
+        if (packet == MO_PACKET_4x4x2) packet = mo_df_packet_for(nf, N, band);
+    }
     MO_CHECK_ARG(method != MO_DF_LBVH || nf <= MAX_TREE_TRIANGLES, "target mesh too large for the LBVH (%lld > %lld)",
                  (long long)nf, (long long)MAX_TREE_TRIANGLES);
     cudaStream_t s = as_stream(stream);
@@ -1048,7 +1076,7 @@ extern "C" int mo_df_build(const float* V, int64_t nv, const int32_t* F, int64_t
     MoDfOptions opt;
     std::memset(&opt, 0, sizeof(opt));
     opt.method = method;
-    opt.packet = MO_PACKET_4x4x2;
+    opt.packet = mo_df_packet_for(nf, N, 0.0f);
     return mo_df_build_ex(V, nv, F, nf, N, params4, &opt, scratch, scratch_bytes, grid_out, status_out, stream);
 }
 

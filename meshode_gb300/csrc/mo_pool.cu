@@ -775,9 +775,11 @@ extern "C" int mo_pool_submit(MoPool* P, const MoRequest* q, int64_t* id_out) {
     MO_CHECK_ARG(q->df_packet >= MO_PACKET_4x4x2 && q->df_packet <= MO_PACKET_LAST, "unknown packet %d",
                  q->df_packet);
     R->method = q->df_method == MO_DF_AUTO ? mo_df_method_for(q->ntf, q->N) : q->df_method;
-    R->packet = q->df_packet;
     MO_CHECK_ARG(q->df_band <= 4.0f && q->df_band == q->df_band, "bad DF band %g", (double)q->df_band);
     R->band = q->df_band < 0.0f ? mo_df_loss_band(q->N) : q->df_band;
+    R->packet = q->df_method == MO_DF_AUTO && q->df_packet == MO_PACKET_4x4x2
+                    ? mo_df_packet_for(q->ntf, q->N, R->band)
+                    : q->df_packet;
     int rc = adam_table(P, q->lr, q->steps, &R->adam_tab);
     if (rc) return rc;
     R->id = P->next_id++;
