@@ -221,11 +221,33 @@ __global__ void k_morton(const float* __restrict__ Vn, const int32_t* __restrict
     codes[f] = (spread10(quant10(c[0])) << 2) | (spread10(quant10(c[1])) << 1) | spread10(quant10(c[2]));
 }
 
-__global__ void k_check_faces(const int32_t* __restrict__ F, int64_t nf, int64_t nv, int* __restrict__ status) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 3 * nf) return;
-    const int v = F[i];
-    if (v < 0 || v >= nv) atomicOr(status, 1);
+// The brute force's triangle records straight from the target: the face's
+// check, its corners' normalisation and its record in one launch (they were
+// three; with a few hundred triangles a launch costs more than its work).  A
+// vertex is normalised once per face that uses it, nine double divisions a
+// triangle, which only small targets can afford.
+constexpr int TRI_RAW_THREADS = 64;
+__global__ void __launch_bounds__(TRI_RAW_THREADS) k_tri_records_raw(const float* __restrict__ V,
+                                                                     const int32_t* __restrict__ F, int64_t nf,
+                                                                     int64_t nv, const double* __restrict__ prm,
+                                                                     float4* __restrict__ tris,
+                                                                     int* __restrict__ status) {
+    const int64_t i = (int64_t)blockIdx.x * TRI_RAW_THREADS + threadIdx.x;
+    if (i >= nf) return;
+    int id[3] = {F[3 * i], F[3 * i + 1], F[3 * i + 2]};
+    if (id[0] < 0 || id[1] < 0 || id[2] < 0 || id[0] >= nv || id[1] >= nv || id[2] >= nv) {
+        atomicOr(status, 1);
+        id[0] = id[1] = id[2] = 0;
+    }
+    const double s = prm[0];
+    float v[9];
+    for (int k = 0; k < 3; ++k)
+        for (int c = 0; c < 3; ++c)
+            v[3 * k + c] = (float)__ddiv_rn(__dsub_rn((double)V[3 * (int64_t)id[k] + c], prm[1 + c]), s);
+    float4 lo, hi;
+    Tri t = make_tri(v, 0, 1, 2, &lo, &hi);
+    if (thin(t)) thin_tri(v, 0, 1, 2, &t);
+    store_tri(tris, (int)i, t);
 }
 
 // Sorted triangle records (leaf order) from the sorted ids.
@@ -726,52 +748,127 @@ static void launch_df_lbvh(int packet, const float4* nodes, const float4* tris, 
 #undef MO_ARGS
 }
 
-// Brute force: one warp per packet of 4 x 4 x 2 voxels with two voxels per
-// lane (the packet and the one 2 above it in z, so a warp covers 4 x 4 x 4),
-// triangles staged through shared memory in chunks and each tested against
-// both voxels of a lane at once on the packed FP32 pipe (tri_d2_2, the same
-// IEEE operations per voxel as tri_d2).  A compact packet lets the
-// warp-wide plane-distance cull skip most tests; a skipped test could not
-// have lowered any lane's best, so every voxel gets the minimum over all
-// triangles, as a test of every pair would.
-constexpr int BF_THREADS = 256, BF_CHUNK = 128;
-constexpr int BF_PX = 4, BF_PY = 4, BF_PZ = 2;
+// Brute force, for targets too small to be worth a tree: a warp (or, on a
+// small grid, `split` warps of a block, each with every split-th triangle) per
+// packet of 4 x 4 x 4 voxels, two voxels per lane on the packed FP32 pipe
+// (tri_d2_2, the same IEEE operations per voxel as tri_d2).
+//
+// A test of a triangle against 64 voxels is ~100 instructions, so the lanes
+// first sort out the triangles that cannot be nearest for any voxel of the
+// packet, one triangle a lane: with c a triangle's centroid, r the radius of
+// its vertices around it, p the packet's centre and R its radius, no voxel's
+// distance is above U = min |p - c| + R, and none to this triangle is below
+// |p - c| - r - R.  CULL_SLACK is far more than these bounds' and the tests'
+// rounding, so what is dropped could not have lowered any voxel's minimum and
+// every voxel gets the minimum over all triangles.
+// Measured (records and grid, us): see mo_df_method_for.
+constexpr int BF_WARPS = 8;
+constexpr int BF_P = 4;  // packet edge, voxels
+constexpr float CULL_SLACK = 4e-6f;
 
 __host__ __device__ __forceinline__ int64_t bf_bricks(int N) {
-    return (int64_t)((N + BF_PX - 1) / BF_PX) * ((N + BF_PY - 1) / BF_PY) * ((N + 2 * BF_PZ - 1) / (2 * BF_PZ));
+    const int64_t b = (N + BF_P - 1) / BF_P;
+    return b * b * b;
 }
 
-__global__ void __launch_bounds__(BF_THREADS) k_df_brute(const float4* __restrict__ tris, int ntri, int N,
-                                                         float band, float band2, float* __restrict__ grid) {
-    __shared__ float4 sh[BF_CHUNK * TRI_F4];
+// Warps per packet: enough packets times warps for one resident wave (32
+// warps an SM); more would only repeat the bounds.
+static int bf_split(int N) {
+    int s = BF_WARPS;
+    while (s > 1 && bf_bricks(N) * s > (int64_t)32 * device_sm_count()) s >>= 1;
+    return s;
+}
+
+// Centroid and squared vertex radius of a record, and the squared distance of
+// the centroid from p.
+__device__ __forceinline__ void tri_sphere(const float4* __restrict__ tris, int i, float px, float py, float pz,
+                                           float* d2, float* r2) {
+    const float4* q = tris + TRI_F4 * (int64_t)i;
+    const float4 r0 = __ldg(q), r1 = __ldg(q + 1), r2v = __ldg(q + 2), r3 = __ldg(q + 3);
+    float cx, cy, cz;
+    if (r3.w != 0.f) {
+        const float gx = (r0.w + r1.w) * (1.f / 3.f), gy = r2v.w * (1.f / 3.f);
+        cx = r0.x + gx * r1.x + gy * r2v.x;
+        cy = r0.y + gx * r1.y + gy * r2v.y;
+        cz = r0.z + gx * r1.z + gy * r2v.z;
+        const float ux = gx - r0.w, vx = gx - r1.w, vy = gy - r2v.w;
+        *r2 = fmaxf(gx * gx, fmaxf(ux * ux, vx * vx + vy * vy - gy * gy)) + gy * gy;
+    } else {
+        cx = (r0.x + r1.x + r2v.x) * (1.f / 3.f);
+        cy = (r0.y + r1.y + r2v.y) * (1.f / 3.f);
+        cz = (r0.z + r1.z + r2v.z) * (1.f / 3.f);
+        *r2 = fmaxf(dot3(r0.x - cx, r0.y - cy, r0.z - cz, r0.x - cx, r0.y - cy, r0.z - cz),
+                    fmaxf(dot3(r1.x - cx, r1.y - cy, r1.z - cz, r1.x - cx, r1.y - cy, r1.z - cz),
+                          dot3(r2v.x - cx, r2v.y - cy, r2v.z - cz, r2v.x - cx, r2v.y - cy, r2v.z - cz)));
+    }
+    *d2 = dot3(cx - px, cy - py, cz - pz, cx - px, cy - py, cz - pz);
+}
+
+__global__ void __launch_bounds__(BF_WARPS * 32) k_df_brute(const float4* __restrict__ tris, int ntri, int N,
+                                                            float band, float band2, int split,
+                                                            float* __restrict__ grid) {
+    __shared__ float sh_u[BF_WARPS];
+    __shared__ float2 sh_best[BF_WARPS][32];
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int bx = (N + BF_PX - 1) / BF_PX, by = (N + BF_PY - 1) / BF_PY;
-    const int64_t brick = (int64_t)blockIdx.x * (BF_THREADS / 32) + w;
-    // a warp past the last packet still stages triangles with its block
-    const bool live = brick < bf_bricks(N);
+    const int part = w & (split - 1);
+    const int64_t brick = ((int64_t)blockIdx.x * BF_WARPS + w) / split;
+    const bool live = brick < bf_bricks(N);  // a warp past the last packet only follows
+    const int nb = (N + BF_P - 1) / BF_P;
     const int64_t b = live ? brick : 0;
-    const int ix = (int)(b % bx), iy = (int)((b / bx) % by), iz = (int)(b / ((int64_t)bx * by));
-    const int x = ix * BF_PX + (lane % BF_PX), y = iy * BF_PY + ((lane / BF_PX) % BF_PY);
-    const int za = iz * 2 * BF_PZ + lane / (BF_PX * BF_PY), zb = za + BF_PZ;
+    const int ix = (int)(b % nb), iy = (int)((b / nb) % nb), iz = (int)(b / ((int64_t)nb * nb));
+    const int x = ix * BF_P + (lane & 3), y = iy * BF_P + ((lane >> 2) & 3);
+    const int za = iz * BF_P + (lane >> 4), zb = za + 2;
     const bool va = live && x < N && y < N && za < N, vb = live && x < N && y < N && zb < N;
     const float Nf = (float)N;
-    const float fx = __fdiv_rn((float)x, Nf), fy = __fdiv_rn((float)y, Nf);
-    const float2 px = bc2(fx), py = bc2(fy);
+    const float2 px = bc2(__fdiv_rn((float)x, Nf)), py = bc2(__fdiv_rn((float)y, Nf));
     const float2 pz = make_float2(__fdiv_rn((float)za, Nf), __fdiv_rn((float)zb, Nf));
     const VoxelBand ba = voxel_band(x, y, za, N, band, band2), bb = voxel_band(x, y, zb, N, band, band2);
     float2 best = make_float2(ba.bound2, bb.bound2);
-    for (int base = 0; base < ntri; base += BF_CHUNK) {
-        const int cnt = min(BF_CHUNK, ntri - base);
-        __syncthreads();
-        for (int k = threadIdx.x; k < cnt * TRI_F4; k += BF_THREADS) sh[k] = tris[TRI_F4 * (int64_t)base + k];
-        __syncthreads();
-        for (int t = 0; t < cnt; ++t) {
-            Tri T;
-            T.r0 = sh[TRI_F4 * t]; T.r1 = sh[TRI_F4 * t + 1]; T.r2 = sh[TRI_F4 * t + 2];
-            T.r3 = sh[TRI_F4 * t + 3]; T.r4 = sh[TRI_F4 * t + 4];
-            const float2 d = tri_d2_2(px, py, pz, T, make_float2(va ? best.x : -1.0f, vb ? best.y : -1.0f));
+    const float half = 0.5f * (BF_P - 1);
+    const float cx = (ix * BF_P + half) / Nf, cy = (iy * BF_P + half) / Nf, cz = (iz * BF_P + half) / Nf;
+    const float R = 1.7320508f * half / Nf;
+    const int first = part + split * lane, stride = 32 * split;
+
+    float u = FLT_MAX;
+    for (int t = first; t < ntri; t += stride) {
+        float d2, r2;
+        tri_sphere(tris, t, cx, cy, cz, &d2, &r2);
+        u = fminf(u, d2);
+    }
+    for (int o = 16; o > 0; o >>= 1) u = fminf(u, __shfl_xor_sync(FULL, u, o));
+    if (lane == 0) sh_u[w] = u;
+    __syncthreads();
+    for (int k = 0; k < split; ++k) u = fminf(u, sh_u[(w & ~(split - 1)) + k]);
+    float U = sqrtf(u) + R;
+    if (band2 != FLT_MAX) U = fminf(U, band + 13.0f / Nf);  // the widest band of any voxel
+    const float reach = U + R + CULL_SLACK;
+
+    for (int base = 0; base < ntri; base += stride) {
+        const int t = base + first;
+        bool keep = live && t < ntri;
+        if (keep) {
+            float d2, r2;
+            tri_sphere(tris, t, cx, cy, cz, &d2, &r2);
+            keep = !(sqrtf(d2) > sqrtf(r2) + reach);  // NaN: tested
+        }
+        unsigned m = __ballot_sync(FULL, keep);
+        while (m) {
+            const int l = __ffs(m) - 1;
+            m &= m - 1;
+            const float2 d = tri_d2_2(px, py, pz, load_tri(tris, base + part + split * l),
+                                      make_float2(va ? best.x : -1.0f, vb ? best.y : -1.0f));
             best.x = fminf(best.x, d.x);
             best.y = fminf(best.y, d.y);
+        }
+    }
+    if (split > 1) {
+        sh_best[w][lane] = best;
+        __syncthreads();
+        if (part != 0) return;
+        for (int k = 1; k < split; ++k) {
+            best.x = fminf(best.x, sh_best[w + k][lane].x);
+            best.y = fminf(best.y, sh_best[w + k][lane].y);
         }
     }
     if (va) grid[((int64_t)za * N + y) * N + x] = best.x < ba.bound2 ? __fsqrt_rn(best.x) : ba.value;
@@ -940,8 +1037,12 @@ extern "C" float mo_df_loss_band(int N) {
 }
 
 extern "C" int mo_df_method_for(int64_t nf, int N) {
-    // Brute force tests every voxel against every triangle; below ~3e8 pair
-    // tests it beats building and walking the tree.
+    // Brute force bounds every packet of voxels against every triangle; below
+    // ~3e8 pairs that beats building and walking the tree (sphere-like and flat
+    // target, us a build).  64^3: 320 triangles 71 against 119, 700 118-184
+    // against 148-160, 1400 207-332 against 185-195; 32^3: 6000 197 against
+    // 288, 24k 850 against 554.  Testing every pair without bounding them first
+    // took 61 us for 320 triangles at 32^3 (31 now), 823 for 6000.
     const double pairs = (double)nf * (double)N * N * N;
     return (nf <= 64 || pairs <= 3.0e8) ? MO_DF_BRUTE : MO_DF_LBVH;
 }
@@ -1022,19 +1123,21 @@ static int df_build_impl(const float* V, int64_t nv, const int32_t* F, int64_t n
             e = cudaMemsetAsync(S.status, 0, sizeof(int) * 4, s);
             if (e != cudaSuccess) { fail(e, "memset"); break; }
         }
-        k_normalize_copy<<<ceil_div(3 * nv, 256), 256, 0, s>>>(V, nv, params4, S.Vn); ::mo::note_launch();
         if (method == MO_DF_BRUTE) {
-            k_check_faces<<<ceil_div(nf, 256), 256, 0, s>>>(F, nf, nv, st); ::mo::note_launch();
-            k_tri_records<<<ceil_div(nf, 256), 256, 0, s>>>(S.Vn, F, nf, nv, nullptr, S.tris, nullptr); ::mo::note_launch();
-            const int64_t nvox = (int64_t)N * N * N;
-            k_df_brute<<<ceil_div(bf_bricks(N), BF_THREADS / 32), BF_THREADS, 0, s>>>(S.tris, (int)nf, N, band,
-                                                                                   band2, grid_out);
+            k_tri_records_raw<<<ceil_div(nf, TRI_RAW_THREADS), TRI_RAW_THREADS, 0, s>>>(V, F, nf, nv, params4, S.tris,
+                                                                                        st);
             ::mo::note_launch();
-            if (counts) {  // every voxel tests every triangle
+            const int64_t nvox = (int64_t)N * N * N;
+            const int split = bf_split(N);
+            k_df_brute<<<ceil_div(bf_bricks(N) * split, BF_WARPS), BF_WARPS * 32, 0, s>>>(S.tris, (int)nf, N, band,
+                                                                                       band2, split, grid_out);
+            ::mo::note_launch();
+            if (counts) {  // every pair of a voxel and a triangle is decided
                 k_add_u64<<<1, 1, 0, s>>>(counts + 1, (unsigned long long)nvox * (unsigned long long)nf);
                 ::mo::note_launch();
             }
         } else {
+            k_normalize_copy<<<ceil_div(3 * nv, 256), 256, 0, s>>>(V, nv, params4, S.Vn); ::mo::note_launch();
             e = issue_tree(S, F, nv, nf, st, s);
             if (e != cudaSuccess) { fail(e, "LBVH build"); break; }
             launch_df_lbvh(packet, S.tnodes, S.tris, (int)nf, N, band, band2, grid_out, st, counts, s);
