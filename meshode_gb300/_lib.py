@@ -84,6 +84,7 @@ _SIGS = {
     "mo_launch_count": (ctypes.c_ulonglong, []),
     "mo_bbox": (_I, [_P, _I64, _P, _P]),
     "mo_norm_params": (_I, [_P, _P, _P]),
+    "mo_bbox_params": (_I, [_P, _I64, _P, _P, _P]),
     "mo_normalize": (_I, [_P, _I64, _P, _I, _P]),
     "mo_df_build_scratch_bytes": (_SZ, [_I64, _I64, _I, _I]),
     "mo_df_build": (_I, [_P, _I64, _P, _I64, _I, _P, _I, _P, _SZ, _P, _P, _P]),

@@ -233,8 +233,7 @@ int phase_a(MoPool* P, Req* R) {
     PCHK(palloc(P, &R->params, 32, s));
     PCHK(palloc(P, &R->status, 16, s));
     PCHK(cudaMemsetAsync(R->status, 0, 16, s));
-    int rc = mo_bbox(tarV, q.ntv, R->bbox, sv);
-    if (!rc) rc = mo_norm_params(R->bbox, R->params, sv);
+    int rc = mo_bbox_params(tarV, q.ntv, R->bbox, R->params, sv);
     if (rc) return rc;
     const int N = q.N;
     if (R->lazy) {

@@ -294,8 +294,7 @@ def InitializeDeformTemplate(tensorV, tensorF, symmetry, grid_resolution, layout
     Fd = _on_device(tensorF, dev)
     bbox = torch.empty(6, dtype=torch.int32, device=dev)
     p.params = torch.empty(4, dtype=torch.float64, device=dev)
-    call("mo_bbox", ptr(Vd), Vd.shape[0], ptr(bbox), s)
-    call("mo_norm_params", ptr(bbox), ptr(p.params), s)
+    call("mo_bbox_params", ptr(Vd), Vd.shape[0], ptr(bbox), ptr(p.params), s)
     nbytes = L.lib().mo_df_build_scratch_bytes(Vd.shape[0], Fd.shape[0], N, int(df_method))
     scratch = torch.empty(int(nbytes), dtype=torch.uint8, device=dev)
     p.grid_linear = torch.empty(N * N * N, dtype=torch.float32, device=dev)

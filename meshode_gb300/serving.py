@@ -150,8 +150,7 @@ class ServingEngine:
             job.status = torch.zeros(4, dtype=torch.int32, device=self.device)
             bbox = torch.empty(6, dtype=torch.int32, device=self.device)
             job.params = torch.empty(4, dtype=torch.float64, device=self.device)
-            call("mo_bbox", ptr(Td), Td.shape[0], ptr(bbox), s)
-            call("mo_norm_params", ptr(bbox), ptr(job.params), s)
+            call("mo_bbox_params", ptr(Td), Td.shape[0], ptr(bbox), ptr(job.params), s)
             N = req.N
             if self.autotuner is not None:
                 method, packet = self.autotuner.df_options(N, TFd.shape[0])
