@@ -269,6 +269,20 @@ int mo_edge_backward_w(const float* V, int64_t nv, const void* csr, int64_t nh, 
 int mo_edge_fwd_bwd(const float* V, int64_t nv, const int32_t* idx, int64_t n_items, int kind, const void* csr,
                     const float* off, const float* w, float* loss_out, float* grad_out, void* stream);
 
+/* The loss of a layer in two launches and its gradient in one
+ * (rigid_loss_layer.py:7-27, graph_loss_layer.py:9-43): *loss (device float) =
+ * sum 0.5 d^2 + r2 * sum 0.5 r^2 over the vertices and the half-edges of idx,
+ * the sums in double; df_grad ([nv,3], may be NULL): the distance term's
+ * gradient, zeroed where 0.5 d^2 >= mask.  mo_layer_backward: grad_out [nv,3] =
+ * distance term (df_grad, or with NULL evaluated here, unmasked) + r2 * edge
+ * term.  Terms and gradients round as mo_dfloss_* and mo_edge_* do. */
+size_t mo_layer_scratch_bytes(int64_t nv, int64_t nh);
+int mo_layer_forward(const float* V, int64_t nv, const float* grid, int N, int layout, const int32_t* idx,
+                     int64_t n_items, int kind, const float* off, float r2, float* df_grad, float mask,
+                     void* scratch, size_t scratch_bytes, float* loss, void* stream);
+int mo_layer_backward(const float* V, int64_t nv, const float* grid, int N, int layout, const void* csr,
+                      int64_t nh, const float* off, const float* df_grad, float r2, float* grad_out, void* stream);
+
 /* Sliced-ELL (32-vertex slices, column-major records) view of the CSR for
  * the fused step: one int32 record per incident half-edge, other | role<<31
  * (role 1 when the vertex is the half-edge's v1), in half-edge order;

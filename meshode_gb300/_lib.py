@@ -117,6 +117,9 @@ _SIGS = {
     "mo_edge_cad_weights": (_I, [_P, _I64, _P, _P]),
     "mo_edge_forward_w": (_I, [_P, _I64, _P, _I64, _I, _P, _P, _P, _P]),
     "mo_edge_backward_w": (_I, [_P, _I64, _P, _I64, _P, _P, _P, _P]),
+    "mo_layer_scratch_bytes": (_SZ, [_I64, _I64]),
+    "mo_layer_forward": (_I, [_P, _I64, _P, _I, _I, _P, _I64, _I, _P, _F, _P, _F, _P, _SZ, _P, _P]),
+    "mo_layer_backward": (_I, [_P, _I64, _P, _I, _I, _P, _I64, _P, _P, _F, _P, _P]),
     "mo_edge_fwd_bwd": (_I, [_P, _I64, _P, _I64, _I, _P, _P, _P, _P, _P, _P]),
     "mo_sell_plan": (_I, [_P, _I64, _I64, _P, _P]),
     "mo_sell_fill": (_I, [_P, _I64, _I64, _P, _P, _P]),

@@ -1,50 +1,11 @@
 // Edge (rigidity) losses: rest offsets, per-half-edge residuals, and the
 // deterministic vertex->half-edge CSR used for the gradient scatter.
 // Reference: src/interface/rigid_layer.cc:11-133, graph_layer.cc:11-135.
-//
-// CSR buffer layout (int32 words):
-//   row_ptr[nv+1] | key[2H] | other[2H] | cursor[nv] | status[1] | pad
-// key = 2*h + role, role 0 when the vertex is the half-edge's v0 (the
-// reference's `g[v0] -= r`), 1 when it is v1 (`g[v1] += r`).  Rows are sorted
-// by key, i.e. in the order the reference's serial loop touches the vertex.
 #include <climits>
 
-#include "mo_common.cuh"
+#include "mo_edge.cuh"
 
 namespace mo {
-
-struct CsrView {
-    int* row_ptr;
-    int* key;
-    int* other;
-    int* cursor;
-    int* status;
-};
-
-static inline CsrView csr_view(void* base, int64_t nv, int64_t nh) {
-    CsrView v;
-    int* p = reinterpret_cast<int*>(base);
-    v.row_ptr = p;
-    v.key = p + (nv + 1);
-    v.other = v.key + 2 * nh;
-    v.cursor = v.other + 2 * nh;
-    v.status = v.cursor + nv;
-    return v;
-}
-
-__device__ __forceinline__ void he_ends(const int32_t* __restrict__ idx, int kind, int64_t h, int& v0, int& v1) {
-    if (kind == MO_EDGES_FACES) {
-        const int64_t f = h / 3;
-        const int j = (int)(h - 3 * f);
-        v0 = idx[3 * f + j];
-        v1 = idx[3 * f + (j == 2 ? 0 : j + 1)];
-    } else {
-        v0 = idx[2 * h];
-        v1 = idx[2 * h + 1];
-    }
-}
-
-__device__ __forceinline__ bool in_range(int v, int64_t nv) { return v >= 0 && (int64_t)v < nv; }
 
 __global__ void k_edge_offsets(const float* __restrict__ V, int64_t nv, const int32_t* __restrict__ idx,
                                int64_t nh, int kind, float* __restrict__ off) {
@@ -170,25 +131,8 @@ __global__ void __launch_bounds__(256) k_edge_backward(const float* __restrict__
                                                        const float* __restrict__ off, float* __restrict__ G) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nv) return;
-    const float px = V[3 * i], py = V[3 * i + 1], pz = V[3 * i + 2];
-    float gx = 0.0f, gy = 0.0f, gz = 0.0f;
-    const int b = row_ptr[i], e = row_ptr[i + 1];
-    for (int k = b; k < e; ++k) {
-        const int kk = key[k];
-        const int64_t h = kk >> 1;
-        const int64_t o = other[k];
-        const float qx = V[3 * o], qy = V[3 * o + 1], qz = V[3 * o + 2];
-        const float ox = off[3 * h], oy = off[3 * h + 1], oz = off[3 * h + 2];
-        if ((kk & 1) == 0) {  // this vertex is v0: g[v0] -= (v1 - v0 - off)
-            gx = SUB(gx, SUB(SUB(qx, px), ox));
-            gy = SUB(gy, SUB(SUB(qy, py), oy));
-            gz = SUB(gz, SUB(SUB(qz, pz), oz));
-        } else {              // this vertex is v1: g[v1] += (v1 - v0 - off)
-            gx = ADD(gx, SUB(SUB(px, qx), ox));
-            gy = ADD(gy, SUB(SUB(py, qy), oy));
-            gz = ADD(gz, SUB(SUB(pz, qz), oz));
-        }
-    }
+    float gx, gy, gz;
+    edge_gather(V, i, row_ptr, key, other, off, gx, gy, gz);
     G[3 * i] = gx; G[3 * i + 1] = gy; G[3 * i + 2] = gz;
 }
 

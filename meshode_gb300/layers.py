@@ -11,6 +11,7 @@ from torch import nn
 from torch.autograd import Function
 
 from . import pyDeform
+from ._lib import MO_EDGES_FACES, MO_EDGES_LIST
 
 
 class RigidLossFunction(Function):
@@ -20,19 +21,16 @@ class RigidLossFunction(Function):
     @staticmethod
     def forward(ctx, src_V, src_F, param_id):
         pid = int(param_id)
-        lossD = pyDeform.DistanceFieldLoss_forward(src_V, pid) * 0.5
-        lossR = pyDeform.RigidEdgeLoss_forward(src_V, src_F, pid) * 0.5
+        loss = pyDeform.LayerLoss_forward(src_V, src_F, pid, MO_EDGES_FACES)
         ctx.save_for_backward(src_V)
         ctx.src_F = src_F
         ctx.pid = pid
-        return lossD.sum() + lossR.sum()
+        return loss
 
     @staticmethod
     def backward(ctx, grad_h):
         (src_V,) = ctx.saved_tensors
-        gD = pyDeform.DistanceFieldLoss_backward(src_V, ctx.pid)
-        gR = pyDeform.RigidEdgeLoss_backward(src_V, ctx.src_F, ctx.pid)
-        return grad_h * (gD + gR), None, None
+        return grad_h * pyDeform.LayerLoss_backward(src_V, ctx.src_F, ctx.pid, MO_EDGES_FACES), None, None
 
 
 class RigidLossLayer(nn.Module):
@@ -65,20 +63,18 @@ class GraphLossFunction(Function):
     def forward(ctx, src_V, src_E, rigidity2, param_id):
         pid = int(param_id)
         r2 = float(rigidity2)
-        lossD, gD = pyDeform.DistanceFieldLoss_fwd_bwd(src_V, pid, mask_thresh=GraphLossFunction.MASK)
-        lossD = lossD * 0.5
-        lossR = pyDeform.GraphEdgeLoss_forward(src_V, src_E, pid) * 0.5
+        loss, gD = pyDeform.LayerLoss_forward(src_V, src_E, pid, MO_EDGES_LIST, r2, GraphLossFunction.MASK)
         ctx.save_for_backward(src_V, gD)
         ctx.src_E = src_E
         ctx.pid = pid
         ctx.r2 = r2
-        return lossD.sum() + lossR.sum() * r2
+        return loss
 
     @staticmethod
     def backward(ctx, grad_h):
         src_V, gD = ctx.saved_tensors
-        gR = pyDeform.GraphEdgeLoss_backward(src_V, ctx.src_E, ctx.pid)
-        return grad_h * (gD + gR * ctx.r2), None, None, None
+        grad = pyDeform.LayerLoss_backward(src_V, ctx.src_E, ctx.pid, MO_EDGES_LIST, ctx.r2, gD)
+        return grad_h * grad, None, None, None
 
 
 class GraphLossLayer(nn.Module):

@@ -492,3 +492,44 @@ def GraphEdgeLoss_forward(tensorV, tensorE, param_id):
 
 def GraphEdgeLoss_backward(tensorV, tensorE, param_id):
     return _edge_backward(tensorV, tensorE, param_id, L.MO_EDGES_LIST)
+
+
+# ---------------------------------------------------------------------------
+# a layer's two terms together
+# ---------------------------------------------------------------------------
+def _layer_inputs(tensorV, idx, param_id, kind):
+    _check_vertices(tensorV)
+    p = GetParams(param_id)
+    _check_indices(idx, 3 if kind == L.MO_EDGES_FACES else 2, "F" if kind == L.MO_EDGES_FACES else "E")
+    p, st = _edge_state(param_id, kind, idx)
+    Vd = _on_device(tensorV, p.device)
+    idx_dev, csr = _csr_for(st, idx, None, Vd.shape[0], p.device)
+    return p, st, Vd, idx_dev, csr
+
+
+def LayerLoss_forward(tensorV, idx, param_id, kind, r2=1.0, mask_thresh=None):
+    """0.5 * sum d^2 + r2 * 0.5 * sum r^2 (0-dim) in one pass over the vertices
+    and the half-edges; with ``mask_thresh`` also the distance term's masked
+    gradient, as DistanceFieldLoss_fwd_bwd's."""
+    p, st, Vd, idx_dev, _ = _layer_inputs(tensorV, idx, param_id, kind)
+    nv = Vd.shape[0]
+    nb = L.lib().mo_layer_scratch_bytes(nv, st.nh)
+    scratch = torch.empty(nb // 8, dtype=torch.float64, device=p.device)
+    loss = torch.empty((), dtype=torch.float32, device=p.device)
+    grad = None if mask_thresh is None else torch.empty(nv, 3, dtype=torch.float32, device=p.device)
+    call("mo_layer_forward", ptr(Vd), nv, ptr(p.grid), p.N, p.layout, ptr(idx_dev), idx_dev.shape[0], kind,
+         ptr(st.offsets), float(r2), ptr(grad), float(mask_thresh or 0.0), ptr(scratch), nb, ptr(loss), stream_ptr())
+    loss = _out(loss, tensorV)
+    return loss if grad is None else (loss, _out(grad, tensorV))
+
+
+def LayerLoss_backward(tensorV, idx, param_id, kind, r2=1.0, df_grad=None):
+    """[V,3]: the distance term's gradient (df_grad, or evaluated here) plus r2
+    times the edge term's."""
+    p, st, Vd, _, csr = _layer_inputs(tensorV, idx, param_id, kind)
+    nv = Vd.shape[0]
+    gd = None if df_grad is None else _on_device(df_grad, p.device)
+    out = torch.empty(nv, 3, dtype=torch.float32, device=p.device)
+    call("mo_layer_backward", ptr(Vd), nv, ptr(p.grid), p.N, p.layout, ptr(csr), st.nh, ptr(st.offsets), ptr(gd),
+         float(r2), ptr(out), stream_ptr())
+    return _out(out, tensorV)
