@@ -200,9 +200,9 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) k_fused_step(const MoPair* __
 
 // ---------------------------------------------------------------------------
 // Many steps of one pair in one cooperative launch, for pairs whose every vertex
-// can have a thread of its own on the chip.  A launch per step is a chain of
-// dependent loads (tile, pair, position, record, neighbour) behind a launch:
-// 7 us a step at 10k vertices.  Here a vertex's position, moments, records and
+// can stay on the chip.  A launch per step is a chain of dependent loads (tile,
+// pair, position, record, neighbour) behind a launch, and from 80k vertices on
+// 370 bytes a vertex from L2.  Here a vertex's position, moments, records and
 // rest offsets stay in registers and shared memory for all steps; a step is one
 // gather of the neighbours' positions (L2), the arithmetic, one store and a grid
 // barrier, beside which the next step's distance lookup and the loss partials
@@ -248,145 +248,222 @@ __device__ __forceinline__ bool run_wait(unsigned* bar, unsigned target) {
     return ok != 0;
 }
 
-template <bool WEIGHTED>
-__global__ void __launch_bounds__(STEP_THREADS, 2) k_fused_run(const __grid_constant__ MoPair P, int nsteps,
-                                                               float* __restrict__ tile_loss, int64_t loss_stride,
-                                                               unsigned* bar) {
-    extern __shared__ float offs[];  // [RUN_REC][3][threads] rest offsets of the kept records
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nt = blockDim.x;
-    const int slice = blockIdx.x * (nt >> 5) + w;
-    const bool live = slice < P.nslices;  // warp-uniform
-    const int i = slice * 32 + lane;
-    const bool valid = live && i < P.nv;
+// K vertices a thread, blocks of up to T threads; LOSS: with the steps' loss
+// partials (else the energy is not summed).  What a thread keeps is 21
+// registers a vertex and, in shared memory, 144 bytes of rest offsets:
+//   T = 256, K = 1: two blocks an SM, all twelve neighbours gathered together;
+//   T = 1024, K = 1: one block, 64 registers, four neighbours at a time;
+//   T = 768, K = 2: one block, 80 registers, its offsets ~all of the shared
+//     memory.  (Three vertices a thread of 512 were slower: 10.3 us a step at
+//     200k vertices, each vertex's gathers waiting for the one's before.)
+// Measured, us a step (a launch per step, here): 10k 4.8, 3.6; 77k 5.6, 4.7;
+// 150k 8.3, 5.8; 200k 10.4, 8.7; 230k 11.8, 9.4.
+constexpr int RUN_WARPS1 = 32, RUN_WARPS2 = 24;
+template <bool WEIGHTED, bool LOSS, int K, int T>
+__global__ void __launch_bounds__(T, T == STEP_THREADS ? 2 : 1)
+    k_fused_run(const __grid_constant__ MoPair P, int nsteps, float* __restrict__ tile_loss, int64_t loss_stride,
+                unsigned* bar) {
+    extern __shared__ float offs[];  // [K][RUN_REC][3][threads] rest offsets of the kept records
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, nt = blockDim.x, warps = nt >> 5;
+    const int slice0 = blockIdx.x * warps * K + w;  // and every warps-th after it
     const float4* __restrict__ R = reinterpret_cast<const float4*>(P.rest);
     float4* const pos0 = reinterpret_cast<float4*>(P.pos0);
     float4* const pos1 = reinterpret_cast<float4*>(P.pos1);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 p = valid ? ((P.t0 & 1) ? pos1 : pos0)[i] : zero;
-    const float4 r0 = valid ? __ldg(R + i) : zero;
-    float* Mm = P.adam_m + 3 * (int64_t)i;
-    float* Vv = P.adam_v + 3 * (int64_t)i;
-    float m0 = 0.f, m1 = 0.f, m2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f;
-    if (valid) {
-        m0 = Mm[0]; m1 = Mm[1]; m2 = Mm[2];
-        v0 = Vv[0]; v1 = Vv[1]; v2 = Vv[2];
-    }
-    const int rb = live ? P.slice_ptr[slice] : 0;
-    const int rows = live ? (P.slice_ptr[slice + 1] - rb) >> 5 : 0;
-    const int* __restrict__ rec = P.sell + rb + lane;
-    const float* __restrict__ recw = WEIGHTED && P.sell_w ? P.sell_w + rb + lane : nullptr;
-    int c[RUN_REC];
-#pragma unroll
-    for (int u = 0; u < RUN_REC; ++u) {
-        c[u] = u < rows ? __ldg(rec + u * 32) : -1;
-        if (c[u] != -1) {
-            const float4 s = __ldg(R + (c[u] & 0x7fffffff));
-            offs[(3 * u) * nt + threadIdx.x] = SUB(s.x, r0.x);
-            offs[(3 * u + 1) * nt + threadIdx.x] = SUB(s.y, r0.y);
-            offs[(3 * u + 2) * nt + threadIdx.x] = SUB(s.z, r0.z);
-        }
-    }
     const int N = P.N;
     const float Nf = (float)N, Cf = (float)((double)(N - 1) - 1e-3);
     const float we = P.w_edge, gh = P.grad_scale;
-    float dsq, gdx, gdy, gdz;
-    auto lookup = [&]() {
-        const DFJet j = (P.layout == MO_LAYOUT_CELL)
-                            ? df_eval_layout<MO_LAYOUT_CELL>(P.grid, N, Nf, Cf, p.x, p.y, p.z)
-                            : (P.layout == MO_LAYOUT_BRICK4)
-                                  ? df_eval_layout<MO_LAYOUT_BRICK4>(P.grid, N, Nf, Cf, p.x, p.y, p.z)
-                                  : df_eval_layout<MO_LAYOUT_LINEAR>(P.grid, N, Nf, Cf, p.x, p.y, p.z);
-        dsq = MUL(j.d, j.d);
-        gdx = df_grad_component(j.d, j.gx);
-        gdy = df_grad_component(j.d, j.gy);
-        gdz = df_grad_component(j.d, j.gz);
+    float3 p[K] = {}, m[K], v[K];
+    int c[K][RUN_REC];
+    bool valid[K];
+    float dsq[K];
+    float3 gd[K];
+    auto rows_of = [&](int slice) { return (P.slice_ptr[slice + 1] - P.slice_ptr[slice]) >> 5; };
+    auto lookup = [&](int j) {
+        const float x = p[j].x, y = p[j].y, z = p[j].z;
+        const DFJet d = (P.layout == MO_LAYOUT_CELL) ? df_eval_layout<MO_LAYOUT_CELL>(P.grid, N, Nf, Cf, x, y, z)
+                        : (P.layout == MO_LAYOUT_BRICK4)
+                            ? df_eval_layout<MO_LAYOUT_BRICK4>(P.grid, N, Nf, Cf, x, y, z)
+                            : df_eval_layout<MO_LAYOUT_LINEAR>(P.grid, N, Nf, Cf, x, y, z);
+        dsq[j] = MUL(d.d, d.d);
+        gd[j] = make_float3(df_grad_component(d.d, d.gx), df_grad_component(d.d, d.gy), df_grad_component(d.d, d.gz));
         if (P.use_mask) {
-            const float mk = (MUL(dsq, 0.5f) < P.mask_thresh) ? 1.0f : 0.0f;
-            gdx = MUL(gdx, mk); gdy = MUL(gdy, mk); gdz = MUL(gdz, mk);
+            const float mk = (MUL(dsq[j], 0.5f) < P.mask_thresh) ? 1.0f : 0.0f;
+            gd[j].x = MUL(gd[j].x, mk); gd[j].y = MUL(gd[j].y, mk); gd[j].z = MUL(gd[j].z, mk);
         }
     };
-    lookup();
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const int slice = slice0 + j * warps;  // warp-uniform
+        const int i = slice * 32 + lane;
+        valid[j] = slice < P.nslices && i < P.nv;
+        p[j] = m[j] = v[j] = make_float3(0.f, 0.f, 0.f);
+        float4 r0 = zero;
+        if (valid[j]) {
+            const float4 q = ((P.t0 & 1) ? pos1 : pos0)[i];
+            p[j] = make_float3(q.x, q.y, q.z);
+            r0 = __ldg(R + i);
+            const float* Mm = P.adam_m + 3 * (int64_t)i;
+            const float* Vv = P.adam_v + 3 * (int64_t)i;
+            m[j] = make_float3(Mm[0], Mm[1], Mm[2]);
+            v[j] = make_float3(Vv[0], Vv[1], Vv[2]);
+        }
+        const int rows = slice < P.nslices ? rows_of(slice) : 0;
+        const int* __restrict__ rec = P.sell + (rows ? P.slice_ptr[slice] : 0) + lane;
+        float* o = offs + j * 3 * RUN_REC * nt + threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < RUN_REC; ++u) {
+            c[j][u] = u < rows ? __ldg(rec + u * 32) : -1;
+            if (c[j][u] != -1) {
+                const float4 s = __ldg(R + (c[j][u] & 0x7fffffff));
+                o[(3 * u) * nt] = SUB(s.x, r0.x);
+                o[(3 * u + 1) * nt] = SUB(s.y, r0.y);
+                o[(3 * u + 2) * nt] = SUB(s.z, r0.z);
+            }
+        }
+        lookup(j);
+    }
     float2 ab = __ldg(reinterpret_cast<const float2*>(P.adam_tab) + P.t0);
     for (int k = 0; k < nsteps; ++k) {
         const int t = P.t0 + k + 1;
         const float4* Vin = (t & 1) ? pos0 : pos1;
         float4* Vout = (t & 1) ? pos1 : pos0;
-        float4 q[RUN_REC];
+        float part[K];
 #pragma unroll
-        for (int u = 0; u < RUN_REC; ++u) q[u] = c[u] != -1 ? Vin[c[u] & 0x7fffffff] : zero;
-        float grx = 0.f, gry = 0.f, grz = 0.f, esq = 0.f;
-        auto edge = [&](int cu, float4 qu, float ox, float oy, float oz, int row) {
-            const float rx = SUB(SUB(qu.x, p.x), ox);
-            const float ry = SUB(SUB(qu.y, p.y), oy);
-            const float rz = SUB(SUB(qu.z, p.z), oz);
-            if (WEIGHTED) {
-                const float we_ = recw ? __ldg(recw + row * 32) : 1.0f;
-                const float l2 = MUL(we_, we_);
-                grx = SUB(grx, MUL(rx, l2)); gry = SUB(gry, MUL(ry, l2)); grz = SUB(grz, MUL(rz, l2));
-                if (cu >= 0) {
-                    const float ex = MUL(rx, we_), ey = MUL(ry, we_), ez = MUL(rz, we_);
-                    esq += ex * ex + ey * ey + ez * ez;
+        for (int j = 0; j < K; ++j) {
+            const int slice = slice0 + j * warps;
+            const int i = slice * 32 + lane;
+            const float* o = offs + j * 3 * RUN_REC * nt + threadIdx.x;
+            const float* __restrict__ recw =
+                WEIGHTED && P.sell_w && slice < P.nslices ? P.sell_w + P.slice_ptr[slice] + lane : nullptr;
+            float grx = 0.f, gry = 0.f, grz = 0.f, esq = 0.f;
+            auto edge = [&](int cu, float4 qu, float ox, float oy, float oz, int row) {
+                const float rx = SUB(SUB(qu.x, p[j].x), ox);
+                const float ry = SUB(SUB(qu.y, p[j].y), oy);
+                const float rz = SUB(SUB(qu.z, p[j].z), oz);
+                if (WEIGHTED) {
+                    const float we_ = recw ? __ldg(recw + row * 32) : 1.0f;
+                    const float l2 = MUL(we_, we_);
+                    grx = SUB(grx, MUL(rx, l2)); gry = SUB(gry, MUL(ry, l2)); grz = SUB(grz, MUL(rz, l2));
+                    if (LOSS && cu >= 0) {
+                        const float ex = MUL(rx, we_), ey = MUL(ry, we_), ez = MUL(rz, we_);
+                        esq += ex * ex + ey * ey + ez * ez;
+                    }
+                } else {
+                    grx = SUB(grx, rx); gry = SUB(gry, ry); grz = SUB(grz, rz);
+                    if (LOSS && cu >= 0) esq += rx * rx + ry * ry + rz * rz;
                 }
-            } else {
-                grx = SUB(grx, rx); gry = SUB(gry, ry); grz = SUB(grz, rz);
-                if (cu >= 0) esq += rx * rx + ry * ry + rz * rz;
-            }
-        };
+            };
+            constexpr int B = T == STEP_THREADS ? RUN_REC : 4;  // gathered together
 #pragma unroll
-        for (int u = 0; u < RUN_REC; ++u)
-            if (c[u] != -1)
-                edge(c[u], q[u], offs[(3 * u) * nt + threadIdx.x], offs[(3 * u + 1) * nt + threadIdx.x],
-                     offs[(3 * u + 2) * nt + threadIdx.x], u);
-        for (int row = RUN_REC; row < rows; ++row) {
-            const int cu = __ldg(rec + row * 32);
-            if (cu == -1) break;  // padding follows the last record
-            const int o = cu & 0x7fffffff;
-            const float4 s = __ldg(R + o);
-            edge(cu, Vin[o], SUB(s.x, r0.x), SUB(s.y, r0.y), SUB(s.z, r0.z), row);
-        }
-        const float gx = MUL(gh, ADD(gdx, MUL(grx, we)));
-        const float gy = MUL(gh, ADD(gdy, MUL(gry, we)));
-        const float gz = MUL(gh, ADD(gdz, MUL(grz, we)));
-        const float part = valid ? 0.5f * dsq + we * (0.5f * esq) : 0.f;
-        if (valid) {
-            if (P.grad_dbg) {
-                P.grad_dbg[3 * (int64_t)i] = gx;
-                P.grad_dbg[3 * (int64_t)i + 1] = gy;
-                P.grad_dbg[3 * (int64_t)i + 2] = gz;
+            for (int u0 = 0; u0 < RUN_REC; u0 += B) {
+                float4 q[B];
+#pragma unroll
+                for (int u = 0; u < B; ++u) q[u] = c[j][u0 + u] != -1 ? Vin[c[j][u0 + u] & 0x7fffffff] : zero;
+#pragma unroll
+                for (int u = 0; u < B; ++u)
+                    if (c[j][u0 + u] != -1)
+                        edge(c[j][u0 + u], q[u], o[(3 * (u0 + u)) * nt], o[(3 * (u0 + u) + 1) * nt],
+                             o[(3 * (u0 + u) + 2) * nt], u0 + u);
             }
-            adam_elem(p.x, gx, m0, v0, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
-            adam_elem(p.y, gy, m1, v1, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
-            adam_elem(p.z, gz, m2, v2, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
-            Vout[i] = make_float4(p.x, p.y, p.z, 0.f);
+            if (c[j][RUN_REC - 1] != -1) {  // the records that were not kept
+                const int rows = rows_of(slice);
+                const int* __restrict__ rec = P.sell + P.slice_ptr[slice] + lane;
+                const float4 r0 = __ldg(R + i);
+                for (int row = RUN_REC; row < rows; ++row) {
+                    const int cu = __ldg(rec + row * 32);
+                    if (cu == -1) break;  // padding follows the last record
+                    const int n = cu & 0x7fffffff;
+                    const float4 s = __ldg(R + n);
+                    edge(cu, Vin[n], SUB(s.x, r0.x), SUB(s.y, r0.y), SUB(s.z, r0.z), row);
+                }
+            }
+            const float gx = MUL(gh, ADD(gd[j].x, MUL(grx, we)));
+            const float gy = MUL(gh, ADD(gd[j].y, MUL(gry, we)));
+            const float gz = MUL(gh, ADD(gd[j].z, MUL(grz, we)));
+            part[j] = 0.f;
+            if (valid[j]) {
+                if (LOSS) part[j] = 0.5f * dsq[j] + we * (0.5f * esq);
+                if (P.grad_dbg) {
+                    P.grad_dbg[3 * (int64_t)i] = gx;
+                    P.grad_dbg[3 * (int64_t)i + 1] = gy;
+                    P.grad_dbg[3 * (int64_t)i + 2] = gz;
+                }
+                adam_elem(p[j].x, gx, m[j].x, v[j].x, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
+                adam_elem(p[j].y, gy, m[j].y, v[j].y, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
+                adam_elem(p[j].z, gz, m[j].z, v[j].z, P.one_minus_b1, P.b2, P.one_minus_b2, P.eps, ab.x, ab.y);
+                Vout[i] = make_float4(p[j].x, p[j].y, p[j].z, 0.f);
+            }
         }
         const bool more = k + 1 < nsteps;
         if (more) run_arrive(bar);
-        if (tile_loss && slice < P.ntiles * TILE_WARPS) {
-            float s = part;
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) tile_loss[(int64_t)k * loss_stride + slice] = s;
+        if (LOSS) {
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                const int slice = slice0 + j * warps;
+                if (slice >= P.ntiles * TILE_WARPS) continue;
+                float s = part[j];
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if (lane == 0) tile_loss[(int64_t)k * loss_stride + slice] = s;
+            }
         }
         if (!more) break;
         ab = __ldg(reinterpret_cast<const float2*>(P.adam_tab) + t);
-        lookup();
+#pragma unroll
+        for (int j = 0; j < K; ++j) lookup(j);
         if (!run_wait(bar, (unsigned)(k + 1) * gridDim.x)) {  // never in a working launch: no result
-            if (valid) pos0[i] = pos1[i] = make_float4(NAN, NAN, NAN, 0.f);
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+                const int i = (slice0 + j * warps) * 32 + lane;
+                if (valid[j]) pos0[i] = pos1[i] = make_float4(NAN, NAN, NAN, 0.f);
+            }
             return;
         }
     }
-    if (valid) {
-        Mm[0] = m0; Mm[1] = m1; Mm[2] = m2;
-        Vv[0] = v0; Vv[1] = v1; Vv[2] = v2;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const int i = (slice0 + j * warps) * 32 + lane;
+        if (!valid[j]) continue;
+        float* Mm = P.adam_m + 3 * (int64_t)i;
+        float* Vv = P.adam_v + 3 * (int64_t)i;
+        Mm[0] = m[j].x; Mm[1] = m[j].y; Mm[2] = m[j].z;
+        Vv[0] = v[j].x; Vv[1] = v[j].y; Vv[2] = v[j].z;
     }
 }
 
-// Warps of a block (an SM's share of the slices, at most 8) and blocks of a run
-// over nslices slices; blocks 0: they do not fit the chip at once.
-static void run_shape(int nslices, int* warps, int* blocks) {
+// Vertices a thread, warps of a block and blocks of a run over nslices slices
+// (blocks 0: they do not fit the chip at once): an SM's share of them in two
+// blocks of up to 8, in one of up to 32, or in one of up to 24 warps twice.
+static void run_shape(int nslices, int* per_thread, int* warps, int* blocks) {
     const int sms = device_sm_count();
-    *warps = std::max(1, std::min(TILE_WARPS, (nslices + sms - 1) / sms));
-    *blocks = (nslices + *warps - 1) / *warps;
-    if (*blocks > 2 * sms) *blocks = 0;  // 8 warps: two blocks an SM (registers)
+    const int share = (nslices + sms - 1) / sms;
+    int max_blocks = sms;
+    if (share <= 2 * TILE_WARPS) {
+        *per_thread = 1;
+        *warps = std::max(1, std::min(TILE_WARPS, share));
+        max_blocks = 2 * sms;
+    } else if (share <= RUN_WARPS1) {
+        *per_thread = 1;
+        *warps = share;
+    } else {
+        *per_thread = 2;
+        *warps = std::min(RUN_WARPS2, (share + 1) / 2);
+    }
+    const int per_block = *warps * *per_thread;
+    *blocks = (nslices + per_block - 1) / per_block;
+    if (*blocks > max_blocks) *blocks = 0;
+}
+
+template <bool WEIGHTED, bool LOSS>
+static const void* run_kernel_of(int per_thread, int warps) {
+    if (per_thread == 2) return (const void*)k_fused_run<WEIGHTED, LOSS, 2, 32 * RUN_WARPS2>;
+    if (warps > TILE_WARPS) return (const void*)k_fused_run<WEIGHTED, LOSS, 1, 32 * RUN_WARPS1>;
+    return (const void*)k_fused_run<WEIGHTED, LOSS, 1, STEP_THREADS>;
+}
+
+static const void* run_kernel(bool weighted, bool loss, int per_thread, int warps) {
+    if (weighted) return loss ? run_kernel_of<true, true>(per_thread, warps) : run_kernel_of<true, false>(per_thread, warps);
+    return loss ? run_kernel_of<false, true>(per_thread, warps) : run_kernel_of<false, false>(per_thread, warps);
 }
 
 // One warp per (pair, launch): lane l sums the pair's tile partials l, l+32,
@@ -490,8 +567,8 @@ extern "C" int mo_fused_step_on_demand(const MoPair* pairs, const MoTile* tiles,
 
 extern "C" int mo_fused_run_fits(int64_t nv) {
     if (nv <= 0 || nv > ((int64_t)1 << 30)) return 0;
-    int warps, blocks;
-    run_shape((int)((nv + 31) / 32), &warps, &blocks);
+    int per_thread, warps, blocks;
+    run_shape((int)((nv + 31) / 32), &per_thread, &warps, &blocks);
     return blocks > 0 ? 1 : 0;
 }
 
@@ -507,8 +584,8 @@ extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float*
                                 loss_stride >= (int64_t)q.ntiles * TILE_WARPS),
                  "loss partials need whole tiles of %d slices", TILE_WARPS);
     MO_CHECK_ARG(q.t0 >= 0 && nsteps <= q.t_end - q.t0, "more steps than the pair has left");
-    int warps, blocks;
-    run_shape(q.nslices, &warps, &blocks);
+    int per_thread, warps, blocks;
+    run_shape(q.nslices, &per_thread, &warps, &blocks);
     MO_CHECK_ARG(blocks > 0, "%d vertices do not fit one launch (mo_fused_run_fits)", q.nv);
     if (tile_loss) {  // the slices past the last one of its tile
         const int pad = q.ntiles * TILE_WARPS - q.nslices;
@@ -516,7 +593,9 @@ extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float*
             MO_CUDA(cudaMemset2DAsync(tile_loss + q.nslices, sizeof(float) * loss_stride, 0, sizeof(float) * pad, nsteps,
                                       as_stream(stream)));
     }
-    const int smem = RUN_REC * 3 * (int)sizeof(float) * 32 * warps;
+    const int smem = RUN_REC * 3 * (int)sizeof(float) * 32 * warps * per_thread;
+    const void* kernel = run_kernel(weighted != 0, tile_loss != nullptr, per_thread, warps);
+    if (smem > 48 * 1024) MO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     for (int done = 0; done < nsteps;) {
         int n = std::min(RUN_CHUNK, nsteps - done);
         MoPair p = q;
@@ -525,8 +604,7 @@ extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float*
         unsigned* bar = sync;
         MO_CUDA(cudaMemsetAsync(sync, 0, 8, as_stream(stream)));
         void* args[] = {&p, &n, &loss, &loss_stride, &bar};
-        MO_CUDA(cudaLaunchCooperativeKernel(weighted ? (const void*)k_fused_run<true> : (const void*)k_fused_run<false>,
-                                            dim3(blocks), dim3(32 * warps), args, smem, as_stream(stream)));
+        MO_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(32 * warps), args, smem, as_stream(stream)));
         ::mo::note_launch();
         done += n;
     }

@@ -2,7 +2,7 @@
 launch per step: positions, moments and losses bit for bit, at one vertex, around
 a slice of 32 and a tile of 8 slices, with more than the 12 records a thread
 keeps, with isolated vertices, with weights, a mask and an odd number of steps,
-in two calls, and at the largest size that fits; one vertex more is refused."""
+in two calls, with one to three vertices a thread, and at the largest size that fits; one vertex more is refused."""
 import numpy as np
 import pytest
 import torch
@@ -54,7 +54,10 @@ def _pairs(target, nv, kind, layout, **kw):
     (1, "plain", L.MO_LAYOUT_CELL, {}), (31, "plain", L.MO_LAYOUT_LINEAR, {}), (33, "star", L.MO_LAYOUT_CELL, {}),
     (256, "plain", L.MO_LAYOUT_BRICK4, {}), (257, "sparse", L.MO_LAYOUT_CELL, {"mask_thresh": 0.5 * 0.03 ** 2}),
     (5000, "cad", L.MO_LAYOUT_CELL, {"w_edge": 0.3}), (9729, "plain", L.MO_LAYOUT_CELL, {}),
-    (40_000, "star", L.MO_LAYOUT_CELL, {"w_edge": 2.0})])
+    (40_000, "star", L.MO_LAYOUT_CELL, {"w_edge": 2.0}),
+    # more than a vertex a thread: two, three, with rows of more than 12 records, weights and a mask
+    (77_900, "plain", L.MO_LAYOUT_CELL, {}), (90_001, "cad", L.MO_LAYOUT_LINEAR, {"w_edge": 0.3}),
+    (160_003, "star", L.MO_LAYOUT_CELL, {}), (200_003, "cad", L.MO_LAYOUT_CELL, {"mask_thresh": 0.5 * 0.03 ** 2})])
 def test_same_bits_as_a_launch_per_step(target, nv, kind, layout, kw):
     a, b = _pairs(target, nv, kind, layout, **kw)
     runner = fused.StepGroupRunner(a.device, 1, a.ntiles, group_steps=27, use_graph=False, weighted=a.sell_w is not None)
