@@ -145,6 +145,12 @@ typedef struct MoDfOptions {
 /* The packet shape of a build of an N^3 grid over nf triangles (band as in
  * MoDfOptions) whose caller names none. */
 int mo_df_packet_for(int64_t nf, int N, float band);
+/* A target's box, normalisation, distance field and grid layout in one call:
+ * mo_bbox_params, mo_df_build and (grid_out, for a layout other than linear)
+ * mo_grid_relayout, then one synchronisation for the status. */
+int mo_template_build(const float* V, int64_t nv, const int32_t* F, int64_t nf, int N, int method, int layout,
+                      int32_t* bbox6, double* params4, void* scratch, size_t scratch_bytes, float* grid_linear_out,
+                      float* grid_out, void* stream);
 /* mo_df_build with explicit build options (opt == NULL: defaults).  method
  * and packet change only the speed, never the grid. */
 int mo_df_build_ex(const float* V, int64_t nv, const int32_t* F, int64_t nf, int N,
@@ -682,6 +688,22 @@ int mo_mlp_tc_wgrad(const float* G, const float* H, int64_t rows, void* pack, in
 int mo_mlp_tc_reduce(const float* partial, int64_t n, const float* wpart2, const float* wpart3, int64_t rows, int W,
                      int m, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3, float* dW4,
                      float* db4, void* stream);
+
+/* x(1) = RK4^steps(x0) under the packed MLP.  ckpt [steps][n][3]: the steps'
+ * start states.  act [steps][mo_ode_act_floats] and u [steps][3][n][3] keep every
+ * evaluation's activations and inputs for the backward pass; act NULL: not
+ * kept, and u is one step's work space. */
+int64_t mo_ode_act_floats(int64_t n, int W);
+int mo_ode_flow(const float* x0, int64_t n, int steps, void* pack, int W, float* ckpt, float* act, float* u,
+                float* out, void* stream);
+/* Its adjoint for dL/dx(1) = a_out: dL/dx0 in dx0 (dx1: work space, [n,3] too)
+ * and the parameters' gradients.  act NULL: every step's evaluations are
+ * repeated.  scratch: mo_ode_backward_floats floats, 128-byte aligned. */
+int64_t mo_ode_backward_floats(int64_t n, int W, int stored);
+int mo_ode_flow_backward(const float* ckpt, int64_t n, int steps, void* pack, int W, int m, float* act, float* u,
+                         const float* a_out, float* scratch, int64_t scratch_floats, float* dx0, float* dx1,
+                         float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3, float* dW4,
+                         float* db4, void* stream);
 
 /* sizeof(MoPair) and sizeof(MoTile) as compiled (host pointers), so that
  * bindings in other languages can check their struct layout. */

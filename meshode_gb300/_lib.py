@@ -90,6 +90,7 @@ _SIGS = {
     "mo_df_build": (_I, [_P, _I64, _P, _I64, _I, _P, _I, _P, _SZ, _P, _P, _P]),
     "mo_df_method_for": (_I, [_I64, _I]),
     "mo_df_loss_band": (_F, [_I]),
+    "mo_template_build": (_I, [_P, _I64, _P, _I64, _I, _I, _I, _P, _P, _P, _SZ, _P, _P, _P]),
     "mo_df_packet_for": (_I, [_I64, _I, _F]),
     "mo_df_build_ex": (_I, [_P, _I64, _P, _I64, _I, _P, _P, _P, _SZ, _P, _P, _P]),
     "mo_df_build_count": (_I, [_P, _I64, _P, _I64, _I, _P, _P, _P, _SZ, _P, _P, _P, _P]),
@@ -151,6 +152,10 @@ _SIGS = {
     "mo_mlp_tc_fwd": (_I, [_P, _P, _I64, _P, _I, _F, _F, _I, _P, _P, _P, _I64, _P]),
     "mo_mlp_tc_bwd": (_I, [_P, _F, _P, _F, _P, _I64, _P, _I, _P, _I64, _P, _P, _P, _P, _P, _P, _I, _P]),
     "mo_mlp_tc_wgrad": (_I, [_P, _P, _I64, _P, _I, _I, _P, _I, _P]),
+    "mo_ode_act_floats": (_I64, [_I64, _I]),
+    "mo_ode_flow": (_I, [_P, _I64, _I, _P, _I, _P, _P, _P, _P, _P]),
+    "mo_ode_backward_floats": (_I64, [_I64, _I, _I]),
+    "mo_ode_flow_backward": (_I, [_P, _I64, _I, _P, _I, _I] + [_P] * 4 + [_I64] + [_P] * 11),
     "mo_mlp_tc_reduce": (_I, [_P, _I64, _P, _P, _I64, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "mo_pack_pos": (_I, [_P, _I64, _P, _P]),
     "mo_unpack_pos": (_I, [_P, _I64, _P, _P]),
@@ -225,7 +230,7 @@ def call(name, *args):
 
 
 def require_cuda():
-    if not torch.cuda.is_available():
+    if not torch.cuda.is_initialized() and not torch.cuda.is_available():
         raise MeshodeError("meshode_gb300 needs a CUDA device (GB300 / sm_103a); none is available")
     lib()
 
@@ -235,5 +240,10 @@ def ptr(t):
 
 
 def stream_ptr(stream=None):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    """A stream's handle (None: the current device's current stream)."""
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    # the handle without a Stream object around it: a call a kernel
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))

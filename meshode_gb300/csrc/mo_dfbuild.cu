@@ -1221,6 +1221,14 @@ extern "C" size_t mo_df_build_scratch_bytes(int64_t nv, int64_t nf, int N, int m
 
 __global__ void k_add_u64(unsigned long long* __restrict__ c, unsigned long long v) { atomicAdd(c, v); }
 
+static int df_status(int status, int64_t nv) {
+    if (status & 1) set_error("face index out of range [0, %lld)", (long long)nv);
+    else if (status & 2) set_error("LBVH traversal stack overflow");
+    else if (status & 4) set_error("LBVH is malformed (refit or traversal bound exceeded)");
+    else return MO_OK;
+    return MO_ERR_DEVICE;
+}
+
 static int df_build_impl(const float* V, int64_t nv, const int32_t* F, int64_t nf, int N, const double* params4,
                          const MoDfOptions* opt, void* scratch, size_t scratch_bytes, float* grid_out,
                          int32_t* status_out, unsigned long long* counts, void* stream) {
@@ -1290,10 +1298,7 @@ static int df_build_impl(const float* V, int64_t nv, const int32_t* F, int64_t n
         int status = 0;
         cudaError_t e = cudaMemcpyAsync(&status, S.status, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) rc = cuda_status(e, "df build status");
-        else if (status & 1) { set_error("face index out of range [0, %lld)", (long long)nv); rc = MO_ERR_DEVICE; }
-        else if (status & 2) { set_error("LBVH traversal stack overflow"); rc = MO_ERR_DEVICE; }
-        else if (status & 4) { set_error("LBVH is malformed (refit or traversal bound exceeded)"); rc = MO_ERR_DEVICE; }
+        rc = e != cudaSuccess ? cuda_status(e, "df build status") : df_status(status, nv);
     }
     if (owned) cudaFreeAsync(owned, s);
     return rc;
@@ -1322,6 +1327,30 @@ extern "C" int mo_df_build(const float* V, int64_t nv, const int32_t* F, int64_t
     opt.method = method;
     opt.packet = mo_df_packet_for(nf, N, 0.0f);
     return mo_df_build_ex(V, nv, F, nf, N, params4, &opt, scratch, scratch_bytes, grid_out, status_out, stream);
+}
+
+extern "C" int mo_template_build(const float* V, int64_t nv, const int32_t* F, int64_t nf, int N, int method,
+                                 int layout, int32_t* bbox6, double* params4, void* scratch, size_t scratch_bytes,
+                                 float* grid_linear_out, float* grid_out, void* stream) {
+    MO_CHECK_ARG(scratch, "null scratch");
+    MO_CHECK_ARG(layout == MO_LAYOUT_LINEAR || grid_out, "null grid pointer");
+    int rc = mo_bbox_params(V, nv, bbox6, params4, stream);
+    if (rc) return rc;
+    cudaStream_t s = as_stream(stream);
+    // the scratch begins with the status words
+    if (scratch_bytes < 4 * sizeof(int)) {
+        set_error("DF build scratch too small: %zu bytes", scratch_bytes);
+        return MO_ERR_SCRATCH;
+    }
+    int32_t* st = plan_scratch(reinterpret_cast<char*>(scratch), nv, nf, MO_DF_BRUTE).status;
+    MO_CUDA(cudaMemsetAsync(st, 0, 4 * sizeof(int), s));
+    rc = mo_df_build(V, nv, F, nf, N, params4, method, scratch, scratch_bytes, grid_linear_out, st, stream);
+    if (!rc && layout != MO_LAYOUT_LINEAR) rc = mo_grid_relayout(grid_linear_out, N, layout, grid_out, stream);
+    if (rc) return rc;
+    int status = 0;
+    MO_CUDA(cudaMemcpyAsync(&status, st, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MO_CUDA(cudaStreamSynchronize(s));
+    return df_status(status, nv);
 }
 
 extern "C" int mo_lbvh_build(const float* V, int64_t nv, const int32_t* F, int64_t nf, const double* params4,

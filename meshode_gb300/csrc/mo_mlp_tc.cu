@@ -1427,3 +1427,124 @@ extern "C" int mo_mlp_tc_reduce(const float* partial, int64_t n, const float* wp
     MO_LAUNCH_CHECK("k_tc_reduce");
     return MO_OK;
 }
+
+// ---------------------------------------------------------------------------
+// The whole RK4 flow and its adjoint, issued in one call each: an evaluation
+// at a few thousand vertices is 10 us of the GPU's time, less than a call
+// through the bindings takes.
+// ---------------------------------------------------------------------------
+namespace {
+constexpr int64_t FLOW_ALIGN = 32;  // floats
+int64_t flow_pad(int64_t floats) { return (floats + FLOW_ALIGN - 1) / FLOW_ALIGN * FLOW_ALIGN; }
+
+// x_next = RK4(x) with the stage inputs in u [3][n][3]; act: the four
+// evaluations' H1, H2, H3 ([3][4][rows][W]) or NULL.
+int flow_step(const float* x, int64_t n, void* pack, int W, double h, float* u, float* act, float* x_next,
+              void* stream) {
+    const int64_t size = mo_mlp_tc_rows(n) * W;
+    const float a[4] = {(float)(h / 2), (float)(h / 2), (float)h, 0.f};
+    const float w[4] = {(float)(h / 6), (float)(h / 3), (float)(h / 3), (float)(h / 6)};
+    for (int k = 0; k < 4; ++k) {
+        const int rc = mo_mlp_tc_fwd(k ? u + (k - 1) * 3 * n : x, x, n, pack, W, a[k], w[k], k == 0,
+                                     k < 3 ? u + k * 3 * n : nullptr, x_next, act ? act + k * size : nullptr,
+                                     act ? 4 * size : 0, stream);
+        if (rc) return rc;
+    }
+    return MO_OK;
+}
+}  // namespace
+
+extern "C" int64_t mo_ode_act_floats(int64_t n, int W) {
+    return n <= 0 || check_width(W) ? 0 : 12 * mo_mlp_tc_rows(n) * W;
+}
+
+extern "C" int64_t mo_ode_backward_floats(int64_t n, int W, int stored) {
+    if (n <= 0 || check_width(W)) return 0;
+    const int64_t rows = mo_mlp_tc_rows(n);
+    return flow_pad(8 * rows * W) + flow_pad(mo_mlp_tc_partial_floats(n, W)) +
+           2 * flow_pad(mo_mlp_tc_wgrad_floats(4 * rows, W)) + 2 * flow_pad(3 * n) +
+           (stored ? 0 : flow_pad(mo_ode_act_floats(n, W)) + flow_pad(9 * n));
+}
+
+extern "C" int mo_ode_flow(const float* x0, int64_t n, int steps, void* pack, int W, float* ckpt, float* act, float* u,
+                           float* out, void* stream) {
+    int rc = check_width(W);
+    if (rc) return rc;
+    MO_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31) && steps >= 1, "bad sizes");
+    if (n == 0) return MO_OK;
+    MO_CHECK_ARG(x0 && pack && ckpt && u && out, "null pointer");
+    MO_CUDA(cudaMemcpyAsync(ckpt, x0, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, as_stream(stream)));
+    const double h = 1.0 / steps;
+    for (int k = 0; k < steps; ++k) {
+        rc = flow_step(ckpt + 3 * n * k, n, pack, W, h, act ? u + 9 * n * k : u,
+                       act ? act + mo_ode_act_floats(n, W) * k : nullptr, k + 1 < steps ? ckpt + 3 * n * (k + 1) : out,
+                       stream);
+        if (rc) return rc;
+    }
+    return MO_OK;
+}
+
+extern "C" int mo_ode_flow_backward(const float* ckpt, int64_t n, int steps, void* pack, int W, int m, float* act,
+                                    float* u, const float* a_out, float* scratch, int64_t scratch_floats, float* dx0,
+                                    float* dx1, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3,
+                                    float* dW4, float* db4, void* stream) {
+    int rc = check_width(W);
+    if (rc) return rc;
+    MO_CHECK_ARG(n > 0 && n < ((int64_t)1 << 31) && steps >= 1, "bad sizes");
+    MO_CHECK_ARG(ckpt && pack && a_out && scratch && dx0 && dx1 && (!act || u), "null pointer");
+    MO_CHECK_ARG(aligned(scratch, 128), "scratch must be 128-byte aligned");
+    const bool stored = act != nullptr;
+    if (scratch_floats < mo_ode_backward_floats(n, W, stored)) {
+        set_error("flow scratch too small: %lld < %lld floats", (long long)scratch_floats,
+                  (long long)mo_ode_backward_floats(n, W, stored));
+        return MO_ERR_SCRATCH;
+    }
+    const int64_t rows = mo_mlp_tc_rows(n), size = rows * W, act_step = mo_ode_act_floats(n, W);
+    float* next = scratch;
+    auto take = [&](int64_t floats) {
+        float* q = next;
+        next += flow_pad(floats);
+        return q;
+    };
+    float* gz = take(8 * size);
+    float* partial = take(mo_mlp_tc_partial_floats(n, W));
+    float* wpart[2] = {take(mo_mlp_tc_wgrad_floats(4 * rows, W)), take(mo_mlp_tc_wgrad_floats(4 * rows, W))};
+    float* gu[2] = {take(3 * n), take(3 * n)};
+    float* dx[2] = {dx0, dx1};
+    if (!stored) {
+        act = take(act_step);
+        u = take(9 * n);
+    }
+    const double h = 1.0 / steps;
+    const float* a = a_out;
+    int evals = 0;
+    for (int k = steps - 1; k >= 0; --k) {
+        const float* x = ckpt + 3 * n * k;
+        float* ak = stored ? act + act_step * k : act;
+        float* uk = stored ? u + 9 * n * k : u;
+        // the recompute's end state is not needed: it goes where this step's
+        // gradient is written next
+        if (!stored) {
+            rc = flow_step(x, n, pack, W, h, uk, ak, dx[k & 1], stream);
+            if (rc) return rc;
+        }
+        // dk4 = a h/6, dk3 = a h/3 + h g4, dk2 = a h/3 + h/2 g3, dk1 = a h/6 + h/2 g2;
+        // dL/dx = a + g4 + g3 + g2 + g1
+        const float ca[4] = {(float)(h / 6), (float)(h / 3), (float)(h / 3), (float)(h / 6)};
+        const float cg[4] = {(float)(h / 2), (float)(h / 2), (float)h, 0.f};
+        for (int e = 3; e >= 0; --e, ++evals) {
+            rc = mo_mlp_tc_bwd(a, ca[e], e == 3 ? nullptr : gu[evals & 1], cg[e], e ? uk + (e - 1) * 3 * n : x, n, pack, W,
+                               ak + e * size, 4 * size, gz + e * size, gz + (4 + e) * size, e == 3 ? a : dx[k & 1],
+                               dx[k & 1], gu[1 - (evals & 1)], partial, evals == 0, stream);
+            if (rc) return rc;
+        }
+        for (int l = 0; l < 2; ++l) {
+            rc = mo_mlp_tc_wgrad(gz + 4 * l * size, ak + 4 * l * size, 4 * rows, pack, W, 2 + l, wpart[l], k == steps - 1,
+                                 stream);
+            if (rc) return rc;
+        }
+        a = dx[k & 1];
+    }
+    return mo_mlp_tc_reduce(partial, n, wpart[0], wpart[1], 4 * rows, W, m, dW1, db1, dW2, db2, dW3, db3, dW4, db4,
+                            stream);
+}

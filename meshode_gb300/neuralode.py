@@ -22,7 +22,8 @@ Every evaluation of the MLP is one fused libmeshode kernel (mo_mlp_tc_fwd:
 the four layers of 128-vertex tiles with their activations kept on chip, and
 the RK4 stage update), its vector-Jacobian product another (mo_mlp_tc_bwd), and
 the hidden weights' gradients a split-K kernel over the four stages of a step
-(mo_mlp_tc_wgrad).  Their contractions run on the tensor cores in FP16 pairs
+(mo_mlp_tc_wgrad); a flow's evaluations are issued by one call (mo_ode_flow,
+mo_ode_flow_backward).  Their contractions run on the tensor cores in FP16 pairs
 that carry 22 bits, accumulated in FP32; everything else is FP32.
 """
 import math
@@ -74,94 +75,6 @@ class _Packed:
                 for sh in ((m, 3), (m,), (m, m), (m,), (m, m), (m,), (3, m), (3,))]
 
 
-def _fwd(P, u, x, a, w, init_acc, unext, acc, store=None, astride=0):
-    """One fused MLP evaluation k = f(u) with the RK4 update
-    unext = x + a*k, acc = (init ? x : acc) + w*k (mo_mlp_tc_fwd); store: the
-    stage's H1 H2 H3 at stride astride."""
-    call("mo_mlp_tc_fwd", ptr(u), ptr(x), u.shape[0], ptr(P.buf), P.M, float(a), float(w), int(init_acc), ptr(unext),
-         ptr(acc), ptr(store), int(astride), stream_ptr())
-
-
-class _StepStore:
-    """The activations of one RK4 step's four evaluations:
-    act [3][4][rows][M] (H1 H2 H3 of stages 1..4; rows: n padded to whole
-    tiles) and the stage inputs u2..u4."""
-
-    def __init__(self, n, M, dev):
-        self.n = int(L.lib().mo_mlp_tc_rows(n)) * M  # floats of one array of one stage
-        self.act = torch.empty(3 * 4 * self.n, dtype=torch.float32, device=dev)
-        self.u = [None, torch.empty(n, 3, dtype=torch.float32, device=dev),
-                  torch.empty(n, 3, dtype=torch.float32, device=dev), torch.empty(n, 3, dtype=torch.float32, device=dev)]
-
-    def stage(self, s):
-        return self.act[s * self.n:], 4 * self.n
-
-    def array(self, a):
-        """Array a (0 H1, 1 H2, 2 H3) of all four stages."""
-        return self.act[a * 4 * self.n:(a + 1) * 4 * self.n]
-
-
-def _rk4_step(P, x, h, st=None):
-    """One classic RK4 step of the fused evaluations; with st, the stages'
-    activations and inputs are kept there.  Returns x_next."""
-    acc = torch.empty_like(x)
-    if st is None:
-        u2, u3, u4 = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
-    else:
-        u2, u3, u4 = st.u[1], st.u[2], st.u[3]
-    ss = [st.stage(k) if st is not None else (None, 0) for k in range(4)]
-    _fwd(P, x, x, h / 2, h / 6, 1, u2, acc, *ss[0])
-    _fwd(P, u2, x, h / 2, h / 3, 0, u3, acc, *ss[1])
-    _fwd(P, u3, x, h, h / 3, 0, u4, acc, *ss[2])
-    _fwd(P, u4, x, 0.0, h / 6, 0, None, acc, *ss[3])
-    return acc
-
-
-class _Backward:
-    """Work buffers of the adjoint: the stage gradients g_z2, g_z3 of the
-    four evaluations of a step ([2][4][rows][M]) and the partial sums of the
-    parameter gradients, added to by every step (each block and split of the
-    kernels adds to its own, in step order) and reduced once at the end."""
-
-    def __init__(self, n, M, dev):
-        lib = L.lib()
-        self.n = n
-        self.rows = int(lib.mo_mlp_tc_rows(n))
-        self.size = self.rows * M
-
-        def floats(k):
-            return torch.empty(int(k), dtype=torch.float32, device=dev)
-
-        self.gz = floats(2 * 4 * self.size)
-        self.partial = floats(lib.mo_mlp_tc_partial_floats(n, M))
-        self.wpart = [floats(lib.mo_mlp_tc_wgrad_floats(4 * self.rows, M)) for _ in range(2)]
-        self.gu = [torch.empty(n, 3, dtype=torch.float32, device=dev) for _ in range(2)]
-        self.dx = [torch.empty(n, 3, dtype=torch.float32, device=dev) for _ in range(2)]
-        self.evals = self.steps = 0
-
-    def stage_vjp(self, P, st, s, u, a, ca, cg, dx_in, dx_out):
-        """Evaluation s (0..3) of the step: dL/dk = ca*a + cg*(dL/du of the
-        evaluation handled before); dx_out = dx_in + dL/du."""
-        act, astride = st.stage(s)
-        prev, out = self.gu[self.evals & 1], self.gu[1 - (self.evals & 1)]
-        call("mo_mlp_tc_bwd", ptr(a), float(ca), ptr(prev) if cg else None, float(cg), ptr(u), self.n, ptr(P.buf), P.M,
-             ptr(act), int(astride), ptr(self.gz[s * self.size:]), ptr(self.gz[(4 + s) * self.size:]), ptr(dx_in),
-             ptr(dx_out), ptr(out), ptr(self.partial), int(self.evals == 0), stream_ptr())
-        self.evals += 1
-
-    def weights(self, P, st):
-        """The hidden weights' gradients of the step's four evaluations."""
-        s = stream_ptr()
-        for k, layer in ((0, 2), (1, 3)):
-            call("mo_mlp_tc_wgrad", ptr(self.gz[4 * k * self.size:]), ptr(st.array(k)), 4 * self.rows, ptr(P.buf), P.M,
-                 layer, ptr(self.wpart[k]), int(self.steps == 0), s)
-        self.steps += 1
-
-    def reduce(self, P, grads):
-        call("mo_mlp_tc_reduce", ptr(self.partial), self.n, ptr(self.wpart[0]), ptr(self.wpart[1]), 4 * self.rows, P.M,
-             P.m, *[ptr(g) for g in grads], stream_ptr())
-
-
 class ODEFlow(Function):
     """x(1) = RK4^steps(x(0)) under the velocity MLP, with an adjoint
     backward on the fused kernels.  store=False: checkpointed (states at
@@ -174,53 +87,41 @@ class ODEFlow(Function):
     def forward(ctx, x0, steps, store, W1, b1, W2, b2, W3, b3, W4, b4):
         P = _Packed((W1, b1, W2, b2, W3, b3, W4, b4))
         steps = int(steps)
-        h = 1.0 / steps
+        1.0 / steps  # a flow has steps
         x = x0.detach().contiguous().float()
         n = x.shape[0]
-        ckpt = torch.empty(steps, n, 3, dtype=torch.float32, device=x.device)
-        ctx.stores = [] if store else None
-        for k in range(steps):
-            ckpt[k].copy_(x)
-            st = _StepStore(n, P.M, x.device) if store else None
-            x = _rk4_step(P, x, h, st)
-            if store:
-                ctx.stores.append(st)
+
+        def floats(*shape):
+            return torch.empty(shape, dtype=torch.float32, device=x.device)
+
+        ckpt = floats(steps, n, 3)
+        act = floats(steps, int(L.lib().mo_ode_act_floats(n, P.M))) if store else None
+        u = floats(steps if store else 1, 3, n, 3)
+        out = torch.empty_like(x)
+        call("mo_ode_flow", ptr(x), n, steps, ptr(P.buf), P.M, ptr(ckpt), ptr(act), ptr(u), ptr(out), stream_ptr())
         ctx.P = P
+        ctx.kept = (act, u) if store else None
         ctx.save_for_backward(ckpt)
         ctx.steps = steps
-        return x
+        return out
 
     @staticmethod
     def backward(ctx, a_out):
         (ckpt,) = ctx.saved_tensors
         P = ctx.P
         steps = ctx.steps
-        h = 1.0 / steps
         n = ckpt.shape[1]
         grads = P.grads()
         a = a_out.contiguous().float()
-        if n > 0 and steps > 0:
-            B = _Backward(n, P.M, a.device)
-            work = None if ctx.stores is not None else _StepStore(n, P.M, a.device)
-            for k in reversed(range(steps)):
-                xk = ckpt[k]
-                if ctx.stores is not None:
-                    st = ctx.stores[k]
-                    ctx.stores[k] = None
-                else:
-                    st = work
-                    _rk4_step(P, xk, h, st)
-                # dk4 = a h/6, dk3 = a h/3 + h g4, dk2 = a h/3 + h/2 g3, dk1 = a h/6 + h/2 g2;
-                # dL/dx = a + g4 + g3 + g2 + g1
-                dx = B.dx[k & 1]
-                B.stage_vjp(P, st, 3, st.u[3], a, h / 6, 0.0, a, dx)
-                B.stage_vjp(P, st, 2, st.u[2], a, h / 3, h, dx, dx)
-                B.stage_vjp(P, st, 1, st.u[1], a, h / 3, h / 2, dx, dx)
-                B.stage_vjp(P, st, 0, xk, a, h / 6, h / 2, dx, dx)
-                B.weights(P, st)
-                a = dx
-            B.reduce(P, grads)
-        ctx.stores = None
+        if n > 0:
+            act, u = ctx.kept if ctx.kept is not None else (None, None)
+            nb = int(L.lib().mo_ode_backward_floats(n, P.M, int(act is not None)))
+            scratch = torch.empty(nb, dtype=torch.float32, device=a.device)
+            dx = [torch.empty(n, 3, dtype=torch.float32, device=a.device) for _ in range(2)]
+            call("mo_ode_flow_backward", ptr(ckpt), n, steps, ptr(P.buf), P.M, P.m, ptr(act), ptr(u), ptr(a),
+                 ptr(scratch), nb, ptr(dx[0]), ptr(dx[1]), *[ptr(g) for g in grads], stream_ptr())
+            a = dx[0]
+        ctx.kept = None
         ctx.P = None
         return (a, None, None) + tuple(grads)
 

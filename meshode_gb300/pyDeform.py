@@ -292,23 +292,17 @@ def InitializeDeformTemplate(tensorV, tensorF, symmetry, grid_resolution, layout
     s = stream_ptr()
     Vd = _on_device(tensorV, dev)
     Fd = _on_device(tensorF, dev)
+    nb = L.lib().mo_grid_bytes(N, p.layout)
+    if nb == 0:
+        raise RuntimeError("unknown grid layout %d" % p.layout)
     bbox = torch.empty(6, dtype=torch.int32, device=dev)
     p.params = torch.empty(4, dtype=torch.float64, device=dev)
-    call("mo_bbox_params", ptr(Vd), Vd.shape[0], ptr(bbox), ptr(p.params), s)
     nbytes = L.lib().mo_df_build_scratch_bytes(Vd.shape[0], Fd.shape[0], N, int(df_method))
     scratch = torch.empty(int(nbytes), dtype=torch.uint8, device=dev)
     p.grid_linear = torch.empty(N * N * N, dtype=torch.float32, device=dev)
-    call("mo_df_build", ptr(Vd), Vd.shape[0], ptr(Fd), Fd.shape[0], N, ptr(p.params), int(df_method),
-         ptr(scratch), nbytes, ptr(p.grid_linear), None, s)
-    del scratch
-    if p.layout == L.MO_LAYOUT_LINEAR:
-        p.grid = p.grid_linear
-    else:
-        nb = L.lib().mo_grid_bytes(N, p.layout)
-        if nb == 0:
-            raise RuntimeError("unknown grid layout %d" % p.layout)
-        p.grid = torch.empty(nb // 4, dtype=torch.float32, device=dev)
-        call("mo_grid_relayout", ptr(p.grid_linear), N, p.layout, ptr(p.grid), s)
+    p.grid = p.grid_linear if p.layout == L.MO_LAYOUT_LINEAR else torch.empty(nb // 4, dtype=torch.float32, device=dev)
+    call("mo_template_build", ptr(Vd), Vd.shape[0], ptr(Fd), Fd.shape[0], N, int(df_method), p.layout, ptr(bbox),
+         ptr(p.params), ptr(scratch), nbytes, ptr(p.grid_linear), ptr(p.grid), s)
     _g_params.append(p)
     return len(_g_params) - 1
 
