@@ -1202,14 +1202,17 @@ extern "C" int mo_df_method_for(int64_t nf, int N) {
 // The lines: below N = 72 the wide packet has too few warps at any triangle
 // count.  With a band the far voxels, whose walks are the ones 64 voxels
 // share best, are cut short, so the wide packet stops paying at N^3 / 48
-// triangles (128^3, 300k: 2.36 for 4x4x2, 2.35 wide, 2.27 for 2x4x4; flat
-// target 1.67, 1.82, 1.27) against about N^3 / 4 on an exact grid (112^3,
-// 500k: 3.89, 4.06, 3.84).
+// triangles against about N^3 / 4 on an exact grid (112^3, 500k: 3.89, 4.06,
+// 3.84).  From N = 120 on, with four times the warps that the chip holds, that
+// line is N^3 / 8: 128^3, 150k: 1.72 for 4x4x2, 1.56 wide, 1.63 for 2x4x4; 300k
+// 2.36, 2.35, 2.27; flat target, 100k 0.97, 1.00, 0.74.  Several builds at once
+// favour the wide packet further, since it takes the fewest instructions (32
+// requests' builds together: 25.5 -> 24.0 with this line, all wide 23.3).
 extern "C" int mo_df_packet_for(int64_t nf, int N, float band) {
     const double vox = (double)N * N * N;
     if (N < 72) return MO_PACKET_2x4x4_TRI2;
-    const bool far_walks = !(band > 0.0f) && N >= 100;
-    if ((double)nf <= vox / (far_walks ? 4.0 : 48.0)) return MO_PACKET_4x4x4;
+    const double share = !(band > 0.0f) && N >= 100 ? 4.0 : N >= 120 ? 8.0 : 48.0;
+    if ((double)nf <= vox / share) return MO_PACKET_4x4x4;
     return N < 100 ? MO_PACKET_2x4x4_TRI2 : MO_PACKET_2x4x4;
 }
 

@@ -17,6 +17,7 @@ from meshode_gb300 import meshgen
     (72, 7776, 0.0, L.MO_PACKET_4x4x4), (72, 7777, 0.0, L.MO_PACKET_2x4x4_TRI2),
     (99, 20214, 0.5, L.MO_PACKET_4x4x4), (99, 20215, 0.5, L.MO_PACKET_2x4x4_TRI2),
     (100, 20833, 0.3, L.MO_PACKET_4x4x4), (100, 20834, 0.3, L.MO_PACKET_2x4x4),
+    (120, 216_000, 0.3, L.MO_PACKET_4x4x4), (120, 216_001, 0.3, L.MO_PACKET_2x4x4),
     (100, 250_000, 0.0, L.MO_PACKET_4x4x4), (100, 250_001, 0.0, L.MO_PACKET_2x4x4),
 ])
 def test_lines(N, nf, band, packet):
