@@ -272,6 +272,16 @@ __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.
 
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
+// Programmatic dependent launch: the evaluations of a flow are a chain of
+// launches, and at a few thousand vertices a launch's start (tensor memory,
+// barriers, the first weights) is a third of its time.  A launch that says so
+// starts beside the one before it and waits here for its results; everything
+// but the packed weights, which no evaluation changes, is read and written
+// after the wait, and with plain loads (a non-coherent one may not see what
+// another running kernel wrote).
+__device__ __forceinline__ void chain_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- parameters ------------------------------------------------------------
 struct Params {
     const float *W1, *b1, *W2, *b2, *W3, *b3, *W4, *b4;
@@ -563,6 +573,7 @@ struct FwdArgs {
     int init_acc;
     float *unext, *accum, *store;
     int64_t astride;
+    int chained;  // the launch before it wrote none of the packed weights
 };
 
 // k = f(u) of the tile's rows; unext = x + a*k, accum = (init ? x : accum) + wgt*k;
@@ -581,6 +592,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
     using C = Cfg<W>;
     extern __shared__ __align__(1024) unsigned char smem[];
     Block<W> B;
+    chain_start();
+    if (!A.chained) chain_wait();  // the packed weights may be what is waited for
     B.init(smem, A.pack);
     const int tiles_all = (int)((A.n + TILE - 1) / TILE);
     const int tiles = (tiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -592,6 +605,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
         __syncwarp();
     } else {
         regs_up();
+        chain_wait();
         constexpr int HC = C::HC, NH = C::NH, G8 = HC / 8;
         const int g = w >> 2, r = 32 * (w & 3) + lane, c0 = g * HC;
         const uint32_t lane_base = B.tmem + ((uint32_t)(32 * (w & 3)) << 16) + c0;
@@ -613,9 +627,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
             const int64_t row = (int64_t)tile * TILE + r;
             ux = uy = uz = 0.f;
             if (row < A.n) {
-                ux = __ldg(A.u + 3 * row);
-                uy = __ldg(A.u + 3 * row + 1);
-                uz = __ldg(A.u + 3 * row + 2);
+                ux = A.u[3 * row];
+                uy = A.u[3 * row + 1];
+                uz = A.u[3 * row + 2];
             }
             hb1 = fmaf(__ldg(misc + M_N1), fmaxf(fmaxf(fabsf(ux), fabsf(uy)), fabsf(uz)), __ldg(misc + M_MB1)) + 0.7f;
             hm1 = fmaxf(hm1, hb1);
@@ -791,6 +805,7 @@ struct BwdArgs {
     float *dx_out, *gu;
     float* partial;      // [blocks * PARTS][16][W]: dW4 (3), db4, dW1 (3), db1, and their rounding errors
     int first;           // partial: 1 set, 0 add
+    int chained;
 };
 
 // The last layer's gate, two layers back through the tensor cores, and the
@@ -803,6 +818,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
     using C = Cfg<W>;
     extern __shared__ __align__(1024) unsigned char smem[];
     Block<W> B;
+    chain_start();
+    if (!A.chained) chain_wait();  // the packed weights may be what is waited for
     B.init(smem, A.pack);
     const int tiles_all = (int)((A.n + TILE - 1) / TILE);
     const int tiles = (tiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -814,6 +831,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
         __syncwarp();
     } else {
         regs_up();
+        chain_wait();
         constexpr int HC = C::HC, NH = C::NH, G8 = HC / 8;
         const int g = w >> 2, r = 32 * (w & 3) + lane, c0 = g * HC;
         const uint32_t lane_base = B.tmem + ((uint32_t)(32 * (w & 3)) << 16) + c0;
@@ -850,8 +868,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
             if (row < A.n) {
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    gd[d] = A.ca * __ldg(A.a + 3 * row + d);
-                    if (A.gprev) gd[d] = fmaf(A.cg, __ldg(A.gprev + 3 * row + d), gd[d]);
+                    gd[d] = A.ca * A.a[3 * row + d];
+                    if (A.gprev) gd[d] = fmaf(A.cg, A.gprev[3 * row + d], gd[d]);
                 }
             }
             if (g == 0) {
@@ -899,7 +917,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
                 for (int k = 0; k < W / 4; ++k) {
                     const int rr = part * (W / 4) + k;
                     const float4 q = rows[rr];
-                    const float x = __ldg(H3 + rr * 8);
+                    const float x = H3[rr * 8];
                     t0 = fmaf(q.x, x, t0);
                     t1 = fmaf(q.y, x, t1);
                     t2 = fmaf(q.z, x, t2);
@@ -973,7 +991,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
             if (g == 0) {
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (row < A.n) {
-                    q = make_float4(__ldg(A.u + 3 * row), __ldg(A.u + 3 * row + 1), __ldg(A.u + 3 * row + 2), 0.f);
+                    q = make_float4(A.u[3 * row], A.u[3 * row + 1], A.u[3 * row + 2], 0.f);
                     if (*B.late) p0 = p1 = p2 = NAN;
                     A.gu[3 * row] = p0;
                     A.gu[3 * row + 1] = p1;
@@ -1102,6 +1120,8 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
     fence_before();
     __syncthreads();
     fence_after();
+    chain_start();
+    chain_wait();
     const uint32_t tmem = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(smem + C::BARS + 32), 0);
     const int o0 = (blockIdx.x / (W / C::NB)) * C::NB, i0 = (blockIdx.x % (W / C::NB)) * C::NB;
     const int64_t per = (A.chunks + gridDim.y - 1) / gridDim.y;
@@ -1233,48 +1253,68 @@ struct ReduceArgs {
     float *dW1, *db1, *dW2, *dbb2, *dW3, *dbb3, *dW4, *db4;
 };
 
-// n values at distance `stride`, summed with their rounding errors (a plain
-// chain of 300 would lose 2e-7)
-__device__ __forceinline__ float sum_exactly(const float* __restrict__ p, int n, int64_t stride) {
+// The sum of n values at distance `stride`, and of its rounding errors (a plain
+// chain of 300 would lose 2e-7).
+__device__ __forceinline__ float2 sum_exactly(const float* p, int n, int64_t stride) {
     float s = 0.f, c = 0.f;
-#pragma unroll 8
+#pragma unroll 4
     for (int k = 0; k < n; ++k) {
-        const float x = __ldg(p + k * stride), t = __fadd_rn(s, x), b = __fsub_rn(t, s);
+        const float x = p[k * stride], t = __fadd_rn(s, x), b = __fsub_rn(t, s);
         c += __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b));
         s = t;
     }
-    return s + c;
+    return make_float2(s, c);
 }
 
-__global__ void __launch_bounds__(256) k_tc_reduce(ReduceArgs A) {
-    const int m = A.m, W = A.W;
-    int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (e < 2 * (int64_t)m * m) {
-        const bool third = e >= (int64_t)m * m;
-        if (third) e -= (int64_t)m * m;
-        (third ? A.dW3 : A.dW2)[e] =
-            sum_exactly((third ? A.w3 : A.w2) + (e / m) * W + e % m, A.splits, (int64_t)W * W);
-        return;
-    }
-    e -= 2 * (int64_t)m * m;
-    if (e < 2 * m) {
+// 32 gradients a block; each warp sums an eighth of their partial sums, the
+// first one the eighths, both with their rounding errors.  (One thread a
+// gradient was 71 us at width 64: a chain of 152 loads and additions on 35
+// blocks; here 10.3, and 51.8 -> 27.4 at width 256.)
+constexpr int RED_PARTS = 8;
+__global__ void __launch_bounds__(32 * RED_PARTS) k_tc_reduce(ReduceArgs A) {
+    __shared__ float2 sh[RED_PARTS][32];
+    chain_wait();
+    const int m = A.m, W = A.W, lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int64_t mm = (int64_t)m * m;
+    int64_t e = (int64_t)blockIdx.x * 32 + lane;
+    const float *p = nullptr, *more = nullptr;  // more: the rounding errors kept beside p's sums
+    float* out = nullptr;
+    int n = 0;
+    int64_t stride = W;
+    if (e < 2 * mm) {
+        const bool third = e >= mm;
+        if (third) e -= mm;
+        p = (third ? A.w3 : A.w2) + (e / m) * W + e % m;
+        out = (third ? A.dW3 : A.dW2) + e;
+        n = A.splits;
+        stride = (int64_t)W * W;
+    } else if ((e -= 2 * mm) < 2 * m) {
         const bool third = e >= m;
         if (third) e -= m;
-        (third ? A.dbb3 : A.dbb2)[e] = sum_exactly((third ? A.db3 : A.db2) + e, A.dbrows, W);
-        return;
+        p = (third ? A.db3 : A.db2) + e;
+        out = (third ? A.dbb3 : A.dbb2) + e;
+        n = A.dbrows;
+    } else if ((e -= 2 * m) < 7 * m + 3) {  // dW4 (3), dW1 (3), db1 of every unit, then db4
+        const int j = (int)(e / m);
+        const int k = e >= 7 * m ? 3 : j < 3 ? j : j + 1, c = e >= 7 * m ? (int)e - 7 * m : (int)(e % m);
+        p = A.small + (int64_t)k * W + c;
+        more = p + 8 * W;
+        out = k < 3 ? A.dW4 + k * m + c : k == 3 ? A.db4 + c : k < 7 ? A.dW1 + 3 * c + k - 4 : A.db1 + c;
+        n = A.rows;
+        stride = 16 * W;
     }
-    e -= 2 * m;
-    // dW4 (3), dW1 (3), db1 of every unit, then db4
-    if (e >= 7 * m + 3) return;
-    const int j = (int)(e / m);
-    const int k = e >= 7 * m ? 3 : j < 3 ? j : j + 1, c = e >= 7 * m ? (int)e - 7 * m : (int)(e % m);
-    const float* p = A.small + (int64_t)k * W + c;
-    float s = sum_exactly(p, A.rows, 16 * W);
-    s += sum_exactly(p + 8 * W, A.rows, 16 * W);
-    if (k < 3) A.dW4[k * m + c] = s;
-    else if (k == 3) A.db4[c] = s;
-    else if (k < 7) A.dW1[3 * c + k - 4] = s;
-    else A.db1[c] = s;
+    const int per = (n + RED_PARTS - 1) / RED_PARTS, k0 = min(n, part * per), k1 = min(n, k0 + per);
+    float2 s = sum_exactly(p + k0 * stride, k1 - k0, stride);
+    if (more) {
+        const float2 q = sum_exactly(more + k0 * stride, k1 - k0, stride);
+        s.y += q.x + q.y;
+    }
+    sh[part][lane] = s;
+    __syncthreads();
+    if (part != 0 || !out) return;
+    const float2 t = sum_exactly(&sh[0][lane].x, RED_PARTS, 64);
+    const float2 c = sum_exactly(&sh[0][lane].y, RED_PARTS, 64);
+    *out = t.x + (t.y + c.x);
 }
 
 template <int W>
@@ -1299,6 +1339,23 @@ int splits_for(int64_t rows, int W) {
 
 using namespace mo;
 using namespace mo::tc;
+
+// A launch that may start beside the one before it (chained; see chain_wait).
+template <class... P, class... Q>
+static cudaError_t launch(void (*kernel)(P...), dim3 grid, int threads, int smem, void* stream, bool chained, Q... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = as_stream(stream);
+    cfg.attrs = &at;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+#define TC_LAUNCH(...) MO_CUDA(launch(__VA_ARGS__))
 
 #define TC_WIDTH(W_, ...)                          \
     do {                                           \
@@ -1345,8 +1402,8 @@ extern "C" int mo_mlp_tc_pack(const float* W1, const float* b1, const float* W2,
     return MO_OK;
 }
 
-extern "C" int mo_mlp_tc_fwd(const float* u, const float* x, int64_t n, void* pack, int W_, float a, float w,
-                             int init_acc, float* unext, float* acc, float* store, int64_t astride, void* stream) {
+static int issue_fwd(const float* u, const float* x, int64_t n, void* pack, int W_, float a, float w, int init_acc,
+                     float* unext, float* acc, float* store, int64_t astride, void* stream, bool chained) {
     int rc = check_width(W_);
     if (rc) return rc;
     MO_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "bad row count %lld", (long long)n);
@@ -1355,21 +1412,22 @@ extern "C" int mo_mlp_tc_fwd(const float* u, const float* x, int64_t n, void* pa
     MO_CHECK_ARG(aligned(pack, 128), "the packed parameters must be 128-byte aligned");
     MO_CHECK_ARG(!store || (aligned(store, 32) && astride >= mo_mlp_tc_rows(n) * W_ && astride % 8 == 0),
                  "store must be 32-byte aligned with an array stride of at least the padded rows times the width");
-    const FwdArgs A{u, x, n, reinterpret_cast<unsigned char*>(pack), a, w, init_acc, unext, acc, store, astride};
-    const int blocks = blocks_for(n);
-    cudaStream_t s = as_stream(stream);
-    TC_WIDTH(W_, {
-        if (store) k_tc_fwd<W, true><<<blocks, THREADS, Cfg<W>::SMEM, s>>>(A);
-        else k_tc_fwd<W, false><<<blocks, THREADS, Cfg<W>::SMEM, s>>>(A);
-    });
+    const FwdArgs A{u, x, n, reinterpret_cast<unsigned char*>(pack), a, w, init_acc, unext, acc, store, astride,
+                    chained};
+    TC_WIDTH(W_, TC_LAUNCH(store ? k_tc_fwd<W, true> : k_tc_fwd<W, false>, blocks_for(n), THREADS, Cfg<W>::SMEM, stream,
+                           chained, A));
     ::mo::note_launch();
-    MO_LAUNCH_CHECK("k_tc_fwd");
     return MO_OK;
 }
 
-extern "C" int mo_mlp_tc_bwd(const float* a, float ca, const float* gprev, float cg, const float* u, int64_t n,
-                             void* pack, int W_, const float* store, int64_t astride, float* gz2, float* gz3,
-                             const float* dx_in, float* dx_out, float* gu, float* partial, int first, void* stream) {
+extern "C" int mo_mlp_tc_fwd(const float* u, const float* x, int64_t n, void* pack, int W, float a, float w,
+                             int init_acc, float* unext, float* acc, float* store, int64_t astride, void* stream) {
+    return issue_fwd(u, x, n, pack, W, a, w, init_acc, unext, acc, store, astride, stream, false);
+}
+
+static int issue_bwd(const float* a, float ca, const float* gprev, float cg, const float* u, int64_t n, void* pack,
+                     int W_, const float* store, int64_t astride, float* gz2, float* gz3, const float* dx_in,
+                     float* dx_out, float* gu, float* partial, int first, void* stream, bool chained) {
     int rc = check_width(W_);
     if (rc) return rc;
     MO_CHECK_ARG(n >= 0 && n < ((int64_t)1 << 31), "bad row count %lld", (long long)n);
@@ -1380,18 +1438,23 @@ extern "C" int mo_mlp_tc_bwd(const float* a, float ca, const float* gprev, float
                      astride >= mo_mlp_tc_rows(n) * W_,
                  "activations and gradients must be 32-byte aligned and padded to whole tiles");
     const BwdArgs A{a,   gprev, ca,  cg,    u,      n,  reinterpret_cast<unsigned char*>(pack), store, astride,
-                    gz2, gz3,   dx_in, dx_out, gu, partial, first};
-    cudaStream_t s = as_stream(stream);
-    TC_WIDTH(W_, { k_tc_bwd<W><<<blocks_for(n), THREADS, Cfg<W>::SMEM, s>>>(A); });
+                    gz2, gz3,   dx_in, dx_out, gu, partial, first, chained};
+    TC_WIDTH(W_, TC_LAUNCH(k_tc_bwd<W>, blocks_for(n), THREADS, Cfg<W>::SMEM, stream, chained, A));
     ::mo::note_launch();
-    MO_LAUNCH_CHECK("k_tc_bwd");
     return MO_OK;
+}
+
+extern "C" int mo_mlp_tc_bwd(const float* a, float ca, const float* gprev, float cg, const float* u, int64_t n,
+                             void* pack, int W, const float* store, int64_t astride, float* gz2, float* gz3,
+                             const float* dx_in, float* dx_out, float* gu, float* partial, int first, void* stream) {
+    return issue_bwd(a, ca, gprev, cg, u, n, pack, W, store, astride, gz2, gz3, dx_in, dx_out, gu, partial, first,
+                     stream, false);
 }
 
 // layer 2: G = gz2, H = H1; layer 3: G = gz3, H = H2 (rows: padded rows of all
 // evaluations, a multiple of 128)
-extern "C" int mo_mlp_tc_wgrad(const float* G, const float* H, int64_t rows, void* pack, int W_, int layer,
-                               float* partial, int first, void* stream) {
+static int issue_wgrad(const float* G, const float* H, int64_t rows, void* pack, int W_, int layer, float* partial,
+                       int first, void* stream, bool chained) {
     int rc = check_width(W_);
     if (rc) return rc;
     MO_CHECK_ARG(rows >= 0 && rows % TILE == 0, "rows must be a multiple of %d", TILE);
@@ -1400,20 +1463,23 @@ extern "C" int mo_mlp_tc_wgrad(const float* G, const float* H, int64_t rows, voi
     MO_CHECK_ARG(G && H && pack && partial, "null pointer");
     MO_CHECK_ARG(aligned(G, 32) && aligned(H, 32), "arrays must be 32-byte aligned");
     const int splits = splits_for(rows, W_);
-    cudaStream_t s = as_stream(stream);
     TC_WIDTH(W_, {
         const uint32_t* mx = reinterpret_cast<const uint32_t*>(reinterpret_cast<unsigned char*>(pack) + Cfg<W>::P_MAX);
         const WgradArgs A{G, H, rows / 64, mx + layer, mx + layer - 2, partial, partial + (int64_t)splits * W * W, first};
-        k_tc_wgrad<W><<<dim3(WCfg<W>::BLOCKS, splits), WTHREADS, WCfg<W>::SMEM, s>>>(A);
+        TC_LAUNCH(k_tc_wgrad<W>, dim3(WCfg<W>::BLOCKS, splits), WTHREADS, WCfg<W>::SMEM, stream, chained, A);
     });
     ::mo::note_launch();
-    MO_LAUNCH_CHECK("k_tc_wgrad");
     return MO_OK;
 }
 
-extern "C" int mo_mlp_tc_reduce(const float* partial, int64_t n, const float* wpart2, const float* wpart3,
-                                int64_t rows, int W_, int m, float* dW1, float* db1, float* dW2, float* db2,
-                                float* dW3, float* db3, float* dW4, float* db4, void* stream) {
+extern "C" int mo_mlp_tc_wgrad(const float* G, const float* H, int64_t rows, void* pack, int W, int layer,
+                               float* partial, int first, void* stream) {
+    return issue_wgrad(G, H, rows, pack, W, layer, partial, first, stream, false);
+}
+
+static int issue_reduce(const float* partial, int64_t n, const float* wpart2, const float* wpart3, int64_t rows,
+                        int W_, int m, float* dW1, float* db1, float* dW2, float* db2, float* dW3, float* db3,
+                        float* dW4, float* db4, void* stream, bool chained) {
     int rc = check_width(W_);
     if (rc) return rc;
     MO_CHECK_ARG(n > 0 && rows > 0 && m > 0 && m <= W_, "bad sizes");
@@ -1422,10 +1488,15 @@ extern "C" int mo_mlp_tc_reduce(const float* partial, int64_t n, const float* wp
     const int64_t ww = (int64_t)splits * W_ * W_;
     const ReduceArgs A{partial, blocks_for(n) * parts_of(W_), wpart2, wpart3, wpart2 + ww, wpart3 + ww, splits,
                        splits * (W_ < 128 ? 2 : 1), W_, m, dW1, db1, dW2, db2, dW3, db3, dW4, db4};
-    k_tc_reduce<<<ceil_div(2 * (int64_t)m * m + 9 * m + 3, 256), 256, 0, as_stream(stream)>>>(A);
+    TC_LAUNCH(k_tc_reduce, ceil_div(2 * (int64_t)m * m + 9 * m + 3, 32), 32 * RED_PARTS, 0, stream, chained, A);
     ::mo::note_launch();
-    MO_LAUNCH_CHECK("k_tc_reduce");
     return MO_OK;
+}
+
+extern "C" int mo_mlp_tc_reduce(const float* partial, int64_t n, const float* wpart2, const float* wpart3,
+                                int64_t rows, int W, int m, float* dW1, float* db1, float* dW2, float* db2,
+                                float* dW3, float* db3, float* dW4, float* db4, void* stream) {
+    return issue_reduce(partial, n, wpart2, wpart3, rows, W, m, dW1, db1, dW2, db2, dW3, db3, dW4, db4, stream, false);
 }
 
 // ---------------------------------------------------------------------------
@@ -1440,14 +1511,14 @@ int64_t flow_pad(int64_t floats) { return (floats + FLOW_ALIGN - 1) / FLOW_ALIGN
 // x_next = RK4(x) with the stage inputs in u [3][n][3]; act: the four
 // evaluations' H1, H2, H3 ([3][4][rows][W]) or NULL.
 int flow_step(const float* x, int64_t n, void* pack, int W, double h, float* u, float* act, float* x_next,
-              void* stream) {
+              void* stream, bool chained) {
     const int64_t size = mo_mlp_tc_rows(n) * W;
     const float a[4] = {(float)(h / 2), (float)(h / 2), (float)h, 0.f};
     const float w[4] = {(float)(h / 6), (float)(h / 3), (float)(h / 3), (float)(h / 6)};
     for (int k = 0; k < 4; ++k) {
-        const int rc = mo_mlp_tc_fwd(k ? u + (k - 1) * 3 * n : x, x, n, pack, W, a[k], w[k], k == 0,
-                                     k < 3 ? u + k * 3 * n : nullptr, x_next, act ? act + k * size : nullptr,
-                                     act ? 4 * size : 0, stream);
+        const int rc = issue_fwd(k ? u + (k - 1) * 3 * n : x, x, n, pack, W, a[k], w[k], k == 0,
+                                 k < 3 ? u + k * 3 * n : nullptr, x_next, act ? act + k * size : nullptr,
+                                 act ? 4 * size : 0, stream, chained || k > 0);
         if (rc) return rc;
     }
     return MO_OK;
@@ -1478,7 +1549,7 @@ extern "C" int mo_ode_flow(const float* x0, int64_t n, int steps, void* pack, in
     for (int k = 0; k < steps; ++k) {
         rc = flow_step(ckpt + 3 * n * k, n, pack, W, h, act ? u + 9 * n * k : u,
                        act ? act + mo_ode_act_floats(n, W) * k : nullptr, k + 1 < steps ? ckpt + 3 * n * (k + 1) : out,
-                       stream);
+                       stream, k > 0);
         if (rc) return rc;
     }
     return MO_OK;
@@ -1525,7 +1596,7 @@ extern "C" int mo_ode_flow_backward(const float* ckpt, int64_t n, int steps, voi
         // the recompute's end state is not needed: it goes where this step's
         // gradient is written next
         if (!stored) {
-            rc = flow_step(x, n, pack, W, h, uk, ak, dx[k & 1], stream);
+            rc = flow_step(x, n, pack, W, h, uk, ak, dx[k & 1], stream, k < steps - 1);
             if (rc) return rc;
         }
         // dk4 = a h/6, dk3 = a h/3 + h g4, dk2 = a h/3 + h/2 g3, dk1 = a h/6 + h/2 g2;
@@ -1533,18 +1604,18 @@ extern "C" int mo_ode_flow_backward(const float* ckpt, int64_t n, int steps, voi
         const float ca[4] = {(float)(h / 6), (float)(h / 3), (float)(h / 3), (float)(h / 6)};
         const float cg[4] = {(float)(h / 2), (float)(h / 2), (float)h, 0.f};
         for (int e = 3; e >= 0; --e, ++evals) {
-            rc = mo_mlp_tc_bwd(a, ca[e], e == 3 ? nullptr : gu[evals & 1], cg[e], e ? uk + (e - 1) * 3 * n : x, n, pack, W,
-                               ak + e * size, 4 * size, gz + e * size, gz + (4 + e) * size, e == 3 ? a : dx[k & 1],
-                               dx[k & 1], gu[1 - (evals & 1)], partial, evals == 0, stream);
+            rc = issue_bwd(a, ca[e], e == 3 ? nullptr : gu[evals & 1], cg[e], e ? uk + (e - 1) * 3 * n : x, n, pack, W,
+                           ak + e * size, 4 * size, gz + e * size, gz + (4 + e) * size, e == 3 ? a : dx[k & 1],
+                           dx[k & 1], gu[1 - (evals & 1)], partial, evals == 0, stream, !stored || evals > 0);
             if (rc) return rc;
         }
         for (int l = 0; l < 2; ++l) {
-            rc = mo_mlp_tc_wgrad(gz + 4 * l * size, ak + 4 * l * size, 4 * rows, pack, W, 2 + l, wpart[l], k == steps - 1,
-                                 stream);
+            rc = issue_wgrad(gz + 4 * l * size, ak + 4 * l * size, 4 * rows, pack, W, 2 + l, wpart[l], k == steps - 1,
+                             stream, true);
             if (rc) return rc;
         }
         a = dx[k & 1];
     }
-    return mo_mlp_tc_reduce(partial, n, wpart[0], wpart[1], 4 * rows, W, m, dW1, db1, dW2, db2, dW3, db3, dW4, db4,
-                            stream);
+    return issue_reduce(partial, n, wpart[0], wpart[1], 4 * rows, W, m, dW1, db1, dW2, db2, dW3, db3, dW4, db4, stream,
+                        true);
 }
