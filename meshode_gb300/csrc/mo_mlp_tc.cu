@@ -56,7 +56,8 @@ struct Cfg {
     static constexpr int STAGE = NS * 128;             // bytes: NS rows x 64 halves
     static constexpr int A_PIECE = KB * TILE * 128;    // bytes of the activations' hi (or lo) image
     static constexpr int TMEM = 4 * NS;                // tensor memory columns: four accumulators of a half
-    static constexpr int PARTS = EPI / W;              // row ranges of the column sums
+    // column sums: 8-column blocks of a warp, and row ranges where there are more warps than blocks
+    static constexpr int SUM_BLOCKS = W == 256 ? 2 : 1, SUM_PARTS = W == 64 ? 2 : 1;
     // shared memory: activation images, weight stages, parameter vectors, rows, barriers
     static constexpr int VECS = 2 * A_PIECE + STAGES * STAGE;
     static constexpr int ROWS = VECS + 9 * 4 * W;
@@ -423,7 +424,6 @@ struct Block {
     __device__ __forceinline__ const float* vec(int v, int c) const {
         return reinterpret_cast<const float*>(sm + C::VECS) + v * W + c;
     }
-    __device__ __forceinline__ float4* rows() const { return reinterpret_cast<float4*>(sm + C::ROWS); }
 
     // Copies the weight stages of images img0, img1 for `tiles` tiles (one thread).
     __device__ void produce(const unsigned char* img0, const unsigned char* img1, int tiles) {
@@ -803,7 +803,7 @@ struct BwdArgs {
     float *gz2, *gz3;    // n-padded x W, blocks of 8 columns
     const float* dx_in;  // dx_out = dx_in + dL/du
     float *dx_out, *gu;
-    float* partial;      // [blocks * PARTS][16][W]: dW4 (3), db4, dW1 (3), db1, and their rounding errors
+    float* partial;      // [blocks][16][W]: dW4 (3), db4, dW1 (3), db1, and their rounding errors
     int first;           // partial: 1 set, 0 add
     int chained;
 };
@@ -811,8 +811,15 @@ struct BwdArgs {
 // The last layer's gate, two layers back through the tensor cores, and the
 // column sums of the small gradients: dW4 from H3 read by column while the
 // first MMAs run, dW1 and db1 from the tile of g_z1, laid out as FP32 in the
-// (then free) activation images; each thread keeps the sums of one column
-// over all of the block's tiles.
+// (then free) activation images; four lanes keep the sums of one column over
+// all of the block's tiles.
+//
+// Bound (n = 49,688, W = 256): 45,000 clocks a tile of issue, waits for the MMAs
+// and shared memory, and 12,000 more behind L2 (256 MB read and written, and H3
+// again).  The activations are asked for half a layer ahead and the columns
+// summed eight by four rows a warp: 105 -> 95.6 us, width 64 at 2,563 rows 12.6 ->
+// 11.0.  A prefetch of them to L2, a tile or a layer ahead, was no faster or
+// slower (117 us); dW4 by shared memory instead of L2 134 against 113.
 template <int W>
 __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
     using C = Cfg<W>;
@@ -838,9 +845,12 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
         const float* misc = reinterpret_cast<const float*>(A.pack + C::P_MISC);
         const float inv2 = __ldg(misc + M_INV2), inv3 = __ldg(misc + M_INV3);
         float* scratch = reinterpret_cast<float*>(smem);
-        float4* rows = B.rows();
-        const int cc = threadIdx.x % W, part = threadIdx.x / W;
-        float s4[3] = {0.f, 0.f, 0.f}, s1[3] = {0.f, 0.f, 0.f}, sb1 = 0.f, sg[3] = {0.f, 0.f, 0.f};
+        float* rows = reinterpret_cast<float*>(smem + C::ROWS);  // [3][TILE]
+        // Column sums: a lane has a column of an 8-column block and every fourth
+        // row, so a warp's access is 128 consecutive bytes of a block.
+        constexpr int SB = C::SUM_BLOCKS, PART_ROWS = TILE / C::SUM_PARTS;
+        const int blk = w % (W / 8), row0 = w / (W / 8) % C::SUM_PARTS * PART_ROWS, cl = lane & 7, rl = lane >> 3;
+        float s4[SB][3] = {}, s1[SB][4] = {}, sg[3] = {0.f, 0.f, 0.f};
         float gm2 = 0.f, gm3 = 0.f;  // bounds of the gradients seen
         auto at8 = [&](int tile, int c) { return (((int64_t)tile * (W / 8) + c / 8) * TILE + r) * 8; };
         // FP32 tile in shared memory, 16-byte chunks swizzled by the row
@@ -861,21 +871,41 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
             }
         };
 
+        // The activations are used half by half, H3, H2, H1; x holds the next
+        // half: a group of 8 columns is asked for as soon as the last half's
+        // group is used up.  (Asked for where they were needed, they were
+        // waited for.)
+        float x[HC];
+        auto ask = [&](int l, int tile, int half, int i) {
+            ldg8(A.store + l * A.astride + at8(tile, half * C::NS + c0 + 8 * i), x + 8 * i);
+        };
+        float ga[3], gp[3];  // the next tile's a and gprev
+        auto ask_row = [&](int tile) {
+            const int64_t row = (int64_t)tile * TILE + r;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                ga[d] = row < A.n ? A.a[3 * row + d] : 0.f;
+                gp[d] = row < A.n && A.gprev ? A.gprev[3 * row + d] : 0.f;
+            }
+        };
+        ask_row(blockIdx.x);
+#pragma unroll
+        for (int i = 0; i < G8; ++i) ask(2, blockIdx.x, 0, i);
         for (int t = 0; t < tiles; ++t) {
             const int tile = blockIdx.x + t * gridDim.x;
             const int64_t row = (int64_t)tile * TILE + r;
-            float gd[3] = {0.f, 0.f, 0.f};
-            if (row < A.n) {
+            float gd[3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    gd[d] = A.ca * A.a[3 * row + d];
-                    if (A.gprev) gd[d] = fmaf(A.cg, A.gprev[3 * row + d], gd[d]);
-                }
+            for (int d = 0; d < 3; ++d) {
+                gd[d] = A.ca * ga[d];
+                if (A.gprev) gd[d] = fmaf(A.cg, gp[d], gd[d]);
             }
             if (g == 0) {
-                rows[r] = make_float4(gd[0], gd[1], gd[2], 0.f);
 #pragma unroll
-                for (int d = 0; d < 3; ++d) sg[d] += gd[d];
+                for (int d = 0; d < 3; ++d) {
+                    rows[d * TILE + r] = gd[d];
+                    sg[d] += gd[d];
+                }
             }
             // g_z3 = (g W4) * softplus'(z3), below |g|_1 max |W4|; g_z2 below that times |W3^T|_1
             const float gb3 = (fabsf(gd[0]) + fabsf(gd[1]) + fabsf(gd[2])) * __ldg(misc + M_M4);
@@ -886,12 +916,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
             const float sc3 = pow2_scale(gb3, &inv_3), sc2 = pow2_scale(gb2, &inv_2);
 #pragma unroll
             for (int h = 0; h < NH; ++h)
-#pragma unroll 2
+#pragma unroll
                 for (int i = 0; i < G8; ++i) {
                     const int c = h * C::NS + c0 + 8 * i;
-                    float v[8], x[8];
+                    float v[8];
                     uint32_t h4[4], l4[4];
-                    ldg8(A.store + 2 * A.astride + at8(tile, c), x);
 #pragma unroll
                     for (int j = 0; j < 8; j += 4) {
                         const float4 wx = ld4(B.vec(V_W4X, c + j)), wy = ld4(B.vec(V_W4Y, c + j));
@@ -902,33 +931,43 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
                                                     __ffma2_rn(f2(gd[1]), zw(wy), __fmul2_rn(f2(gd[0]), zw(wx))));
                         v[j] = p.x; v[j + 1] = p.y; v[j + 2] = q.x; v[j + 3] = q.y;
                     }
-                    gate8(v, x, 1.0f);
+                    gate8(v, x + 8 * i, 1.0f);
+                    if (h + 1 < NH) ask(2, tile, h + 1, i);
+                    else ask(1, tile, 0, i);
                     stg8(A.gz3 + at8(tile, c), v);
                     split8(v, sc3, h4, l4);
                     B.put8(r, c, h4, l4);
                 }
             B.publish();
             epi_sync();
-            {   // dW4 += g^T H3
-                const float* H3 = A.store + 2 * A.astride +
-                                  ((int64_t)tile * (W / 8) + cc / 8) * TILE * 8 + (cc & 7);
-                float t0 = 0.f, t1 = 0.f, t2 = 0.f;
+            {   // dW4 += g^T H3, from L2 (beside the first MMAs)
+                const float* H3 = A.store + 2 * A.astride + ((int64_t)tile * (W / 8) + blk) * TILE * 8 + cl;
 #pragma unroll 8
-                for (int k = 0; k < W / 4; ++k) {
-                    const int rr = part * (W / 4) + k;
-                    const float4 q = rows[rr];
-                    const float x = H3[rr * 8];
-                    t0 = fmaf(q.x, x, t0);
-                    t1 = fmaf(q.y, x, t1);
-                    t2 = fmaf(q.z, x, t2);
+                for (int k = 0; k < PART_ROWS / 4; ++k) {
+                    const int rr = row0 + 4 * k + rl;
+                    const float g0 = rows[rr], g1 = rows[TILE + rr], g2 = rows[2 * TILE + rr];
+#pragma unroll
+                    for (int q = 0; q < SB; ++q) {
+                        const float h = H3[(q * 16 * TILE + rr) * 8];
+                        s4[q][0] = fmaf(g0, h, s4[q][0]);
+                        s4[q][1] = fmaf(g1, h, s4[q][1]);
+                        s4[q][2] = fmaf(g2, h, s4[q][2]);
+                    }
                 }
-                s4[0] += t0; s4[1] += t1; s4[2] += t2;
             }
+            float e3[3] = {0.f, 0.f, 0.f};  // this row's dx (group 0) or u (group 1)
             // two layers back
             float p0 = 0.f, p1 = 0.f, p2 = 0.f;
 #pragma unroll
             for (int l = 0; l < 2; ++l) {
-                const float* H = A.store + (l == 0 ? A.astride : 0);
+                if (l == 1) {
+                    if (t + 1 < tiles) ask_row(tile + gridDim.x);
+                    const float* e = g == 0 ? A.dx_in : A.u;
+                    if (g < 2 && row < A.n) {
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) e3[d] = e[3 * row + d];
+                    }
+                }
                 const float f = l == 0 ? inv_3 * inv3 : inv_2 * inv2;
                 float v[HC];
                 uint32_t ph[G8][4], pl[G8][4];
@@ -950,9 +989,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
                     }
                 };
                 if (NH == 2) {
-                    float x[HC];
-#pragma unroll
-                    for (int i = 0; i < G8; ++i) ldg8(H + at8(tile, c0 + 8 * i), x + 8 * i);
                     B.wait_result();
 #pragma unroll
                     for (int i = 0; i < G8; ++i) tmem_sum4(lane_base + 8 * i, C::NS, v + 8 * i);
@@ -960,12 +996,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
 #pragma unroll
                     for (int i = 0; i < G8; ++i) {
                         gate8(v + 8 * i, x + 8 * i, f);
+                        ask(1 - l, tile, 1, i);
                         finish8(v + 8 * i, c0 + 8 * i, ph[i], pl[i]);
                     }
                 }
-                float x[HC];
-#pragma unroll
-                for (int i = 0; i < G8; ++i) ldg8(H + at8(tile, (NH - 1) * C::NS + c0 + 8 * i), x + 8 * i);
                 B.wait_result();
                 if (NH == 2) {
 #pragma unroll
@@ -981,6 +1015,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
                     uint32_t h4[4], l4[4];
                     tmem_sum4(lane_base + 8 * i, C::NS, q);
                     gate8(q, x + 8 * i, f);
+                    if (l == 0) ask(0, tile, 0, i);
+                    else if (t + 1 < tiles) ask(2, tile + gridDim.x, 0, i);
                     finish8(q, c, h4, l4);
                     if (l == 0) B.put8(r, c, h4, l4);
                     else put_scratch(c, q);
@@ -988,63 +1024,69 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
                 if (l == 0) B.publish();
             }
             B.row_sums(p0, p1, p2, g, r);
-            if (g == 0) {
-                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (row < A.n) {
-                    q = make_float4(A.u[3 * row], A.u[3 * row + 1], A.u[3 * row + 2], 0.f);
-                    if (*B.late) p0 = p1 = p2 = NAN;
-                    A.gu[3 * row] = p0;
-                    A.gu[3 * row + 1] = p1;
-                    A.gu[3 * row + 2] = p2;
-                    A.dx_out[3 * row] = A.dx_in[3 * row] + p0;
-                    A.dx_out[3 * row + 1] = A.dx_in[3 * row + 1] + p1;
-                    A.dx_out[3 * row + 2] = A.dx_in[3 * row + 2] + p2;
-                }
-                rows[r] = q;
+            if (g == 0 && row < A.n) {
+                if (*B.late) p0 = p1 = p2 = NAN;
+                A.gu[3 * row] = p0;
+                A.gu[3 * row + 1] = p1;
+                A.gu[3 * row + 2] = p2;
+                A.dx_out[3 * row] = e3[0] + p0;
+                A.dx_out[3 * row + 1] = e3[1] + p1;
+                A.dx_out[3 * row + 2] = e3[2] + p2;
             }
-            epi_sync();
-            {   // dW1 += g_z1^T u, db1 += g_z1
-                float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
-#pragma unroll 8
-                for (int k = 0; k < W / 4; ++k) {
-                    const int rr = part * (W / 4) + k;
-                    const float4 q = rows[rr];
-                    const float x = scratch[rr * W + ((((cc >> 2) ^ (rr & 7)) << 2) | (cc & 3))];
-                    t0 = fmaf(q.x, x, t0);
-                    t1 = fmaf(q.y, x, t1);
-                    t2 = fmaf(q.z, x, t2);
-                    t3 += x;
-                }
-                s1[0] += t0; s1[1] += t1; s1[2] += t2; sb1 += t3;
-            }
-            epi_sync();
-        }
-        // db4: the rows of group 0, by the first three columns of its first threads
-        float sb4 = 0.f;
-        {
-            float* x = reinterpret_cast<float*>(smem + C::ROWS);
-            if (g == 0) {
+            if (g == 1) {
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    for (int o = 16; o > 0; o >>= 1) sg[d] += __shfl_xor_sync(0xffffffffu, sg[d], o);
-                    if (lane == 0) x[4 * d + w] = sg[d];
+                for (int d = 0; d < 3; ++d) rows[d * TILE + r] = e3[d];
+            }
+            epi_sync();
+            {   // dW1 += g_z1^T u, db1 += g_z1 (every other row of a lane's eight: no two lanes in a bank)
+#pragma unroll 4
+                for (int k = 0; k < PART_ROWS / 4; ++k) {
+                    const int rr = row0 + 8 * (k >> 1) + (k & 1) + 2 * rl;
+                    const float u0 = rows[rr], u1 = rows[TILE + rr], u2 = rows[2 * TILE + rr];
+#pragma unroll
+                    for (int q = 0; q < SB; ++q) {
+                        const int c = 8 * (blk + 16 * q) + cl;
+                        const float x1 = scratch[rr * W + ((((c >> 2) ^ (rr & 7)) << 2) | (c & 3))];
+                        s1[q][0] = fmaf(u0, x1, s1[q][0]);
+                        s1[q][1] = fmaf(u1, x1, s1[q][1]);
+                        s1[q][2] = fmaf(u2, x1, s1[q][2]);
+                        s1[q][3] += x1;
+                    }
                 }
             }
             epi_sync();
-            if (threadIdx.x < 3) {
-                const float* q = x + 4 * threadIdx.x;
-                sb4 = (q[0] + q[1]) + (q[2] + q[3]);
+        }
+        // a column's four lanes (and row ranges) together; db4: the rows of group 0
+        float* sums = scratch;  // [SUM_PARTS][8][W]: dW4 (3), -, dW1 (3), db1
+        float* xs = reinterpret_cast<float*>(smem + C::ROWS);
+#pragma unroll
+        for (int q = 0; q < SB; ++q)
+#pragma unroll
+            for (int d = 0; d < 7; ++d) {
+                float v = d < 3 ? s4[q][d < 3 ? d : 0] : s1[q][d < 3 ? 0 : d - 3];
+                v += __shfl_xor_sync(0xffffffffu, v, 8);
+                v += __shfl_xor_sync(0xffffffffu, v, 16);
+                if (lane < 8) sums[(row0 / PART_ROWS * 8 + d + (d >= 3)) * W + 8 * (blk + 16 * q) + cl] = v;
+            }
+        if (g == 0) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                for (int o = 16; o > 0; o >>= 1) sg[d] += __shfl_xor_sync(0xffffffffu, sg[d], o);
+                if (lane == 0) xs[4 * d + w] = sg[d];
             }
         }
+        epi_sync();
         // the sums over all launches of a backward pass, with their rounding errors beside them
-        float* out = A.partial + ((int64_t)blockIdx.x * C::PARTS + part) * 16 * W + cc;
-        const float s[8] = {s4[0], s4[1], s4[2], sb4, s1[0], s1[1], s1[2], sb1};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const float h = A.first ? 0.f : out[k * W], y = A.first ? s[k] : __fadd_rn(s[k], out[(8 + k) * W]);
+        for (int e = threadIdx.x; e < 8 * W; e += EPI) {
+            const int k = e / W, c = e % W;
+            float v = sums[e];
+            if (C::SUM_PARTS == 2) v += sums[8 * W + e];
+            if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
+            float* out = A.partial + (int64_t)blockIdx.x * 16 * W + e;
+            const float h = A.first ? 0.f : *out, y = A.first ? v : __fadd_rn(v, out[8 * W]);
             const float t = __fadd_rn(h, y), b = __fsub_rn(t, h);
-            out[k * W] = t;
-            out[(8 + k) * W] = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(y, b));
+            *out = t;
+            out[8 * W] = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(y, b));
         }
         const uint32_t m2 = __reduce_max_sync(0xffffffffu, __float_as_uint(gm2));
         const uint32_t m3 = __reduce_max_sync(0xffffffffu, __float_as_uint(gm3));
@@ -1328,7 +1370,6 @@ int set_attrs() {
 
 int64_t tiles_of(int64_t n) { return (n + TILE - 1) / TILE; }
 int blocks_for(int64_t n) { return (int)std::min<int64_t>(tiles_of(n), device_sm_count()); }
-int parts_of(int W) { return EPI / W; }
 int splits_for(int64_t rows, int W) {
     const int blocks = W == 256 ? 4 : 1;
     return (int)std::max<int64_t>(1, std::min<int64_t>(device_sm_count() / blocks, rows / 64));
@@ -1376,7 +1417,7 @@ extern "C" size_t mo_mlp_tc_pack_bytes(int W) {
 }
 extern "C" int64_t mo_mlp_tc_partial_floats(int64_t n, int W) {
     if (n <= 0 || (W != 64 && W != 128 && W != 256)) return 0;
-    return (int64_t)blocks_for(n) * parts_of(W) * 16 * W;
+    return (int64_t)blocks_for(n) * 16 * W;
 }
 extern "C" int64_t mo_mlp_tc_wgrad_floats(int64_t rows, int W) {
     if (rows <= 0 || (W != 64 && W != 128 && W != 256)) return 0;
@@ -1486,7 +1527,7 @@ static int issue_reduce(const float* partial, int64_t n, const float* wpart2, co
     MO_CHECK_ARG(partial && wpart2 && wpart3 && dW1 && db1 && dW2 && db2 && dW3 && db3 && dW4 && db4, "null pointer");
     const int splits = splits_for(rows, W_);
     const int64_t ww = (int64_t)splits * W_ * W_;
-    const ReduceArgs A{partial, blocks_for(n) * parts_of(W_), wpart2, wpart3, wpart2 + ww, wpart3 + ww, splits,
+    const ReduceArgs A{partial, blocks_for(n), wpart2, wpart3, wpart2 + ww, wpart3 + ww, splits,
                        splits * (W_ < 128 ? 2 : 1), W_, m, dW1, db1, dW2, db2, dW3, db3, dW4, db4};
     TC_LAUNCH(k_tc_reduce, ceil_div(2 * (int64_t)m * m + 9 * m + 3, 32), 32 * RED_PARTS, 0, stream, chained, A);
     ::mo::note_launch();
