@@ -5,20 +5,17 @@
 // Mesh::ConstructDistanceField (mesh.cc:106-152), whose
 // igl::point_mesh_squared_distance query (mesh.cc:140) returns the exact
 // squared distance to the nearest triangle; the grid stores its sqrt.
-#include <cooperative_groups.h>
-
 #include <cfloat>
 #include <cmath>
 #include <cstring>
 #include <mutex>
 
+#include "mo_bbox.cuh"
 #include "mo_common.cuh"
 #include "mo_df_trav.cuh"
 #include "mo_lbvh.cuh"
 
 namespace mo {
-
-namespace cg = cooperative_groups;
 
 // ---------------------------------------------------------------------------
 // Normalisation
@@ -70,57 +67,15 @@ __device__ __forceinline__ void norm_params(const int* bb, double* __restrict__ 
 
 __global__ void k_norm_params(const int* __restrict__ bb, double* __restrict__ prm) { norm_params(bb, prm); }
 
-// The box, and with prm the normalisation, in one launch: a cluster of eight
-// blocks, which can wait for one another without a word in memory that
-// somebody would have to clear first.  The thread count is a multiple of
-// three, so a thread keeps one coordinate and the reads are consecutive; a
-// warp reduces each coordinate by itself and its leaders put it into the
-// first block's shared memory.  Eight SMs read ~1 TB/s: past BBOX_CLUSTER_MAX
-// vertices the whole chip and two launches more are faster.
+// The box, and with prm the normalisation, in one launch.
 // Measured, us: 10k vertices 9.0 (box, clearing, parameters) -> 5.2;
 // 178k 25.6 -> 12.2.
-constexpr int BBOX_BLOCKS = 8, BBOX_THREADS = 960, BBOX_UNROLL = 16;
-constexpr int64_t BBOX_CLUSTER_MAX = 1 << 20;
-
 __global__ void __cluster_dims__(BBOX_BLOCKS, 1, 1) __launch_bounds__(BBOX_THREADS)
     k_bbox_cluster(const float* __restrict__ V, int64_t n, int* __restrict__ bb, double* __restrict__ prm) {
-    static_assert(BBOX_THREADS % 96 == 0, "whole warps, and a coordinate a thread");
     __shared__ int box[6];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int tid = (int)threadIdx.x, c = tid % 3;
-    if (tid < 6) box[tid] = tid < 3 ? INT_MAX : INT_MIN;
-    cluster.sync();
-    int lo = INT_MAX, hi = INT_MIN;
-    constexpr int64_t STRIDE = (int64_t)BBOX_BLOCKS * BBOX_THREADS;
-    const int64_t total = 3 * n;
-    for (int64_t i = (int64_t)blockIdx.x * BBOX_THREADS + tid; i < total; i += STRIDE * BBOX_UNROLL) {
-        float f[BBOX_UNROLL];
-#pragma unroll
-        for (int k = 0; k < BBOX_UNROLL; ++k) f[k] = i + k * STRIDE < total ? __ldg(V + i + k * STRIDE) : NAN;
-#pragma unroll
-        for (int k = 0; k < BBOX_UNROLL; ++k) {
-            if (f[k] != f[k]) continue;  // NaN never wins a comparison in the reference
-            const int o = float_to_ordered(f[k]);
-            lo = min(lo, o);
-            hi = max(hi, o);
-        }
-    }
-    int* first = cluster.map_shared_rank(box, 0);
-    for (int k = 0; k < 3; ++k) {  // lanes of coordinate k
-        const unsigned lanes = __ballot_sync(0xffffffffu, c == k);
-        if (c != k) continue;
-        lo = __reduce_min_sync(lanes, lo);
-        hi = __reduce_max_sync(lanes, hi);
-        if ((tid & 31) == __ffs(lanes) - 1) {
-            atomicMin(&first[k], lo);
-            atomicMax(&first[3 + k], hi);
-        }
-    }
-    cluster.sync();
-    if (blockIdx.x == 0 && tid == 0) {
-        for (int k = 0; k < 6; ++k) bb[k] = box[k];
-        if (prm) norm_params(box, prm);
-    }
+    if (!bbox_cluster<false>(V, n, box)) return;
+    for (int k = 0; k < 6; ++k) bb[k] = box[k];
+    if (prm) norm_params(box, prm);
 }
 
 // normalize.cc:21 / :42, evaluated in double (the reference's FT) once per

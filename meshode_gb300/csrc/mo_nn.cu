@@ -3,7 +3,7 @@
 //   ii = cKDTree(src).query(tar, k=1);  loss = 0.5 * sum |src[ii] - tar|^2.
 //
 // The query builds an LBVH over the source points (Morton codes in the points'
-// bounding cube, stable radix sort, Karras tree, refit: the same stages as the
+// bounding cube, stable radix sort, Karras tree, node boxes: the stages of the
 // distance-field build) and walks it once per target point, one thread per
 // query, queries taken in Morton order so a warp's queries are neighbours.
 // Distances are squared Euclidean in double, summed x, y, z like cKDTree's
@@ -12,6 +12,7 @@
 // index wins.
 #include <cfloat>
 
+#include "mo_bbox.cuh"
 #include "mo_common.cuh"
 #include "mo_lbvh.cuh"
 
@@ -19,12 +20,17 @@ namespace mo {
 namespace {
 
 constexpr int NN_STACK = 64;
+constexpr int CHUNK = 256;
+
+// Points and queries are sorted in one go, the queries' codes above the points'.
+bool sort_together(int64_t np, int64_t nq) { return np + nq < ((int64_t)1 << 30); }
+constexpr uint32_t QUERY = 1u << 30;
 
 struct NnScratch {
     int* bbox;        // 6 ordered ints
     float4* cube;     // lo.xyz, 1/extent
     int* status;
-    uint32_t* codes_a;
+    uint32_t* codes_a;  // points, then queries
     uint32_t* codes_b;
     int* ids_a;
     int* ids_b;
@@ -32,13 +38,9 @@ struct NnScratch {
     float4* boxes;
     int* parent;
     int* flags;
+    int2* range;
+    float4* chunks;   // boxes of CHUNK leaves
     int* hist;
-    float* rootbox;
-    uint32_t* qcodes_a;
-    uint32_t* qcodes_b;
-    int* qids_a;
-    int* qids_b;
-    int* qhist;
     size_t bytes;
 };
 
@@ -55,21 +57,19 @@ NnScratch plan(char* base, int64_t np, int64_t nq) {
     s.bbox = reinterpret_cast<int*>(take(32));
     s.cube = reinterpret_cast<float4*>(take(16));
     s.status = reinterpret_cast<int*>(take(16));
-    s.rootbox = reinterpret_cast<float*>(take(32));
-    s.codes_a = reinterpret_cast<uint32_t*>(take(4 * (size_t)np));
-    s.codes_b = reinterpret_cast<uint32_t*>(take(4 * (size_t)np));
-    s.ids_a = reinterpret_cast<int*>(take(4 * (size_t)np));
-    s.ids_b = reinterpret_cast<int*>(take(4 * (size_t)np));
+    const size_t all = (size_t)np + (size_t)nq;
+    s.codes_a = reinterpret_cast<uint32_t*>(take(4 * all));
+    s.codes_b = reinterpret_cast<uint32_t*>(take(4 * all));
+    s.ids_a = reinterpret_cast<int*>(take(4 * all));
+    s.ids_b = reinterpret_cast<int*>(take(4 * all));
     s.nodes = reinterpret_cast<float4*>(take(64 * (size_t)(np > 1 ? np - 1 : 1)));
     s.boxes = reinterpret_cast<float4*>(take(32 * (size_t)np));
     s.parent = reinterpret_cast<int*>(take(8 * (size_t)np));
     s.flags = reinterpret_cast<int*>(take(4 * (size_t)np));
-    s.hist = reinterpret_cast<int*>(take(4 * radix_hist_ints((int)np)));
-    s.qcodes_a = reinterpret_cast<uint32_t*>(take(4 * (size_t)nq));
-    s.qcodes_b = reinterpret_cast<uint32_t*>(take(4 * (size_t)nq));
-    s.qids_a = reinterpret_cast<int*>(take(4 * (size_t)nq));
-    s.qids_b = reinterpret_cast<int*>(take(4 * (size_t)nq));
-    s.qhist = reinterpret_cast<int*>(take(4 * radix_hist_ints((int)nq)));
+    s.range = reinterpret_cast<int2*>(take(8 * (size_t)np));
+    s.chunks = reinterpret_cast<float4*>(take(32 * (size_t)((np + CHUNK - 1) / CHUNK)));
+    const size_t most = sort_together(np, nq) ? all : (size_t)(np > nq ? np : nq);
+    s.hist = reinterpret_cast<int*>(take(4 * radix_hist_ints((int)most)));
     s.bytes = o;
     return s;
 }
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) k_pt_bbox(const float* __restrict__ P, in
 }
 
 // The cube the Morton codes quantise: lower corner and 1/longest extent.
-__global__ void k_pt_cube(const int* __restrict__ bb, float4* __restrict__ cube) {
+__device__ void pt_cube(const int* bb, float4* __restrict__ cube) {
     float lo[3], ext = 0.f;
     for (int c = 0; c < 3; ++c) {
         lo[c] = bb[c] == INT_MAX ? 0.f : ordered_to_float(bb[c]);
@@ -116,27 +116,144 @@ __global__ void k_pt_cube(const int* __restrict__ bb, float4* __restrict__ cube)
     *cube = make_float4(lo[0], lo[1], lo[2], ext > 0.f && isfinite(ext) ? 1.0f / ext : 0.f);
 }
 
+__global__ void k_pt_cube(const int* __restrict__ bb, float4* __restrict__ cube) { pt_cube(bb, cube); }
+
+__global__ void __cluster_dims__(BBOX_BLOCKS, 1, 1) __launch_bounds__(BBOX_THREADS)
+    k_pt_cube_cluster(const float* __restrict__ P, int64_t n, float4* __restrict__ cube) {
+    __shared__ int box[6];
+    if (bbox_cluster<true>(P, n, box)) pt_cube(box, cube);
+}
+
 __device__ __forceinline__ uint32_t pt_code(const float* __restrict__ p, float4 cube) {
     return morton30((p[0] - cube.x) * cube.w, (p[1] - cube.y) * cube.w, (p[2] - cube.z) * cube.w);
 }
 
-__global__ void k_pt_morton(const float* __restrict__ P, int64_t n, const float4* __restrict__ cube,
-                            uint32_t* __restrict__ codes, int* __restrict__ ids) {
+// Codes of the points, and behind them of the queries.
+__global__ void k_pt_morton(const float* __restrict__ P, int64_t np, const float* __restrict__ Q, int64_t nq,
+                            const float4* __restrict__ cube, uint32_t* __restrict__ codes, int* __restrict__ ids) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    codes[i] = pt_code(P + 3 * i, *cube);
-    ids[i] = (int)i;
+    if (i >= np + nq) return;
+    const bool query = i >= np;
+    const int64_t j = query ? i - np : i;
+    codes[i] = pt_code(query ? Q + 3 * j : P + 3 * j, *cube) | (query ? QUERY : 0u);
+    ids[i] = (int)j;
 }
 
-// Leaf k's box is its point (NaN coordinates give an empty box, never nearest).
-__global__ void k_pt_leaves(const float* __restrict__ P, const int* __restrict__ order, int n,
-                            float4* __restrict__ boxes) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const float* p = P + 3 * (int64_t)order[k];
-    boxes[2 * (int64_t)k] = make_float4(p[0], p[1], p[2], 0.f);
-    boxes[2 * (int64_t)k + 1] = make_float4(p[0], p[1], p[2], 0.f);
+struct Box {
+    float3 lo, hi;
+    __device__ void none() { lo = make_float3(NAN, NAN, NAN); hi = lo; }
+    __device__ __forceinline__ void add(float3 l, float3 h) {
+        lo = make_float3(fminf(lo.x, l.x), fminf(lo.y, l.y), fminf(lo.z, l.z));
+        hi = make_float3(fmaxf(hi.x, h.x), fmaxf(hi.y, h.y), fmaxf(hi.z, h.z));
+    }
+    __device__ __forceinline__ void add(const float4* __restrict__ b) {  // (lo, hi) pair
+        const float4 l = __ldg(b), h = __ldg(b + 1);
+        add(make_float3(l.x, l.y, l.z), make_float3(h.x, h.y, h.z));
+    }
+    __device__ __forceinline__ void warp() {
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned F = 0xffffffffu;
+            const float3 l = make_float3(__shfl_xor_sync(F, lo.x, o), __shfl_xor_sync(F, lo.y, o), __shfl_xor_sync(F, lo.z, o));
+            const float3 h = make_float3(__shfl_xor_sync(F, hi.x, o), __shfl_xor_sync(F, hi.y, o), __shfl_xor_sync(F, hi.z, o));
+            add(l, h);
+        }
+    }
+};
+
+// Leaf k's box is its point (a NaN coordinate stays out of its ancestors'
+// boxes; such a point is never nearest).  Also the boxes of CHUNK leaves.
+__global__ void __launch_bounds__(CHUNK) k_pt_leaves(const float* __restrict__ P, const int* __restrict__ order, int n,
+                                                     float4* __restrict__ boxes, float4* __restrict__ chunks) {
+    __shared__ Box sh[CHUNK / 32];
+    const int k = blockIdx.x * CHUNK + threadIdx.x;
+    Box b;
+    b.none();
+    if (k < n) {
+        const float* p = P + 3 * (int64_t)order[k];
+        b.lo = b.hi = make_float3(p[0], p[1], p[2]);
+        boxes[2 * (int64_t)k] = make_float4(p[0], p[1], p[2], 0.f);
+        boxes[2 * (int64_t)k + 1] = make_float4(p[0], p[1], p[2], 0.f);
+    }
+    b.warp();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = b;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < CHUNK / 32; ++w) b.add(sh[w].lo, sh[w].hi);
+    chunks[2 * (int64_t)blockIdx.x] = make_float4(b.lo.x, b.lo.y, b.lo.z, 0.f);
+    chunks[2 * (int64_t)blockIdx.x + 1] = make_float4(b.hi.x, b.hi.y, b.hi.z, 0.f);
 }
+
+__device__ __forceinline__ void write_box(float4* nodes, int slot, const Box& b) {  // slot: 2 * node + side
+    float* r = reinterpret_cast<float*>(nodes + 4 * (int64_t)(slot >> 1) + 2 * (slot & 1));
+    r[0] = b.lo.x; r[1] = b.lo.y; r[2] = b.lo.z;
+    r[4] = b.hi.x; r[5] = b.hi.y; r[6] = b.hi.z;
+}
+
+// Every node's box, into its parent's record, from its leaves: a thread for up
+// to NB_SMALL of them, a warp for up to NB_WIDE, else the whole block, which
+// takes the chunks inside the node whole.  All nodes at once: climbing the tree
+// (k_refit) is a chain of its depth in atomics and fences, 43 us for 50k
+// points against 13.0 here.
+constexpr int NB_THREADS = 256, NB_SMALL = 16, NB_WIDE = 1024;
+__global__ void __launch_bounds__(NB_THREADS) k_pt_boxes(const float4* __restrict__ boxes,
+                                                         const float4* __restrict__ chunks, int n,
+                                                         const int2* __restrict__ range,
+                                                         const int* __restrict__ parent, float4* __restrict__ nodes) {
+    __shared__ int n_wide, wide[NB_THREADS];
+    __shared__ Box sh[NB_THREADS / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * NB_THREADS + threadIdx.x;
+    if (threadIdx.x == 0) n_wide = 0;
+    __syncthreads();
+    Box b;
+    b.none();
+    if (i < n) {  // leaf i
+        b.add(boxes + 2 * (int64_t)i);
+        write_box(nodes, parent[n - 1 + i], b);
+    }
+    int2 r = make_int2(0, -1);
+    if (i > 0 && i < n - 1) r = range[i];  // the root's box is nobody's
+    const int size = r.y - r.x + 1;
+    if (size > 0 && size <= NB_SMALL) {
+        b.none();
+#pragma unroll 4
+        for (int k = r.x; k <= r.y; ++k) b.add(boxes + 2 * (int64_t)k);
+        write_box(nodes, parent[i], b);
+    } else if (size > NB_WIDE) {
+        wide[atomicAdd(&n_wide, 1)] = i;
+    }
+    unsigned m = __ballot_sync(0xffffffffu, size > NB_SMALL && size <= NB_WIDE);
+    while (m) {
+        const int l = __ffs(m) - 1;
+        m &= m - 1;
+        const int first = __shfl_sync(0xffffffffu, r.x, l), last = __shfl_sync(0xffffffffu, r.y, l);
+        b.none();
+        for (int k = first + lane; k <= last; k += 32) b.add(boxes + 2 * (int64_t)k);
+        b.warp();
+        if (lane == l) write_box(nodes, parent[i], b);
+    }
+    __syncthreads();
+    const int cnt = n_wide;
+    for (int q = 0; q < cnt; ++q) {
+        const int node = wide[q];
+        r = range[node];
+        // leaves [r.x, c0 * CHUNK), chunks [c0, c1), leaves [c1 * CHUNK, r.y]
+        const int c0 = (r.x + CHUNK - 1) / CHUNK, c1 = (r.y + 1) / CHUNK;
+        b.none();
+        for (int k = r.x + threadIdx.x; k < c0 * CHUNK; k += NB_THREADS) b.add(boxes + 2 * (int64_t)k);
+        for (int k = c0 + threadIdx.x; k < c1; k += NB_THREADS) b.add(chunks + 2 * (int64_t)k);
+        for (int k = c1 * CHUNK + threadIdx.x; k <= r.y; k += NB_THREADS) b.add(boxes + 2 * (int64_t)k);
+        b.warp();
+        if (lane == 0) sh[w] = b;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < NB_THREADS / 32; ++k) b.add(sh[k].lo, sh[k].hi);
+            write_box(nodes, parent[node], b);
+        }
+        __syncthreads();
+    }
+}
+static_assert(NB_WIDE >= 2 * CHUNK, "a wide node holds a chunk");
 
 // Squared distance of two points, summed x, y, z in double with every product
 // and sum rounded on its own (no fused multiply-add): cKDTree's evaluation.
@@ -165,16 +282,63 @@ __device__ __forceinline__ void take(double d, int id, double& best, int& best_i
     }
 }
 
-// The boxes are culled in float: a box whose lower bound exceeds `lim` (the best
-// double distance, a relative 1e-7 up, rounded up to float) lies farther than
-// the best, by more than the double evaluation's rounding, so the result is
-// that of opening every box at or below the best in double.  Double arithmetic
-// (2 lanes a clock and SM) is left to the points that pass: about one in five
-// leaves.  (All boxes in double: 788 us for 50k queries over 50k points.)
-__global__ void __launch_bounds__(128) k_nn(const float4* __restrict__ nodes, const int* __restrict__ order,
-                                            const float* __restrict__ P, int np, const float* __restrict__ Q,
-                                            const int* __restrict__ qorder, int nq, int32_t* __restrict__ idx_out,
-                                            double* __restrict__ d2_out, int* __restrict__ status) {
+// A query's nearest point so far.  Distances are compared in float as long as
+// that decides: box_lb of a point is at most its double distance, and NN_UP times
+// it (plus NN_TINY, for what underflows) at least.  The points that may still be
+// nearest wait in a short list; only they are measured in double (2 lanes a
+// clock and SM), when the list is full and at the end: about one per query.
+constexpr int NN_LIST = 4;
+constexpr float NN_UP = 1.0f + 1e-6f, NN_TINY = 1e-37f;
+
+struct Nearest {
+    float lo = INFINITY;   // least lower bound in the list
+    float lim = INFINITY;  // upper bound of the nearest distance: what lies beyond is not opened
+    int n = 0;
+    int leaf[NN_LIST];     // sorted points
+
+    // The exact nearest of the list (and of `best`, `best_id` before it).
+    __device__ void resolve(const float4* __restrict__ boxes, const int* __restrict__ order, double qx, double qy,
+                            double qz, double& best, int& best_id) {
+        for (int k = 0; k < n; ++k) {
+            const float4 p = __ldg(boxes + 2 * (int64_t)leaf[k]);
+            take(pt_d2(qx, qy, qz, p.x, p.y, p.z), order[leaf[k]], best, best_id);
+        }
+        n = 0;
+    }
+    // A point whose lower bound d is not above lim.
+    __device__ __forceinline__ void add(int k, float d, const float4* __restrict__ boxes,
+                                        const int* __restrict__ order, double qx, double qy, double qz, double& best,
+                                        int& best_id) {
+        const float up = fmaf(d, NN_UP, NN_TINY);
+        if (up < lo) {  // nearer than everything before it
+            n = 0;
+            best = DBL_MAX;
+            best_id = -1;
+            lo = d;
+        }
+        lo = fminf(lo, d);
+        lim = fminf(lim, up);
+        if (n == NN_LIST) resolve(boxes, order, qx, qy, qz, best, best_id);
+        leaf[0] = n == 0 ? k : leaf[0];
+        leaf[1] = n == 1 ? k : leaf[1];
+        leaf[2] = n == 2 ? k : leaf[2];
+        leaf[3] = n == 3 ? k : leaf[3];
+        ++n;
+    }
+};
+static_assert(NN_LIST == 4, "add writes four entries");
+
+// One query a thread, queries in Morton order.  Measured: 50k queries over 50k
+// points 788 us with every box in double, 150 with every passing point in
+// double, 65.5 with the list.  A walk of the whole warp together, opening what
+// any of its queries needs, was slower at every size from 1k to 200k points and
+// queries (50k: by 120 us): neighbours in Morton order share little below
+// the upper levels.
+__global__ void __launch_bounds__(128) k_nn(const float4* __restrict__ nodes, const float4* __restrict__ boxes,
+                                            const int* __restrict__ order, const float* __restrict__ P, int np,
+                                            const float* __restrict__ Q, const int* __restrict__ qorder, int nq,
+                                            int32_t* __restrict__ idx_out, double* __restrict__ d2_out,
+                                            int* __restrict__ status) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nq) return;
     const int q = qorder[t];
@@ -191,14 +355,11 @@ __global__ void __launch_bounds__(128) k_nn(const float4* __restrict__ nodes, co
     if (np == 1) {
         take(pt_d2(qx, qy, qz, P[0], P[1], P[2]), 0, best, best_id);
     } else {
-        float lim = INFINITY;
-        // a leaf's box is its point
-        auto leaf = [&](int k, float4 at) {
-            const double d = pt_d2(qx, qy, qz, at.x, at.y, at.z);
-            if (d <= best) {
-                take(d, order[k], best, best_id);
-                lim = __double2float_ru(best * (1.0 + 1e-7));
-            }
+        Nearest near;
+        // a leaf's box is its point; one that is not finite is never nearest
+        auto leaf = [&](int k, float4 at, float d) {
+            if (d <= near.lim && isfinite(at.x) && isfinite(at.y) && isfinite(at.z))
+                near.add(k, d, boxes, order, qx, qy, qz, best, best_id);
         };
         int stack[NN_STACK];
         int sp = 0, node = 0;
@@ -214,9 +375,9 @@ __global__ void __launch_bounds__(128) k_nn(const float4* __restrict__ nodes, co
             const float dl = box_lb(fx, fy, fz, a, b), dr = box_lb(fx, fy, fz, c, d);
             // boxes at exactly the best distance are opened too: a lower index
             // may tie
-            if (L < 0 && dl <= lim) leaf(~L, a);
-            if (R < 0 && dr <= lim) leaf(~R, c);
-            const bool wl = L >= 0 && dl <= lim, wr = R >= 0 && dr <= lim;
+            if (L < 0) leaf(~L, a, dl);
+            if (R < 0) leaf(~R, c, dr);
+            const bool wl = L >= 0 && dl <= near.lim, wr = R >= 0 && dr <= near.lim;
             if (wl && wr) {
                 if (sp >= NN_STACK) {  // cannot happen for trees of depth <= 64
                     atomicOr(status, 2);
@@ -234,6 +395,7 @@ __global__ void __launch_bounds__(128) k_nn(const float4* __restrict__ nodes, co
                 node = stack[--sp];
             }
         }
+        near.resolve(boxes, order, qx, qy, qz, best, best_id);
     }
     if (best_id < 0) atomicOr(status, 8);  // every source coordinate non-finite
     idx_out[q] = best_id < 0 ? 0 : best_id;
@@ -422,28 +584,36 @@ extern "C" int mo_nn_query(const float* P, int64_t np, const float* Q, int64_t n
     do {
         cudaError_t e = cudaMemsetAsync(S.status, 0, 16, s);
         if (e != cudaSuccess) { rc = cuda_status(e, "memset"); break; }
-        k_pt_bbox_init<<<1, 32, 0, s>>>(S.bbox); ::mo::note_launch();
-        k_pt_bbox<<<std::min(ceil_div(np, 256), 4 * device_sm_count()), 256, 0, s>>>(P, np, S.bbox);
+        if (np <= BBOX_CLUSTER_MAX) {
+            k_pt_cube_cluster<<<BBOX_BLOCKS, BBOX_THREADS, 0, s>>>(P, np, S.cube); ::mo::note_launch();
+        } else {
+            k_pt_bbox_init<<<1, 32, 0, s>>>(S.bbox); ::mo::note_launch();
+            k_pt_bbox<<<std::min(ceil_div(np, 256), 4 * device_sm_count()), 256, 0, s>>>(P, np, S.bbox);
+            ::mo::note_launch();
+            k_pt_cube<<<1, 1, 0, s>>>(S.bbox, S.cube); ::mo::note_launch();
+        }
+        // the queries in Morton order of the same cube
+        k_pt_morton<<<ceil_div(np + nq, 256), 256, 0, s>>>(P, np, Q, nq, S.cube, S.codes_a, S.ids_a);
         ::mo::note_launch();
-        k_pt_cube<<<1, 1, 0, s>>>(S.bbox, S.cube); ::mo::note_launch();
-        k_pt_morton<<<ceil_div(np, 256), 256, 0, s>>>(P, np, S.cube, S.codes_a, S.ids_a); ::mo::note_launch();
-        e = radix_sort_pairs(S.codes_a, S.ids_a, S.codes_b, S.ids_b, (int)np, 30, S.hist, s);
-        if (e != cudaSuccess) { rc = cuda_status(e, "radix_sort_pairs"); break; }
-        // queries in Morton order of the same cube
-        k_pt_morton<<<ceil_div(nq, 256), 256, 0, s>>>(Q, nq, S.cube, S.qcodes_a, S.qids_a); ::mo::note_launch();
-        e = radix_sort_pairs(S.qcodes_a, S.qids_a, S.qcodes_b, S.qids_b, (int)nq, 30, S.qhist, s);
+        if (sort_together(np, nq)) {
+            e = radix_sort_pairs(S.codes_a, S.ids_a, S.codes_b, S.ids_b, (int)(np + nq), 31, S.hist, s);
+        } else {
+            e = radix_sort_pairs(S.codes_a, S.ids_a, S.codes_b, S.ids_b, (int)np, 30, S.hist, s);
+            if (e == cudaSuccess)
+                e = radix_sort_pairs(S.codes_a + np, S.ids_a + np, S.codes_b + np, S.ids_b + np, (int)nq, 30, S.hist, s);
+        }
         if (e != cudaSuccess) { rc = cuda_status(e, "radix_sort_pairs"); break; }
         if (np > 1) {
-            k_pt_leaves<<<ceil_div(np, 256), 256, 0, s>>>(P, S.ids_a, (int)np, S.boxes); ::mo::note_launch();
-            k_karras<<<ceil_div(np - 1, 256), 256, 0, s>>>(S.codes_a, (int)np, S.nodes, S.parent, S.flags,
-                                                           nullptr);
+            k_pt_leaves<<<ceil_div(np, CHUNK), CHUNK, 0, s>>>(P, S.ids_a, (int)np, S.boxes, S.chunks);
             ::mo::note_launch();
-            k_refit<<<ceil_div(np, 256), 256, 0, s>>>(S.boxes, (int)np, S.nodes, S.parent, S.flags, S.rootbox,
-                                                       S.status);
+            k_karras<<<ceil_div(np - 1, 256), 256, 0, s>>>(S.codes_a, (int)np, S.nodes, S.parent, S.flags, S.range);
+            ::mo::note_launch();
+            k_pt_boxes<<<ceil_div(np, NB_THREADS), NB_THREADS, 0, s>>>(S.boxes, S.chunks, (int)np, S.range, S.parent,
+                                                                       S.nodes);
             ::mo::note_launch();
         }
-        k_nn<<<ceil_div(nq, 128), 128, 0, s>>>(S.nodes, S.ids_a, P, (int)np, Q, S.qids_a, (int)nq, idx_out, d2_out,
-                                               S.status);
+        k_nn<<<ceil_div(nq, 128), 128, 0, s>>>(S.nodes, S.boxes, S.ids_a, P, (int)np, Q, S.ids_a + np, (int)nq, idx_out,
+                                               d2_out, S.status);
         ::mo::note_launch();
         e = cudaGetLastError();
         if (e != cudaSuccess) { rc = cuda_status(e, "nn kernels"); break; }
