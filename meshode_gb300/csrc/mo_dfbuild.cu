@@ -149,13 +149,14 @@ __device__ __forceinline__ float diff_prod(float a, float b, float c, float d) {
     return __fadd_rn(__fmaf_rn(a, b, -w), __fmaf_rn(-c, d, w));
 }
 
-// A triangle whose angle at a has a sine below 0.1 gets its normal from
+// A triangle whose angle at a has a sine below 0.01 gets its normal from
 // rounding-free products: the plain cross product is off by up to ~1e-7 / sine
 // in direction, and in a frame that is that far from orthonormal the distance
 // of a far point is wrong by as much (for an exactly repeated vertex the
 // contracted products leave a normal of any direction), below what the boxes
 // around the triangle bound, so the grid would depend on the visit order.
-constexpr float THIN2 = 0.01f;
+// Down to 0.01 the error stays inside the boxes' widening and the walk's slack.
+constexpr float THIN2 = 1e-4f;
 // |cross|^2 below which a thin triangle is measured by its segments: its
 // height is then below 1e-8, and the square loses digits.
 constexpr float THIN_NN = 1e-30f;
