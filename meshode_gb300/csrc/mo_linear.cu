@@ -403,12 +403,14 @@ struct CgArgs {
 };
 
 // All blocks of the (cooperative) grid; `target` grows by gridDim.x per call.
+// The release publishes the writes that the block's barrier put before it, the
+// acquire holds for the threads behind the second one.  (With a full fence beside
+// each an iteration took 23.6 us instead of 21.6.)
 // A wait of more than two seconds, or another block's, ends the solve: false.
 __device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned target) {
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         ok = 1;
         unsigned v, stop;
@@ -427,7 +429,6 @@ __device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned target) {
                 }
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return ok != 0;

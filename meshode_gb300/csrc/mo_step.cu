@@ -212,12 +212,12 @@ __global__ void __launch_bounds__(STEP_THREADS, 4) k_fused_step(const MoPair* __
 constexpr int RUN_REC = 12;  // records a thread keeps (a closed mesh's six neighbours twice); further ones are re-read
 constexpr int RUN_CHUNK = 4096;  // steps of a launch
 
+// The block's writes come before the release, by its barrier, and the release
+// publishes them all; run_wait's acquire, before its block's barrier, is as good
+// for every thread behind it.  (A full fence beside each cost 0.5 us a step.)
 __device__ __forceinline__ void run_arrive(unsigned* bar) {
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-    }
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
 }
 
 // Waits until every block has arrived `target` times in total; after two seconds
@@ -242,7 +242,6 @@ __device__ __forceinline__ bool run_wait(unsigned* bar, unsigned target) {
                 }
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return ok != 0;
@@ -255,9 +254,9 @@ __device__ __forceinline__ bool run_wait(unsigned* bar, unsigned target) {
 //   T = 1024, K = 1: one block, 64 registers, four neighbours at a time;
 //   T = 768, K = 2: one block, 80 registers, its offsets ~all of the shared
 //     memory.  (Three vertices a thread of 512 were slower: 10.3 us a step at
-//     200k vertices, each vertex's gathers waiting for the one's before.)
-// Measured, us a step (a launch per step, here): 10k 4.8, 3.6; 77k 5.6, 4.7;
-// 150k 8.3, 5.8; 200k 10.4, 8.7; 230k 11.8, 9.4.
+//     200k vertices against 8.7, each vertex's gathers waiting for the one's before.)
+// Measured, us a step (a launch per step, here): 10k 4.7, 2.65; 77k 5.6, 3.5;
+// 150k 8.3, 5.4; 200k 10.4, 7.9; 230k 11.8, 8.5.
 constexpr int RUN_WARPS1 = 32, RUN_WARPS2 = 24;
 template <bool WEIGHTED, bool LOSS, int K, int T>
 __global__ void __launch_bounds__(T, T == STEP_THREADS ? 2 : 1)
