@@ -248,20 +248,27 @@ __device__ __forceinline__ void tmem_ld8(uint32_t a, float (&v)[8]) {
         : "r"(a)
         : "memory");
 }
-// ... of four accumulators at distance d, added
-__device__ __forceinline__ void tmem_sum4(uint32_t a, uint32_t d, float* v) {
-    float p[8], q[8], r[8], s[8];
+// ... of two accumulators, added (all four in flight held 32 results, which k_tc_bwd
+// paid for: 95.6 us against 93.2)
+__device__ __forceinline__ void tmem_sum2(uint32_t a, uint32_t b, float (&v)[8]) {
+    float p[8], q[8];
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%32];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%33];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%34];\n"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%35];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%16];\n"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%17];\n"
         "tcgen05.wait::ld.sync.aligned;"
-        : MO_TC_R8(p), MO_TC_R8(q), MO_TC_R8(r), MO_TC_R8(s)
-        : "r"(a), "r"(a + d), "r"(a + 2 * d), "r"(a + 3 * d)
+        : MO_TC_R8(p), MO_TC_R8(q)
+        : "r"(a), "r"(b)
         : "memory");
 #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = (p[j] + q[j]) + (r[j] + s[j]);
+    for (int j = 0; j < 8; ++j) v[j] = p[j] + q[j];
+}
+// ... of four accumulators at distance d, added
+__device__ __forceinline__ void tmem_sum4(uint32_t a, uint32_t d, float* v) {
+    float s[8], t[8];
+    tmem_sum2(a, a + d, s);
+    tmem_sum2(a + 2 * d, a + 3 * d, t);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = s[j] + t[j];
 }
 
 // A block starts with 640 x 96 registers; the epilogue's four warpgroups take
