@@ -406,11 +406,11 @@ def df_roofline(specs, meshes, ids, tuner, sm_mhz):
 
 
 def df_brute_roofline(sm_mhz):
-    """The brute-force DF build (k_df_brute: every voxel against every
-    triangle, triangles staged through shared memory) on the ico-5 workload's
+    """The brute-force DF build (k_df_brute: every packet of voxels against
+    every triangle, 32 triangles bounded at a time) on the ico-5 workload's
     target (20,480 triangles) at 64^3, exact grid (no band): point-triangle
-    pair tests per second against the FP32 SIMT peak, beside the LBVH build
-    of the same grid (the method the library picks at this size)."""
+    pairs decided per second, beside the LBVH build of the same grid (the
+    method the library picks at this size)."""
     import ctypes
     from meshode_gb300 import _lib as L, meshgen
     from meshode_gb300._lib import call, ptr, stream_ptr
@@ -438,14 +438,11 @@ def df_brute_roofline(sm_mhz):
         grids[name] = grid
     tests = float(N ** 3) * Fd.shape[0]
     rate = tests / (out["brute_ms"] * 1e-3)
-    peak = 152 * 128 * 2 * sm_mhz * 1e6
-    out.update({"kernel": "k_df_brute", "N": N, "target_tris": int(Fd.shape[0]), "pair_tests": tests,
-                "pair_tests_per_s": rate, "fp32_flops_per_s": rate * TRI_FLOPS, "fp32_peak_flops_per_s": peak,
-                "fp32_frac": rate * TRI_FLOPS / peak,
+    out.update({"kernel": "k_df_brute", "N": N, "target_tris": int(Fd.shape[0]), "pairs": tests,
+                "pairs_per_s": rate, "sm_mhz": sm_mhz,
                 "grids_equal": bool(torch.equal(grids["brute"], grids["lbvh"])),
-                "note": "whole build timed (normalisation and triangle records included, < 1%%); FLOPs = tests x "
-                        "%d (a full test; the plane-distance cull makes most cheaper, so an upper bound)"
-                        % TRI_FLOPS})
+                "note": "whole build timed (normalisation and triangle records included, < 1%); most pairs are "
+                        "decided by the bounds of a packet of 64 voxels, so pairs are not FP32 work"})
     return out
 
 
@@ -803,13 +800,14 @@ def ode_config():
             "torch_autograd_ms_per_iteration": plain, "torch_autograd_peak_extra_mem_gb": plain_mem / 1e9,
             "tflops": flops / (ours * 1e-3) / 1e12,
             "fp32_peak_tflops": 152 * 128 * 2 * 2.07e9 / 1e12,
-            "kernels": "mo_mlp_fwd (fused 4-layer evaluation + RK4 update per 64-vertex tile), mo_mlp_bwd "
-                       "(fused vector-Jacobian product), mo_mlp_wgrad (split-K 256x256 weight gradients): "
-                       "FP32 SIMT with packed FFMA2, no library GEMM",
+            "kernels": "mo_mlp_tc_fwd (fused 4-layer evaluation + RK4 update per 128-vertex tile), mo_mlp_tc_bwd "
+                       "(fused vector-Jacobian product), mo_mlp_tc_wgrad (split-K 256x256 weight gradients): "
+                       "tcgen05 in FP16 pairs (three products each) with FP32 accuracy, no library GEMM",
             "note": "checkpointed adjoint: recomputes each RK4 step's activations (4/3 of the FLOPs) to hold "
                     "one step's activations instead of all 80 stage evaluations'; stored_activations: the same "
                     "fit keeping them (same gradients bit for bit); torch_autograd: the same fp32 model through "
-                    "torch (cuBLAS) autograd, every activation stored"}
+                    "torch (cuBLAS) autograd, every activation stored; tflops counts an FP32 product once (it takes "
+                    "three FP16 ones)"}
 
 
 # ---------------------------------------------------------------------------

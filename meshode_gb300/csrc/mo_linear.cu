@@ -31,9 +31,10 @@ namespace {
 
 constexpr int CG_ROWS = 341;      // vertices a block of the solver handles at a time, a thread per coordinate
 constexpr int CG_THREADS = 1024;  // one block per SM
-constexpr int CG_MIN_ROWS = 64;   // vertices a block should have before another block is used
+constexpr int CG_MIN_ROWS = 16;   // vertices a block should have before another block is used
 constexpr int CG_CHECK = 32;      // iterations between convergence checks
 constexpr int CG_MAX_BLOCKS = 512;
+constexpr int CG_ROW_BYTES = 160 * 1024;  // shared memory for a block's rows of the matrix
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -456,17 +457,43 @@ __device__ __forceinline__ void block_sum3(double v, double* sh, double* out) {
     __syncthreads();
 }
 
-// The totals of the blocks' partial sums (every block adds them in the same order).
-__device__ __forceinline__ void grid_sum3(const double* part, double* out) {
+// The block's sums of v per coordinate (as block_sum3's) into its place of part.
+__device__ __forceinline__ void store_partial(double v, double* sh, double* part) {
+    sh[threadIdx.x] = v;
+    __syncthreads();
     const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (c >= 3) return;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < (CG_ROWS + 31) / 32; ++k) {
+        const int row = lane + 32 * k;
+        if (row < CG_ROWS) s[k & 3] += sh[3 * row + c];
+    }
+    double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) part[3 * blockIdx.x + c] = t;
+}
+
+// The totals of the blocks' partial sums (every block adds them in the same
+// order): then(c, total) in one thread per coordinate, before all go on.
+template <class Then>
+__device__ __forceinline__ void grid_sum3(const double* part, Then then) {
+    constexpr int BATCH = 5;  // 160 blocks
+    const int c = threadIdx.x >> 5, lane = threadIdx.x & 31, n = (int)gridDim.x;
     if (c < 3) {
         double s = 0.0;
-#pragma unroll 4
-        for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(part + 3 * b + c);
+        for (int b0 = lane; b0 < n; b0 += 32 * BATCH) {
+            double v[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) v[j] = b0 + 32 * j < n ? __ldcg(part + 3 * (b0 + 32 * j) + c) : 0.0;
+            s += ((v[0] + v[1]) + (v[2] + v[3])) + v[4];
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) out[c] = s;
+        if (lane == 0) then(c, s);
     }
+    __syncthreads();
 }
 
 // Every iteration of the conjugate gradients in one cooperative launch.  (Before:
@@ -475,14 +502,25 @@ __device__ __forceinline__ void grid_sum3(const double* part, double* out) {
 // Three grid barriers an iteration:
 //   A p and p.Ap | alpha; x, r, z = r / diag and r.z | beta; p = z + beta p and
 //   its cell sums
+// (Sums that are their own barrier, every block polling every block's slot, were
+// slower: 24 us an iteration at 15k vertices; the polling fills L2.)
 // p is double-buffered, so the cell sums can be taken of z + beta p while the
 // vertices write it.  A block owns a contiguous range of vertices, a thread one
-// coordinate of a vertex; with at most CG_ROWS vertices (ONE) x and r stay in
-// registers.  Bound: the FP64 pipe (2 lanes a clock and SM) in A p, two
-// operations a neighbour and coordinate, and the latency of the barriers.
+// coordinate of a vertex; with at most CG_ROWS vertices (ONE) x, r, z and p stay in
+// registers, and the block's rows of the matrix in shared memory where they fit.
+// Bound: latency (a trip to L2 for the neighbours, one for the cells, three
+// barriers of ~2,500 clocks and two sums of ~5,000 in between), and from ~30k
+// vertices the FP64 pipe (2 lanes a clock and SM) in A p, two operations a
+// neighbour and coordinate.
+// Measured, us an iteration: 4k vertices 17.2, 15k 15.8, 41k 18.8 (20.5, 16.8, 20.2
+// with the rows read from L2, two more loads a vertex and chains of eleven
+// additions).  Eight lanes a cell instead of a warp: 41k 25; fewer than 16 vertices
+// a block were not tried, 64 took 5% longer at 2k to 8k.
 template <bool ONE>
 __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
-    __shared__ double sh[CG_THREADS];
+    extern __shared__ int4 rows[];  // ONE: this block's rows, if they fit
+    __shared__ double sh[CG_THREADS], sh2[CG_THREADS];
+    __shared__ int longest;
     __shared__ double sum[3], rz[3], bb[3], coef[3];
     __shared__ double rel_sh;
     const int64_t per = (A.nv + gridDim.x - 1) / gridDim.x;
@@ -493,7 +531,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
     double* PU = PA + 3 * CG_MAX_BLOCKS;
     double* PR = PU + 3 * CG_MAX_BLOCKS;
     unsigned target = 0;
-    double x = 0, r = 0, di = 0;  // ONE: this thread's vertex
+    double x = 0, r = 0, di = 0, z = 0, pv = 0;  // ONE: this thread's vertex
 
     // a vertex's neighbours and cell
     struct Row {
@@ -511,8 +549,22 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
         }
         return w;
     };
-    Row mine{};  // ONE
-    if (ONE && i0 < i1) mine = row_of(i0);
+    Row mine{};      // ONE
+    int stride = 1;  // of its entries
+    if (ONE) {
+        if (i0 < i1) mine = row_of(i0);
+        // entry k of the block's v-th vertex at rows[k * per + v]: no two of a warp's in a bank
+        if (tid == 0) longest = 0;
+        __syncthreads();
+        if (i0 < i1) atomicMax(&longest, mine.n);
+        __syncthreads();
+        if (longest * per <= CG_ROW_BYTES / (int64_t)sizeof(int4)) {
+            for (int k = c; k < mine.n; k += 3) rows[k * per + tid / 3] = mine.q[k];
+            mine.q = rows + tid / 3;
+            stride = (int)per;
+        }
+        __syncthreads();
+    }
     // coordinate c of A v for vertex i; v in rows of 4
     auto apply = [&](const double* v, int64_t i, double vi) {
         const Row w = ONE ? mine : row_of(i);
@@ -522,7 +574,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
         const int n = w.n;
 #pragma unroll 6
         for (int k = 0; k < n; ++k) {
-            const int4 e = __ldg(q + k);
+            const int4 e = ONE ? q[k * stride] : __ldg(q + k);
             y += __hiloint2double(e.w, e.z) * (vi - __ldcg(v + 4 * (int64_t)e.x + c));
         }
         y += w.w2 * cs;
@@ -556,11 +608,6 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
             if (lane == 0) A.cellsum[q] = s;
         }
     };
-    auto store_partial = [&](double* part, double v) {
-        block_sum3(v, sh, sum);
-        if (tid < 3) part[3 * blockIdx.x + tid] = sum[tid];
-    };
-
     // r = B - A x0 (B in r), z = r / diag, p = z
     double* p = A.p;
     double* pn = A.p + 4 * A.nv;
@@ -575,6 +622,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
             x = x0;
             r = rc;
             di = d;
+            pv = zc;
         } else {
             A.x[3 * i + c] = x0;
             A.r[3 * i + c] = rc;
@@ -585,11 +633,11 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
         sz += rc * zc;
         sb += b * b;
     }
-    store_partial(PU, sz);
-    store_partial(PR, sb);
+    store_partial(sz, sh, PU);
+    store_partial(sb, sh2, PR);
     if (!grid_sync(A.bar, target += gridDim.x)) return;
-    grid_sum3(PU, rz);
-    grid_sum3(PR, bb);
+    grid_sum3(PU, [&](int k, double v) { rz[k] = v; });
+    grid_sum3(PR, [&](int k, double v) { bb[k] = v; });
     if (A.ref) cells([&](int64_t j, int k) { return __ldcg(A.z + 4 * j + k); });
     if (!grid_sync(A.bar, target += gridDim.x)) return;
 
@@ -597,48 +645,48 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
     double rel = INFINITY;
     while (it < A.max_iter) {
         const bool check = (it + 1) % CG_CHECK == 0 || it + 1 == A.max_iter;
-        double y = 0, pi = 0, acc = 0.0;
+        double y = 0, acc = 0.0;
         for (int64_t i = i0; i < i1; i += CG_ROWS) {
-            pi = p[4 * i + c];
+            const double pi = ONE ? pv : p[4 * i + c];
             y = apply(p, i, pi);
             acc += pi * y;
             if (!ONE) pn[4 * i + c] = y;  // A p waits where the next p will be
         }
-        store_partial(PA, acc);
+        store_partial(acc, sh, PA);
         if (!grid_sync(A.bar, target += gridDim.x)) return;
-        grid_sum3(PA, sum);
-        if (tid < 96 && (tid & 31) == 0) coef[tid >> 5] = sum[tid >> 5] > 0.0 ? rz[tid >> 5] / sum[tid >> 5] : 0.0;
-        __syncthreads();
+        grid_sum3(PA, [&](int k, double v) { coef[k] = v > 0.0 ? rz[k] / v : 0.0; });
         const double alpha = coef[c];
         double s = 0.0, rr = 0.0;
         for (int64_t i = i0; i < i1; i += CG_ROWS) {
-            double rc, zc;
+            double rc;
             if (ONE) {
-                x += alpha * pi;
+                x += alpha * pv;
                 r -= alpha * y;
                 rc = r;
-                zc = rc * di;
+                z = rc * di;
             } else {
                 A.x[3 * i + c] += alpha * p[4 * i + c];
                 rc = A.r[3 * i + c] -= alpha * pn[4 * i + c];
-                zc = rc * A.dinv[3 * i + c];
+                z = rc * A.dinv[3 * i + c];
             }
-            A.z[4 * i + c] = zc;
-            s += rc * zc;
+            A.z[4 * i + c] = z;
+            s += rc * z;
             if (check) rr += rc * rc;
         }
-        store_partial(PU, s);
-        if (check) store_partial(PR, rr);
+        store_partial(s, sh, PU);
+        if (check) store_partial(rr, sh2, PR);
         if (!grid_sync(A.bar, target += gridDim.x)) return;
-        grid_sum3(PU, sum);
+        grid_sum3(PU, [&](int k, double v) {
+            coef[k] = rz[k] > 0.0 ? v / rz[k] : 0.0;
+            rz[k] = v;
+        });
         ++it;
         if (check) {
-            grid_sum3(PR, coef);
-            __syncthreads();
+            grid_sum3(PR, [&](int k, double v) { sum[k] = v; });
             if (tid == 0) {
                 double m = 0.0;
                 for (int k = 0; k < 3; ++k) {
-                    const double v = bb[k] > 0.0 ? sqrt(coef[k] / bb[k]) : sqrt(coef[k]);
+                    const double v = bb[k] > 0.0 ? sqrt(sum[k] / bb[k]) : sqrt(sum[k]);
                     if (m < v) m = v;
                 }
                 rel_sh = m;
@@ -647,14 +695,11 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
             rel = rel_sh;
             if (!(rel > A.tol)) break;
         }
-        if (tid < 96 && (tid & 31) == 0) {
-            const int k = tid >> 5;
-            coef[k] = rz[k] > 0.0 ? sum[k] / rz[k] : 0.0;
-            rz[k] = sum[k];
-        }
-        __syncthreads();
         const double beta = coef[c];
-        for (int64_t i = i0; i < i1; i += CG_ROWS) pn[4 * i + c] = fma(beta, p[4 * i + c], A.z[4 * i + c]);
+        for (int64_t i = i0; i < i1; i += CG_ROWS) {
+            if (ONE) pn[4 * i + c] = pv = fma(beta, pv, z);
+            else pn[4 * i + c] = fma(beta, p[4 * i + c], A.z[4 * i + c]);
+        }
         if (A.ref) {
             const double b0 = coef[0], b1 = coef[1], b2 = coef[2];
             cells([&](int64_t j, int k) {
@@ -808,8 +853,11 @@ int solve_on(float* V, int64_t nv, const int32_t* F, int64_t nf, const int32_t* 
                     S.x, S.r, S.dinv, S.z, S.p, S.cellsum, S.partial, S.result, S.bar, tol, max_iter};
         void* argv[] = {&args};
         const bool one = (nv + blocks - 1) / blocks <= CG_ROWS;
-        e = cudaLaunchCooperativeKernel(one ? (const void*)k_lin_cg<true> : (const void*)k_lin_cg<false>, dim3(blocks),
-                                        dim3(CG_THREADS), argv, 0, s);
+        const void* kernel = one ? (const void*)k_lin_cg<true> : (const void*)k_lin_cg<false>;
+        const int smem = one ? CG_ROW_BYTES : 0;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess)
+            e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(CG_THREADS), argv, smem, s);
         ::mo::note_launch();
         if (e != cudaSuccess) { fail(e, "k_lin_cg"); break; }
         double result[2];

@@ -34,3 +34,21 @@ def test_against_direct_solve(cuda, orc, n, cut, ncells):
     assert res <= 1e-13 and it > 0
     diag = float(np.linalg.norm(V.max(0) - V.min(0)))
     assert np.abs(X.cpu().numpy() - want).max() <= 1e-6 * diag
+
+
+def test_a_vertex_with_a_thousand_neighbours(cuda, orc):
+    """A block's rows that do not fit its shared memory."""
+    rng = np.random.Generator(np.random.PCG64(5))
+    n = 1500
+    V = rng.uniform(0.2, 0.8, (n, 3)).astype(np.float32)
+    k = np.arange(1, 1200)
+    F = np.stack([np.zeros_like(k), k, k + 1], 1).astype(np.int32)
+    ref = (np.arange(n) // 25).astype(np.int32)
+    G = np.stack([V[ref == g].mean(0) for g in range(ref.max() + 1)]).astype(np.float32)
+    E = np.stack([np.arange(8), np.arange(8) + 1201], 1).astype(np.int32)
+    want = orc.solve_linear(V, F, E, ref, G, 1.0, 0)
+    X = torch.from_numpy(V.copy()).cuda()
+    it, res = PD.SolveLinear(X, torch.from_numpy(F), torch.from_numpy(E), torch.from_numpy(ref), torch.from_numpy(G),
+                             1.0, 0)
+    assert res <= 1e-13 and it > 0
+    assert np.abs(X.cpu().numpy() - want).max() <= 1e-6 * float(np.linalg.norm(V.max(0) - V.min(0)))
