@@ -409,6 +409,9 @@ int mo_fused_step_on_demand(const MoPair* pairs, const MoTile* tiles, const int3
  * launch k of mo_fused_step leaves them for tiles of 8 slices.  sync: two words
  * of device memory.  A wait inside that runs out leaves NaN positions. */
 int mo_fused_run_fits(int64_t nv);
+/* Whether it fits and is the faster way for a pair whose longest row of records
+ * (mo_sell_plan) is max_rows. */
+int mo_fused_run_pays(int64_t nv, int max_rows);
 int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float* tile_loss, int64_t loss_stride,
                  uint32_t* sync, void* stream);
 /* pair_loss[k*npairs + p] (double) = sum, in a fixed order, of the tile

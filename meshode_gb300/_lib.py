@@ -130,6 +130,7 @@ _SIGS = {
     "mo_fused_step_weighted": (_I, [_P, _P, _P, _I, _I, _P, _I, _P]),
     "mo_fused_step_on_demand": (_I, [_P, _P, _P, _I, _I, _P, _I, _P]),
     "mo_fused_run_fits": (_I, [_I64]),
+    "mo_fused_run_pays": (_I, [_I64, _I]),
     "mo_fused_run": (_I, [_P, _I, _I, _P, _I64, _P, _P]),
     "mo_pair_loss": (_I, [_P, _I, _I, _I, _P, _P, _P]),
     "mo_abi_sizes": (_I, [ctypes.POINTER(_SZ), ctypes.POINTER(_SZ)]),

@@ -369,12 +369,42 @@ __global__ void __launch_bounds__(T, T == STEP_THREADS ? 2 : 1)
                 const int rows = rows_of(slice);
                 const int* __restrict__ rec = P.sell + P.slice_ptr[slice] + lane;
                 const float4 r0 = __ldg(R + i);
-                for (int row = RUN_REC; row < rows; ++row) {
-                    const int cu = __ldg(rec + row * 32);
-                    if (cu == -1) break;  // padding follows the last record
-                    const int n = cu & 0x7fffffff;
-                    const float4 s = __ldg(R + n);
-                    edge(cu, Vin[n], SUB(s.x, r0.x), SUB(s.y, r0.y), SUB(s.z, r0.z), row);
+                if (T == STEP_THREADS) {
+                    // a vertex of a CAD mesh can have hundreds: four at a time, their
+                    // numbers a round ahead (5,912 vertices with up to 60: 18.3 us a step
+                    // one after the other, 6.3 so, 10.7 with a launch per step)
+                    constexpr int MORE = 4;
+                    int cu[MORE];
+#pragma unroll
+                    for (int u = 0; u < MORE; ++u) cu[u] = RUN_REC + u < rows ? __ldg(rec + (RUN_REC + u) * 32) : -1;
+                    for (int row = RUN_REC; row < rows; row += MORE) {
+                        float4 q[MORE], s[MORE];
+#pragma unroll
+                        for (int u = 0; u < MORE; ++u) {
+                            const int n = cu[u] != -1 ? cu[u] & 0x7fffffff : i;
+                            q[u] = Vin[n];
+                            s[u] = __ldg(R + n);
+                        }
+                        int cn[MORE];
+#pragma unroll
+                        for (int u = 0; u < MORE; ++u)
+                            cn[u] = row + MORE + u < rows ? __ldg(rec + (row + MORE + u) * 32) : -1;
+#pragma unroll
+                        for (int u = 0; u < MORE; ++u)
+                            if (cu[u] != -1)
+                                edge(cu[u], q[u], SUB(s[u].x, r0.x), SUB(s[u].y, r0.y), SUB(s[u].z, r0.z), row + u);
+                        if (cu[MORE - 1] == -1) break;  // padding follows the last record
+#pragma unroll
+                        for (int u = 0; u < MORE; ++u) cu[u] = cn[u];
+                    }
+                } else {  // no registers for that: see mo_fused_run_pays
+                    for (int row = RUN_REC; row < rows; ++row) {
+                        const int cu = __ldg(rec + row * 32);
+                        if (cu == -1) break;  // padding follows the last record
+                        const int n = cu & 0x7fffffff;
+                        const float4 s = __ldg(R + n);
+                        edge(cu, Vin[n], SUB(s.x, r0.x), SUB(s.y, r0.y), SUB(s.z, r0.z), row);
+                    }
                 }
             }
             const float gx = MUL(gh, ADD(gd[j].x, MUL(grx, we)));
@@ -569,6 +599,17 @@ extern "C" int mo_fused_run_fits(int64_t nv) {
     int per_thread, warps, blocks;
     run_shape((int)((nv + 31) / 32), &per_thread, &warps, &blocks);
     return blocks > 0 ? 1 : 0;
+}
+
+// With more than 512 vertices an SM the records past the kept ones are read one
+// after the other, 0.26 us a step for each of the longest row: with nine of them
+// a launch per step is as fast (93k vertices with up to 60 records: 10.8 us against
+// 17.0; without long rows 6.7 against 4.5).
+extern "C" int mo_fused_run_pays(int64_t nv, int max_rows) {
+    if (nv <= 0 || nv > ((int64_t)1 << 30)) return 0;
+    int per_thread, warps, blocks;
+    run_shape((int)((nv + 31) / 32), &per_thread, &warps, &blocks);
+    return blocks > 0 && (warps <= TILE_WARPS || max_rows <= RUN_REC + 8) ? 1 : 0;
 }
 
 extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float* tile_loss, int64_t loss_stride,

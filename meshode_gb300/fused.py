@@ -168,6 +168,16 @@ class Pair:
         return p
 
 
+    def run_pays(self):
+        """Whether all steps in one launch (run) are the faster way."""
+        lib = L.lib()
+        if lib.mo_fused_run_pays(self.nv, 2 ** 31 - 1):
+            return True  # however long its rows
+        if not lib.mo_fused_run_pays(self.nv, 0):
+            return False
+        rows = int((self.slice_ptr[1:] - self.slice_ptr[:-1]).max().item()) // 32
+        return bool(lib.mo_fused_run_pays(self.nv, rows))
+
     def run(self, nsteps, record_loss=False):
         """The next nsteps steps in one launch (mo_fused_run); the per-step
         losses (float64 [nsteps]) or None."""
@@ -322,8 +332,8 @@ def fused_fit(pid, src_V_norm, steps, lr=1e-3, group_steps=25, use_graph=True, w
     cad_loss_layer.py:9-31, on the weighted step).  Returns
     (final normalised positions [nv,3] on the device, per-step losses or None)."""
     pr = pair_from_template(pid, src_V_norm, steps, lr=lr, w_edge=w_edge, mask_thresh=mask_thresh)
-    if pr.steps > 0 and L.lib().mo_fused_run_fits(pr.nv):
-        # every vertex has a thread on the chip: all steps in one launch
+    if pr.steps > 0 and pr.run_pays():
+        # every vertex stays on the chip: all steps in one launch
         losses = pr.run(pr.steps, record_loss)
         return pr.positions(), losses
     runner = StepGroupRunner(pr.device, 1, pr.ntiles, group_steps=group_steps, use_graph=use_graph,

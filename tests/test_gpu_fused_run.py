@@ -88,3 +88,30 @@ def test_largest_and_refused(target):
     c = _pairs(target, hi, "plain", L.MO_LAYOUT_CELL)[0]
     with pytest.raises(RuntimeError, match="do not fit"):
         c.run(1)
+
+
+def test_long_rows(target):
+    """Vertices with hundreds of records: the same bits as a launch per step, and
+    the rule that keeps large pairs with such rows on a launch per step."""
+    lib = L.lib()
+    assert lib.mo_fused_run_pays(5000, 10 ** 6) == 1 and lib.mo_fused_run_pays(77_824, 10 ** 6) == 1
+    assert lib.mo_fused_run_pays(77_825, 20) == 1 and lib.mo_fused_run_pays(77_825, 21) == 0
+    assert lib.mo_fused_run_pays(10 ** 7, 1) == 0 and lib.mo_fused_run_pays(0, 1) == 0
+    for nv, fan in ((700, 200), (90_000, 40)):
+        V, F = _mesh(nv, "plain")
+        k = np.arange(fan)
+        F = np.concatenate([F, np.stack([np.full(fan, 5), 10 + k, 11 + k], 1)]).astype(np.int32)
+        pid = PD.InitializeDeformTemplate(*target, 0, 32)
+        X = torch.from_numpy(V).cuda()
+        PD.NormalizeByTemplate(X, pid)
+        PD.StoreRigidityInformation(X, torch.from_numpy(F).cuda(), pid)
+        X = X + 0.01 * torch.sin(40 * X)
+        a, b = [fused.pair_from_template(pid, X, 9) for _ in range(2)]
+        assert b.run_pays() == (nv == 700)
+        runner = fused.StepGroupRunner(a.device, 1, a.ntiles, group_steps=9, use_graph=False)
+        runner.upload([a], [0])
+        runner.run_group()
+        a.t = 9
+        b.run(9)
+        assert torch.equal(a.positions(), b.positions())
+        PD.ReleaseTemplate(pid)
