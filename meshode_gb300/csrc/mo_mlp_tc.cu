@@ -23,7 +23,7 @@
 //   k_tc_pack   parameters -> operand images (the exact shared-memory layout:
 //               K-major rows of 64 halves, 128-byte swizzle), in the order
 //               the kernels stream them
-//   k_tc_fwd    one evaluation of 128-vertex tiles and the RK4 update
+//   k_tc_fwd    evaluations of 128-vertex tiles and the RK4 update: one, or a flow's
 //   k_tc_bwd    one vector-Jacobian product of 128-vertex tiles
 //   k_tc_wgrad  dW += G^T H over the rows of a step's four evaluations
 //   k_tc_reduce partial sums -> gradients, once per backward pass
@@ -280,9 +280,9 @@ __device__ __forceinline__ void regs_down() { asm volatile("setmaxnreg.dec.sync.
 
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
 
-// Programmatic dependent launch: the evaluations of a flow are a chain of
-// launches, and at a few thousand vertices a launch's start (tensor memory,
-// barriers, the first weights) is a third of its time.  A launch that says so
+// Programmatic dependent launch: an adjoint (and a flow whose blocks have one or
+// two tiles) is a chain of launches, and at a few thousand vertices a launch's
+// start (tensor memory, barriers, the first weights) is a third of its time.  A launch that says so
 // starts beside the one before it and waits here for its results; everything
 // but the packed weights, which no evaluation changes, is read and written
 // after the wait, and with plain loads (a non-coherent one may not see what
@@ -519,14 +519,15 @@ struct Block {
         fence_after();
     }
 
-    // Sums of the four column groups' values (group order), in group 0.
+    // Sums of the four column groups' values (group order), in group 0 or in ALL.
+    template <bool ALL = false>
     __device__ __forceinline__ void row_sums(float& v0, float& v1, float& v2, int g, int r) {
         float* x = reinterpret_cast<float*>(sm + C::ROWS);
         x[g * TILE + r] = v0;
         x[(4 + g) * TILE + r] = v1;
         x[(8 + g) * TILE + r] = v2;
         epi_sync();
-        if (g == 0) {
+        if (ALL || g == 0) {
             v0 = ((x[r] + x[TILE + r]) + x[2 * TILE + r]) + x[3 * TILE + r];
             v1 = ((x[4 * TILE + r] + x[5 * TILE + r]) + x[6 * TILE + r]) + x[7 * TILE + r];
             v2 = ((x[8 * TILE + r] + x[9 * TILE + r]) + x[10 * TILE + r]) + x[11 * TILE + r];
@@ -572,15 +573,21 @@ __device__ __forceinline__ void split8(const float* v, float sc, uint32_t* hi, u
 }
 
 // ---- evaluation ------------------------------------------------------------
+// One evaluation, or the 4 * steps of a flow.  A step's first evaluation reads the
+// state x + s*3n (u for the first of all), the others the one before's unext +
+// s*ustep + (k-1)*3n; the state after step s goes to next + s*3n, the last to accum.
 struct FwdArgs {
     const float *u, *x;
     int64_t n;
     unsigned char* pack;
-    float a, wgt;
+    float a, a2, wgt, wgt1;  // of evaluations 0 and 1, 2; 0 and 3, 1 and 2
     int init_acc;
     float *unext, *accum, *store;
     int64_t astride;
     int chained;  // the launch before it wrote none of the packed weights
+    int evals;
+    int64_t ustep;
+    float* next;
 };
 
 // k = f(u) of the tile's rows; unext = x + a*k, accum = (init ? x : accum) + wgt*k;
@@ -594,7 +601,16 @@ struct FwdArgs {
 // beside the first half's epilogue.  No more than 32 results are held in
 // registers at a time (64 spilled, and a spill goes to L2: shared memory leaves
 // 20 KB of L1).
-template <int W, bool STORE>
+//
+// A row's flow needs no other row, so a flow is one launch: a block takes its
+// tiles through evaluation after evaluation, and the next one's layer 1 runs
+// beside the last layers of this one across the evaluations too.  SERIAL: one
+// tile a block, whose next evaluation can only begin when this one's k is there;
+// the row's state stays in registers.  (A launch an evaluation before: 20 steps of
+// 200,003 vertices, W = 256: 14.1 ms, 13.6 here; 10 steps of 2,563 with their
+// gradient, W = 64: 869 us, 758 here; of 49,688, 20 steps with the adjoint: 22.4 and
+// 21.4 ms.)
+template <int W, bool STORE, bool SERIAL>
 __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
     using C = Cfg<W>;
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -603,12 +619,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
     if (!A.chained) chain_wait();  // the packed weights may be what is waited for
     B.init(smem, A.pack);
     const int tiles_all = (int)((A.n + TILE - 1) / TILE);
-    const int tiles = (tiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int tiles = SERIAL ? 1 : (tiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int items = tiles * A.evals;  // evaluation by evaluation
     const int w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (w >= EPI / 32) {
         regs_down();
-        if (w == EPI / 32 && lane == 0) B.produce(A.pack, A.pack + C::IMAGE, tiles);
-        if (w == EPI / 32 + 1) B.issue(tiles);
+        if (w == EPI / 32 && lane == 0) B.produce(A.pack, A.pack + C::IMAGE, items);
+        if (w == EPI / 32 + 1) B.issue(items);
         __syncwarp();
     } else {
         regs_up();
@@ -622,6 +639,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
 
         uint32_t hi[G8][4], lo[G8][4];  // the first half of layer 1 of the next tile
         float inv1 = 0.f, hb1 = 0.f, sc1 = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+        float sx[3] = {0.f, 0.f, 0.f}, sa[3] = {0.f, 0.f, 0.f};  // SERIAL: the row's state, its next one
+        // an item's evaluation and tile; its place in the store (a step's three
+        // layers have four evaluations each)
+        auto eval_of = [&](int i) { return SERIAL ? i : i / tiles; };
+        auto tile_of = [&](int i, int e) { return (int)blockIdx.x + (i - e * tiles) * (int)gridDim.x; };
+        auto place = [&](int i) {
+            if (!STORE) return 0;
+            const int e = eval_of(i);
+            return (12 * (e >> 2) + (e & 3)) * tiles_all + tile_of(i, e);
+        };
         auto at8 = [&](int tile, int c) { return (((int64_t)tile * (W / 8) + c / 8) * TILE + r) * 8; };
         auto keep = [&](int l, int tile, int c, const float* v) {  // the training pass keeps every layer
             if (STORE) {
@@ -630,13 +657,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
             }
         };
         // A row's layer-1 activations are below |W1|_1 |u|_inf + max b1 + ln 2.
-        auto begin1 = [&](int tile) {
-            const int64_t row = (int64_t)tile * TILE + r;
-            ux = uy = uz = 0.f;
-            if (row < A.n) {
-                ux = A.u[3 * row];
-                uy = A.u[3 * row + 1];
-                uz = A.u[3 * row + 2];
+        auto begin1 = [&](int item) {
+            if (!SERIAL || item == 0) {
+                const int e = eval_of(item), k = e & 3;
+                const int64_t row = (int64_t)tile_of(item, e) * TILE + r, s3n = (int64_t)(e >> 2) * 3 * A.n;
+                const float* u = e == 0   ? A.u
+                                 : k == 0 ? A.x + s3n
+                                          : A.unext + (e >> 2) * A.ustep + (k - 1) * 3 * A.n;
+                ux = uy = uz = 0.f;
+                if (row < A.n) {
+                    ux = u[3 * row];
+                    uy = u[3 * row + 1];
+                    uz = u[3 * row + 2];
+                }
+                if (SERIAL) {
+                    sx[0] = ux;
+                    sx[1] = uy;
+                    sx[2] = uz;
+                }
             }
             hb1 = fmaf(__ldg(misc + M_N1), fmaxf(fmaxf(fabsf(ux), fabsf(uy)), fabsf(uz)), __ldg(misc + M_MB1)) + 0.7f;
             hm1 = fmaxf(hm1, hb1);
@@ -683,20 +721,41 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
             keep(2, tile, c, v);
         };
         // k and the RK4 update
-        auto finish = [&](int tile) {
-            const int64_t row = (int64_t)tile * TILE + r;
+        auto finish = [&](int item) {
+            const int e = eval_of(item), k = e & 3;
+            const int64_t row = (int64_t)tile_of(item, e) * TILE + r, s3n = (int64_t)(e >> 2) * 3 * A.n;
             float k0 = p0.x + p0.y, k1 = p1.x + p1.y, k2 = p2.x + p2.y;
-            B.row_sums(k0, k1, k2, g, r);
-            if (g == 0 && row < A.n) {
-                const float kv[3] = {k0 + __ldg(misc + M_B4), k1 + __ldg(misc + M_B4 + 1), k2 + __ldg(misc + M_B4 + 2)};
-                const bool late = *B.late != 0;
+            B.template row_sums<SERIAL>(k0, k1, k2, g, r);
+            if ((!SERIAL && g > 0) || row >= A.n) return;
+            const float kv[3] = {k0 + __ldg(misc + M_B4), k1 + __ldg(misc + M_B4 + 1), k2 + __ldg(misc + M_B4 + 2)};
+            const bool late = *B.late != 0;
+            const float* x = A.x + s3n;
+            float* unext = k < 3 && A.unext ? A.unext + (e >> 2) * A.ustep + k * 3 * A.n : nullptr;
+            float* accum = (e | 3) + 1 < A.evals ? A.next + s3n : A.accum;
+            const float a = k == 2 ? A.a2 : A.a, wgt = k == 1 || k == 2 ? A.wgt1 : A.wgt;
+            const bool init = k == 0 && A.init_acc;
+            float un[3];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const int64_t q = 3 * row + d;
-                    const float k = late ? NAN : kv[d];
-                    if (A.unext) A.unext[q] = fmaf(A.a, k, A.x[q]);
-                    A.accum[q] = fmaf(A.wgt, k, A.init_acc ? A.x[q] : A.accum[q]);
+            for (int d = 0; d < 3; ++d) {
+                const int64_t q = 3 * row + d;
+                const float kd = late ? NAN : kv[d];
+                if (SERIAL) {
+                    un[d] = fmaf(a, kd, sx[d]);
+                    sa[d] = fmaf(wgt, kd, k == 0 ? sx[d] : sa[d]);
+                    if (k == 3) un[d] = sx[d] = sa[d];
+                    if (g == 0) {
+                        if (k < 3) unext[q] = un[d];
+                        else accum[q] = sa[d];
+                    }
+                } else {
+                    if (unext) unext[q] = fmaf(a, kd, x[q]);
+                    accum[q] = fmaf(wgt, kd, init ? x[q] : accum[q]);
                 }
+            }
+            if (SERIAL) {
+                ux = un[0];
+                uy = un[1];
+                uz = un[2];
             }
         };
         // the accumulators of the half that is ready
@@ -706,18 +765,34 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
             for (int i = 0; i < G8; ++i) tmem_sum4(lane_base + 8 * i, C::NS, v + 8 * i);
         };
 
-        begin1(blockIdx.x);
+        begin1(0);
 #pragma unroll
-        for (int i = 0; i < G8; ++i) layer1(blockIdx.x, c0 + 8 * i, hi[i], lo[i]);
+        for (int i = 0; i < G8; ++i) layer1(place(0), c0 + 8 * i, hi[i], lo[i]);
         float f3 = 0.f;
-        for (int t = 0; t <= tiles; ++t) {
-            const int tile = blockIdx.x + t * gridDim.x, prev = tile - gridDim.x;
+        for (int t = 0; t <= items; ++t) {
+            const int tile = place(t);
             constexpr int c1 = (NH - 1) * C::NS;  // the second half's first column
-            const float f2_ = inv1 * inv2, hb = hb1;
+            float f2_, hb;
             {
                 float z[HC];
-                if (t > 0) take(z);  // layer 3 of the previous tile is done: the images are free
-                if (t < tiles) {
+                if (t > 0) take(z);  // layer 3 of the previous item is done: the images are free
+                auto last = [&]() {
+                    const int prev = place(t - 1);
+                    if (NH == 1) p0 = p1 = p2 = f2(0.f);
+#pragma unroll
+                    for (int i = 0; i < G8; ++i) layer3(prev, c1 + c0 + 8 * i, z + 8 * i, f3);
+                    finish(t - 1);
+                };
+                if (SERIAL && t > 0) {
+                    last();
+                    if (t == items) break;
+                    begin1(t);
+#pragma unroll
+                    for (int i = 0; i < G8; ++i) layer1(tile, c0 + 8 * i, hi[i], lo[i]);
+                }
+                f2_ = inv1 * inv2;
+                hb = hb1;
+                if (t < items) {
 #pragma unroll
                     for (int i = 0; i < G8; ++i) B.put8(r, c0 + 8 * i, hi[i], lo[i]);
                     if (NH == 2) {
@@ -730,14 +805,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
                     }
                     B.publish();
                 }
-                if (t > 0) {
-                    if (NH == 1) p0 = p1 = p2 = f2(0.f);
-#pragma unroll
-                    for (int i = 0; i < G8; ++i) layer3(prev, c1 + c0 + 8 * i, z + 8 * i, f3);
-                    finish(prev);
-                }
+                if (!SERIAL && t > 0) last();
             }
-            if (t == tiles) break;
+            if (t == items) break;
             // layer 2: activations below sum(W2+) max h1 + max b2 + ln 2
             const float hb2 = fmaf(__ldg(misc + M_N2), hb, __ldg(misc + M_MB2)) + 0.7f;
             hm2 = fmaxf(hm2, hb2);
@@ -773,10 +843,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
                 B.put8(r, c, h4, l4);
             }
             B.publish();
-            if (t + 1 < tiles) {
-                begin1(tile + gridDim.x);
+            if (!SERIAL && t + 1 < items) {
+                // its input is at least `tiles` items old, and between two items
+                // every thread has met the others (row_sums) unless there are two
+                if (tiles == 2) epi_sync();
+                const int then = place(t + 1);
+                begin1(t + 1);
 #pragma unroll
-                for (int i = 0; i < G8; ++i) layer1(tile + gridDim.x, c0 + 8 * i, hi[i], lo[i]);
+                for (int i = 0; i < G8; ++i) layer1(then, c0 + 8 * i, hi[i], lo[i]);
             }
             if (NH == 2) {
                 float z[HC];
@@ -1368,8 +1442,10 @@ __global__ void __launch_bounds__(32 * RED_PARTS) k_tc_reduce(ReduceArgs A) {
 
 template <int W>
 int set_attrs() {
-    MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
-    MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
+    MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
+    MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
+    MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
+    MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
     MO_CUDA(cudaFuncSetAttribute(k_tc_bwd<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
     MO_CUDA(cudaFuncSetAttribute(k_tc_wgrad<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, WCfg<W>::SMEM));
     return MO_OK;
@@ -1460,9 +1536,9 @@ static int issue_fwd(const float* u, const float* x, int64_t n, void* pack, int 
     MO_CHECK_ARG(aligned(pack, 128), "the packed parameters must be 128-byte aligned");
     MO_CHECK_ARG(!store || (aligned(store, 32) && astride >= mo_mlp_tc_rows(n) * W_ && astride % 8 == 0),
                  "store must be 32-byte aligned with an array stride of at least the padded rows times the width");
-    const FwdArgs A{u, x, n, reinterpret_cast<unsigned char*>(pack), a, w, init_acc, unext, acc, store, astride,
-                    chained};
-    TC_WIDTH(W_, TC_LAUNCH(store ? k_tc_fwd<W, true> : k_tc_fwd<W, false>, blocks_for(n), THREADS, Cfg<W>::SMEM, stream,
+    const FwdArgs A{u,     x,   n,     reinterpret_cast<unsigned char*>(pack), a, 0.f, w, 0.f, init_acc,
+                    unext, acc, store, astride, chained, 1, 0, nullptr};
+    TC_WIDTH(W_, TC_LAUNCH(store ? k_tc_fwd<W, true, false> : k_tc_fwd<W, false, false>, blocks_for(n), THREADS, Cfg<W>::SMEM, stream,
                            chained, A));
     ::mo::note_launch();
     return MO_OK;
@@ -1556,10 +1632,41 @@ namespace {
 constexpr int64_t FLOW_ALIGN = 32;  // floats
 int64_t flow_pad(int64_t floats) { return (floats + FLOW_ALIGN - 1) / FLOW_ALIGN * FLOW_ALIGN; }
 
+// The steps of a flow that one launch takes, or 0: a launch an evaluation.  Where
+// some blocks have two tiles and others one, the ones would wait for their k while
+// the twos need not.  FLOW_ITEMS keeps a launch below 20 ms (17 us a tile and
+// evaluation at W = 256).
+constexpr int64_t FLOW_ITEMS = 1024;
+int flow_launch_steps(int64_t n, int steps) {
+    const int64_t tiles = tiles_of(n), sms = device_sm_count();
+    if (tiles > sms && tiles < 2 * sms) return 0;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(steps, FLOW_ITEMS / (4 * ((tiles + sms - 1) / sms))));
+}
+
+// `steps` RK4 steps of states ckpt [steps][n][3], the last one to out, with the
+// stage inputs in u ([3][n][3] every ustep floats); act: a step's four evaluations'
+// H1, H2, H3 ([3][4][rows][W]), one step after the other, or NULL.
+int flow_launch(float* ckpt, int64_t n, int steps, void* pack, int W_, double h, float* u, int64_t ustep, float* act,
+                float* out, void* stream, bool chained) {
+    MO_CHECK_ARG(aligned(pack, 128), "the packed parameters must be 128-byte aligned");
+    MO_CHECK_ARG(!act || aligned(act, 32), "the activations must be 32-byte aligned");
+    const FwdArgs A{ckpt, ckpt, n, reinterpret_cast<unsigned char*>(pack), (float)(h / 2), (float)h, (float)(h / 6),
+                    (float)(h / 3), 1, u, out, act, 4 * mo_mlp_tc_rows(n) * W_, chained, 4 * steps, ustep,
+                    ckpt + 3 * n};
+    const bool serial = tiles_of(n) <= device_sm_count();
+    TC_WIDTH(W_, TC_LAUNCH(act ? (serial ? k_tc_fwd<W, true, true> : k_tc_fwd<W, true, false>)
+                               : (serial ? k_tc_fwd<W, false, true> : k_tc_fwd<W, false, false>),
+                           blocks_for(n), THREADS, Cfg<W>::SMEM, stream, chained, A));
+    ::mo::note_launch();
+    return MO_OK;
+}
+
 // x_next = RK4(x) with the stage inputs in u [3][n][3]; act: the four
 // evaluations' H1, H2, H3 ([3][4][rows][W]) or NULL.
 int flow_step(const float* x, int64_t n, void* pack, int W, double h, float* u, float* act, float* x_next,
               void* stream, bool chained) {
+    if (flow_launch_steps(n, 1))
+        return flow_launch(const_cast<float*>(x), n, 1, pack, W, h, u, 0, act, x_next, stream, chained);
     const int64_t size = mo_mlp_tc_rows(n) * W;
     const float a[4] = {(float)(h / 2), (float)(h / 2), (float)h, 0.f};
     const float w[4] = {(float)(h / 6), (float)(h / 3), (float)(h / 3), (float)(h / 6)};
@@ -1594,6 +1701,15 @@ extern "C" int mo_ode_flow(const float* x0, int64_t n, int steps, void* pack, in
     MO_CHECK_ARG(x0 && pack && ckpt && u && out, "null pointer");
     MO_CUDA(cudaMemcpyAsync(ckpt, x0, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, as_stream(stream)));
     const double h = 1.0 / steps;
+    if (const int some = flow_launch_steps(n, steps)) {
+        for (int k = 0; k < steps && !rc; k += some) {
+            const int m = std::min(some, steps - k);
+            rc = flow_launch(ckpt + 3 * n * k, n, m, pack, W, h, act ? u + 9 * n * k : u, act ? 9 * n : 0,
+                             act ? act + mo_ode_act_floats(n, W) * k : nullptr,
+                             k + m < steps ? ckpt + 3 * n * (k + m) : out, stream, k > 0);
+        }
+        return rc;
+    }
     for (int k = 0; k < steps; ++k) {
         rc = flow_step(ckpt + 3 * n * k, n, pack, W, h, act ? u + 9 * n * k : u,
                        act ? act + mo_ode_act_floats(n, W) * k : nullptr, k + 1 < steps ? ckpt + 3 * n * (k + 1) : out,
