@@ -24,7 +24,7 @@
 //               K-major rows of 64 halves, 128-byte swizzle), in the order
 //               the kernels stream them
 //   k_tc_fwd    evaluations of 128-vertex tiles and the RK4 update: one, or a flow's
-//   k_tc_bwd    one vector-Jacobian product of 128-vertex tiles
+//   k_tc_bwd    vector-Jacobian products of 128-vertex tiles: one, or a step's four
 //   k_tc_wgrad  dW += G^T H over the rows of a step's four evaluations
 //   k_tc_reduce partial sums -> gradients, once per backward pass
 //
@@ -33,6 +33,8 @@
 // so a warp whose lanes are rows moves 1 KB of consecutive bytes per access.
 // Every wait is bounded in time; one that runs out leaves NaN in the outputs.
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "mo_common.cuh"
 
@@ -889,6 +891,15 @@ struct BwdArgs {
     int chained;
 };
 
+// A step's four products, last evaluation first: product j has the arrays of
+// evaluation 3 - j, the inputs u - j*3n (x for the last), the weights ca or ca1 and
+// cg, cg1 or cg2, the product before's dx_out and gradient.  (A type of its own: with
+// these fields the other kernel spilled 172 bytes a thread instead of 104.)
+struct StepArgs : BwdArgs {
+    float ca1, cg1, cg2;
+    const float* x;
+};
+
 // The last layer's gate, two layers back through the tensor cores, and the
 // column sums of the small gradients: dW4 from H3 read by column while the
 // first MMAs run, dW1 and db1 from the tile of g_z1, laid out as FP32 in the
@@ -901,8 +912,13 @@ struct BwdArgs {
 // summed eight by four rows a warp: 105 -> 95.6 us, width 64 at 2,563 rows 12.6 ->
 // 11.0.  A prefetch of them to L2, a tile or a layer ahead, was no faster or
 // slower (117 us); dW4 by shared memory instead of L2 134 against 113.
-template <int W>
-__global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
+//
+// STEP: a step's four products, for one tile a block, whose row keeps its gradient in
+// registers (10 steps of 2,563 rows with their flow, W = 64: 758 -> 703 us).  With more
+// tiles a block the same launch was slower than four (W = 256, 49,688 rows: 22.1 ms
+// against 21.4: 304 bytes of spills a thread against 104).
+template <int W, bool STEP>
+__global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(std::conditional_t<STEP, StepArgs, BwdArgs> A) {
     using C = Cfg<W>;
     extern __shared__ __align__(1024) unsigned char smem[];
     Block<W> B;
@@ -910,12 +926,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
     if (!A.chained) chain_wait();  // the packed weights may be what is waited for
     B.init(smem, A.pack);
     const int tiles_all = (int)((A.n + TILE - 1) / TILE);
-    const int tiles = (tiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int tiles = STEP ? 1 : (tiles_all - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int items = STEP ? 4 : tiles;
     const int w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (w >= EPI / 32) {
         regs_down();
-        if (w == EPI / 32 && lane == 0) B.produce(A.pack + 3 * C::IMAGE, A.pack + 2 * C::IMAGE, tiles);
-        if (w == EPI / 32 + 1) B.issue(tiles);
+        if (w == EPI / 32 && lane == 0) B.produce(A.pack + 3 * C::IMAGE, A.pack + 2 * C::IMAGE, items);
+        if (w == EPI / 32 + 1) B.issue(items);
         __syncwarp();
     } else {
         regs_up();
@@ -931,7 +948,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
         // row, so a warp's access is 128 consecutive bytes of a block.
         constexpr int SB = C::SUM_BLOCKS, PART_ROWS = TILE / C::SUM_PARTS;
         const int blk = w % (W / 8), row0 = w / (W / 8) % C::SUM_PARTS * PART_ROWS, cl = lane & 7, rl = lane >> 3;
-        float s4[SB][3] = {}, s1[SB][4] = {}, sg[3] = {0.f, 0.f, 0.f};
         float gm2 = 0.f, gm3 = 0.f;  // bounds of the gradients seen
         auto at8 = [&](int tile, int c) { return (((int64_t)tile * (W / 8) + c / 8) * TILE + r) * 8; };
         // FP32 tile in shared memory, 16-byte chunks swizzled by the row
@@ -960,7 +976,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
         auto ask = [&](int l, int tile, int half, int i) {
             ldg8(A.store + l * A.astride + at8(tile, half * C::NS + c0 + 8 * i), x + 8 * i);
         };
-        float ga[3], gp[3];  // the next tile's a and gprev
+        float ga[3], gp[3];  // the next item's a and gprev
         auto ask_row = [&](int tile) {
             const int64_t row = (int64_t)tile * TILE + r;
 #pragma unroll
@@ -972,202 +988,225 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(BwdArgs A) {
         ask_row(blockIdx.x);
 #pragma unroll
         for (int i = 0; i < G8; ++i) ask(2, blockIdx.x, 0, i);
-        for (int t = 0; t < tiles; ++t) {
-            const int tile = blockIdx.x + t * gridDim.x;
-            const int64_t row = (int64_t)tile * TILE + r;
-            float gd[3];
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                gd[d] = A.ca * ga[d];
-                if (A.gprev) gd[d] = fmaf(A.cg, gp[d], gd[d]);
-            }
-            if (g == 0) {
+        for (int j = 0; j < (STEP ? 4 : 1); ++j) {
+            float s4[SB][3] = {}, s1[SB][4] = {}, sg[3] = {0.f, 0.f, 0.f};
+            for (int t = 0; t < tiles; ++t) {
+                // the tile's place in the arrays of the evaluations, and the next item's
+                const int tile = STEP ? (int)blockIdx.x - j * tiles_all : (int)blockIdx.x + t * (int)gridDim.x;
+                const int then = STEP ? tile - tiles_all : tile + (int)gridDim.x;
+                const bool more = STEP ? j < 3 : t + 1 < tiles;
+                const int64_t row = (int64_t)(STEP ? (int)blockIdx.x : tile) * TILE + r;
+                float gd[3];
+                float ca = A.ca, cg = A.cg;
+                if constexpr (STEP) {
+                    if (j == 1 || j == 2) ca = A.ca1;
+                    if (j > 0) cg = j == 1 ? A.cg1 : A.cg2;
+                }
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    rows[d * TILE + r] = gd[d];
-                    sg[d] += gd[d];
+                    gd[d] = ca * ga[d];
+                    if ((STEP && j > 0) || A.gprev) gd[d] = fmaf(cg, gp[d], gd[d]);
                 }
-            }
-            // g_z3 = (g W4) * softplus'(z3), below |g|_1 max |W4|; g_z2 below that times |W3^T|_1
-            const float gb3 = (fabsf(gd[0]) + fabsf(gd[1]) + fabsf(gd[2])) * __ldg(misc + M_M4);
-            const float gb2 = gb3 * __ldg(misc + M_N3);
-            gm3 = fmaxf(gm3, gb3);
-            gm2 = fmaxf(gm2, gb2);
-            float inv_3, inv_2;
-            const float sc3 = pow2_scale(gb3, &inv_3), sc2 = pow2_scale(gb2, &inv_2);
+                if (g == 0) {
 #pragma unroll
-            for (int h = 0; h < NH; ++h)
-#pragma unroll
-                for (int i = 0; i < G8; ++i) {
-                    const int c = h * C::NS + c0 + 8 * i;
-                    float v[8];
-                    uint32_t h4[4], l4[4];
-#pragma unroll
-                    for (int j = 0; j < 8; j += 4) {
-                        const float4 wx = ld4(B.vec(V_W4X, c + j)), wy = ld4(B.vec(V_W4Y, c + j));
-                        const float4 wz = ld4(B.vec(V_W4Z, c + j));
-                        const float2 p = __ffma2_rn(f2(gd[2]), xy(wz),
-                                                    __ffma2_rn(f2(gd[1]), xy(wy), __fmul2_rn(f2(gd[0]), xy(wx))));
-                        const float2 q = __ffma2_rn(f2(gd[2]), zw(wz),
-                                                    __ffma2_rn(f2(gd[1]), zw(wy), __fmul2_rn(f2(gd[0]), zw(wx))));
-                        v[j] = p.x; v[j + 1] = p.y; v[j + 2] = q.x; v[j + 3] = q.y;
+                    for (int d = 0; d < 3; ++d) {
+                        rows[d * TILE + r] = gd[d];
+                        sg[d] += gd[d];
                     }
-                    gate8(v, x + 8 * i, 1.0f);
-                    if (h + 1 < NH) ask(2, tile, h + 1, i);
-                    else ask(1, tile, 0, i);
-                    stg8(A.gz3 + at8(tile, c), v);
-                    split8(v, sc3, h4, l4);
-                    B.put8(r, c, h4, l4);
                 }
-            B.publish();
-            epi_sync();
-            {   // dW4 += g^T H3, from L2 (beside the first MMAs)
-                const float* H3 = A.store + 2 * A.astride + ((int64_t)tile * (W / 8) + blk) * TILE * 8 + cl;
+                // g_z3 = (g W4) * softplus'(z3), below |g|_1 max |W4|; g_z2 below that times |W3^T|_1
+                const float gb3 = (fabsf(gd[0]) + fabsf(gd[1]) + fabsf(gd[2])) * __ldg(misc + M_M4);
+                const float gb2 = gb3 * __ldg(misc + M_N3);
+                gm3 = fmaxf(gm3, gb3);
+                gm2 = fmaxf(gm2, gb2);
+                float inv_3, inv_2;
+                const float sc3 = pow2_scale(gb3, &inv_3), sc2 = pow2_scale(gb2, &inv_2);
+#pragma unroll
+                for (int h = 0; h < NH; ++h)
+#pragma unroll
+                    for (int i = 0; i < G8; ++i) {
+                        const int c = h * C::NS + c0 + 8 * i;
+                        float v[8];
+                        uint32_t h4[4], l4[4];
+#pragma unroll
+                        for (int j = 0; j < 8; j += 4) {
+                            const float4 wx = ld4(B.vec(V_W4X, c + j)), wy = ld4(B.vec(V_W4Y, c + j));
+                            const float4 wz = ld4(B.vec(V_W4Z, c + j));
+                            const float2 p = __ffma2_rn(f2(gd[2]), xy(wz),
+                                                        __ffma2_rn(f2(gd[1]), xy(wy), __fmul2_rn(f2(gd[0]), xy(wx))));
+                            const float2 q = __ffma2_rn(f2(gd[2]), zw(wz),
+                                                        __ffma2_rn(f2(gd[1]), zw(wy), __fmul2_rn(f2(gd[0]), zw(wx))));
+                            v[j] = p.x; v[j + 1] = p.y; v[j + 2] = q.x; v[j + 3] = q.y;
+                        }
+                        gate8(v, x + 8 * i, 1.0f);
+                        if (h + 1 < NH) ask(2, tile, h + 1, i);
+                        else ask(1, tile, 0, i);
+                        stg8(A.gz3 + at8(tile, c), v);
+                        split8(v, sc3, h4, l4);
+                        B.put8(r, c, h4, l4);
+                    }
+                B.publish();
+                epi_sync();
+                {   // dW4 += g^T H3, from L2 (beside the first MMAs)
+                    const float* H3 = A.store + 2 * A.astride + ((int64_t)tile * (W / 8) + blk) * TILE * 8 + cl;
 #pragma unroll 8
-                for (int k = 0; k < PART_ROWS / 4; ++k) {
-                    const int rr = row0 + 4 * k + rl;
-                    const float g0 = rows[rr], g1 = rows[TILE + rr], g2 = rows[2 * TILE + rr];
+                    for (int k = 0; k < PART_ROWS / 4; ++k) {
+                        const int rr = row0 + 4 * k + rl;
+                        const float g0 = rows[rr], g1 = rows[TILE + rr], g2 = rows[2 * TILE + rr];
 #pragma unroll
-                    for (int q = 0; q < SB; ++q) {
-                        const float h = H3[(q * 16 * TILE + rr) * 8];
-                        s4[q][0] = fmaf(g0, h, s4[q][0]);
-                        s4[q][1] = fmaf(g1, h, s4[q][1]);
-                        s4[q][2] = fmaf(g2, h, s4[q][2]);
+                        for (int q = 0; q < SB; ++q) {
+                            const float h = H3[(q * 16 * TILE + rr) * 8];
+                            s4[q][0] = fmaf(g0, h, s4[q][0]);
+                            s4[q][1] = fmaf(g1, h, s4[q][1]);
+                            s4[q][2] = fmaf(g2, h, s4[q][2]);
+                        }
                     }
                 }
-            }
-            float e3[3] = {0.f, 0.f, 0.f};  // this row's dx (group 0) or u (group 1)
-            // two layers back
-            float p0 = 0.f, p1 = 0.f, p2 = 0.f;
+                float e3[3] = {0.f, 0.f, 0.f};  // this row's dx (group 0) or u (group 1)
+                // two layers back
+                float p0 = 0.f, p1 = 0.f, p2 = 0.f;
 #pragma unroll
-            for (int l = 0; l < 2; ++l) {
-                if (l == 1) {
-                    if (t + 1 < tiles) ask_row(tile + gridDim.x);
-                    const float* e = g == 0 ? A.dx_in : A.u;
-                    if (g < 2 && row < A.n) {
+                for (int l = 0; l < 2; ++l) {
+                    if (l == 1) {
+                        if (!STEP && more) ask_row(then);
+                        const float* e = g == 0 ? A.dx_in : A.u;
+                        if constexpr (STEP)
+                            if (j > 0) e = g == 0 ? A.dx_out : j == 3 ? A.x : A.u - j * 3 * A.n;
+                        if (g < 2 && row < A.n) {
 #pragma unroll
-                        for (int d = 0; d < 3; ++d) e3[d] = e[3 * row + d];
+                            for (int d = 0; d < 3; ++d) e3[d] = e[3 * row + d];
+                        }
                     }
-                }
-                const float f = l == 0 ? inv_3 * inv3 : inv_2 * inv2;
-                float v[HC];
-                uint32_t ph[G8][4], pl[G8][4];
-                // one 8-column group: l = 0 g_z2 -> global and images, l = 1 g_z1 -> g_u
-                auto finish8 = [&](float* q, int c, uint32_t* h4, uint32_t* l4) {
-                    if (l == 0) {
-                        const float o[8] = {q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]};
-                        stg8(A.gz2 + at8(tile, c), o);
-                        split8(q, sc2, h4, l4);
-                        return;
-                    }
+                    const float f = l == 0 ? inv_3 * inv3 : inv_2 * inv2;
+                    float v[HC];
+                    uint32_t ph[G8][4], pl[G8][4];
+                    // one 8-column group: l = 0 g_z2 -> global and images, l = 1 g_z1 -> g_u
+                    auto finish8 = [&](float* q, int c, uint32_t* h4, uint32_t* l4) {
+                        if (l == 0) {
+                            const float o[8] = {q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]};
+                            stg8(A.gz2 + at8(tile, c), o);
+                            split8(q, sc2, h4, l4);
+                            return;
+                        }
 #pragma unroll
-                    for (int j = 0; j < 8; j += 4) {
-                        const float4 x = ld4(B.vec(V_W1X, c + j)), y = ld4(B.vec(V_W1Y, c + j));
-                        const float4 z = ld4(B.vec(V_W1Z, c + j));
-                        p0 = fmaf(q[j + 3], x.w, fmaf(q[j + 2], x.z, fmaf(q[j + 1], x.y, fmaf(q[j], x.x, p0))));
-                        p1 = fmaf(q[j + 3], y.w, fmaf(q[j + 2], y.z, fmaf(q[j + 1], y.y, fmaf(q[j], y.x, p1))));
-                        p2 = fmaf(q[j + 3], z.w, fmaf(q[j + 2], z.z, fmaf(q[j + 1], z.y, fmaf(q[j], z.x, p2))));
+                        for (int j = 0; j < 8; j += 4) {
+                            const float4 x = ld4(B.vec(V_W1X, c + j)), y = ld4(B.vec(V_W1Y, c + j));
+                            const float4 z = ld4(B.vec(V_W1Z, c + j));
+                            p0 = fmaf(q[j + 3], x.w, fmaf(q[j + 2], x.z, fmaf(q[j + 1], x.y, fmaf(q[j], x.x, p0))));
+                            p1 = fmaf(q[j + 3], y.w, fmaf(q[j + 2], y.z, fmaf(q[j + 1], y.y, fmaf(q[j], y.x, p1))));
+                            p2 = fmaf(q[j + 3], z.w, fmaf(q[j + 2], z.z, fmaf(q[j + 1], z.y, fmaf(q[j], z.x, p2))));
+                        }
+                    };
+                    if (NH == 2) {
+                        B.wait_result();
+#pragma unroll
+                        for (int i = 0; i < G8; ++i) tmem_sum4(lane_base + 8 * i, C::NS, v + 8 * i);
+                        B.release_half();
+#pragma unroll
+                        for (int i = 0; i < G8; ++i) {
+                            gate8(v + 8 * i, x + 8 * i, f);
+                            ask(1 - l, tile, 1, i);
+                            finish8(v + 8 * i, c0 + 8 * i, ph[i], pl[i]);
+                        }
                     }
-                };
-                if (NH == 2) {
                     B.wait_result();
+                    if (NH == 2) {
 #pragma unroll
-                    for (int i = 0; i < G8; ++i) tmem_sum4(lane_base + 8 * i, C::NS, v + 8 * i);
-                    B.release_half();
+                        for (int i = 0; i < G8; ++i) {
+                            if (l == 0) B.put8(r, c0 + 8 * i, ph[i], pl[i]);
+                            else put_scratch(c0 + 8 * i, v + 8 * i);
+                        }
+                    }
 #pragma unroll
                     for (int i = 0; i < G8; ++i) {
-                        gate8(v + 8 * i, x + 8 * i, f);
-                        ask(1 - l, tile, 1, i);
-                        finish8(v + 8 * i, c0 + 8 * i, ph[i], pl[i]);
+                        const int c = (NH - 1) * C::NS + c0 + 8 * i;
+                        float q[8];
+                        uint32_t h4[4], l4[4];
+                        tmem_sum4(lane_base + 8 * i, C::NS, q);
+                        gate8(q, x + 8 * i, f);
+                        if (l == 0) ask(0, tile, 0, i);
+                        else if (more) ask(2, then, 0, i);
+                        finish8(q, c, h4, l4);
+                        if (l == 0) B.put8(r, c, h4, l4);
+                        else put_scratch(c, q);
                     }
+                    if (l == 0) B.publish();
                 }
-                B.wait_result();
-                if (NH == 2) {
-#pragma unroll
-                    for (int i = 0; i < G8; ++i) {
-                        if (l == 0) B.put8(r, c0 + 8 * i, ph[i], pl[i]);
-                        else put_scratch(c0 + 8 * i, v + 8 * i);
+                B.template row_sums<STEP>(p0, p1, p2, g, r);
+                if (STEP) {
+                    const bool late = *B.late != 0;
+                    gp[0] = row >= A.n ? 0.f : late ? NAN : p0;
+                    gp[1] = row >= A.n ? 0.f : late ? NAN : p1;
+                    gp[2] = row >= A.n ? 0.f : late ? NAN : p2;
+                }
+                if (g == 0 && row < A.n) {
+                    if (*B.late) p0 = p1 = p2 = NAN;
+                    if (!STEP) {
+                        A.gu[3 * row] = p0;
+                        A.gu[3 * row + 1] = p1;
+                        A.gu[3 * row + 2] = p2;
                     }
+                    A.dx_out[3 * row] = e3[0] + p0;
+                    A.dx_out[3 * row + 1] = e3[1] + p1;
+                    A.dx_out[3 * row + 2] = e3[2] + p2;
                 }
+                if (g == 1) {
 #pragma unroll
-                for (int i = 0; i < G8; ++i) {
-                    const int c = (NH - 1) * C::NS + c0 + 8 * i;
-                    float q[8];
-                    uint32_t h4[4], l4[4];
-                    tmem_sum4(lane_base + 8 * i, C::NS, q);
-                    gate8(q, x + 8 * i, f);
-                    if (l == 0) ask(0, tile, 0, i);
-                    else if (t + 1 < tiles) ask(2, tile + gridDim.x, 0, i);
-                    finish8(q, c, h4, l4);
-                    if (l == 0) B.put8(r, c, h4, l4);
-                    else put_scratch(c, q);
+                    for (int d = 0; d < 3; ++d) rows[d * TILE + r] = e3[d];
                 }
-                if (l == 0) B.publish();
-            }
-            B.row_sums(p0, p1, p2, g, r);
-            if (g == 0 && row < A.n) {
-                if (*B.late) p0 = p1 = p2 = NAN;
-                A.gu[3 * row] = p0;
-                A.gu[3 * row + 1] = p1;
-                A.gu[3 * row + 2] = p2;
-                A.dx_out[3 * row] = e3[0] + p0;
-                A.dx_out[3 * row + 1] = e3[1] + p1;
-                A.dx_out[3 * row + 2] = e3[2] + p2;
-            }
-            if (g == 1) {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) rows[d * TILE + r] = e3[d];
-            }
-            epi_sync();
-            {   // dW1 += g_z1^T u, db1 += g_z1 (every other row of a lane's eight: no two lanes in a bank)
+                epi_sync();
+                {   // dW1 += g_z1^T u, db1 += g_z1 (every other row of a lane's eight: no two lanes in a bank)
 #pragma unroll 4
-                for (int k = 0; k < PART_ROWS / 4; ++k) {
-                    const int rr = row0 + 8 * (k >> 1) + (k & 1) + 2 * rl;
-                    const float u0 = rows[rr], u1 = rows[TILE + rr], u2 = rows[2 * TILE + rr];
+                    for (int k = 0; k < PART_ROWS / 4; ++k) {
+                        const int rr = row0 + 8 * (k >> 1) + (k & 1) + 2 * rl;
+                        const float u0 = rows[rr], u1 = rows[TILE + rr], u2 = rows[2 * TILE + rr];
 #pragma unroll
-                    for (int q = 0; q < SB; ++q) {
-                        const int c = 8 * (blk + 16 * q) + cl;
-                        const float x1 = scratch[rr * W + ((((c >> 2) ^ (rr & 7)) << 2) | (c & 3))];
-                        s1[q][0] = fmaf(u0, x1, s1[q][0]);
-                        s1[q][1] = fmaf(u1, x1, s1[q][1]);
-                        s1[q][2] = fmaf(u2, x1, s1[q][2]);
-                        s1[q][3] += x1;
+                        for (int q = 0; q < SB; ++q) {
+                            const int c = 8 * (blk + 16 * q) + cl;
+                            const float x1 = scratch[rr * W + ((((c >> 2) ^ (rr & 7)) << 2) | (c & 3))];
+                            s1[q][0] = fmaf(u0, x1, s1[q][0]);
+                            s1[q][1] = fmaf(u1, x1, s1[q][1]);
+                            s1[q][2] = fmaf(u2, x1, s1[q][2]);
+                            s1[q][3] += x1;
+                        }
                     }
                 }
+                epi_sync();
             }
-            epi_sync();
-        }
-        // a column's four lanes (and row ranges) together; db4: the rows of group 0
-        float* sums = scratch;  // [SUM_PARTS][8][W]: dW4 (3), -, dW1 (3), db1
-        float* xs = reinterpret_cast<float*>(smem + C::ROWS);
+            // a column's four lanes (and row ranges) together; db4: the rows of group 0
+                float* sums = scratch;  // [SUM_PARTS][8][W]: dW4 (3), -, dW1 (3), db1
+                float* xs = reinterpret_cast<float*>(smem + C::ROWS);
 #pragma unroll
-        for (int q = 0; q < SB; ++q)
+                for (int q = 0; q < SB; ++q)
 #pragma unroll
-            for (int d = 0; d < 7; ++d) {
-                float v = d < 3 ? s4[q][d < 3 ? d : 0] : s1[q][d < 3 ? 0 : d - 3];
-                v += __shfl_xor_sync(0xffffffffu, v, 8);
-                v += __shfl_xor_sync(0xffffffffu, v, 16);
-                if (lane < 8) sums[(row0 / PART_ROWS * 8 + d + (d >= 3)) * W + 8 * (blk + 16 * q) + cl] = v;
-            }
-        if (g == 0) {
+                    for (int d = 0; d < 7; ++d) {
+                        float v = d < 3 ? s4[q][d < 3 ? d : 0] : s1[q][d < 3 ? 0 : d - 3];
+                        v += __shfl_xor_sync(0xffffffffu, v, 8);
+                        v += __shfl_xor_sync(0xffffffffu, v, 16);
+                        if (lane < 8) sums[(row0 / PART_ROWS * 8 + d + (d >= 3)) * W + 8 * (blk + 16 * q) + cl] = v;
+                    }
+                if (g == 0) {
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                for (int o = 16; o > 0; o >>= 1) sg[d] += __shfl_xor_sync(0xffffffffu, sg[d], o);
-                if (lane == 0) xs[4 * d + w] = sg[d];
-            }
-        }
-        epi_sync();
-        // the sums over all launches of a backward pass, with their rounding errors beside them
-        for (int e = threadIdx.x; e < 8 * W; e += EPI) {
-            const int k = e / W, c = e % W;
-            float v = sums[e];
-            if (C::SUM_PARTS == 2) v += sums[8 * W + e];
-            if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
-            float* out = A.partial + (int64_t)blockIdx.x * 16 * W + e;
-            const float h = A.first ? 0.f : *out, y = A.first ? v : __fadd_rn(v, out[8 * W]);
-            const float t = __fadd_rn(h, y), b = __fsub_rn(t, h);
-            *out = t;
-            out[8 * W] = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(y, b));
+                    for (int d = 0; d < 3; ++d) {
+                        for (int o = 16; o > 0; o >>= 1) sg[d] += __shfl_xor_sync(0xffffffffu, sg[d], o);
+                        if (lane == 0) xs[4 * d + w] = sg[d];
+                    }
+                }
+                epi_sync();
+                // the sums over all products of a backward pass, with their rounding errors beside them
+                for (int e = threadIdx.x; e < 8 * W; e += EPI) {
+                    const int k = e / W, c = e % W;
+                    float v = sums[e];
+                    if (C::SUM_PARTS == 2) v += sums[8 * W + e];
+                    if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
+                    float* out = A.partial + (int64_t)blockIdx.x * 16 * W + e;
+                    const bool first = A.first && j == 0;
+                    const float h = first ? 0.f : *out, y = first ? v : __fadd_rn(v, out[8 * W]);
+                    const float t = __fadd_rn(h, y), b = __fsub_rn(t, h);
+                    *out = t;
+                    out[8 * W] = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(y, b));
+                }
+            if (STEP && j < 3) epi_sync();
         }
         const uint32_t m2 = __reduce_max_sync(0xffffffffu, __float_as_uint(gm2));
         const uint32_t m3 = __reduce_max_sync(0xffffffffu, __float_as_uint(gm3));
@@ -1446,7 +1485,8 @@ int set_attrs() {
     MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
     MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
     MO_CUDA(cudaFuncSetAttribute(k_tc_fwd<W, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
-    MO_CUDA(cudaFuncSetAttribute(k_tc_bwd<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
+    MO_CUDA(cudaFuncSetAttribute(k_tc_bwd<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
+    MO_CUDA(cudaFuncSetAttribute(k_tc_bwd<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<W>::SMEM));
     MO_CUDA(cudaFuncSetAttribute(k_tc_wgrad<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, WCfg<W>::SMEM));
     return MO_OK;
 }
@@ -1538,8 +1578,8 @@ static int issue_fwd(const float* u, const float* x, int64_t n, void* pack, int 
                  "store must be 32-byte aligned with an array stride of at least the padded rows times the width");
     const FwdArgs A{u,     x,   n,     reinterpret_cast<unsigned char*>(pack), a, 0.f, w, 0.f, init_acc,
                     unext, acc, store, astride, chained, 1, 0, nullptr};
-    TC_WIDTH(W_, TC_LAUNCH(store ? k_tc_fwd<W, true, false> : k_tc_fwd<W, false, false>, blocks_for(n), THREADS, Cfg<W>::SMEM, stream,
-                           chained, A));
+    TC_WIDTH(W_, TC_LAUNCH(store ? k_tc_fwd<W, true, false> : k_tc_fwd<W, false, false>, blocks_for(n), THREADS,
+                           Cfg<W>::SMEM, stream, chained, A));
     ::mo::note_launch();
     return MO_OK;
 }
@@ -1563,7 +1603,7 @@ static int issue_bwd(const float* a, float ca, const float* gprev, float cg, con
                  "activations and gradients must be 32-byte aligned and padded to whole tiles");
     const BwdArgs A{a,   gprev, ca,  cg,    u,      n,  reinterpret_cast<unsigned char*>(pack), store, astride,
                     gz2, gz3,   dx_in, dx_out, gu, partial, first, chained};
-    TC_WIDTH(W_, TC_LAUNCH(k_tc_bwd<W>, blocks_for(n), THREADS, Cfg<W>::SMEM, stream, chained, A));
+    TC_WIDTH(W_, TC_LAUNCH((k_tc_bwd<W, false>), blocks_for(n), THREADS, Cfg<W>::SMEM, stream, chained, A));
     ::mo::note_launch();
     return MO_OK;
 }
@@ -1728,6 +1768,8 @@ extern "C" int mo_ode_flow_backward(const float* ckpt, int64_t n, int steps, voi
     MO_CHECK_ARG(n > 0 && n < ((int64_t)1 << 31) && steps >= 1, "bad sizes");
     MO_CHECK_ARG(ckpt && pack && a_out && scratch && dx0 && dx1 && (!act || u), "null pointer");
     MO_CHECK_ARG(aligned(scratch, 128), "scratch must be 128-byte aligned");
+    MO_CHECK_ARG(aligned(pack, 128), "the packed parameters must be 128-byte aligned");
+    MO_CHECK_ARG(!act || aligned(act, 32), "the activations must be 32-byte aligned");
     const bool stored = act != nullptr;
     if (scratch_floats < mo_ode_backward_floats(n, W, stored)) {
         set_error("flow scratch too small: %lld < %lld floats", (long long)scratch_floats,
@@ -1767,11 +1809,21 @@ extern "C" int mo_ode_flow_backward(const float* ckpt, int64_t n, int steps, voi
         // dL/dx = a + g4 + g3 + g2 + g1
         const float ca[4] = {(float)(h / 6), (float)(h / 3), (float)(h / 3), (float)(h / 6)};
         const float cg[4] = {(float)(h / 2), (float)(h / 2), (float)h, 0.f};
-        for (int e = 3; e >= 0; --e, ++evals) {
-            rc = issue_bwd(a, ca[e], e == 3 ? nullptr : gu[evals & 1], cg[e], e ? uk + (e - 1) * 3 * n : x, n, pack, W,
-                           ak + e * size, 4 * size, gz + e * size, gz + (4 + e) * size, e == 3 ? a : dx[k & 1],
-                           dx[k & 1], gu[1 - (evals & 1)], partial, evals == 0, stream, !stored || evals > 0);
-            if (rc) return rc;
+        if (tiles_of(n) <= device_sm_count()) {
+            const bool chained = !stored || k < steps - 1;
+            const StepArgs A{{a, nullptr, ca[3], cg[3], uk + 6 * n, n, reinterpret_cast<unsigned char*>(pack),
+                              ak + 3 * size, 4 * size, gz + 3 * size, gz + 7 * size, a, dx[k & 1], nullptr, partial,
+                              k == steps - 1, chained},
+                             ca[2], cg[2], cg[1], x};
+            TC_WIDTH(W, TC_LAUNCH((k_tc_bwd<W, true>), blocks_for(n), THREADS, Cfg<W>::SMEM, stream, chained, A));
+            ::mo::note_launch();
+        } else {
+            for (int e = 3; e >= 0; --e, ++evals) {
+                rc = issue_bwd(a, ca[e], e == 3 ? nullptr : gu[evals & 1], cg[e], e ? uk + (e - 1) * 3 * n : x, n, pack,
+                               W, ak + e * size, 4 * size, gz + e * size, gz + (4 + e) * size, e == 3 ? a : dx[k & 1],
+                               dx[k & 1], gu[1 - (evals & 1)], partial, evals == 0, stream, !stored || evals > 0);
+                if (rc) return rc;
+            }
         }
         for (int l = 0; l < 2; ++l) {
             rc = issue_wgrad(gz + 4 * l * size, ak + 4 * l * size, 4 * rows, pack, W, 2 + l, wpart[l], k == steps - 1,
