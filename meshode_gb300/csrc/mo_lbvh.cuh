@@ -1,7 +1,8 @@
 // LBVH pieces shared by the distance-field build (triangles) and the
 // nearest-point queries (points): 30-bit Morton codes, the Karras (HPG 2012)
-// radix tree over sorted codes, and the bottom-up box refit.  The kernels are
-// defined in mo_dfbuild.cu.
+// radix tree over sorted codes, and the bottom-up box refit (mo_lbvh_build's
+// plain boxes; the other trees take their boxes from their leaves).  The kernels
+// are defined in mo_dfbuild.cu.
 //
 // Node layout: internal node i (of n-1) is 4 float4 =
 //   (left lo.xyz, left id) (left hi.xyz, right id) (right lo.xyz, -) (right hi.xyz, -)
