@@ -53,26 +53,53 @@ def init_params(hidden=256, seed=4, device="cuda"):
 MLP_WIDTH = 256  # the fused kernels' hidden width; narrower MLPs run zero-padded
 
 
+def _shapes(m):
+    return ((m, 3), (m,), (m, m), (m,), (m, m), (m,), (3, m), (3,))
+
+
 class _Packed:
     """The parameters as the fused kernels take them (mo_mlp_tc_pack): split
     and laid out for the tensor cores, zero-padded to the kernels' width
     (exact: a padded unit's pre-activation and outgoing weights are 0)."""
 
     def __init__(self, params):
-        params = [p.detach().float().contiguous() for p in params]
+        params = [p.detach() for p in params]
+        dev = params[0].device
         m = params[0].shape[0]
         if m > MLP_WIDTH:
             raise RuntimeError("hidden width %d exceeds the fused kernels' %d" % (m, MLP_WIDTH))
-        self.m = m
+        self.units = m
+        if m == 0 or any(tuple(p.shape) != s for p, s in zip(params, _shapes(m))):
+            # hidden layers of different widths: all padded to the kernels' width,
+            # which a larger or differently shaped parameter does not fit
+            m = MLP_WIDTH
+            params = [self._pad(p, s, dev) for p, s in zip(params[:7], _shapes(m))] + [self._bias4(params[7])]
+        params = [p.to(dev, torch.float32).contiguous() for p in params]
+        self.m = m  # as packed
         self.M = int(L.lib().mo_mlp_tc_width(m))
-        self.dev = params[0].device
-        self.buf = torch.empty(int(L.lib().mo_mlp_tc_pack_bytes(self.M)), dtype=torch.uint8, device=self.dev)
+        self.dev = dev
+        self.buf = torch.empty(int(L.lib().mo_mlp_tc_pack_bytes(self.M)), dtype=torch.uint8, device=dev)
         call("mo_mlp_tc_pack", *[ptr(p) for p in params], m, ptr(self.buf), stream_ptr())
 
+    @staticmethod
+    def _pad(t, shape, dev):
+        out = torch.zeros(shape, dtype=torch.float32, device=dev)
+        out[tuple(slice(0, k) for k in t.shape)] = t
+        return out
+
+    @staticmethod
+    def _bias4(t):
+        if t.numel() < 3:
+            raise RuntimeError("b4 needs 3 values, got shape %s" % (tuple(t.shape),))
+        return t.reshape(-1)[:3]
+
     def grads(self):
-        m = self.m
-        return [torch.zeros(sh, dtype=torch.float32, device=self.dev)
-                for sh in ((m, 3), (m,), (m, m), (m,), (m, m), (m,), (3, m), (3,))]
+        return [torch.zeros(sh, dtype=torch.float32, device=self.dev) for sh in _shapes(self.m)]
+
+    def unpad(self, grads):
+        if self.m == self.units:
+            return grads
+        return [g[tuple(slice(0, k) for k in s)].contiguous() for g, s in zip(grads, _shapes(self.units))]
 
 
 class ODEFlow(Function):
@@ -87,7 +114,10 @@ class ODEFlow(Function):
     def forward(ctx, x0, steps, store, W1, b1, W2, b2, W3, b3, W4, b4):
         P = _Packed((W1, b1, W2, b2, W3, b3, W4, b4))
         steps = int(steps)
-        1.0 / steps  # a flow has steps
+        if steps == 0:
+            raise ZeroDivisionError("a flow has at least one step")
+        if x0.dim() != 2 or x0.shape[1] != 3:
+            raise RuntimeError("x0 must be [n, 3], got %s" % (tuple(x0.shape),))
         x = x0.detach().contiguous().float()
         n = x.shape[0]
 
@@ -123,7 +153,7 @@ class ODEFlow(Function):
             a = dx[0]
         ctx.kept = None
         ctx.P = None
-        return (a, None, None) + tuple(grads)
+        return (a, None, None) + tuple(P.unpad(grads))
 
 
 class FitLossFunction(Function):
