@@ -114,7 +114,9 @@ cudaError_t exclusive_scan_i32(int* data, int n, int* total, cudaStream_t s) {
 // 30-bit codes: 75 us at 20k to 50k keys, 130 us at 355k.)
 //
 // hist: counts [4][256] | tickets [4] | words [passes][tiles][256], zeroed per sort;
-// a word is state << 30 | count, state 1: the tile's count, 2: inclusive prefix.
+// a word is state << BITS | count, state 1: the tile's count, 2: inclusive prefix.
+// 30 bits hold the count of a digit up to 2^30 - 1 keys; from 2^30 on the words
+// have 64 bits, twice the bytes to clear and to look back over.
 // ---------------------------------------------------------------------------
 constexpr int RS_WARPS = 8, RS_PASSES = 4, RS_HEAD = RS_PASSES * 256 + 64;
 // keys per thread: small sorts take small tiles, so that more SMs share them
@@ -123,7 +125,27 @@ constexpr int RS_SMALL = 1 << 17;
 static int rs_rounds(int n) { return n <= RS_SMALL ? 2 : 8; }
 static int rs_tiles(int n) { return ceil_div(n > 0 ? n : 1, RS_WARPS * 32 * rs_rounds(n)); }
 
-size_t radix_hist_ints(int n) { return (size_t)RS_HEAD + (size_t)RS_PASSES * 256 * (size_t)rs_tiles(n); }
+constexpr int RS_WIDE = 1 << 30;
+static size_t rs_word_ints(int n) { return 256 * (size_t)rs_tiles(n) * (n >= RS_WIDE ? 2 : 1); }  // of a pass
+
+size_t radix_hist_ints(int n) { return (size_t)RS_HEAD + RS_PASSES * rs_word_ints(n); }
+
+__device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_relaxed(uint64_t* p, uint64_t v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint64_t ld_relaxed(const uint64_t* p) {
+    uint64_t v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
 
 __global__ void __launch_bounds__(256) k_rs_count(const uint32_t* __restrict__ keys, int n, int passes,
                                                   int* __restrict__ hist) {
@@ -139,10 +161,12 @@ __global__ void __launch_bounds__(256) k_rs_count(const uint32_t* __restrict__ k
         if (h[p][threadIdx.x]) atomicAdd(hist + 256 * p + threadIdx.x, h[p][threadIdx.x]);
 }
 
-template <int ROUNDS>
+template <int ROUNDS, class Word>
 __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ kin, const int* __restrict__ vin,
                                                  uint32_t* __restrict__ kout, int* __restrict__ vout, int n, int pass,
-                                                 int* __restrict__ hist, uint32_t* __restrict__ words) {
+                                                 int* __restrict__ hist, Word* __restrict__ words) {
+    constexpr int BITS = 8 * sizeof(Word) - 2;
+    constexpr Word COUNT = ((Word)1 << BITS) - 1;
     __shared__ int wh[RS_WARPS][256];
     __shared__ int warp_sum[8];
     __shared__ int tile_sh;
@@ -180,9 +204,8 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
     int mine = 0;
 #pragma unroll
     for (int ww = 0; ww < RS_WARPS; ++ww) mine += wh[ww][d];
-    uint32_t* my = words + (int64_t)tile * 256 + d;
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(my), "r"((tile == 0 ? 2u << 30 : 1u << 30) | (uint32_t)mine)
-                 : "memory");
+    Word* my = words + (int64_t)tile * 256 + d;
+    st_relaxed(my, (Word)(tile == 0 ? 2 : 1) << BITS | (Word)mine);
     const int total = hist[256 * pass + d];
     int x = total;
 #pragma unroll
@@ -199,28 +222,21 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
         constexpr int BATCH = 16;
         unsigned long long t0 = 0, now;
         for (int t = tile - 1; t >= 0;) {
-            uint32_t v[BATCH];
+            Word v[BATCH];
 #pragma unroll
-            for (int k = 0; k < BATCH; ++k) {
-                v[k] = 0u;
-                if (t - k >= 0)
-                    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];"
-                                 : "=r"(v[k])
-                                 : "l"(words + (int64_t)(t - k) * 256 + d)
-                                 : "memory");
-            }
+            for (int k = 0; k < BATCH; ++k) v[k] = t - k >= 0 ? ld_relaxed(words + (int64_t)(t - k) * 256 + d) : 0;
             bool end = false, stalled = false;
 #pragma unroll
             for (int k = 0; k < BATCH; ++k) {
                 if (end || stalled || t < 0) continue;
-                const uint32_t st = v[k] >> 30;
-                if (st == 0u) {
+                const int st = (int)(v[k] >> BITS);
+                if (st == 0) {
                     stalled = true;
                     continue;
                 }
-                prefix += (int)(v[k] & 0x3fffffffu);
+                prefix += (int)(v[k] & COUNT);
                 --t;
-                end = st == 2u;
+                end = st == 2;
             }
             if (end) break;
             if (stalled) {  // a predecessor has not published yet; two seconds at most
@@ -229,8 +245,7 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
                 if (now - t0 > 2000000000ull) break;
             }
         }
-        asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(my), "r"((2u << 30) | (uint32_t)(prefix + mine))
-                     : "memory");
+        st_relaxed(my, (Word)2 << BITS | (Word)(prefix + mine));
     }
     int run = base + prefix;
 #pragma unroll
@@ -256,16 +271,17 @@ cudaError_t radix_sort_pairs(uint32_t* keys_a, int* vals_a, uint32_t* keys_b, in
                              int bits, int* hist, cudaStream_t s) {
     if (n <= 1) return cudaSuccess;
     const int tiles = rs_tiles(n), passes = (bits + 7) / 8;
-    cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * ((size_t)RS_HEAD + (size_t)passes * 256 * tiles), s);
+    cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * ((size_t)RS_HEAD + passes * rs_word_ints(n)), s);
     if (e != cudaSuccess) return e;
     k_rs_count<<<std::min(ceil_div(n, 1024), 2 * device_sm_count()), 256, 0, s>>>(keys_a, n, passes, hist);
     ::mo::note_launch();
     uint32_t *ki = keys_a, *ko = keys_b;
     int *vi = vals_a, *vo = vals_b;
     for (int p = 0; p < passes; ++p) {
-        uint32_t* words = reinterpret_cast<uint32_t*>(hist) + RS_HEAD + (size_t)p * 256 * tiles;
+        uint32_t* words = reinterpret_cast<uint32_t*>(hist) + RS_HEAD + p * rs_word_ints(n);
         if (rs_rounds(n) == 2) k_rs_pass<2><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words);
-        else k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words);
+        else if (n < RS_WIDE) k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words);
+        else k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, reinterpret_cast<uint64_t*>(words));
         ::mo::note_launch();
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

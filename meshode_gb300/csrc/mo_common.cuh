@@ -84,8 +84,8 @@ cudaError_t exclusive_scan_i32(int* data, int n, int* total, cudaStream_t s);
 
 // Stable LSD radix sort of (uint32 key, int32 value) pairs over the low
 // `bits` bits.  Buffers *_a hold the input; the sorted result is returned in
-// *_a as well (ping-pong through *_b).  hist must hold radix_hist_ints(n) ints;
-// n < 2^30.
+// *_a as well (ping-pong through *_b).  hist (8-byte aligned) must hold
+// radix_hist_ints(n) ints.
 cudaError_t radix_sort_pairs(uint32_t* keys_a, int* vals_a, uint32_t* keys_b, int* vals_b,
                              int n, int bits, int* hist, cudaStream_t s);
 size_t radix_hist_ints(int n);
