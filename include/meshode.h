@@ -50,6 +50,13 @@ int mo_version(void);
 /* Kernel launches issued by this library since it was loaded (launches
  * replayed from a captured CUDA graph are not included). */
 unsigned long long mo_launch_count(void);
+/* In place: (key, value) pairs by key (below 2^bits), stable, n < 2^31;
+ * the sort inside the tree builds and the nearest-point query.  max_wait_ns:
+ * how long a tile waits for those before it until it does their counting
+ * itself (the builds and the query use 2 s); the order does not depend on it. */
+size_t mo_sort_pairs_scratch_bytes(int64_t n);
+int mo_sort_pairs(uint32_t* keys, int32_t* vals, int64_t n, int bits, void* scratch, size_t scratch_bytes,
+                  uint64_t max_wait_ns, void* stream);
 
 /* ------------------------------------------------------------------------
  * Normalisation by the target's transform.

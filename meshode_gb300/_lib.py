@@ -82,6 +82,8 @@ _SIGS = {
     "mo_last_error": (ctypes.c_char_p, []),
     "mo_version": (_I, []),
     "mo_launch_count": (ctypes.c_ulonglong, []),
+    "mo_sort_pairs_scratch_bytes": (_SZ, [_I64]),
+    "mo_sort_pairs": (_I, [_P, _P, _I64, _I, _P, _SZ, ctypes.c_uint64, _P]),
     "mo_bbox": (_I, [_P, _I64, _P, _P]),
     "mo_norm_params": (_I, [_P, _P, _P]),
     "mo_bbox_params": (_I, [_P, _I64, _P, _P, _P]),

@@ -109,7 +109,9 @@ cudaError_t exclusive_scan_i32(int* data, int n, int* total, cudaStream_t s) {
 // a tile ranks its keys (per-warp ranks from __match_any_sync, warps in order),
 // publishes its digit counts and adds up its predecessors' by looking back over
 // their published words, 16 at a time, until one holds an inclusive prefix.
-// Tiles take their number from a counter, so every predecessor is running.
+// Tiles take their number from a counter, so every predecessor is running.  A tile
+// that has waited for one for too long all the same counts the keys before its own
+// by itself, which needs nobody: the order is complete whatever the waits did.
 // (Before: histogram, single-CTA scan and scatter per digit, 12 launches for
 // 30-bit codes: 75 us at 20k to 50k keys, 130 us at 355k.)
 //
@@ -164,12 +166,14 @@ __global__ void __launch_bounds__(256) k_rs_count(const uint32_t* __restrict__ k
 template <int ROUNDS, class Word>
 __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ kin, const int* __restrict__ vin,
                                                  uint32_t* __restrict__ kout, int* __restrict__ vout, int n, int pass,
-                                                 int* __restrict__ hist, Word* __restrict__ words) {
+                                                 int* __restrict__ hist, Word* __restrict__ words,
+                                                 unsigned long long max_wait) {
     constexpr int BITS = 8 * sizeof(Word) - 2;
     constexpr Word COUNT = ((Word)1 << BITS) - 1;
     __shared__ int wh[RS_WARPS][256];
     __shared__ int warp_sum[8];
     __shared__ int tile_sh;
+    __shared__ int before[256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, shift = 8 * pass;
     if (threadIdx.x == 0) tile_sh = atomicAdd(hist + RS_PASSES * 256 + pass, 1);
     for (int d = threadIdx.x; d < RS_WARPS * 256; d += 256) (&wh[0][0])[d] = 0;
@@ -218,6 +222,7 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
     int base = x - total;
     for (int k = 0; k < w; ++k) base += warp_sum[k];
     int prefix = 0;
+    bool lost = false;
     if (tile > 0) {
         constexpr int BATCH = 16;
         unsigned long long t0 = 0, now;
@@ -239,13 +244,25 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
                 end = st == 2;
             }
             if (end) break;
-            if (stalled) {  // a predecessor has not published yet; two seconds at most
+            if (stalled) {  // a predecessor has not published yet
                 asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
                 if (t0 == 0) t0 = now;
-                if (now - t0 > 2000000000ull) break;
+                lost = now - t0 >= max_wait;
+                if (lost) break;
             }
         }
-        st_relaxed(my, (Word)2 << BITS | (Word)(prefix + mine));
+        if (!lost) st_relaxed(my, (Word)2 << BITS | (Word)(prefix + mine));
+    }
+    if (__syncthreads_or(lost)) {
+        before[d] = 0;
+        __syncthreads();
+        const int64_t first = (int64_t)tile * RS_WARPS * ROUNDS * 32;
+        for (int64_t i = d; i < first; i += 256) atomicAdd(&before[(kin[i] >> shift) & 255u], 1);
+        __syncthreads();
+        if (lost) {
+            prefix = before[d];
+            st_relaxed(my, (Word)2 << BITS | (Word)(prefix + mine));
+        }
     }
     int run = base + prefix;
 #pragma unroll
@@ -259,7 +276,7 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
     for (int r = 0; r < ROUNDS; ++r) {
         if (wbeg + r * 32 + lane < n) {
             const int pos = wh[w][digit[r]] + rank[r];
-            if ((unsigned)pos < (unsigned)n) {  // always, unless a wait ran out
+            if ((unsigned)pos < (unsigned)n) {  // always, unless somebody else writes to the scratch
                 kout[pos] = key[r];
                 vout[pos] = val[r];
             }
@@ -268,7 +285,7 @@ __global__ void __launch_bounds__(256) k_rs_pass(const uint32_t* __restrict__ ki
 }
 
 cudaError_t radix_sort_pairs(uint32_t* keys_a, int* vals_a, uint32_t* keys_b, int* vals_b, int n,
-                             int bits, int* hist, cudaStream_t s) {
+                             int bits, int* hist, cudaStream_t s, uint64_t max_wait_ns) {
     if (n <= 1) return cudaSuccess;
     const int tiles = rs_tiles(n), passes = (bits + 7) / 8;
     cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int) * ((size_t)RS_HEAD + passes * rs_word_ints(n)), s);
@@ -279,9 +296,13 @@ cudaError_t radix_sort_pairs(uint32_t* keys_a, int* vals_a, uint32_t* keys_b, in
     int *vi = vals_a, *vo = vals_b;
     for (int p = 0; p < passes; ++p) {
         uint32_t* words = reinterpret_cast<uint32_t*>(hist) + RS_HEAD + p * rs_word_ints(n);
-        if (rs_rounds(n) == 2) k_rs_pass<2><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words);
-        else if (n < RS_WIDE) k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words);
-        else k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, reinterpret_cast<uint64_t*>(words));
+        if (rs_rounds(n) == 2)
+            k_rs_pass<2><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words, max_wait_ns);
+        else if (n < RS_WIDE)
+            k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, words, max_wait_ns);
+        else
+            k_rs_pass<8><<<tiles, 256, 0, s>>>(ki, vi, ko, vo, n, p, hist, reinterpret_cast<uint64_t*>(words),
+                                                 max_wait_ns);
         ::mo::note_launch();
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -298,6 +319,28 @@ cudaError_t radix_sort_pairs(uint32_t* keys_a, int* vals_a, uint32_t* keys_b, in
 }
 
 }  // namespace mo
+
+extern "C" size_t mo_sort_pairs_scratch_bytes(int64_t n) {
+    if (n < 0 || n > INT_MAX) return 0;
+    return sizeof(int) * mo::radix_hist_ints((int)n) + 8 * (size_t)n;
+}
+
+extern "C" int mo_sort_pairs(uint32_t* keys, int32_t* vals, int64_t n, int bits, void* scratch, size_t scratch_bytes,
+                             uint64_t max_wait_ns, void* stream) {
+    MO_CHECK_ARG(n >= 0 && n <= INT_MAX, "bad number of keys");
+    MO_CHECK_ARG(bits >= 1 && bits <= 32, "keys have 1 to 32 bits, got %d", bits);
+    if (n <= 1) return MO_OK;
+    MO_CHECK_ARG(keys && vals && scratch && mo::aligned(scratch, 8), "null or misaligned pointer");
+    if (scratch_bytes < mo_sort_pairs_scratch_bytes(n)) {
+        mo::set_error("sort scratch too small: %zu < %zu", scratch_bytes, mo_sort_pairs_scratch_bytes(n));
+        return MO_ERR_SCRATCH;
+    }
+    int* hist = reinterpret_cast<int*>(scratch);
+    uint32_t* keys_b = reinterpret_cast<uint32_t*>(hist + mo::radix_hist_ints((int)n));
+    MO_CUDA(mo::radix_sort_pairs(keys, vals, keys_b, reinterpret_cast<int*>(keys_b + n), (int)n, bits, hist,
+                                 mo::as_stream(stream), max_wait_ns));
+    return MO_OK;
+}
 
 extern "C" const char* mo_last_error(void) { return mo::g_err; }
 extern "C" int mo_version(void) { return 100; }

@@ -85,9 +85,10 @@ cudaError_t exclusive_scan_i32(int* data, int n, int* total, cudaStream_t s);
 // Stable LSD radix sort of (uint32 key, int32 value) pairs over the low
 // `bits` bits.  Buffers *_a hold the input; the sorted result is returned in
 // *_a as well (ping-pong through *_b).  hist (8-byte aligned) must hold
-// radix_hist_ints(n) ints.
+// radix_hist_ints(n) ints.  max_wait_ns: when a tile stops waiting for those before
+// it and does their counting itself; the result does not depend on it.
 cudaError_t radix_sort_pairs(uint32_t* keys_a, int* vals_a, uint32_t* keys_b, int* vals_b,
-                             int n, int bits, int* hist, cudaStream_t s);
+                             int n, int bits, int* hist, cudaStream_t s, uint64_t max_wait_ns = 2000000000);
 size_t radix_hist_ints(int n);
 
 }  // namespace mo
