@@ -633,9 +633,13 @@ extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float*
             MO_CUDA(cudaMemset2DAsync(tile_loss + q.nslices, sizeof(float) * loss_stride, 0, sizeof(float) * pad, nsteps,
                                       as_stream(stream)));
     }
-    const int smem = RUN_REC * 3 * (int)sizeof(float) * 32 * warps * per_thread;
+    auto smem_of = [](int slices) { return RUN_REC * 3 * (int)sizeof(float) * 32 * slices; };
+    const int smem = smem_of(warps * per_thread);
     const void* kernel = run_kernel(weighted != 0, tile_loss != nullptr, per_thread, warps);
-    if (smem > 48 * 1024) MO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    // a limit belongs to the kernel and not to a call: every thread sets the kernel's largest
+    if (per_thread == 2 || warps > TILE_WARPS)
+        MO_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     smem_of(per_thread == 2 ? 2 * RUN_WARPS2 : RUN_WARPS1)));
     for (int done = 0; done < nsteps;) {
         int n = std::min(RUN_CHUNK, nsteps - done);
         MoPair p = q;
