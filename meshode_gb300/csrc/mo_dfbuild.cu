@@ -506,12 +506,14 @@ __device__ __forceinline__ Obb load_obb(const float4* obb, int i, float3* ns) {
 
 // A node of at most DF_BUCKET triangles under a parent of at most DF_BUCKET
 // lies inside a bucket: the walk tests the bucket's triangles and never reads
-// its box (nor visits its parent), so none is made.
+// its box (nor visits its parent), so none is made.  The root is visited however
+// few triangles it has, so its children have boxes.
 __device__ __forceinline__ bool inside_bucket(const int2* __restrict__ range, const int* __restrict__ parent, int i) {
     const int2 r = range[i];
     if (i == 0 || r.y - r.x + 1 > DF_BUCKET) return false;
-    const int2 pr = range[parent[i] >> 1];
-    return pr.y - pr.x + 1 <= DF_BUCKET;
+    const int up = parent[i] >> 1;
+    const int2 pr = range[up];
+    return up != 0 && pr.y - pr.x + 1 <= DF_BUCKET;
 }
 
 // Boxes of the internal nodes whose subtree holds at most OBB_EXACT
