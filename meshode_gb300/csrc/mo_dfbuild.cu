@@ -843,13 +843,18 @@ static void launch_df_lbvh(int packet, const float4* nodes, const float4* tris, 
 // packet, one triangle a lane: with c a triangle's centroid, r the radius of
 // its vertices around it, p the packet's centre and R its radius, no voxel's
 // distance is above U = min |p - c| + R, and none to this triangle is below
-// |p - c| - r - R.  CULL_SLACK is far more than these bounds' and the tests'
-// rounding, so what is dropped could not have lowered any voxel's minimum and
-// every voxel gets the minimum over all triangles.
+// |p - c| - r - R.  Both sides give way by CULL_SLACK of 1 + |p - c| + r (the
+// coordinates are below that; a target need not lie in the unit cube), far more
+// than these bounds' and the tests' rounding, so what is dropped could not have
+// lowered any voxel's minimum and every voxel gets the minimum over all
+// triangles.
 // Measured (records and grid, us): see mo_df_method_for.
 constexpr int BF_WARPS = 8;
 constexpr int BF_P = 4;  // packet edge, voxels
-constexpr float CULL_SLACK = 4e-6f;
+constexpr float CULL_SLACK = 2e-6f;
+// The nearest centroid is that of the least |p - c|^2 + CULL_R2 r^2, whose r is at
+// most |p - c| / sqrt(CULL_R2): the slack of U without a root per triangle.
+constexpr float CULL_R2 = 1.f / 1024, CULL_R = 32.f;
 
 __host__ __device__ __forceinline__ int64_t bf_bricks(int N) {
     const int64_t b = (N + BF_P - 1) / BF_P;
@@ -919,15 +924,16 @@ __global__ void __launch_bounds__(BF_WARPS * 32) k_df_brute(const float4* __rest
     for (int t = first; t < ntri; t += stride) {
         float d2, r2;
         tri_sphere(tris, t, cx, cy, cz, &d2, &r2);
-        u = fminf(u, d2);
+        u = fminf(u, fmaf(r2, CULL_R2, d2));
     }
     for (int o = 16; o > 0; o >>= 1) u = fminf(u, __shfl_xor_sync(FULL, u, o));
     if (lane == 0) sh_u[w] = u;
     __syncthreads();
     for (int k = 0; k < split; ++k) u = fminf(u, sh_u[(w & ~(split - 1)) + k]);
-    float U = sqrtf(u) + R;
+    u = sqrtf(u);
+    float U = u + CULL_SLACK * (1.f + (1.f + CULL_R) * u) + R;
     if (band2 != FLT_MAX) U = fminf(U, band + 13.0f / Nf);  // the widest band of any voxel
-    const float reach = U + R + CULL_SLACK;
+    const float reach = U + R + CULL_SLACK;  // beside r, and with 1 - CULL_SLACK of |p - c|
 
     for (int base = 0; base < ntri; base += stride) {
         const int t = base + first;
@@ -935,7 +941,7 @@ __global__ void __launch_bounds__(BF_WARPS * 32) k_df_brute(const float4* __rest
         if (keep) {
             float d2, r2;
             tri_sphere(tris, t, cx, cy, cz, &d2, &r2);
-            keep = !(sqrtf(d2) > sqrtf(r2) + reach);  // NaN: tested
+            keep = !((1.f - CULL_SLACK) * sqrtf(d2) > fmaf(sqrtf(r2), 1.f + CULL_SLACK, reach));  // NaN: tested
         }
         unsigned m = __ballot_sync(FULL, keep);
         while (m) {
