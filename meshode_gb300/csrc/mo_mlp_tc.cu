@@ -31,7 +31,9 @@
 // Activations and gradients between kernels are FP32 in blocks of 8 columns:
 // element (row, c) of a 128-row tile at ((tile*(W/8) + c/8)*128 + row)*8 + c%8,
 // so a warp whose lanes are rows moves 1 KB of consecutive bytes per access.
-// Every wait is bounded in time; one that runs out leaves NaN in the outputs.
+// Every wait is bounded in time; one that runs out leaves NaN in the outputs of
+// its call and in the packed weights' scales, and so in whatever later calls make
+// with them and from what it left.
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -64,7 +66,7 @@ struct Cfg {
     static constexpr int VECS = 2 * A_PIECE + STAGES * STAGE;
     static constexpr int ROWS = VECS + 9 * 4 * W;
     static constexpr int BARS = ROWS + 3 * 2048;
-    static constexpr int SMEM = BARS + 160;
+    static constexpr int SMEM = BARS + 160;           // see Block::init
     // mean relative truncation of a layer's sums (see the top)
     static constexpr float TRUNCATED = W == 256 ? 4e-8f : 0.f;
     // packed parameters (bytes)
@@ -169,6 +171,12 @@ __device__ __forceinline__ void ldg8(const float* p, float* v) {
                  : "l"(p));
 }
 
+// The packed weights' scales after a wait that ran out.
+__device__ __forceinline__ void spoil(float* misc) {
+    reinterpret_cast<volatile float*>(misc)[M_INV2] = NAN;
+    reinterpret_cast<volatile float*>(misc)[M_INV3] = NAN;
+}
+
 // ---- barriers, copies, MMA -------------------------------------------------
 __device__ __forceinline__ void bar_init(uint32_t bar, int count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -186,18 +194,22 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
 }
 // Waits for the phase; after two seconds (or once another wait of the block
 // ran out) it sets *late and returns: the block then runs to its end without
-// waiting and its outputs are overwritten with NaN.
-__device__ __forceinline__ void bar_wait(uint32_t bar, uint32_t parity, volatile int* late) {
-    if (bar_try(bar, parity)) return;
+// waiting and its outputs are overwritten with NaN.  OWN: for what this thread
+// itself has in flight, which is waited for (two seconds) whatever ran out.
+// False: the wait ran out.
+template <bool OWN = false>
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* late) {
+    if (bar_try(bar, parity)) return true;
     unsigned long long t0, t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
     while (!bar_try(bar, parity)) {
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (*late || t - t0 > 2000000000ull) {
+        if ((!OWN && *late) || t - t0 > 2000000000ull) {
             *late = 1;
-            return;
+            return false;
         }
     }
+    return true;
 }
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, int bytes, uint32_t bar) {
@@ -232,6 +244,14 @@ __device__ __forceinline__ void commit(uint32_t bar) {
     asm volatile(
         "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
+        : "memory");
+}
+// ... if the elected lane says so
+__device__ __forceinline__ void commit_if(uint32_t bar, bool ok) {
+    asm volatile(
+        "{\n.reg .pred p, q;\nelect.sync _|q, 0xffffffff;\nsetp.ne.and.b32 p, %1, 0, q;\n"
+        "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar),
+        "r"((uint32_t)ok)
         : "memory");
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -383,7 +403,7 @@ template <int W>
 struct Block {
     using C = Cfg<W>;
     unsigned char* sm;
-    uint32_t a, stage0, full, empty, a_ready, d_ready, drained, tmem;  // shared-memory addresses; tensor memory base
+    uint32_t a, stage0, full, empty, a_ready, d_ready, drained, idle, tmem;  // shared-memory addresses; tensor memory base
     volatile int* late;
     int done = 0;  // results waited for (epilogue)
 
@@ -396,7 +416,9 @@ struct Block {
         a_ready = empty + 8 * STAGES;
         d_ready = a_ready + 8;
         drained = d_ready + 8;
-        const int slot = C::BARS + 8 * (2 * STAGES + 3);
+        idle = drained + 8;
+        const int slot = C::BARS + 8 * (2 * STAGES + 4);
+        static_assert(8 * (2 * STAGES + 4) + 16 <= 160, "barriers, tensor memory address, late");
         late = reinterpret_cast<volatile int*>(smem + slot + 8);
         if (threadIdx.x >> 5 == EPI / 32 + 1) {  // the MMA warp
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(a + slot),
@@ -412,6 +434,7 @@ struct Block {
             bar_init(a_ready, EPI);
             bar_init(d_ready, 1);
             bar_init(drained, EPI);
+            bar_init(idle, 1);
             *late = (a & 1023u) ? 1 : 0;  // the operand images need 1 KB alignment
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -430,6 +453,12 @@ struct Block {
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(C::TMEM));
     }
 
+    // If a wait ran out, the calls after this one make NaN (one thread, when all
+    // others' waits are behind them).
+    __device__ __forceinline__ void hand_on(unsigned char* pack) const {
+        if (*late) spoil(reinterpret_cast<float*>(pack + C::P_MISC));
+    }
+
     __device__ __forceinline__ const float* vec(int v, int c) const {
         return reinterpret_cast<const float*>(sm + C::VECS) + v * W + c;
     }
@@ -441,11 +470,12 @@ struct Block {
             for (int l = 0; l < 2; ++l)
                 for (int s = 0; s < C::IMG_STAGES; ++s, ++it) {
                     const int st = it % STAGES;
-                    if (it >= STAGES) bar_wait(empty + 8 * st, (it / STAGES - 1) & 1, late);
+                    if (it >= STAGES && !bar_wait(empty + 8 * st, (it / STAGES - 1) & 1, late)) goto end;
                     bulk_load(stage0 + st * C::STAGE, (l ? img1 : img0) + (size_t)s * C::STAGE, C::STAGE, full + 8 * st);
                 }
+    end:
         // none of its copies is in flight when the block ends
-        for (int k = max(0, it - STAGES); k < it; ++k) bar_wait(full + 8 * (k % STAGES), (k / STAGES) & 1, late);
+        for (int k = max(0, it - STAGES); k < it; ++k) bar_wait<true>(full + 8 * (k % STAGES), (k / STAGES) & 1, late);
     }
 
     // Issues the MMAs of two layers for `tiles` tiles (one warp).  An MMA takes 65
@@ -454,6 +484,7 @@ struct Block {
         const uint64_t bd = smem_desc(stage0, 16);
         int st = 0, emptied = 0;
         uint32_t parity = 0;  // of stage st's current use
+        bool filled = true;   // a stage whose copy was not waited for is not handed back
         for (int t = 0; t < 2 * tiles; ++t) {
             bar_wait(a_ready, t & 1, late);
             fence_after();
@@ -471,9 +502,9 @@ struct Block {
                     // hi * lo: the weights' lo stages are done with
 #pragma unroll
                     for (int i = 0; i < C::KBH; ++i) {
-                        bar_wait(full + 8 * st, parity, late);
+                        filled &= bar_wait(full + 8 * st, parity, late);
                         block(ad + i * (TILE * 128 >> 4), bd + st * (C::STAGE >> 4), d + i * DB, true);
-                        commit(empty + 8 * st);
+                        commit_if(empty + 8 * st, filled);
                         if (++st == STAGES) {
                             st = 0;
                             parity ^= 1;
@@ -484,7 +515,7 @@ struct Block {
 #pragma unroll
                     for (int i = 0; i < C::KBH; ++i) {
                         hs[i] = st;
-                        bar_wait(full + 8 * st, parity, late);
+                        filled &= bar_wait(full + 8 * st, parity, late);
                         block(ad + i * (TILE * 128 >> 4) + (C::A_PIECE >> 4), bd + st * (C::STAGE >> 4), d + i * DB,
                               false);
                         if (++st == STAGES) {
@@ -495,13 +526,17 @@ struct Block {
 #pragma unroll
                     for (int i = 0; i < C::KBH; ++i) {
                         block(ad + i * (TILE * 128 >> 4), bd + hs[i] * (C::STAGE >> 4), d + i * DB, false);
-                        commit(empty + 8 * hs[i]);
+                        commit_if(empty + 8 * hs[i], filled);
                     }
                     ad += C::KBH * (TILE * 128 >> 4);
                     d += C::KBH * DB;
                 }
                 commit(d_ready);
             }
+        }
+        if (__any_sync(0xffffffffu, *late)) {  // nobody else has waited for the last MMAs then
+            commit(idle);
+            bar_wait<true>(idle, 0, late);
         }
     }
 
@@ -869,6 +904,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_fwd(FwdArgs A) {
             uint32_t* mx = reinterpret_cast<uint32_t*>(A.pack + C::P_MAX);
             atomicMax(mx, m1);
             atomicMax(mx + 1, m2);
+            if (w == 0) B.hand_on(A.pack);
         }
     }
     B.finish();
@@ -1198,7 +1234,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(std::conditional_t<STEP, 
                     const int k = e / W, c = e % W;
                     float v = sums[e];
                     if (C::SUM_PARTS == 2) v += sums[8 * W + e];
-                    if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
+                    if (*B.late || isnan(inv2)) v = NAN;
+                    else if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
                     float* out = A.partial + (int64_t)blockIdx.x * 16 * W + e;
                     const bool first = A.first && j == 0;
                     const float h = first ? 0.f : *out, y = first ? v : __fadd_rn(v, out[8 * W]);
@@ -1214,6 +1251,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(std::conditional_t<STEP, 
             uint32_t* mx = reinterpret_cast<uint32_t*>(A.pack + C::P_MAX);
             atomicMax(mx + 2, m2);
             atomicMax(mx + 3, m3);
+            if (w == 0) B.hand_on(A.pack);
         }
     }
     B.finish();
@@ -1249,6 +1287,7 @@ struct WgradArgs {
     const float *G, *H;  // rows x W, blocks of 8 columns
     int64_t chunks;      // 64-row chunks
     const uint32_t *gmax, *hmax;
+    float* misc;
     float *partial, *db;
     int first;
 };
@@ -1257,7 +1296,7 @@ template <int W>
 __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
     using C = WCfg<W>;
     extern __shared__ __align__(1024) unsigned char smem[];
-    const uint32_t sm = s32(smem), full = sm + C::BARS, done = full + 16, slot = done + 16;
+    const uint32_t sm = s32(smem), full = sm + C::BARS, done = full + 16, slot = done + 16, idle = slot + 16;
     volatile int* late = reinterpret_cast<volatile int*>(smem + C::BARS + 40);
     const int w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     if (w == EPI / 32) {
@@ -1270,6 +1309,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             bar_init(full + 8 * i, EPI);
             bar_init(done + 8 * i, 1);
         }
+        bar_init(idle, 1);
         *late = (sm & 1023u) ? 1 : 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -1309,12 +1349,17 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             for (int q = 0; q < C::ROWS / 16; ++q) mma(d, gh + 128 * q, hh + 128 * q, inst, true);
             commit(done + 8 * s);
         }
+        if (__any_sync(0xffffffffu, *late)) {  // nobody else has waited for the last MMAs then
+            commit(idle);
+            bar_wait<true>(idle, 0, late);
+        }
         __syncwarp();
     } else {
         constexpr int NC = C::NB / 4;            // accumulator columns of a thread
         constexpr int IT = C::NB / 64;           // items (8 columns x 32 rows) of a warp per operand
         const int c8 = C::NB < 128 ? (w & 7) : w;
         float ginv, hinv;
+        const bool was_late = isnan(A.misc[M_INV2]);
         const float gs = pow2_scale(__uint_as_float(*A.gmax), &ginv), hs = pow2_scale(__uint_as_float(*A.hmax), &hinv);
         const uint32_t lane_base = tmem + ((uint32_t)(32 * (w & 3)) << 16) + (w >> 2) * NC;
         float acc[NC];
@@ -1380,12 +1425,14 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             drain(k & 1);
         }
         const int o = 32 * (w & 3) + lane;
+        const bool bad = *late || was_late;
+        if (bad) spoil(A.misc);
         if (C::NB == 128 || o < C::NB) {
             float* out = A.partial + ((int64_t)blockIdx.y * W + o0 + o) * W + i0 + (w >> 2) * NC;
 #pragma unroll
             for (int j = 0; j < NC; ++j) {
                 const float x = acc[j] * ginv * hinv;
-                const float v = *late ? NAN : fmaf(x, 2e-8f, x);  // the mean loss of 4-step chains
+                const float v = bad ? NAN : fmaf(x, 2e-8f, x);  // the mean loss of 4-step chains
                 out[j] = A.first ? v : out[j] + v;
             }
         }
@@ -1396,7 +1443,10 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             if (lane == 0) {
                 float* out = A.db + ((int64_t)blockIdx.y * C::DB + (C::NB < 128 ? w >> 3 : 0)) * W + o0 + 8 * c8;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) out[j] = A.first ? cs[j] : out[j] + cs[j];
+                for (int j = 0; j < 8; ++j) {
+                    const float v = bad ? NAN : cs[j];
+                    out[j] = A.first ? v : out[j] + v;
+                }
             }
         }
     }
@@ -1628,8 +1678,9 @@ static int issue_wgrad(const float* G, const float* H, int64_t rows, void* pack,
     MO_CHECK_ARG(aligned(G, 32) && aligned(H, 32), "arrays must be 32-byte aligned");
     const int splits = splits_for(rows, W_);
     TC_WIDTH(W_, {
-        const uint32_t* mx = reinterpret_cast<const uint32_t*>(reinterpret_cast<unsigned char*>(pack) + Cfg<W>::P_MAX);
-        const WgradArgs A{G, H, rows / 64, mx + layer, mx + layer - 2, partial, partial + (int64_t)splits * W * W, first};
+        uint32_t* mx = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(pack) + Cfg<W>::P_MAX);
+        const WgradArgs A{G, H, rows / 64, mx + layer, mx + layer - 2,
+                          reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(pack) + Cfg<W>::P_MISC), partial, partial + (int64_t)splits * W * W, first};
         TC_LAUNCH(k_tc_wgrad<W>, dim3(WCfg<W>::BLOCKS, splits), WTHREADS, WCfg<W>::SMEM, stream, chained, A);
     });
     ::mo::note_launch();
