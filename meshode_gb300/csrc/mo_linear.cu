@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "mo_common.cuh"
+#include "mo_wait.cuh"
 
 namespace mo {
 namespace {
@@ -407,7 +408,7 @@ struct CgArgs {
 // The release publishes the writes that the block's barrier put before it, the
 // acquire holds for the threads behind the second one.  (With a full fence beside
 // each an iteration took 23.6 us instead of 21.6.)
-// A wait of more than two seconds, or another block's, ends the solve: false.
+// A wait of more than two seconds of polling, or another block's, ends the solve: false.
 __device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned target) {
     __shared__ int ok;
     __syncthreads();
@@ -415,15 +416,15 @@ __device__ __forceinline__ bool grid_sync(unsigned* bar, unsigned target) {
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         ok = 1;
         unsigned v, stop;
-        unsigned long long t0 = 0, t;
+        WaitLimit limit(0);
         for (int n = 0;; ++n) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if ((int)(v - target) >= 0) break;
             if ((n & 1023) == 1023) {
-                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-                if (t0 == 0) t0 = t;
+                const uint32_t now = wait_clock();
+                if (n == 1023) limit = WaitLimit(now);  // a clock reading a millisecond, none for a short wait
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(stop) : "l"(bar + 1) : "memory");
-                if (stop || t - t0 > 2000000000ull) {
+                if (stop || limit.over(now)) {
                     atomicExch(bar + 1, 1u);
                     ok = 0;
                     break;

@@ -39,6 +39,7 @@
 #include <type_traits>
 
 #include "mo_common.cuh"
+#include "mo_wait.cuh"
 
 namespace mo {
 namespace tc {
@@ -192,7 +193,7 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
                  : "memory");
     return ok != 0;
 }
-// Waits for the phase; after two seconds (or once another wait of the block
+// Waits for the phase; after two seconds of polling (or once another wait of the block
 // ran out) it sets *late and returns: the block then runs to its end without
 // waiting and its outputs are overwritten with NaN.  OWN: for what this thread
 // itself has in flight, which is waited for (two seconds) whatever ran out.
@@ -200,11 +201,9 @@ __device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
 template <bool OWN = false>
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* late) {
     if (bar_try(bar, parity)) return true;
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    WaitLimit limit(wait_clock());
     while (!bar_try(bar, parity)) {
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if ((!OWN && *late) || t - t0 > 2000000000ull) {
+        if (limit.over(wait_clock()) || (!OWN && *late)) {
             *late = 1;
             return false;
         }

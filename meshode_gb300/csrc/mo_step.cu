@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "mo_lazydf.cuh"
+#include "mo_wait.cuh"
 
 namespace mo {
 
@@ -221,21 +222,21 @@ __device__ __forceinline__ void run_arrive(unsigned* bar) {
 }
 
 // Waits until every block has arrived `target` times in total; after two seconds
-// (or another block's) it gives up: false.
+// of polling (or another block's) it gives up: false.
 __device__ __forceinline__ bool run_wait(unsigned* bar, unsigned target) {
     __shared__ int ok;
     if (threadIdx.x == 0) {
         ok = 1;
         unsigned v, stop;
-        unsigned long long t0 = 0, t;
+        WaitLimit limit(0);
         for (int n = 0;; ++n) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if ((int)(v - target) >= 0) break;
             if ((n & 1023) == 1023) {
-                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-                if (t0 == 0) t0 = t;
+                const uint32_t now = wait_clock();
+                if (n == 1023) limit = WaitLimit(now);  // a clock reading a millisecond, none for a short wait
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(stop) : "l"(bar + 1) : "memory");
-                if (stop || t - t0 > 2000000000ull) {
+                if (stop || limit.over(now)) {
                     atomicExch(bar + 1, 1u);
                     ok = 0;
                     break;
