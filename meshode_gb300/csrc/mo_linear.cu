@@ -848,17 +848,23 @@ int solve_on(float* V, int64_t nv, const int32_t* F, int64_t nf, const int32_t* 
         const int32_t* cref = with_rot ? nullptr : ref;
         k_lin_merge<<<ceil_div(nv, 128), 128, 0, s>>>(nv, row_ptr, other, key, S.w, S.nbr, S.nnbr); ::mo::note_launch();
         // one block per SM, fewer where blocks would have too few vertices for the barriers to pay
-        const int blocks = (int)std::max<int64_t>(
+        int blocks = (int)std::max<int64_t>(
             1, std::min<int64_t>(std::min(device_sm_count(), CG_MAX_BLOCKS), (nv + CG_MIN_ROWS - 1) / CG_MIN_ROWS));
         CgArgs args{nv, ng, row_ptr, S.nbr, S.nnbr, cref, S.cellw, S.cell_ptr, S.cell_mem, c0, S.V0, S.diag,
                     S.x, S.r, S.dinv, S.z, S.p, S.cellsum, S.partial, S.result, S.bar, tol, max_iter};
         void* argv[] = {&args};
-        const bool one = (nv + blocks - 1) / blocks <= CG_ROWS;
-        const void* kernel = one ? (const void*)k_lin_cg<true> : (const void*)k_lin_cg<false>;
-        const int smem = one ? CG_ROW_BYTES : 0;
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess)
-            e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(CG_THREADS), argv, smem, s);
+        // half of them as long as the process has only a part of the SMs (a partition of
+        // the device): one block always fits
+        for (;; blocks /= 2) {
+            const bool one = (nv + blocks - 1) / blocks <= CG_ROWS;
+            const void* kernel = one ? (const void*)k_lin_cg<true> : (const void*)k_lin_cg<false>;
+            const int smem = one ? CG_ROW_BYTES : 0;
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e == cudaSuccess)
+                e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(CG_THREADS), argv, smem, s);
+            if (e != cudaErrorCooperativeLaunchTooLarge || blocks == 1) break;
+            cudaGetLastError();
+        }
         ::mo::note_launch();
         if (e != cudaSuccess) { fail(e, "k_lin_cg"); break; }
         double result[2];
