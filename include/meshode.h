@@ -31,6 +31,7 @@ extern "C" {
 #define MO_ERR_CUDA 2    /* CUDA runtime error */
 #define MO_ERR_SCRATCH 3 /* caller scratch too small */
 #define MO_ERR_DEVICE 4  /* a kernel reported an error through its status word */
+#define MO_ERR_TOO_LARGE 5 /* the process' part of the GPU cannot hold the call's blocks at once; nothing has run */
 
 #define MO_LAYOUT_LINEAR 0 /* [z][y][x] float, 4*N^3 bytes */
 #define MO_LAYOUT_CELL 1   /* per cell (x,y,z < N-1) its 8 corners, 32 B = one sector */
@@ -414,7 +415,9 @@ int mo_fused_step_on_demand(const MoPair* pairs, const MoTile* tiles, const int3
  * (mo_fused_run_fits).  Results are mo_fused_step's, bit for bit.  tile_loss
  * (may be NULL): the loss partials of step k at tile_loss + k*loss_stride, as
  * launch k of mo_fused_step leaves them for tiles of 8 slices.  sync: two words
- * of device memory.  A wait inside that runs out leaves NaN positions. */
+ * of device memory.  A wait inside that runs out leaves NaN positions.
+ * MO_ERR_TOO_LARGE: in a context with a part of the device's SMs; mo_fused_step
+ * takes the pair as it is. */
 int mo_fused_run_fits(int64_t nv);
 /* Whether it fits and is the faster way for a pair whose longest row of records
  * (mo_sell_plan) is max_rows. */

@@ -11,7 +11,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_lib", "libmeshode.so")
 
-MO_OK, MO_ERR_INVALID, MO_ERR_CUDA, MO_ERR_SCRATCH, MO_ERR_DEVICE = 0, 1, 2, 3, 4
+MO_OK, MO_ERR_INVALID, MO_ERR_CUDA, MO_ERR_SCRATCH, MO_ERR_DEVICE, MO_ERR_TOO_LARGE = 0, 1, 2, 3, 4, 5
 MO_LAYOUT_LINEAR, MO_LAYOUT_CELL, MO_LAYOUT_BRICK4 = 0, 1, 2
 MO_PACKET_4x4x2, MO_PACKET_8x4x1, MO_PACKET_4x2x4, MO_PACKET_2x4x4, MO_PACKET_8x2x2 = 0, 1, 2, 3, 4
 MO_PACKET_4x4x4, MO_PACKET_2x4x8, MO_PACKET_8x4x2 = 5, 6, 7
@@ -194,7 +194,7 @@ _lib = None
 
 
 class MeshodeError(RuntimeError):
-    pass
+    status = None  # of the call that failed
 
 
 def lib():
@@ -222,7 +222,9 @@ def check(rc, what=""):
     if rc != MO_OK:
         msg = lib().mo_last_error()
         msg = msg.decode() if msg else ""
-        raise MeshodeError("%s failed (status %d): %s" % (what, rc, msg))
+        err = MeshodeError("%s failed (status %d): %s" % (what, rc, msg))
+        err.status = rc
+        raise err
 
 
 def call(name, *args):

@@ -649,7 +649,14 @@ extern "C" int mo_fused_run(const MoPair* pair, int weighted, int nsteps, float*
         unsigned* bar = sync;
         MO_CUDA(cudaMemsetAsync(sync, 0, 8, as_stream(stream)));
         void* args[] = {&p, &n, &loss, &loss_stride, &bar};
-        MO_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(32 * warps), args, smem, as_stream(stream)));
+        const cudaError_t e =
+            cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(32 * warps), args, smem, as_stream(stream));
+        if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
+            cudaGetLastError();
+            set_error("%d blocks do not fit this context's SMs at once", blocks);
+            return MO_ERR_TOO_LARGE;
+        }
+        MO_CUDA(e);
         ::mo::note_launch();
         done += n;
     }

@@ -334,8 +334,13 @@ def fused_fit(pid, src_V_norm, steps, lr=1e-3, group_steps=25, use_graph=True, w
     pr = pair_from_template(pid, src_V_norm, steps, lr=lr, w_edge=w_edge, mask_thresh=mask_thresh)
     if pr.steps > 0 and pr.run_pays():
         # every vertex stays on the chip: all steps in one launch
-        losses = pr.run(pr.steps, record_loss)
-        return pr.positions(), losses
+        try:
+            losses = pr.run(pr.steps, record_loss)
+            return pr.positions(), losses
+        except L.MeshodeError as e:
+            if e.status != L.MO_ERR_TOO_LARGE:
+                raise
+            # a part of the SMs only: a launch per step
     runner = StepGroupRunner(pr.device, 1, pr.ntiles, group_steps=group_steps, use_graph=use_graph,
                              weighted=pr.sell_w is not None)
     losses = []

@@ -6,6 +6,11 @@ import subprocess
 import sys
 
 import pytest
+import torch
+
+from meshode_gb300 import _lib as L
+from meshode_gb300 import fused, meshgen
+from meshode_gb300 import pyDeform as PD
 
 pytestmark = pytest.mark.gpu
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -97,10 +102,34 @@ print("OK")
 '''
 
 
-@pytest.mark.parametrize("what", ["solve"])
+@pytest.mark.parametrize("what", ["solve", "fit"])
 def test_part_of_the_gpu(cuda, what):
     r = subprocess.run([sys.executable, "-c", BODY, ROOT, what], capture_output=True, text=True, timeout=300)
     out = r.stdout + r.stderr
     if "SKIP" in r.stdout:
         pytest.skip(r.stdout.strip())
     assert r.returncode == 0 and r.stdout.rstrip().endswith("OK"), out
+
+
+@pytest.mark.parametrize("record", [False, True])
+def test_fit_goes_on_with_a_launch_per_step(cuda, record, monkeypatch):
+    V, F = meshgen.cubesphere(20)
+    V, F = torch.from_numpy((0.4 * V + 0.5).astype("float32")), torch.from_numpy(F.astype("int32"))
+    pid = PD.InitializeDeformTemplate(V, F, 0, 32)
+    PD.StoreRigidityInformation(V, F, pid)
+    X = V + 0.01 * torch.sin(40 * V)
+    want, losses = fused.fused_fit(pid, X, 30, record_loss=record)
+    real = fused.call
+
+    def call(name, *args):
+        if name == "mo_fused_run":
+            err = L.MeshodeError("too large")
+            err.status = L.MO_ERR_TOO_LARGE
+            raise err
+        return real(name, *args)
+
+    monkeypatch.setattr(fused, "call", call)
+    got, losses2 = fused.fused_fit(pid, X, 30, record_loss=record)
+    PD.ReleaseTemplate(pid)
+    assert torch.equal(got, want)
+    assert losses is None and losses2 is None if not record else torch.allclose(losses, losses2, rtol=1e-6, atol=0)
