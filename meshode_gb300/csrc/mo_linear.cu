@@ -36,6 +36,7 @@ constexpr int CG_MIN_ROWS = 16;   // vertices a block should have before another
 constexpr int CG_CHECK = 32;      // iterations between convergence checks
 constexpr int CG_MAX_BLOCKS = 512;
 constexpr int CG_ROW_BYTES = 160 * 1024;  // shared memory for a block's rows of the matrix
+constexpr int CG_MERGE = 128;     // half-edges of a vertex whose neighbours are merged
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -366,23 +367,30 @@ __global__ void k_lin_rhs_rot(int64_t nv, const int* __restrict__ row_ptr, const
 // ---- CG --------------------------------------------------------------------
 // A vertex's unique neighbours with their summed weights, in the order of
 // their first half-edge: a closed mesh names every neighbour twice, and the
-// product with A is bound by the FP64 pipe (2 lanes a clock and SM).
+// product with A is bound by the FP64 pipe (2 lanes a clock and SM).  One thread
+// looks at every pair of a vertex's half-edges, so past CG_MERGE of them they stay
+// as they are.  Measured, ms a solve with one hub (merged, not): 200 half-edges
+// 3.6, 3.15; 400 10.0, 8.2; 1600 121, 74; 3200 452, 257 (of which the vertex ->
+// half-edge list 147).
 __global__ void k_lin_merge(int64_t nv, const int* __restrict__ row_ptr, const int* __restrict__ other,
                             const int* __restrict__ key, const double* __restrict__ w, int4* __restrict__ nbr,
                             int32_t* __restrict__ nnbr) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nv) return;
     const int b = row_ptr[i], e = row_ptr[i + 1];
+    const bool merge = e - b <= CG_MERGE;
     int n = 0;
     for (int k = b; k < e; ++k) {
         const int o = other[k];
         if (o == i) continue;  // a self-loop's entries cancel
-        bool seen = false;
-        for (int j = b; j < k && !seen; ++j) seen = other[j] == o;
-        if (seen) continue;
         double s = w[key[k] >> 1];
-        for (int j = k + 1; j < e; ++j)
-            if (other[j] == o) s += w[key[j] >> 1];
+        if (merge) {
+            bool seen = false;
+            for (int j = b; j < k && !seen; ++j) seen = other[j] == o;
+            if (seen) continue;
+            for (int j = k + 1; j < e; ++j)
+                if (other[j] == o) s += w[key[j] >> 1];
+        }
         nbr[b + n] = make_int4(o, 0, __double2loint(s), __double2hiint(s));
         ++n;
     }
