@@ -88,13 +88,13 @@ enum Misc { M_INV2, M_INV3, M_B4, M_N1 = 5, M_MB1, M_N2, M_MB2, M_M4, M_N3 };
 // ---- small pieces ----------------------------------------------------------
 __device__ __forceinline__ uint32_t s32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// The power of two that brings a magnitude mx into [2^14, 2^15), and its
-// inverse.  The exponents are clamped so that the product of a row's and a
-// matrix's inverse is a normal float: rows keep full precision down to 2e-25
-// (LO = -40, HI = 96), matrices down to 2^-16 (HI = 30).
+// The power of two that brings a magnitude mx into [2^14, 2^15), up to the largest
+// finite one, and its inverse.  Small ones stay smaller, so that the product of a
+// row's and a matrix's inverse is a normal float: rows keep full precision down to
+// 2e-25 (HI = 96), matrices down to 2^-16 (HI = 30).
 template <int HI = 96>
 __device__ __forceinline__ float pow2_scale(float mx, float* inv) {
-    const int e = min(max(141 - ((__float_as_int(mx) >> 23) & 255), -40), HI);
+    const int e = min(max(141 - ((__float_as_int(mx) >> 23) & 255), 141 - 254), HI);
     *inv = __int_as_float((127 - e) << 23);
     return __int_as_float((127 + e) << 23);
 }
@@ -1430,7 +1430,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             float* out = A.partial + ((int64_t)blockIdx.y * W + o0 + o) * W + i0 + (w >> 2) * NC;
 #pragma unroll
             for (int j = 0; j < NC; ++j) {
-                const float x = acc[j] * ginv * hinv;
+                const float x = acc[j] * (ginv * hinv);
                 const float v = bad ? NAN : fmaf(x, 2e-8f, x);  // the mean loss of 4-step chains
                 out[j] = A.first ? v : out[j] + v;
             }
