@@ -1423,6 +1423,9 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             bar_wait(done + 8 * (k & 1), (k >> 1) & 1, late);
             drain(k & 1);
         }
+        // the two inverse scales as two factors of about the same size: neither alone overflows
+        const int e = (__float_as_int(ginv) >> 23) + (__float_as_int(hinv) >> 23) - 254, e1 = e >> 1;
+        const float s1 = __int_as_float((127 + e1) << 23), s2 = __int_as_float((127 + e - e1) << 23);
         const int o = 32 * (w & 3) + lane;
         const bool bad = *late || was_late;
         if (bad) spoil(A.misc);
@@ -1430,7 +1433,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) k_tc_wgrad(WgradArgs A) {
             float* out = A.partial + ((int64_t)blockIdx.y * W + o0 + o) * W + i0 + (w >> 2) * NC;
 #pragma unroll
             for (int j = 0; j < NC; ++j) {
-                const float x = acc[j] * (ginv * hinv);
+                const float x = acc[j] * s1 * s2;
                 const float v = bad ? NAN : fmaf(x, 2e-8f, x);  // the mean loss of 4-step chains
                 out[j] = A.first ? v : out[j] + v;
             }

@@ -5,6 +5,7 @@ array's scale, as in test_gpu_mlp_tc.py)."""
 import pytest
 import torch
 
+from meshode_gb300 import _lib as L
 from meshode_gb300 import neuralode
 
 pytestmark = pytest.mark.gpu
@@ -63,3 +64,32 @@ def test_large_gradients(cuda, m, top):
     assert ((got[0].double() - want[0]).abs().max(1).values <= 1e-5 * row).all()
     for a, b in zip(got[1:], want[1:]):
         assert (a.double() - b).abs().max() <= 1e-5 * b.abs().max()
+
+
+@pytest.mark.parametrize("W", [64, 128, 256])
+@pytest.mark.parametrize("gmax,hmax", [(1e38, 1e38), (1e38, 1e-3), (1e-3, 1e38), (1e-20, 1e30), (1.0, 1.0)])
+def test_weight_gradient_scales(cuda, W, gmax, hmax):
+    """The arrays' two scales, whose product is no float: sums that are zero stay
+    zero, others are right."""
+    rows, s, lib = 1024, L.stream_ptr(), L.lib()
+    P = neuralode._Packed(neuralode.init_params(W, 5, cuda))
+    bounds = P.buf[-32:-16].view(torch.float32)  # of |H1|, |H2|, |G2|, |G3|
+    bounds.copy_(torch.tensor([hmax, hmax, gmax, gmax]))
+    g = torch.Generator().manual_seed(W)
+    G, H = [(torch.rand(rows * W, generator=g) * 2 - 1).to(cuda) for _ in range(2)]
+    H *= hmax
+    n = int(lib.mo_mlp_tc_wgrad_floats(rows, W))
+
+    def sums(G):
+        part = torch.full((n,), float("nan"), device=cuda)
+        L.call("mo_mlp_tc_wgrad", L.ptr(G), L.ptr(H), rows, L.ptr(P.buf), W, 2, L.ptr(part), 1, s)
+        splits = n // (W * W + (2 if W < 128 else 1) * W)
+        return part[:splits * W * W].view(splits, W, W).double().sum(0)
+
+    assert (sums(torch.zeros_like(G)) == 0).all()
+    scale = gmax if gmax * hmax < 1e35 else 1e35 / hmax if 1e35 / hmax > gmax * 2.0 ** -16 else None
+    if scale is not None:  # the sums are finite, and G not 17 binades below its bound
+        got = sums(G * scale)
+        cols = [t.double().view(rows // 128, W // 8, 128, 8).permute(0, 2, 1, 3).reshape(rows, W) for t in (G * scale, H)]
+        want = cols[0].t() @ cols[1]
+        assert (got - want).abs().max() <= 1e-5 * want.abs().max()
