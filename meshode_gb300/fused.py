@@ -21,6 +21,7 @@ from ._lib import call, ptr, stream_ptr
 PAIR_BYTES = ctypes.sizeof(L.MoPair)
 TILE_BYTES = ctypes.sizeof(L.MoTile)
 SLICES_PER_TILE = 8
+RUN_LOSS_STEPS = 4096  # steps of a run whose loss partials are held at once (120 MB at the most vertices)
 # int32 word offsets of the per-group fields inside a MoPair row
 _OFF_T0 = L.MoPair.t0.offset // 4
 _OFF_TILE0 = L.MoPair.tile0.offset // 4
@@ -180,20 +181,26 @@ class Pair:
 
     def run(self, nsteps, record_loss=False):
         """The next nsteps steps in one launch (mo_fused_run); the per-step
-        losses (float64 [nsteps]) or None."""
+        losses (float64 [nsteps]) or None.  With them RUN_LOSS_STEPS at a time:
+        every step leaves a float a slice."""
         nt = tiles_for(self.nslices)
-        row = self.struct(self.t, 0, nt)
         stride = nt * SLICES_PER_TILE
-        partial = torch.empty(nsteps * stride, dtype=torch.float32, device=self.device) if record_loss else None
         sync = torch.empty(2, dtype=torch.int32, device=self.device)
-        call("mo_fused_run", ctypes.byref(row), int(self.sell_w is not None), int(nsteps), ptr(partial), stride,
-             ptr(sync), stream_ptr())
-        self.t += nsteps
+        weighted = int(self.sell_w is not None)
         if not record_loss:
+            call("mo_fused_run", ctypes.byref(self.struct(self.t, 0, nt)), weighted, int(nsteps), None, stride,
+                 ptr(sync), stream_ptr())
+            self.t += nsteps
             return None
-        table = torch.from_numpy(np.frombuffer(bytes(row), np.uint8).copy()).to(self.device)
         out = torch.empty(nsteps, dtype=torch.float64, device=self.device)
-        call("mo_pair_loss", ptr(table), 1, nt, int(nsteps), ptr(partial), ptr(out), stream_ptr())
+        partial = torch.empty(min(nsteps, RUN_LOSS_STEPS) * stride, dtype=torch.float32, device=self.device)
+        for k in range(0, nsteps, RUN_LOSS_STEPS):
+            n = min(RUN_LOSS_STEPS, nsteps - k)
+            row = self.struct(self.t, 0, nt)
+            call("mo_fused_run", ctypes.byref(row), weighted, n, ptr(partial), stride, ptr(sync), stream_ptr())
+            self.t += n
+            table = torch.from_numpy(np.frombuffer(bytes(row), np.uint8).copy()).to(self.device)
+            call("mo_pair_loss", ptr(table), 1, nt, n, ptr(partial), ptr(out[k:]), stream_ptr())
         return out
 
 
