@@ -28,6 +28,7 @@ from . import objio
 from ._lib import call, ptr, stream_ptr
 
 DEFAULT_LAYOUT = L.MO_LAYOUT_CELL
+GRID_AT_ONCE = 1 << 30  # bytes of a laid-out grid up to which it is made in the call that builds the field
 
 
 class _EdgeState:
@@ -300,9 +301,15 @@ def InitializeDeformTemplate(tensorV, tensorF, symmetry, grid_resolution, layout
     nbytes = L.lib().mo_df_build_scratch_bytes(Vd.shape[0], Fd.shape[0], N, int(df_method))
     scratch = torch.empty(int(nbytes), dtype=torch.uint8, device=dev)
     p.grid_linear = torch.empty(N * N * N, dtype=torch.float32, device=dev)
-    p.grid = p.grid_linear if p.layout == L.MO_LAYOUT_LINEAR else torch.empty(nb // 4, dtype=torch.float32, device=dev)
-    call("mo_template_build", ptr(Vd), Vd.shape[0], ptr(Fd), Fd.shape[0], N, int(df_method), p.layout, ptr(bbox),
+    # a large grid is laid out when the build has been checked and its scratch is free again
+    layout = p.layout if nb <= GRID_AT_ONCE else L.MO_LAYOUT_LINEAR
+    p.grid = p.grid_linear if layout == L.MO_LAYOUT_LINEAR else torch.empty(nb // 4, dtype=torch.float32, device=dev)
+    call("mo_template_build", ptr(Vd), Vd.shape[0], ptr(Fd), Fd.shape[0], N, int(df_method), layout, ptr(bbox),
          ptr(p.params), ptr(scratch), nbytes, ptr(p.grid_linear), ptr(p.grid), s)
+    if layout != p.layout:
+        del scratch
+        p.grid = torch.empty(nb // 4, dtype=torch.float32, device=dev)
+        call("mo_grid_relayout", ptr(p.grid_linear), N, p.layout, ptr(p.grid), s)
     _g_params.append(p)
     return len(_g_params) - 1
 
