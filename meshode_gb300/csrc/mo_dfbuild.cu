@@ -1012,10 +1012,13 @@ static BuildScratch plan_scratch(char* base, int64_t nv, int64_t nf, int method)
         s.boxes = reinterpret_cast<float4*>(take(sizeof(float4) * 2 * (size_t)nf));
         s.parent = reinterpret_cast<int*>(take(sizeof(int) * (size_t)(2 * nf)));
         s.flags = reinterpret_cast<int*>(take(sizeof(int) * (size_t)nf));
-        s.hist = reinterpret_cast<int*>(take(sizeof(int) * radix_hist_ints((int)nf)));
         s.range = reinterpret_cast<int2*>(take(sizeof(int2) * (size_t)(nf > 1 ? nf - 1 : 1)));
+        // the sort is over before the boxes are made: its words (8 bytes a key) lie where they go
+        const size_t sort = o + align256(sizeof(int) * radix_hist_ints((int)nf));
+        s.hist = reinterpret_cast<int*>(base ? base + o : nullptr);
         s.obb = reinterpret_cast<float4*>(take(sizeof(float4) * 4 * (size_t)(nf > 1 ? nf - 1 : 1)));
         s.tnodes = reinterpret_cast<float4*>(take(sizeof(float4) * NODE_F4 * (size_t)(nf > 1 ? nf - 1 : 1)));
+        o = std::max(o, sort);
     } else {
         s.codes_a = s.codes_b = nullptr;
         s.ids_a = s.ids_b = nullptr;
