@@ -36,6 +36,7 @@ constexpr int CG_MIN_ROWS = 16;   // vertices a block should have before another
 constexpr int CG_CHECK = 32;      // iterations between convergence checks
 constexpr int CG_MAX_BLOCKS = 512;
 constexpr int CG_ROW_BYTES = 160 * 1024;  // shared memory for a block's rows of the matrix
+constexpr int CG_FEW = 8;         // members of a cell that one lane sums
 constexpr int CG_MERGE = 128;     // half-edges of a vertex whose neighbours are merged
 
 size_t a256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -525,7 +526,11 @@ __device__ __forceinline__ void grid_sum3(const double* part, Then then) {
 // with the rows read from L2, two more loads a vertex and chains of eleven
 // additions).  Eight lanes a cell instead of a warp: 41k 25; fewer than 16 vertices
 // a block were not tried, 64 took 5% longer at 2k to 8k.
-template <bool ONE>
+//
+// MANY (four turns of a warp a sum and more; a cell a vertex at 15k, 100k and 300k
+// vertices, where the kernels before took 40, 60 and 123 us an iteration): 39, 158 and
+// 447 us with a warp a sum, 20, 32 and 71 so; cells of 16 at 300k 80 and 82.
+template <bool ONE, bool MANY>
 __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
     extern __shared__ int4 rows[];  // ONE: this block's rows, if they fit
     __shared__ double sh[CG_THREADS], sh2[CG_THREADS];
@@ -591,7 +596,8 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
     };
     // cellsum = sums of value(member, coordinate) over the cells: a warp per
     // coordinate of a cell, its loads in flight together, or a block where cells
-    // are large
+    // are large.  MANY: more sums than the grid's warps take in a few turns; a warp
+    // takes up to 32 at once, and a lane each of those with few members
     auto cells = [&](auto value) {
         if (A.nv >= A.ng * 1024) {
             for (int64_t g = blockIdx.x; g < A.ng; g += gridDim.x) {
@@ -606,6 +612,39 @@ __global__ void __launch_bounds__(CG_THREADS) k_lin_cg(CgArgs A) {
             return;
         }
         const int lane = tid & 31;
+        if (MANY) {
+            const int64_t sums = 3 * A.ng, warps = (int64_t)gridDim.x * (CG_THREADS / 32);
+            const int at_once = (int)min((int64_t)32, (sums + warps - 1) / warps);
+            for (int64_t q0 = (blockIdx.x + gridDim.x * (int64_t)(tid >> 5)) * at_once; q0 < sums;
+                 q0 += warps * at_once) {
+                const int64_t q = q0 + lane, g = q / 3;
+                const int k0 = (int)(q - 3 * g);
+                int b = 0, n = -1;
+                if (lane < at_once && q < sums) {
+                    b = A.cell_ptr[g];
+                    n = A.cell_ptr[g + 1] - b;
+                    if (n <= CG_FEW) {
+                        double s = 0.0;
+                        for (int k = b; k < b + n; ++k) s += value(A.cell_mem[k], k0);
+                        A.cellsum[q] = s;
+                    }
+                }
+                unsigned m = __ballot_sync(0xffffffffu, n > CG_FEW);
+                while (m) {
+                    const int l = __ffs(m) - 1;
+                    m &= m - 1;
+                    const int b0 = __shfl_sync(0xffffffffu, b, l), e = b0 + __shfl_sync(0xffffffffu, n, l);
+                    const int kl = __shfl_sync(0xffffffffu, k0, l);
+                    double s = 0.0;
+#pragma unroll 4
+                    for (int k = b0 + lane; k < e; k += 32) s += value(A.cell_mem[k], kl);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                    if (lane == l) A.cellsum[q] = s;
+                }
+            }
+            return;
+        }
         for (int64_t q = blockIdx.x + gridDim.x * (int64_t)(tid >> 5); q < 3 * A.ng; q += gridDim.x * (CG_THREADS / 32)) {
             const int64_t g = q / 3;
             const int k0 = (int)(q - 3 * g), e = A.cell_ptr[g + 1];
@@ -865,7 +904,9 @@ int solve_on(float* V, int64_t nv, const int32_t* F, int64_t nf, const int32_t* 
         // the device): one block always fits
         for (;; blocks /= 2) {
             const bool one = (nv + blocks - 1) / blocks <= CG_ROWS;
-            const void* kernel = one ? (const void*)k_lin_cg<true> : (const void*)k_lin_cg<false>;
+            const bool many = cref && nv < ng * 1024 && 3 * ng > (int64_t)4 * blocks * (CG_THREADS / 32);
+            const void* kernel = many ? (one ? (const void*)k_lin_cg<true, true> : (const void*)k_lin_cg<false, true>)
+                                      : (one ? (const void*)k_lin_cg<true, false> : (const void*)k_lin_cg<false, false>);
             const int smem = one ? CG_ROW_BYTES : 0;
             e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e == cudaSuccess)
