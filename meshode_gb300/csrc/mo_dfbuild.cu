@@ -851,6 +851,9 @@ static void launch_df_lbvh(int packet, const float4* nodes, const float4* tris, 
 // Measured (records and grid, us): see mo_df_method_for.
 constexpr int BF_WARPS = 8;
 constexpr int BF_P = 4;  // packet edge, voxels
+// Triangles that are all tested: bounding them first costs as much (a template at
+// 400^3, us, bounded and not: 1 triangle 598, 501; 4 746, 698; 8 921, 947).
+constexpr int BF_TEST_ALL = 4;
 constexpr float CULL_SLACK = 2e-6f;
 // The nearest centroid is that of the least |p - c|^2 + CULL_R2 r^2, whose r is at
 // most |p - c| / sqrt(CULL_R2): the slack of U without a root per triangle.
@@ -902,11 +905,11 @@ __global__ void __launch_bounds__(BF_WARPS * 32) k_df_brute(const float4* __rest
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int part = w & (split - 1);
-    const int64_t brick = ((int64_t)blockIdx.x * BF_WARPS + w) / split;
-    const bool live = brick < bf_bricks(N);  // a warp past the last packet only follows
-    const int nb = (N + BF_P - 1) / BF_P;
-    const int64_t b = live ? brick : 0;
-    const int ix = (int)(b % nb), iy = (int)((b / nb) % nb), iz = (int)(b / ((int64_t)nb * nb));
+    // 32-bit: at most 2^27 packets (N <= 2048), and several warps a packet only for few
+    const unsigned nb = (N + BF_P - 1) / BF_P, brick = (blockIdx.x * BF_WARPS + w) >> (__ffs(split) - 1);
+    const bool live = brick < nb * nb * nb;  // a warp past the last packet only follows
+    const unsigned b = live ? brick : 0, by = b / nb;
+    const int ix = (int)(b - by * nb), iy = (int)(by % nb), iz = (int)(by / nb);
     const int x = ix * BF_P + (lane & 3), y = iy * BF_P + ((lane >> 2) & 3);
     const int za = iz * BF_P + (lane >> 4), zb = za + 2;
     const bool va = live && x < N && y < N && za < N, vb = live && x < N && y < N && zb < N;
@@ -916,12 +919,13 @@ __global__ void __launch_bounds__(BF_WARPS * 32) k_df_brute(const float4* __rest
     const VoxelBand ba = voxel_band(x, y, za, N, band, band2), bb = voxel_band(x, y, zb, N, band, band2);
     float2 best = make_float2(ba.bound2, bb.bound2);
     const float half = 0.5f * (BF_P - 1);
-    const float cx = (ix * BF_P + half) / Nf, cy = (iy * BF_P + half) / Nf, cz = (iz * BF_P + half) / Nf;
-    const float R = 1.7320508f * half / Nf;
+    const float rN = 1.0f / Nf;
+    const float cx = (ix * BF_P + half) * rN, cy = (iy * BF_P + half) * rN, cz = (iz * BF_P + half) * rN;
+    const float R = 1.7320508f * half * rN;
     const int first = part + split * lane, stride = 32 * split;
 
     float u = FLT_MAX;
-    for (int t = first; t < ntri; t += stride) {
+    for (int t = first; t < ntri && ntri > BF_TEST_ALL; t += stride) {
         float d2, r2;
         tri_sphere(tris, t, cx, cy, cz, &d2, &r2);
         u = fminf(u, fmaf(r2, CULL_R2, d2));
@@ -932,13 +936,13 @@ __global__ void __launch_bounds__(BF_WARPS * 32) k_df_brute(const float4* __rest
     for (int k = 0; k < split; ++k) u = fminf(u, sh_u[(w & ~(split - 1)) + k]);
     u = sqrtf(u);
     float U = u + CULL_SLACK * (1.f + (1.f + CULL_R) * u) + R;
-    if (band2 != FLT_MAX) U = fminf(U, band + 13.0f / Nf);  // the widest band of any voxel
+    if (band2 != FLT_MAX) U = fminf(U, band + 13.0f * rN);  // the widest band of any voxel
     const float reach = U + R + CULL_SLACK;  // beside r, and with 1 - CULL_SLACK of |p - c|
 
     for (int base = 0; base < ntri; base += stride) {
         const int t = base + first;
         bool keep = live && t < ntri;
-        if (keep) {
+        if (keep && ntri > BF_TEST_ALL) {
             float d2, r2;
             tri_sphere(tris, t, cx, cy, cz, &d2, &r2);
             keep = !((1.f - CULL_SLACK) * sqrtf(d2) > fmaf(sqrtf(r2), 1.f + CULL_SLACK, reach));  // NaN: tested
