@@ -38,7 +38,7 @@ extern "C" {
 #define MO_LAYOUT_BRICK4 2 /* 4x4x4 bricks of 256 B, bricks and voxels [z][y][x], N padded to 4 */
 
 #define MO_DF_AUTO 0
-#define MO_DF_BRUTE 1 /* shared-memory-tiled brute force (small targets) */
+#define MO_DF_BRUTE 1 /* brute force over packets of voxels (small targets) */
 #define MO_DF_LBVH 2  /* Morton codes + radix sort + Karras LBVH + warp packet traversal */
 
 #define MO_EDGES_FACES 0 /* idx = F[m,3]; half-edge 3f+j = (F[f][j], F[f][(j+1)%3]) */
@@ -670,7 +670,8 @@ int mo_mlp_wgrad(const float* A, const float* B, int64_t rows, int splits, float
  * W = mo_mlp_tc_width(m) = 64, 128 or 256; -1 for other m).  Arrays of n rows x
  * W columns are padded to mo_mlp_tc_rows(n) rows (whole 128-row tiles) and
  * stored in blocks of 8 columns: element (row, c) of tile t at
- * ((t*(W/8) + c/8)*128 + row)*8 + c%8. */
+ * ((t*(W/8) + c/8)*128 + row)*8 + c%8.  A wait inside that runs out leaves NaN in
+ * the call's outputs and in the pack, and so in all that later calls make. */
 int mo_mlp_tc_width(int m);
 int64_t mo_mlp_tc_rows(int64_t n);
 size_t mo_mlp_tc_pack_bytes(int W);

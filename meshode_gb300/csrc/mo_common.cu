@@ -104,7 +104,8 @@ cudaError_t exclusive_scan_i32(int* data, int n, int* total, cudaStream_t s) {
 }
 
 // ---------------------------------------------------------------------------
-// Stable LSD radix sort, 8-bit digits, one kernel per digit.  One pass over the
+// Stable LSD radix sort, 8-bit digits, one kernel per digit by decoupled look-back
+// (Merrill and Garland 2016; for sorting Adinets and Merrill 2022).  One pass over the
 // keys counts every digit of every pass; then each pass is a single kernel:
 // a tile ranks its keys (per-warp ranks from __match_any_sync, warps in order),
 // publishes its digit counts and adds up its predecessors' by looking back over

@@ -5,7 +5,8 @@
 //
 // The row-major FP32 kernels of the C ABI (mo_mlp_*), all arithmetic on the SIMT
 // pipes (packed FFMA2).  The velocity field itself runs on mo_mlp_tc.cu's
-// tensor-core kernels (3 to 6 times these kernels' speed, the same accuracy).
+// tensor-core kernels (3 to 6 times these kernels' speed; their accuracy beside
+// these kernels' stands there).
 //
 //   k_mlp_fwd    one MLP evaluation of a 64-vertex tile with its RK4 stage
 //                update: the 3-wide input layer, the two 256x256 layers and

@@ -4,11 +4,13 @@
 // W = 64, 128 or 256; a narrower hidden layer is zero-padded to the next W).
 //
 // FP32 accuracy from FP16 products.  Every operand x of a contraction is
-// scaled by a power of two (per row for activations and their gradients, per
-// matrix for weights, per array for the weight gradients) so that its largest
-// magnitude lies in [2^14, 2^15), and split into hi = fp16(x) and
-// lo = fp16(x - hi): 22 bits, full over 17 binades below the maximum.  A
-// product is hi*hi + hi*lo + lo*hi (lo*lo is below 2^-24 of it), accumulated
+// scaled by a power of two so that a bound of its magnitude lies in [2^14, 2^15):
+// the largest magnitude of a weight matrix; for a row of activations or their
+// gradients what its inputs and the weights' norms allow, up to a few binades above
+// its values; for the weight gradients the largest such bound that any call on the
+// packed parameters has seen.  It is split into hi = fp16(x) and lo = fp16(x - hi):
+// 22 bits down to 2^-17 of the bound, a bit less for every binade below, nothing
+// below 2^-39.  A product is hi*hi + hi*lo + lo*hi (lo*lo is below 2^-24 of it), accumulated
 // in FP32 in tensor memory.  That accumulation truncates toward zero: of a
 // 256-long sum of positive activations times weights of both signs, chains of
 // 16 / 8 / 4 / 2 / 1 steps (K = 16 each) lose 2.8 / 1.5 / 0.9 / 0.6 / 0.4 e-7
@@ -18,7 +20,16 @@
 // accumulators of W/64 steps, of 4 for the weight gradients), the accumulators are added in FP32 registers
 // with rounding to nearest, and the mean loss that is left is given back: the
 // split weights are those of W * (1 + loss), the weight gradients are scaled at
-// the end (constants fitted to FP64 gradients).
+// the end (constants fitted to FP64 gradients; they are right on average for sums of
+// positive activations and a bias of their size, 2e-8 to 6e-8, for others).
+// Against FP64 and beside the FP32 kernels of mo_mlp.cu (relative L2 errors of
+// states and gradients, widths 64 and 256, two steps): Xavier weights 0.4e-7 to
+// 1.5e-7 (0.7e-7 to 2.2e-7); weights of lognormal size, one weight 1e3 times the
+// others: 0.3 to 1.3 of theirs; weights of 1e-3 and 1e-6 of Xavier's: states 1.9e-7
+// and 2.7e-7 (1.4e-7 and 1.6e-7), gradients 0.4 to 1.0 of theirs; rows or columns that
+// differ tenfold either way: below 3e-7.  Beyond that the bounds leave fewer bits:
+// with one weight 1e5 times the others states are 2e-6 to 3e-6 off (0.5e-6 to 2e-6)
+// and weight gradients up to 2e-3, more where the flow itself grows to 1e9.
 //
 //   k_tc_pack   parameters -> operand images (the exact shared-memory layout:
 //               K-major rows of 64 halves, 128-byte swizzle), in the order
@@ -1209,39 +1220,39 @@ __global__ void __launch_bounds__(THREADS, 1) k_tc_bwd(std::conditional_t<STEP, 
                 epi_sync();
             }
             // a column's four lanes (and row ranges) together; db4: the rows of group 0
-                float* sums = scratch;  // [SUM_PARTS][8][W]: dW4 (3), -, dW1 (3), db1
-                float* xs = reinterpret_cast<float*>(smem + C::ROWS);
+            float* sums = scratch;  // [SUM_PARTS][8][W]: dW4 (3), -, dW1 (3), db1
+            float* xs = reinterpret_cast<float*>(smem + C::ROWS);
 #pragma unroll
-                for (int q = 0; q < SB; ++q)
+            for (int q = 0; q < SB; ++q)
 #pragma unroll
-                    for (int d = 0; d < 7; ++d) {
-                        float v = d < 3 ? s4[q][d < 3 ? d : 0] : s1[q][d < 3 ? 0 : d - 3];
-                        v += __shfl_xor_sync(0xffffffffu, v, 8);
-                        v += __shfl_xor_sync(0xffffffffu, v, 16);
-                        if (lane < 8) sums[(row0 / PART_ROWS * 8 + d + (d >= 3)) * W + 8 * (blk + 16 * q) + cl] = v;
-                    }
-                if (g == 0) {
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        for (int o = 16; o > 0; o >>= 1) sg[d] += __shfl_xor_sync(0xffffffffu, sg[d], o);
-                        if (lane == 0) xs[4 * d + w] = sg[d];
-                    }
+                for (int d = 0; d < 7; ++d) {
+                    float v = d < 3 ? s4[q][d < 3 ? d : 0] : s1[q][d < 3 ? 0 : d - 3];
+                    v += __shfl_xor_sync(0xffffffffu, v, 8);
+                    v += __shfl_xor_sync(0xffffffffu, v, 16);
+                    if (lane < 8) sums[(row0 / PART_ROWS * 8 + d + (d >= 3)) * W + 8 * (blk + 16 * q) + cl] = v;
                 }
-                epi_sync();
-                // the sums over all products of a backward pass, with their rounding errors beside them
-                for (int e = threadIdx.x; e < 8 * W; e += EPI) {
-                    const int k = e / W, c = e % W;
-                    float v = sums[e];
-                    if (C::SUM_PARTS == 2) v += sums[8 * W + e];
-                    if (*B.late || isnan(inv2)) v = NAN;
-                    else if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
-                    float* out = A.partial + (int64_t)blockIdx.x * 16 * W + e;
-                    const bool first = A.first && j == 0;
-                    const float h = first ? 0.f : *out, y = first ? v : __fadd_rn(v, out[8 * W]);
-                    const float t = __fadd_rn(h, y), b = __fsub_rn(t, h);
-                    *out = t;
-                    out[8 * W] = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(y, b));
+            if (g == 0) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    for (int o = 16; o > 0; o >>= 1) sg[d] += __shfl_xor_sync(0xffffffffu, sg[d], o);
+                    if (lane == 0) xs[4 * d + w] = sg[d];
                 }
+            }
+            epi_sync();
+            // the sums over all products of a backward pass, with their rounding errors beside them
+            for (int e = threadIdx.x; e < 8 * W; e += EPI) {
+                const int k = e / W, c = e % W;
+                float v = sums[e];
+                if (C::SUM_PARTS == 2) v += sums[8 * W + e];
+                if (*B.late || isnan(inv2)) v = NAN;
+                else if (k == 3) v = c < 3 ? (xs[4 * c] + xs[4 * c + 1]) + (xs[4 * c + 2] + xs[4 * c + 3]) : 0.f;
+                float* out = A.partial + (int64_t)blockIdx.x * 16 * W + e;
+                const bool first = A.first && j == 0;
+                const float h = first ? 0.f : *out, y = first ? v : __fadd_rn(v, out[8 * W]);
+                const float t = __fadd_rn(h, y), b = __fsub_rn(t, h);
+                *out = t;
+                out[8 * W] = __fadd_rn(__fsub_rn(h, __fsub_rn(t, b)), __fsub_rn(y, b));
+            }
             if (STEP && j < 3) epi_sync();
         }
         const uint32_t m2 = __reduce_max_sync(0xffffffffu, __float_as_uint(gm2));

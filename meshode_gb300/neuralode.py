@@ -20,11 +20,12 @@ the graph/DF losses, back-propagating through the stored RK4 graph.  Here:
 
 The evaluations of the MLP are one fused libmeshode kernel (mo_mlp_tc_fwd:
 the four layers of 128-vertex tiles with their activations kept on chip, and
-the RK4 stage update; a flow's evaluations are one launch of it), its vector-Jacobian product another (mo_mlp_tc_bwd), and
-the hidden weights' gradients a split-K kernel over the four stages of a step
-(mo_mlp_tc_wgrad); a flow's evaluations are issued by one call (mo_ode_flow,
-mo_ode_flow_backward).  Their contractions run on the tensor cores in FP16 pairs
-that carry 22 bits, accumulated in FP32; everything else is FP32.
+the RK4 stage update; a flow's evaluations are one launch of it), its
+vector-Jacobian product another (mo_mlp_tc_bwd), and the hidden weights'
+gradients a split-K kernel over the four stages of a step (mo_mlp_tc_wgrad); a
+flow's evaluations are issued by one call (mo_ode_flow, mo_ode_flow_backward).
+Their contractions run on the tensor cores in FP16 pairs that carry 22 bits,
+accumulated in FP32; everything else is FP32.
 """
 import math
 
