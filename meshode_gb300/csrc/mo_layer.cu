@@ -7,9 +7,11 @@
 // 2-8 us for 10k vertices, each behind its own call from the host (445 us for
 // an evaluation with its gradient, 291 now, nearly all of it the host), and 12
 // bytes a half-edge written and read twice.  Here the terms are summed where
-// they are made.  Every term is rounded as before; the sums are kept in
-// double, a block's in the order of its threads, so the loss is the same in
-// every run.
+// they are made.  Every term is rounded as before; a thread's sum keeps its
+// rounding errors, a block's is in double in the order of its threads, so the loss
+// is the same in every run.
+#include <algorithm>
+
 #include "mo_df_eval.cuh"
 #include "mo_edge.cuh"
 
@@ -28,22 +30,41 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
     return v;  // thread 0
 }
 
-// Blocks [0, vblocks): 0.5 d^2 of a vertex a thread (and with GRAD the
+// A sum of floats that are not negative and its rounding errors (Knuth's two-sum):
+// as good as double for a fraction of the time of 2 FP64 lanes a clock and SM.
+struct Sum {
+    float hi = 0.f, lo = 0.f;
+    __device__ __forceinline__ void add(float x) {
+        const float t = ADD(hi, x), b = SUB(t, hi);
+        lo = ADD(lo, ADD(SUB(hi, SUB(t, b)), SUB(x, b)));
+        hi = t;
+    }
+    __device__ __forceinline__ double value() const { return isfinite(hi) ? (double)hi + (double)lo : (double)hi; }
+};
+
+// Blocks of a kind at most: past them a thread takes several vertices or half-edges,
+// since a block's sum in double costs 5 FP64 instructions a thread.  (With one each and
+// all sums in double a loss over 60 M half-edges took 1640 us, as separate calls 890.
+// 378 here.)
+constexpr int LAYER_BLOCKS = 2048;
+static int layer_blocks(int64_t n) { return (int)std::min<int64_t>((n + LAYER_THREADS - 1) / LAYER_THREADS, LAYER_BLOCKS); }
+
+// Blocks [0, vblocks): 0.5 d^2 of the vertices (and with GRAD the
 // distance term's gradient, zeroed where 0.5 d^2 >= mask).  The others:
-// 0.5 r^2 of a half-edge a thread.  partial[block] = the block's sum.
+// 0.5 r^2 of the half-edges.  partial[block] = the block's sum.
 template <int LAYOUT, bool GRAD>
 __global__ void __launch_bounds__(LAYER_THREADS)
     k_layer_forward(const float* __restrict__ V, int64_t nv, const float* __restrict__ grid, int N, float Nf, float Cf,
                     const int32_t* __restrict__ idx, int64_t nh, int kind, const float* __restrict__ off, int vblocks,
                     float mask, double* __restrict__ partial, float* __restrict__ grad) {
     __shared__ double sh[LAYER_THREADS / 32];
-    double sum = 0.0;
+    Sum sum;
     if ((int)blockIdx.x < vblocks) {
-        const int64_t i = (int64_t)blockIdx.x * LAYER_THREADS + threadIdx.x;
-        if (i < nv) {
+        for (int64_t i = (int64_t)blockIdx.x * LAYER_THREADS + threadIdx.x; i < nv;
+             i += (int64_t)vblocks * LAYER_THREADS) {
             const DFJet j = df_eval<LAYOUT, GRAD>(grid, N, Nf, Cf, V[3 * i], V[3 * i + 1], V[3 * i + 2]);
             const float half = MUL(MUL(j.d, j.d), 0.5f);
-            sum = (double)half;
+            sum.add(half);
             if (GRAD) {
                 const float m = half < mask ? 1.0f : 0.0f;
                 grad[3 * i] = MUL(df_grad_component(j.d, j.gx), m);
@@ -52,22 +73,21 @@ __global__ void __launch_bounds__(LAYER_THREADS)
             }
         }
     } else {
-        const int64_t h = (int64_t)(blockIdx.x - vblocks) * LAYER_THREADS + threadIdx.x;
-        if (h < nh) {
+        const int64_t step = (int64_t)(gridDim.x - vblocks) * LAYER_THREADS;
+#pragma unroll 2
+        for (int64_t h = (int64_t)(blockIdx.x - vblocks) * LAYER_THREADS + threadIdx.x; h < nh; h += step) {
             int v0, v1;
             he_ends(idx, kind, h, v0, v1);
-            if (!in_range(v0, nv) || !in_range(v1, nv)) {
-                sum = (double)__int_as_float(0x7fc00000);
-            } else {
-                for (int c = 0; c < 3; ++c) {
-                    const float r = SUB(SUB(V[3 * (int64_t)v1 + c], V[3 * (int64_t)v0 + c]), off[3 * h + c]);
-                    sum += (double)MUL(MUL(r, r), 0.5f);
-                }
+            const bool ok = in_range(v0, nv) && in_range(v1, nv);
+            for (int c = 0; c < 3; ++c) {
+                const float r = ok ? SUB(SUB(V[3 * (int64_t)v1 + c], V[3 * (int64_t)v0 + c]), off[3 * h + c])
+                                   : __int_as_float(0x7fc00000);
+                sum.add(MUL(MUL(r, r), 0.5f));
             }
         }
     }
-    sum = block_sum(sum, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = sum;
+    const double total = block_sum(sum.value(), sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = total;
 }
 
 // loss = sum of the vertex blocks + r2 * sum of the edge blocks, the two sums
@@ -130,7 +150,7 @@ using namespace mo;
 
 extern "C" size_t mo_layer_scratch_bytes(int64_t nv, int64_t nh) {
     if (nv < 0 || nh < 0) return 0;
-    return sizeof(double) * ((size_t)ceil_div(nv, LAYER_THREADS) + (size_t)ceil_div(nh, LAYER_THREADS) + 1);
+    return sizeof(double) * ((size_t)layer_blocks(nv) + (size_t)layer_blocks(nh) + 1);
 }
 
 extern "C" int mo_layer_forward(const float* V, int64_t nv, const float* grid, int N, int layout, const int32_t* idx,
@@ -148,7 +168,7 @@ extern "C" int mo_layer_forward(const float* V, int64_t nv, const float* grid, i
     }
     cudaStream_t s = as_stream(stream);
     double* partial = reinterpret_cast<double*>(scratch);
-    const int vblocks = ceil_div(nv, LAYER_THREADS), blocks = vblocks + ceil_div(nh, LAYER_THREADS);
+    const int vblocks = layer_blocks(nv), blocks = vblocks + layer_blocks(nh);
     const float Nf = (float)N, Cf = far_offset(N);
     if (blocks > 0) {
 #define MO_LAYER(LAYOUT, GRAD)                                                                                     \
