@@ -70,7 +70,7 @@ int mo_bbox(const float* V, int64_t n, int32_t* bbox6, void* stream);
 /* params4 (device double[4]) = {scale, tx, ty, tz}:
  * scale = 1.1 * longest extent, t = min - 0.05*scale (mesh.cc:79-82). */
 int mo_norm_params(const int32_t* bbox6, double* params4, void* stream);
-/* mo_bbox and mo_norm_params in one call (one launch up to 2^20 vertices). */
+/* mo_bbox and mo_norm_params in one call (one launch up to 600,000 vertices). */
 int mo_bbox_params(const float* V, int64_t n, int32_t* bbox6, double* params4, void* stream);
 /* In place: v = (v - t)/scale (inverse == 0) or v = v*scale + t
  * (inverse != 0), evaluated in double and rounded to float like

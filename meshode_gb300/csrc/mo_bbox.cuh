@@ -10,10 +10,12 @@ namespace mo {
 
 // The thread count is a multiple of three, so a thread keeps one coordinate and
 // the reads are consecutive; a warp reduces each coordinate by itself and its
-// leaders put it into the first block's shared memory.  Eight SMs read ~1
-// TB/s: past BBOX_CLUSTER_MAX points the whole chip and more launches are faster.
+// leaders put it into the first block's shared memory.  Eight SMs read ~0.25
+// TB/s: past BBOX_CLUSTER_MAX points the whole chip and more launches are faster (box
+// and parameters, us, inputs not in L2: 400k 23 against 30, 600k 31 against 32, 800k 39
+// against 32).
 constexpr int BBOX_BLOCKS = 8, BBOX_THREADS = 960, BBOX_UNROLL = 16;
-constexpr int64_t BBOX_CLUSTER_MAX = 1 << 20;
+constexpr int64_t BBOX_CLUSTER_MAX = 600000;
 
 // Called by all threads of the cluster; box: six ints of shared memory.  True in
 // one thread, where box then holds the extremes (ordered ints: min x, y, z, max
