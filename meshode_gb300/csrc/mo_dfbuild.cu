@@ -1176,7 +1176,10 @@ extern "C" int mo_df_method_for(int64_t nf, int N) {
 // triangles against about N^3 / 4 on an exact grid (112^3, 500k: 3.89, 4.06,
 // 3.84).  From N = 120 on, with four times the warps that the chip holds, that
 // line is N^3 / 8: 128^3, 150k: 1.72 for 4x4x2, 1.56 wide, 1.63 for 2x4x4; 300k
-// 2.36, 2.35, 2.27; flat target, 100k 0.97, 1.00, 0.74.  Several builds at once
+// 2.36, 2.35, 2.27; flat target, 100k 0.97, 1.00, 0.74.  Against the line is an
+// exact sphere, whose centre is equally far from every triangle: warps there walk
+// most of the tree, and a wide one longest (355k 128^3 19.8 for 4x4x2, 23.5 wide; 4M
+// 256^3 146 and 216, where a displaced one takes 62 and 48).  Several builds at once
 // favour the wide packet further, since it takes the fewest instructions (32
 // requests' builds together: 25.5 -> 24.0 with this line, all wide 23.3).
 extern "C" int mo_df_packet_for(int64_t nf, int N, float band) {
